@@ -35,7 +35,6 @@ enum BatchSlot {
   BS_P_FACE,     // k_p_face (FlatBlock)
   BS_P_DPDX,     // k_p_dpdx (is_dpdx_tolerance)
   BS_ZERO_FLUX,  // k_zero_flux
-  BS_T_COEF,     // k_T_coef
   BS_T_CELL,     // k_T_cell (FlatBlock)
   BS_T_FACE,     // k_T_face (FlatBlock)
   BS_COUNT
@@ -259,13 +258,7 @@ __global__ void __launch_bounds__(BLK) kb_zero_flux(BatchArgs A) {
   });
 }
 template <class R, int W>
-__global__ void __launch_bounds__(BLK, wider(4, W)) kb_T_coef(BatchArgs A) {
-  batch_items<BS_T_COEF, R>(A, [&](const BatchInst<R> &I, BatchBlock b) {
-    T_coef_body<R>(I.d, I.g, I.F, I.P, I.ctl, b);
-  });
-}
-template <class R, int W>
-__global__ void __launch_bounds__(CB3, wider(minb<R>(5, TCELL_MINB_F), W)) kb_T_cell(BatchArgs A) {
+__global__ void __launch_bounds__(CB3, wider(minb<R>(TCELL_MINB, TCELL_MINB_F), W)) kb_T_cell(BatchArgs A) {
   batch_items<BS_T_CELL, R, FlatBlock>(A, [&](const BatchInst<R> &I, FlatBlock b) {
     T_cell_body<false, R>(I.d, I.g, I.F, I.P, I.ctl, b);
   });
@@ -361,11 +354,7 @@ __global__ void __launch_bounds__(BLK) kg_zero_flux(const __grid_constant__ Batc
   group_item<R, BatchBlock>(L, [&](const BatchInst<R> &I, BatchBlock b) { zero_flux_body<R>(I.d, I.g, I.F, I.ctl, b); });
 }
 template <class R>
-__global__ void __launch_bounds__(BLK, 4) kg_T_coef(const __grid_constant__ BatchGroup<R> L) {
-  group_item<R, BatchBlock>(L, [&](const BatchInst<R> &I, BatchBlock b) { T_coef_body<R>(I.d, I.g, I.F, I.P, I.ctl, b); });
-}
-template <class R>
-__global__ void __launch_bounds__(CB3, minb<R>(5, TCELL_MINB_F)) kg_T_cell(const __grid_constant__ BatchGroup<R> L) {
+__global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) kg_T_cell(const __grid_constant__ BatchGroup<R> L) {
   group_item<R, FlatBlock>(L, [&](const BatchInst<R> &I, FlatBlock b) { T_cell_body<false, R>(I.d, I.g, I.F, I.P, I.ctl, b); });
 }
 template <class R>

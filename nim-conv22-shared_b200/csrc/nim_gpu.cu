@@ -212,7 +212,7 @@ int verify_mesh(const nim_mesh_desc *m, const Dims &d, std::vector<int> &perm) {
   if ((int64_t)NT * (NR + 1) * (NZ + 1) != m->nnode || d.Nc != m->nmesh || d.NF != m->nface || d.NBF != m->nbcface)
     return NIM_ERR_BAD_ARG;
   // The sweep kernels index with 32-bit integers (fewer registers, so fewer
-  // spills); their largest offset is 19 x the cell count (MT_A, 18 rows).
+  // spills); their largest offset is 19 x the cell count.
   // 2^31 / 20 = 107 M cells is beyond what one GPU's memory holds in FP64.
   if ((int64_t)d.Nc * 20 >= (int64_t)INT32_MAX) return NIM_ERR_BAD_ARG;
   perm.assign(d.NF, -1);
@@ -469,8 +469,6 @@ int launch_temperature(nim_ctx *x, cudaStream_t s, const GeoT<R> &g, const Field
   const Dims &d = x->d;
   k_zero_flux<<<grid(2 * d.plane), BLK, 0, s>>>(d, g, F, x->ctl);
   TRY(mark(x, "k_zero_flux"));
-  k_T_coef<<<dim3(3, x->nblk_c), BLK, 0, s>>>(d, g, F, x->phys, x->ctl);
-  TRY(mark(x, "k_T_coef"));
   if constexpr (std::is_same<R, float>::value) {
     if (x->cell_quad) {  // the float mirror: four theta-adjacent cells a thread
       const dim3 gq((d.NT + 127) / 128, (d.NR + 3) / 4, d.NZ);
@@ -498,7 +496,7 @@ int launch_parallel(nim_ctx *x, const GeoT<R> &g, const FieldsT<R> &F, int lowp)
   k_iter_end<<<1, 1, 0, s>>>(x->ctl, x->phys, lowp);
   TRY(mark(x, "k_iter_end"));
   CK(cudaGetLastError());
-  x->kernels_per_iter = x->phys.dpdx_tolerance ? 12 : 11;
+  x->kernels_per_iter = x->phys.dpdx_tolerance ? 11 : 10;
   x->launches += x->kernels_per_iter;
   return NIM_OK;
 }
@@ -816,6 +814,7 @@ static int setup_levels(nim_ctx *x) {
   const Dims &d = x->d;
   const size_t Nc = d.Nc;
   TRY(dalloc(x, &x->F.MTF4, 8 * Nc));
+  TRY(dalloc(x, &x->F.MT4, 9 * Nc));
   TRY(dalloc(x, &x->F.RDT, Nc));
   // counting sort of the cells by level
   const int nlev = (d.NT - 1) + 2 * (d.NR - 1) + 3 * (d.NZ - 1) + 1;
@@ -1144,8 +1143,7 @@ static int create_impl(const nim_mesh_desc *m, const nim_params *p, nim_ctx *x, 
   TRY(dalloc(x, &F.MA, 18 * Nc));
   TRY(dalloc(x, &F.MF4, 8 * Nc));
   TRY(dalloc(x, &F.MF, 15 * Nc));
-  TRY(dalloc(x, &F.MTF, 15 * Nc));
-  TRY(dalloc(x, &F.MTA, 18 * Nc));
+  TRY(dalloc(x, &F.MTF, 12 * Nc));
   if (x->seq || p->formulation == 1) TRY(dalloc(x, &F.Bv, 3 * Nc));
   if (p->formulation == 1) {
     TRY(dalloc(x, &F.N1, 22 * Nc));
@@ -1181,8 +1179,7 @@ static int create_impl(const nim_mesh_desc *m, const nim_params *p, nim_ctx *x, 
     TRY(dalloc(x, &H.Rp, Nc));
     TRY(dalloc(x, &H.MF4, 8 * Nc));
     TRY(dalloc(x, &H.MF, 15 * Nc));
-    TRY(dalloc(x, &H.MTF, 15 * Nc));
-    TRY(dalloc(x, &H.MTA, 18 * Nc));
+    TRY(dalloc(x, &H.MTF, 12 * Nc));
     TRY(dalloc(x, &H.dpd, 3 * Nc));
   }
   TRY(dalloc(x, &F.part, 8 * (size_t)std::max(x->nblk_c, grid(2 * d.NT * d.NZ))));
@@ -1698,7 +1695,6 @@ int fused_occupancy(FusedBatch &B, int sms) {
   TRY(persistent_blocks(kb_p_face<R, W>, CB3, sms, b[BS_P_FACE]));
   TRY(persistent_blocks(kb_p_dpdx<R, W>, BLK, sms, b[BS_P_DPDX]));
   TRY(persistent_blocks(kb_zero_flux<R, W>, BLK, sms, b[BS_ZERO_FLUX]));
-  TRY(persistent_blocks(kb_T_coef<R, W>, BLK, sms, b[BS_T_COEF]));
   TRY(persistent_blocks(kb_T_cell<R, W>, CB3, sms, b[BS_T_CELL]));
   TRY(persistent_blocks(kb_T_face<R, W>, BLK, sms, b[BS_T_FACE]));
   return NIM_OK;
@@ -1728,7 +1724,6 @@ int fused_slots(FusedBatch &B) {
   if (u[BS_P_FACE]) kb_p_face<R, W><<<b[BS_P_FACE], t3, 0, s>>>(A);
   if (u[BS_P_DPDX]) kb_p_dpdx<R, W><<<b[BS_P_DPDX], BLK, 0, s>>>(A);
   if (u[BS_ZERO_FLUX]) kb_zero_flux<R, W><<<b[BS_ZERO_FLUX], BLK, 0, s>>>(A);
-  if (u[BS_T_COEF]) kb_T_coef<R, W><<<b[BS_T_COEF], BLK, 0, s>>>(A);
   if (u[BS_T_CELL]) kb_T_cell<R, W><<<b[BS_T_CELL], t3, 0, s>>>(A);
   if (u[BS_T_FACE]) kb_T_face<R, W><<<b[BS_T_FACE], BLK, 0, s>>>(A);
   CK(cudaGetLastError());
@@ -1754,7 +1749,6 @@ void group_launch(int slot, const BatchGroup<R> &L, cudaStream_t s) {
     case BS_P_FACE: kg_p_face<R><<<nb, t3, 0, s>>>(L); break;
     case BS_P_DPDX: kg_p_dpdx<R><<<nb, BLK, 0, s>>>(L); break;
     case BS_ZERO_FLUX: kg_zero_flux<R><<<nb, BLK, 0, s>>>(L); break;
-    case BS_T_COEF: kg_T_coef<R><<<nb, BLK, 0, s>>>(L); break;
     case BS_T_CELL: kg_T_cell<R><<<nb, t3, 0, s>>>(L); break;
     case BS_T_FACE: kg_T_face<R><<<nb, BLK, 0, s>>>(L); break;
     default:
@@ -1921,7 +1915,6 @@ int fused_setup(FusedBatch &B, int32_t n, nim_ctx *const *ctx) {
       G[BS_P_BC_COPY] = gb;
       if (x->phys.dpdx_tolerance) G[BS_P_DPDX] = BatchGrid{(unsigned)x->nblk_c, 1u, 1u};
       G[BS_ZERO_FLUX] = BatchGrid{(unsigned)grid(2 * d.plane), 1u, 1u};
-      G[BS_T_COEF] = BatchGrid{3u, (unsigned)x->nblk_c, 1u};
       G[BS_T_CELL] = f3;
       G[BS_T_FACE] = f8;
       for (int q = 0; q < BS_COUNT; ++q) B.use[ph][q] = B.use[ph][q] || G[q].x > 0;
@@ -2755,8 +2748,7 @@ int dual_alloc(nim_ctx *x) {
   TRY(dalloc(x, &H.MA, 18 * Nc));
   TRY(dalloc(x, &H.MF4, 8 * Nc));
   TRY(dalloc(x, &H.MF, 15 * Nc));
-  TRY(dalloc(x, &H.MTF, 15 * Nc));
-  TRY(dalloc(x, &H.MTA, 18 * Nc));
+  TRY(dalloc(x, &H.MTF, 12 * Nc));
   TRY(dalloc(x, &H.dpd, 3 * Nc));
   H.part = x->F.part;  // per-block partial sums: FP64, shared
   TRY(dalloc(x, &x->ctlD, 1));

@@ -96,8 +96,8 @@ struct FieldsT {
   R *MA;      // [18][Nc] velocity M_A (per step scratch)
   R *MF4;     // [8][Nc]
   R *MF;      // [15][Nc]  M_F1..3(k) at 5(d-1)+k-1
-  R *MTF;     // [15][Nc]  MT_F1..3
-  R *MTA;     // [18][Nc]  MT_A(q, d) at 3(q-1) + d-1 (float: 1/MT_A(5, d) at q = 5)
+  R *MTF;     // [12][Nc]  the cell's own terms of MT_F1..3 (TDir): G1, G3, H2, H4 of direction d at 4(d-1)
+  R *MT4;     // [9][Nc]   its terms of MT_F4 (TDir): r, m, p of direction d at 3(d-1) (reference order only)
   R *dpd;     // [3][Nc]   dpdx_old, dpdy_old, dpdz_old
   // reference-order schedule: sources stored before the ordered sweeps
   R *Bv;      // [3][Nc]   R_C + R_D + R_B of u, v, w
@@ -183,7 +183,7 @@ constexpr int BLK = 256;
 constexpr int VC2_MINB = 3;  // resident blocks per SM asked of k_vel_cell2 (56 registers)
 // resident blocks per SM the float instantiations of the pass kernels ask
 // for: computing in float they need about half the FP64 registers
-constexpr int VC2_MINB_F = 3, PSRC_MINB_F = 4, PFACE_MINB_F = 5, TCELL_MINB_F = 5, TFACE_MINB_F = 4;
+constexpr int VC2_MINB_F = 3, PSRC_MINB_F = 4, PFACE_MINB_F = 5, TCELL_MINB = 3, TCELL_MINB_F = 5, TFACE_MINB_F = 4;
 constexpr int VCN_MINB = 2;  // k_vel_cellN (four float cells a thread)
 constexpr int PSN_MINB = 2;  // k_p_srcN (four float or two FP64 cells a thread)
 constexpr int TCN_MINB = 2;  // k_T_cellN (four float cells a thread)
@@ -838,28 +838,6 @@ __device__ __forceinline__ void form_Fd(const V Ai[6], const V A2[6], V G[5]) {
   G[3] = Ai[0] / (V(2.) * Ai[4]);
   G[4] = A2[1] / (V(2.) * A2[4]);
   G[0] = G[1] + G[2] + V(2.) * G[3] + V(2.) * G[4];
-}
-
-// form_Fd and form_F4 with slot 4 holding 1/A4 (the float MT_A of the FP32
-// phase): the same terms with each division by A4 a multiplication
-template <class V>
-__device__ __forceinline__ void form_Fd_rcp(const V Ai[6], const V A2[6], V G[5]) {
-  G[1] = Ai[2] - Ai[0] * Ai[5] * Ai[4];
-  G[2] = A2[3] - A2[1] * A2[4] + A2[1] * A2[5] * A2[4];
-  G[3] = V(0.5) * Ai[0] * Ai[4];
-  G[4] = V(0.5) * A2[1] * A2[4];
-  G[0] = G[1] + G[2] + V(2) * G[3] + V(2) * G[4];
-}
-template <class V>
-__device__ __forceinline__ void form_F4_rcp(const V A[3][6], V DT, V F4[8]) {
-  F4[1] = V(0.5) * (A[0][4] + A[1][4] + A[2][4] - V(1) / DT);
-  F4[2] = -(A[0][5] * A[0][4]);
-  F4[3] = (A[0][5] - V(1)) * A[0][4];
-  F4[4] = -(A[1][5] * A[1][4]);
-  F4[5] = (A[1][5] - V(1)) * A[1][4];
-  F4[6] = -(A[2][5] * A[2][4]);
-  F4[7] = (A[2][5] - V(1)) * A[2][4];
-  F4[0] = F4[1] + F4[2] + F4[3] + F4[4] + F4[5] + F4[6] + F4[7];
 }
 
 template <class R>
@@ -3220,57 +3198,116 @@ __global__ void __launch_bounds__(BLK) k_zero_flux(Dims d, GeoT<R> g, FieldsT<R>
   zero_flux_body<R>(d, g, F, ctl, LaunchBlock{});
 }
 
-// ---- K7a: calculate_temperature_nim_constants_formulation2, first part
-// (nim.f90:334-464): MT_A(1:6) of every cell and direction, from the cell
-// velocities of this pass.  One thread per (direction, cell) and no
-// barriers: in FP64 the divisions of the NIM series make this the one
-// instruction-bound piece of the pass, and every warp can issue.
-// Grid (3, ceil(Nc/BLK)): blockIdx.x is the direction, so the three
-// directions of the same cells run side by side and share their loads.
-// The float instantiation (the FP32 phase) computes in float with
-// nim_direction_f32, which makes it bound by its bytes.
-template <class R, class BI>
-__device__ __forceinline__ void T_coef_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+// ---- K7: calculate_temperature_nim_constants_formulation2 (nim.f90:334-500)
+// of one direction of one cell.  MT_F1..3 of a +xi face mix the constants of
+// the face's two cells, but every product in them takes its factors from one
+// cell (form_Fd):
+//   MT_F(2) = G1 of the lower cell, MT_F(3) = H2 of the upper one,
+//   MT_F(4) = G3 of the lower cell, MT_F(5) = H4 of the upper one,
+//   MT_F(1) = G1 + H2 + 2 G3 + 2 H4,
+// so a cell forms its own four terms and the face sweep adds them up: MT_A
+// never goes to memory and a cell needs no neighbour's MT_A.  r, m, p are
+// the direction's terms of MT_F4: 1/A5, -(A6/A5), (A6 - 1)/A5.
+template <class V>
+struct TDir {
+  V G1, G3, H2, H4, r, m, p;
+};
+template <class R>
+__device__ __forceinline__ TDir<Ar<R>> T_direction(Ar<R> u, Ar<R> k, Ar<R> gminus, Ar<R> gplus, double v_limit) {
+  using V = Ar<R>;
+  TDir<V> t;
+  V A[6];
+  if constexpr (std::is_same<R, float>::value) {
+    nim_direction_f32(u, k, gminus, gplus, A);
+    const V q = V(1) / A[4];  // A5 = 4h/k > 0: every division by it a multiplication
+    t.G1 = A[2] - A[0] * A[5] * q;
+    t.G3 = V(0.5) * A[0] * q;
+    t.H2 = A[3] - A[1] * q + A[1] * A[5] * q;
+    t.H4 = V(0.5) * A[1] * q;
+    t.r = q;
+    t.m = -(A[5] * q);
+    t.p = (A[5] - V(1)) * q;
+  } else {
+    nim_direction<V>(u, k, gminus, gplus, v_limit, A);
+    t.G1 = A[2] - (A[0] * A[5] / A[4]);
+    t.G3 = A[0] / (V(2.) * A[4]);
+    t.H2 = A[3] - A[1] / A[4] + A[1] * A[5] / A[4];
+    t.H4 = A[1] / (V(2.) * A[4]);
+    t.r = V(1.) / A[4];
+    t.m = -(A[5] / A[4]);
+    t.p = (A[5] - V(1.)) / A[4];
+  }
+  return t;
+}
+// direction dd (1..3) of cell c, from the cell velocities of this pass
+template <class R>
+__device__ __forceinline__ TDir<Ar<R>> T_direction_of(const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, int Nc,
+                                                      int c, int dd) {
+  using V = Ar<R>;
+  const V ut = V(0.5) * (F.c[0][c] + F.co[0][c]);
+  const V vt = V(0.5) * (F.c[1][c] + F.co[1][c]);
+  const V wt = V(0.5) * (F.c[2][c] + F.co[2][c]);
+  const V u = contravariant(g.xi, Nc, c, dd, ut, vt, wt);
+  return T_direction<R>(u, g.gij[(dd - 1 + 3 * (dd - 1)) * Nc + c] * pv<V>(P.alpha, P.d_alpha),
+                        g.gfd[(2 * (dd - 1)) * Nc + c], g.gfd[(2 * (dd - 1) + 1) * Nc + c], P.v_limit);
+}
+// MT_F4 (nim.f90:466-475) from the three directions' terms
+template <class V>
+__device__ __forceinline__ void T_form_F4(const V r[3], const V m[3], const V p[3], V DT, V F4[8]) {
+  F4[1] = V(0.5) * (r[0] + r[1] + r[2] - V(1.) / DT);
+  F4[2] = m[0];
+  F4[3] = p[0];
+  F4[4] = m[1];
+  F4[5] = p[1];
+  F4[6] = m[2];
+  F4[7] = p[2];
+  F4[0] = F4[1] + F4[2] + F4[3] + F4[4] + F4[5] + F4[6] + F4[7];
+}
+// MT_F1..3 of the +xi_dd face between cells c (lower) and c2 (upper)
+template <class R>
+__device__ __forceinline__ void T_form_Fd(const FieldsT<R> &F, int Nc, int c, int c2, int dd, Ar<R> Fd[5]) {
+  using V = Ar<R>;
+  const R *row = F.MTF + 4 * (dd - 1) * Nc;
+  Fd[1] = row[c];
+  Fd[3] = row[Nc + c];
+  Fd[2] = row[2 * Nc + c2];
+  Fd[4] = row[3 * Nc + c2];
+  Fd[0] = Fd[1] + Fd[2] + V(2.) * Fd[3] + V(2.) * Fd[4];
+}
+
+// The reference order's temperature constants: the TDir terms of every cell
+// and direction stored for k_T_cell(src) and the ordered sweep.
+// Grid (3, ceil(Nc/BLK)): blockIdx.x is the direction.
+template <class R>
+__global__ void __launch_bounds__(BLK, 4) k_T_coef(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   if (ctl->done) return;
   const int c = blockIdx.y * BLK + threadIdx.x;
   if (c >= d.Nc) return;
-  const int dd = blockIdx.x + 1;
-  const int Nc = d.Nc;
-  if constexpr (std::is_same<R, float>::value) {
-    const float ut = 0.5f * (F.c[0][c] + F.co[0][c]);
-    const float vt = 0.5f * (F.c[1][c] + F.co[1][c]);
-    const float wt = 0.5f * (F.c[2][c] + F.co[2][c]);
-    const float u = ut * g.xi[(dd - 1) * Nc + c] + vt * g.xi[(dd + 2) * Nc + c] + wt * g.xi[(dd + 5) * Nc + c];
-    float A[6];
-    nim_direction_f32(u, g.gij[(dd - 1 + 3 * (dd - 1)) * Nc + c] * (float)P.alpha, g.gfd[(2 * (dd - 1)) * Nc + c],
-                      g.gfd[(2 * (dd - 1) + 1) * Nc + c], A);
-    A[4] = 1.f / A[4];  // k_T_cell, the one reader, only divides by A4 (A4 = 4h/k > 0)
-    for (int q = 0; q < 6; ++q) F.MTA[(3 * q + dd - 1) * Nc + c] = A[q];
-  } else {
-    using V = Ar<R>;
-    const V ut = V(0.5) * (F.c[0][c] + F.co[0][c]);
-    const V vt = V(0.5) * (F.c[1][c] + F.co[1][c]);
-    const V wt = V(0.5) * (F.c[2][c] + F.co[2][c]);
-    const V u = contravariant(g.xi, Nc, c, dd, ut, vt, wt);
-    V A[6];
-    nim_direction<V>(u, g.gij[(dd - 1 + 3 * (dd - 1)) * Nc + c] * pv<V>(P.alpha, P.d_alpha),
-                     g.gfd[(2 * (dd - 1)) * Nc + c], g.gfd[(2 * (dd - 1) + 1) * Nc + c], P.v_limit, A);
-    for (int q = 0; q < 6; ++q) F.MTA[(3 * q + dd - 1) * Nc + c] = A[q];
-  }
-}
-template <class R>
-__global__ void __launch_bounds__(BLK, 4) k_T_coef(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  T_coef_body<R>(d, g, F, P, ctl, LaunchBlock{});
+  const int y = blockIdx.x, Nc = d.Nc;
+  const TDir<Ar<R>> t = T_direction_of(g, F, P, Nc, c, y + 1);
+  R *row = F.MTF + 4 * y * Nc, *q = F.MT4 + 3 * y * Nc;
+  row[c] = t.G1;
+  row[Nc + c] = t.G3;
+  row[2 * Nc + c] = t.H2;
+  row[3 * Nc + c] = t.H4;
+  q[c] = t.r;
+  q[Nc + c] = t.m;
+  q[2 * Nc + c] = t.p;
 }
 
-// ---- K7b: the rest of calculate_temperature_nim_constants_formulation2
-// (MT_F4, MT_F1..3, nim.f90:466-500), calculate_R_D_T (nse.f90:2000-2134)
-// and the cell update of T (1017-1026).  Block (CB, 3): thread y forms MT_F
-// of direction y+1 from MT_A of the cell and of its +neighbour, and two of
-// the six cross derivatives; thread 0 assembles MT_F4, R_D_T and the update
-// in the reference's order.
-// SRC_ONLY (reference-order schedule): store MT_F4 and R_D_T and leave the
-// update to k_seq_T.
+// ---- K7, the cell kernel: the temperature constants, calculate_R_D_T
+// (nse.f90:2000-2134) and the cell update of T (1017-1026).  Block (CB, 3):
+// thread y forms the NIM constants of direction y+1 (its TDir terms of
+// MT_F1..3 go to memory for the face sweep, those of MT_F4 stay on chip) and
+// two of the six cross derivatives; thread 0 assembles MT_F4, R_D_T and the
+// update in the reference's order.
+// Bound by latency and, in FP64, by its divisions.  Forming the constants
+// here moves 616 bytes a cell in this kernel and k_T_face together; with
+// MT_A (18 words) and MT_F (15) written and read through memory by a kernel
+// of their own it was 952.  128x128x96: FP64 T_coef + T_cell 305 -> 289 us,
+// float (k_T_cellN) 128 -> 91 us, and k_T_faceN 51 -> 45 us.
+// SRC_ONLY (reference-order schedule): the constants are k_T_coef's; store
+// MT_F4 and R_D_T and leave the update to k_seq_T.
 template <bool SRC_ONLY, class R, class BI>
 __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   using V = Ar<R>;
@@ -3278,7 +3315,7 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, con
   __shared__ BlockRed red;
   red_init<1>(red);
   __shared__ V sX[3][2][CB];   // cross derivatives
-  __shared__ V sF4[8][CB];     // MT_F4, formed by thread 1
+  __shared__ V sF[3][3][CB];   // r, m, p of MT_F4 by direction
   __shared__ V sG[CB];         // G1 dT/dx + G2 dT/dy + G3 dT/dz, by thread 2
   const int par = parity(ctl);
   const bool first = ctl->first;
@@ -3287,48 +3324,33 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, con
   const bool active = patch_cell(d, x, blockIdx);
   const int c = x.c;
   double e[1] = {0.};
-  const size_t Nc = d.Nc, NF = d.NF;
+  const int Nc = d.Nc, NF = d.NF;
   const R *T = F.f[4] + par * NF;
   int f[7];
   cell_faces(d, x, f);
   if (active) by_dir(threadIdx.y, [&](auto D) {
     constexpr int dd = decltype(D)::value, y = dd - 1;
-    const R *MA = F.MTA + (size_t)y * Nc;  // MT_A(q, dd) at MA[3q Nc]
-    V G[5] = {V(0.), V(0.), V(0.), V(0.), V(0.)};
-    if (x.has_nb(d, 2 * dd)) {
-      const int c2 = x.nb(d, 2 * dd).c;
-      V A[6], A2[6];
-      for (int q = 0; q < 6; ++q) A[q] = MA[3 * q * Nc + c];
-      A2[0] = A2[2] = V(0.);  // not used by form_Fd
-      A2[1] = MA[3 * Nc + c2];
-      A2[3] = MA[9 * Nc + c2];
-      A2[4] = MA[12 * Nc + c2];
-      A2[5] = MA[15 * Nc + c2];
-      if constexpr (std::is_same<R, float>::value)
-        form_Fd_rcp(A, A2, G);
-      else
-        form_Fd(A, A2, G);
+    if (SRC_ONLY) {
+      const R *q = F.MT4 + 3 * y * Nc;
+      for (int n = 0; n < 3; ++n) sF[y][n][tx] = q[n * Nc + c];
+    } else {
+      const TDir<V> t = T_direction_of(g, F, P, Nc, c, dd);
+      R *row = F.MTF + 4 * y * Nc;
+      row[c] = t.G1;
+      row[Nc + c] = t.G3;
+      row[2 * Nc + c] = t.H2;
+      row[3 * Nc + c] = t.H4;
+      sF[y][0][tx] = t.r;
+      sF[y][1][tx] = t.m;
+      sF[y][2][tx] = t.p;
     }
-    for (int k = 0; k < 5; ++k) F.MTF[(size_t)(5 * (dd - 1) + k) * Nc + c] = G[k];
     // cross derivatives of calculate_R_D_T: y=0 pxy,pzy  y=1 pyx,pzx  y=2 pxz,pyz
     constexpr int e2 = (y == 0) ? 2 : (y == 1) ? 1 : 3;
     constexpr int fa = (y == 1) ? 4 : 2, fb = (y == 1) ? 3 : 1;
     sX[y][0][tx] = V(0.5) * (tangential(d, T, x, (y == 2) ? 2 : fa, e2) - tangential(d, T, x, (y == 2) ? 1 : fb, e2));
     sX[y][1][tx] = (y == 2) ? V(0.5) * (tangential(d, T, x, 4, 3) - tangential(d, T, x, 3, 3))
                             : V(0.5) * (tangential(d, T, x, 6, e2) - tangential(d, T, x, 5, e2));
-    if (y == 1) {  // MT_F4 (nim.f90:466-475)
-      V Am[3][6];
-      for (int k = 0; k < 3; ++k) {
-        Am[k][4] = F.MTA[(size_t)(12 + k) * Nc + c];
-        Am[k][5] = F.MTA[(size_t)(15 + k) * Nc + c];
-      }
-      V F4[8];
-      if constexpr (std::is_same<R, float>::value)
-        form_F4_rcp(Am, V(P.DT), F4);
-      else
-        form_F4(Am, V(P.DT), F4);
-      for (int k = 0; k < 8; ++k) sF4[k][tx] = F4[k];
-    } else if (y == 2) {  // the leading G_i d_i T terms of R_D_T, in source order
+    if (y == 2) {  // the leading G_i d_i T terms of R_D_T, in source order
       const V px = (T[f[2]] - T[f[1]]) / V(2.);
       const V py = (T[f[4]] - T[f[3]]) / V(2.);
       const V pz = (T[f[6]] - T[f[5]]) / V(2.);
@@ -3337,8 +3359,13 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, con
   });
   __syncthreads();
   if (active && threadIdx.y == 0) {
-    V F4[8];
-    for (int k = 0; k < 8; ++k) F4[k] = sF4[k][tx];
+    V r[3], m[3], p[3], F4[8];
+    for (int n = 0; n < 3; ++n) {
+      r[n] = sF[n][0][tx];
+      m[n] = sF[n][1][tx];
+      p[n] = sF[n][2][tx];
+    }
+    T_form_F4(r, m, p, V(P.DT), F4);
     const V pxy = sX[0][0][tx], pzy = sX[0][1][tx], pyx = sX[1][0][tx], pzx = sX[1][1][tx];
     const V pxz = sX[2][0][tx], pyz = sX[2][1][tx];
     const R *gij = g.gij;
@@ -3357,18 +3384,16 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, con
   if (!SRC_ONLY && d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 4);
 }
 template <bool SRC_ONLY, class R>
-__global__ void __launch_bounds__(CB3, minb<R>(5, TCELL_MINB_F)) k_T_cell(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) k_T_cell(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   T_cell_body<SRC_ONLY, R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
 // ---- K7b, NP cells per thread (the float mirror's parallel passes,
 // n_theta % NP == 0): k_T_cell over NP theta-adjacent cells with NP-wide
-// vector loads and stores (as k_vel_cellN).  Thread y forms MT_F of
-// direction y+1 (the +theta neighbour's MT_A is the group's own vector
-// shifted by one cell, and one single load for the last cell) and two of the
-// six cross derivatives of T; thread 1 forms MT_F4, thread 2 the G_i d_i T
-// prefix; thread 0 assembles R_D_T and the cell update.  Each cell's
-// arithmetic is k_T_cell's.
+// vector loads and stores (as k_vel_cellN).  Thread y forms the NIM
+// constants of direction y+1 and two of the six cross derivatives of T;
+// thread 2 also the G_i d_i T prefix; thread 0 assembles MT_F4, R_D_T and
+// the cell update.  Each cell's arithmetic is k_T_cell's.
 template <class R, int NP>
 __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   using V = Ar<R>;
@@ -3376,7 +3401,7 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
   __shared__ BlockRed red;
   red_init<1>(red);
   __shared__ V sX[3][2][CB * NP];  // cross derivatives
-  __shared__ V sF4[8][CB * NP];    // MT_F4, formed by thread 1
+  __shared__ V sF[3][3][CB * NP];  // r, m, p of MT_F4 by direction
   __shared__ V sG[CB * NP];        // G1 dT/dx + G2 dT/dy + G3 dT/dz, by thread 2
   const int par = parity(ctl);
   const bool first = ctl->first;
@@ -3410,55 +3435,40 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
   double e[1] = {0.};
   if (active) by_dir(threadIdx.y, [&](auto D) {
     constexpr int dd = decltype(D)::value, y = dd - 1;
-    const R *MA = F.MTA + (size_t)y * Nc;  // MT_A(q, dd) at MA[3q Nc]
-    // MT_F of direction dd (nim.f90:477-500) from MT_A of the cells and of
-    // their +dd neighbours
-    {
-      const bool nb = (dd == 1) ? (j < NR - 1) : (dd == 3) ? (k < d.NZ - 1) : true;
-      R A[6][NP];
+    {  // the NIM constants of direction dd (T_direction_of)
+      V u[NP];
+      {
+        const R *xd = g.xi + (dd - 1) * Nc;
+        R a[NP], b[NP], xi[NP];
 #pragma unroll
-      for (int q = 0; q < 6; ++q) ldN<R, NP>(MA + 3 * q * Nc, c, A[q]);
-      V G[5][NP];
+        for (int q = 0; q < 3; ++q) {
+          ldN<R, NP>(F.c[q], c, a);
+          ldN<R, NP>(F.co[q], c, b);
+          ldN<R, NP>(xd + 3 * q * Nc, c, xi);
 #pragma unroll
-      for (int p = 0; p < NP; ++p)
-        for (int s = 0; s < 5; ++s) G[s][p] = V(0.);
-      if (nb) {
-        const int slots[4] = {1, 3, 4, 5};
-        R B[6][NP];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int q = slots[u];
-          if (dd == 2) {
-#pragma unroll
-            for (int p = 0; p + 1 < NP; ++p) B[q][p] = A[q][p + 1];
-            B[q][NP - 1] = MA[3 * q * Nc + c - i + ipn];
-          } else {
-            ldN<R, NP>(MA + 3 * q * Nc, c + (dd == 1 ? NT : pl), B[q]);
+          for (int p = 0; p < NP; ++p) {
+            const V tp = (V(0.5) * (a[p] + b[p])) * xi[p];
+            u[p] = (q == 0) ? tp : u[p] + tp;
           }
         }
+      }
+      R kd[NP], gm[NP], gp[NP], out[4][NP];
+      ldN<R, NP>(g.gij + 4 * (dd - 1) * Nc, c, kd);
+      ldN<R, NP>(g.gfd + 2 * (dd - 1) * Nc, c, gm);
+      ldN<R, NP>(g.gfd + (2 * (dd - 1) + 1) * Nc, c, gp);
 #pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          V a[6], a2[6], gg[5];
-          for (int q = 0; q < 6; ++q) a[q] = A[q][p];
-          a2[0] = a2[2] = V(0.);  // not used by form_Fd
-          a2[1] = B[1][p];
-          a2[3] = B[3][p];
-          a2[4] = B[4][p];
-          a2[5] = B[5][p];
-          if constexpr (std::is_same<R, float>::value)
-            form_Fd_rcp(a, a2, gg);
-          else
-            form_Fd(a, a2, gg);
-          for (int s = 0; s < 5; ++s) G[s][p] = gg[s];
-        }
+      for (int p = 0; p < NP; ++p) {
+        const TDir<V> t = T_direction<R>(u[p], kd[p] * pv<V>(P.alpha, P.d_alpha), gm[p], gp[p], P.v_limit);
+        out[0][p] = t.G1;
+        out[1][p] = t.G3;
+        out[2][p] = t.H2;
+        out[3][p] = t.H4;
+        sF[y][0][tx * NP + p] = t.r;
+        sF[y][1][tx * NP + p] = t.m;
+        sF[y][2][tx * NP + p] = t.p;
       }
 #pragma unroll
-      for (int s = 0; s < 5; ++s) {
-        R out[NP];
-#pragma unroll
-        for (int p = 0; p < NP; ++p) out[p] = G[s][p];
-        stN<R, NP>(F.MTF + (size_t)(5 * (dd - 1) + s) * Nc, c, out);
-      }
+      for (int n = 0; n < 4; ++n) stN<R, NP>(F.MTF + (4 * (dd - 1) + n) * Nc, c, out[n]);
     }
     // T's faces of the NP cells
     R o[7][NP];
@@ -3508,26 +3518,6 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
             V(0.5) * (along(rlo, rhi, o[4][p], av[p + 1], bv[p + 1]) - along(rlo, rhi, o[3][p], av[p], bv[p]));
         sX[1][1][tx * NP + p] =
             V(0.5) * (along(rlo, rhi, o[6][p], zA[p], zB[p]) - along(rlo, rhi, o[5][p], za[p], zb[p]));
-      }
-      // MT_F4 (nim.f90:466-475)
-      R a4[3][NP], a5[3][NP];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        ldN<R, NP>(F.MTA + (size_t)(12 + q) * Nc, c, a4[q]);
-        ldN<R, NP>(F.MTA + (size_t)(15 + q) * Nc, c, a5[q]);
-      }
-#pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        V Am[3][6], F4[8];
-        for (int q = 0; q < 3; ++q) {
-          Am[q][4] = a4[q][p];
-          Am[q][5] = a5[q][p];
-        }
-        if constexpr (std::is_same<R, float>::value)
-          form_F4_rcp(Am, V(P.DT), F4);
-        else
-          form_F4(Am, V(P.DT), F4);
-        for (int q = 0; q < 8; ++q) sF4[q][tx * NP + p] = F4[q];
       }
     } else {
       const int rka = NT * (j + (NR + 1) * ka), rkb = NT * (j + (NR + 1) * kb);
@@ -3583,8 +3573,13 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const int e2 = tx * NP + p;
-      V F4[8];
-      for (int q = 0; q < 8; ++q) F4[q] = sF4[q][e2];
+      V r[3], m[3], q3[3], F4[8];
+      for (int q = 0; q < 3; ++q) {
+        r[q] = sF[q][0][e2];
+        m[q] = sF[q][1][e2];
+        q3[q] = sF[q][2][e2];
+      }
+      T_form_F4(r, m, q3, V(P.DT), F4);
       const V pxy = sX[0][0][e2], pzy = sX[0][1][e2], pyx = sX[1][0][e2], pzx = sX[1][1][e2];
       const V pxz = sX[2][0][e2], pyz = sX[2][1][e2];
       const V RDT = pv<V>(P.alpha, P.d_alpha) * (sG[e2] - gs[0][p] * pxy - gs[1][p] * pyx - gs[2][p] * pxz -
@@ -3625,7 +3620,7 @@ __device__ __forceinline__ void T_face_body(const Dims &d, const GeoT<R> &g, con
       if (!x.has_nb(d, 2 * dd)) continue;
       const Cell x2 = x.nb(d, 2 * dd);
       V Fd[5];
-      for (int k = 0; k < 5; ++k) Fd[k] = F.MTF[(5 * (dd - 1) + k) * Nc + c];
+      T_form_Fd(F, Nc, c, x2.c, dd, Fd);
       const int fo = x.face(d, 2 * dd);
       const V nw = stored<R>(face_update(d, T, F.c[3], F.co[3], Fd, g.dg[(2 * (dd - 1)) * Nc + c],
                                               g.dg[(2 * (dd - 1) + 1) * Nc + c], dd, x, x2, V(P.w[3])));
@@ -3817,8 +3812,28 @@ __global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoT<R> g, Fi
       cno[NP - 1] = F.co[3][cw];
     }
     R Fd[5][NP], dg0[NP], dg1[NP];
+    {  // T_form_Fd: the lower cells' G1, G3 and the upper cells' H2, H4
+      const R *row = F.MTF + 4 * (dd - 1) * Nc;
+      ldN<R, NP>(row, c, Fd[1]);
+      ldN<R, NP>(row + Nc, c, Fd[3]);
+      if (dd == 2) {
+        R t[NP];
+        const int cw = c - i + ipn;
+        ldN<R, NP>(row + 2 * Nc, c, t);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) ldN<R, NP>(F.MTF + (size_t)(5 * (dd - 1) + q) * Nc, c, Fd[q]);
+        for (int p = 0; p + 1 < NP; ++p) Fd[2][p] = t[p + 1];
+        Fd[2][NP - 1] = row[2 * Nc + cw];
+        ldN<R, NP>(row + 3 * Nc, c, t);
+#pragma unroll
+        for (int p = 0; p + 1 < NP; ++p) Fd[4][p] = t[p + 1];
+        Fd[4][NP - 1] = row[3 * Nc + cw];
+      } else {
+        ldN<R, NP>(row + 2 * Nc, c + (dd == 1 ? NT : pl), Fd[2]);
+        ldN<R, NP>(row + 3 * Nc, c + (dd == 1 ? NT : pl), Fd[4]);
+      }
+#pragma unroll
+      for (int p = 0; p < NP; ++p) Fd[0][p] = (V)Fd[1][p] + Fd[2][p] + V(2) * Fd[3][p] + V(2) * Fd[4][p];
+    }
     ldN<R, NP>(g.dg + (size_t)(2 * (dd - 1)) * Nc, c, dg0);
     ldN<R, NP>(g.dg + (size_t)(2 * (dd - 1) + 1) * Nc, c, dg1);
     constexpr int e1 = (dd == 1) ? 2 : 1, e2 = (dd == 3) ? 2 : 3;  // tr1(dd), tr2(dd)
@@ -4115,7 +4130,7 @@ __global__ void __launch_bounds__(BLK) k_seq_T(Dims d, Geo g, Fields F, Phys P, 
         if (!x.has_nb(d, 2 * dd)) continue;
         const Cell x2 = x.nb(d, 2 * dd);
         double Fd[5];
-        for (int k = 0; k < 5; ++k) Fd[k] = F.MTF[(size_t)(5 * (dd - 1) + k) * Nc + c];
+        T_form_Fd(F, (int)Nc, c, x2.c, dd, Fd);
         const int fo = x.face(d, 2 * dd);
         const double old = LdCoh::ld(T, fo);
         const double nwf = face_update_cv<LdCoh>(d, T, nw, LdCoh::ld(F.c[3], x2.c), F.co[3], Fd,
