@@ -483,6 +483,14 @@ int nim_gpu_selftest_wait_timeout(nim_ctx *ctx, int32_t tries);
    exponential NIM coefficients, nim.f90:190-194, call it). */
 int nim_gpu_selftest_exp(const double *x, double *y, int64_t n);
 
+/* Self-test of the straight-line quotients the FP64 sweeps use in place of
+   IEEE divisions (no counterpart in the reference): q[i] = a[i] / b[i], which
+   must be the correctly rounded quotient, n <= 2^28.  Operands outside that
+   form's range (zero, subnormal, non-finite, exponents beyond +-480, divisors
+   with a significand above 2 - 2^-20) are divided.  Allocates and frees its
+   device buffers; default stream. */
+int nim_gpu_selftest_quot(const double *a, const double *b, double *q, int64_t n);
+
 /* Self-test of the temperature's NIM coefficients of one direction
    (nim.f90:334-464, with gminus = gplus = 1): A[6i + q] = coefficient q+1
    for the contravariant velocity u[i] and diffusion coefficient k[i] > 0,

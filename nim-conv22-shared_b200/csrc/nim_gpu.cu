@@ -2711,6 +2711,26 @@ extern "C" int nim_gpu_selftest_exp(const double *x, double *y, int64_t n) {
   return st;
 }
 
+extern "C" int nim_gpu_selftest_quot(const double *a, const double *b, double *q, int64_t n) {
+  if (n < 0 || n > (int64_t)1 << 28) return NIM_ERR_BAD_ARG;
+  if (n == 0) return NIM_OK;
+  if (!a || !b || !q) return NIM_ERR_BAD_ARG;
+  double *dev = nullptr;
+  const size_t bytes = sizeof(double) * n;
+  int st = cudaMalloc(&dev, 3 * bytes) == cudaSuccess ? NIM_OK : NIM_ERR_CUDA;
+  if (st == NIM_OK && (cudaMemcpy(dev, a, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+                       cudaMemcpy(dev + n, b, bytes, cudaMemcpyHostToDevice) != cudaSuccess))
+    st = NIM_ERR_CUDA;
+  if (st == NIM_OK) {
+    const int64_t blocks = std::min<int64_t>((n + BLK - 1) / BLK, 148 * 16);
+    k_quot_selftest<<<(unsigned)blocks, BLK>>>(dev, dev + n, dev + 2 * n, n);
+    if (cudaGetLastError() != cudaSuccess || cudaMemcpy(q, dev + 2 * n, bytes, cudaMemcpyDeviceToHost) != cudaSuccess)
+      st = NIM_ERR_CUDA;
+  }
+  cudaFree(dev);
+  return st;
+}
+
 // ---- tangent-linear steps (forward mode): a dual copy of the iterate and
 // geometry advanced by the dual instantiations of the step's kernels
 namespace {

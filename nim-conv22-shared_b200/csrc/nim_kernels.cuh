@@ -31,6 +31,7 @@
 #include <type_traits>
 
 #include "nim_common.cuh"
+#include "nim_div.cuh"
 #include "nim_exp.cuh"
 #include "nim_dual.cuh"
 
@@ -692,7 +693,7 @@ __global__ void k_apply_dirichlet(Dims d, Geo g, Fields F) {
 // NIM coefficients of one direction for contravariant speed u and
 // diffusivity k: M_A(d,1:6) / MT_A(d,1:6) (nim.f90:181-287, 354-460).
 template <class V>
-__device__ __forceinline__ void nim_direction(V u, V k, V gminus, V gplus, double v_limit, V A[6]) {
+__device__ __forceinline__ void nim_direction_general(V u, V k, V gminus, V gplus, double v_limit, V A[6]) {
   const V a = V(1.);
   const V Re = 2 * a * u / k;
   if (fabs(Re) > v_limit) {
@@ -723,6 +724,77 @@ __device__ __forceinline__ void nim_direction(V u, V k, V gminus, V gplus, doubl
     A[5] = V(0.5) + (u) / (V(6.) * k) - (U[3]) / (V(90.) * K[3]) + (U[5]) / (V(945.) * K[5]) - -((U[7]) / (V(9450.) * K[7])) +
            (U[9]) / (V(93555.) * K[9]);
   }
+}
+
+__device__ __noinline__ void nim_direction_slow(double u, double k, double gminus, double gplus, double v_limit,
+                                                double *A) {
+  nim_direction_general<double>(u, k, gminus, gplus, v_limit, A);
+}
+
+// The same coefficients in straight-line code (FP64), bit for bit those of
+// nim_direction_general, which takes over for operands outside the ranges
+// below.  Every division is a quot() over the reciprocal of its divisor, so
+// the quotients overlap (nim_div.cuh); divisors that differ by an exact
+// factor of two share one: 13 quotients over 7 divisors in the series, 11
+// over 8 in the exponential form, against 25 and 11 serial divisions.
+// 128x128x96 from rest (series): k_T_cell 289 -> 205 us, FP64 pipe-bound
+// before; 150x101x77 237 -> 170 us.  And the series stops at the last term that can
+// change its sum: for |Re| <= 0.01, i.e. x = |u/k| <= 0.005, a term below a
+// quarter ulp of the partial sum it is added to leaves it as it is, which
+// holds from x^7/4725 (1.7e-20 of A(1), A(2)), x^6/945 (1.65e-17 against
+// sums of 0.5 whose half spacing is at least 2.7e-17, A(3), A(4)),
+// 3 x^6/4725 (1e-17 of A(5)) and x^7/9450 (8.3e-21 against 0.5, A(6)) on.
+__device__ __forceinline__ void nim_direction_fast(double u, double k, double gminus, double gplus, double v_limit,
+                                                   double A[6]) {
+  const Recip rk = recip(k);
+  const double uk = quot(u, rk), Re = 2 * uk;  // 2 a u / k: the doubling is exact
+  bool ok = div_ok<60>(k) && fabs(u) < 0x1p60;
+  if (!(fabs(Re) > v_limit)) {
+    // a tiny or zero u only makes terms that the sums absorb
+    ok = ok && fabs(Re) <= 0.01;
+    const double U2 = u * u, U3 = u * U2, U4 = U2 * U2, U5 = U2 * U3;
+    const double K2 = k * k, K3 = k * K2, K4 = K2 * K2, K5 = K2 * K3, K6 = K3 * K3;
+    const Recip r3k = recip(3. * k), r3K2 = recip(3. * K2), r45K3 = recip(45. * K3), r45K4 = recip(45. * K4),
+                r945K5 = recip(945. * K5), r945K6 = recip(945. * K6);
+    ok = ok && div_ok<480>(r3k.b) && div_ok<480>(r3K2.b) && div_ok<480>(r45K3.b) && div_ok<480>(r45K4.b) &&
+         div_ok<480>(r945K5.b) && div_ok<480>(r945K6.b);
+    const double a0 = quot(1., rk), a1 = quot(u, r3K2), a3 = quot(U3, r45K4), a5 = 2 * quot(U5, r945K6);
+    A[0] = (-a0 - a1 + a3 - a5) * gplus;
+    A[1] = (-a0 + a1 - a3 + a5) * gminus;
+    const double b1 = 0.5 * uk, b2 = 0.5 * quot(U2, r3K2), b4 = 0.5 * quot(U4, r45K4);
+    A[2] = (-0.5 - b1 - b2 + b4) * gplus;
+    A[3] = (-0.5 + b1 - b2 + b4) * gminus;
+    A[4] = quot(1., r3k) - quot(U2, r45K3) + 2 * quot(U4, r945K5);
+    A[5] = 0.5 + 0.5 * quot(u, r3k) - 0.5 * quot(U3, r45K3) + quot(U5, r945K5);
+  } else {
+    // |Re| < 200 keeps e and 1/e, and with the bounds on k and u every
+    // product below, far from the ends of the exponent range
+    ok = ok && fabs(Re) < 200. && div_ok<80>(u);
+    const double e = nim_exp(Re);
+    const Recip re = recip(e), ru = recip(u);
+    const double ie = quot(1., re), iu = quot(1., ru);
+    const Recip r1 = recip(k * (ie - 1.)), r2 = recip(k * (1. - e)), ruu = recip(u * u), rRe = recip(Re);
+    A[0] = (quot(2., r1) + iu) * gplus;
+    A[1] = (-quot(2., r2) - iu) * gminus;
+    A[2] = quot(u, r1) * gplus;
+    A[3] = quot(u, r2) * gminus;
+    const bool pos = Re > 0;
+    const Recip rd = recip(pos ? -ie + 1. : -1. + e);
+    const double num = pos ? u * (ie + 1.) : u * (1. + e);
+    const double dif = -k + quot(num, rd);
+    A[4] = quot(dif, ruu);
+    A[5] = quot(pos ? 1. : e, rd) - quot(1., rRe);
+    ok = ok && div_ok<300>(e) && div_ok<400>(r1.b) && div_ok<400>(r2.b) && div_ok<400>(ruu.b) && div_ok<400>(Re) &&
+         div_ok<400>(rd.b) && num_ok<400>(num) && num_ok<400>(dif);
+  }
+  if (!ok) nim_direction_slow(u, k, gminus, gplus, v_limit, A);
+}
+template <class V>
+__device__ __forceinline__ void nim_direction(V u, V k, V gminus, V gplus, double v_limit, V A[6]) {
+  if constexpr (std::is_same<V, double>::value)
+    nim_direction_fast(u, k, gminus, gplus, v_limit, A);
+  else
+    nim_direction_general<V>(u, k, gminus, gplus, v_limit, A);
 }
 
 // The temperature's NIM coefficients in float for the FP32 phase.  With
@@ -775,6 +847,12 @@ __device__ __forceinline__ void nim_direction_f32(float u, float k, float gminus
 __global__ void k_exp_selftest(const double *x, double *y, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = nim_exp(x[i]);
+}
+
+// quotients by nim_div.cuh where it accepts the operands, else a division
+__global__ void k_quot_selftest(const double *a, const double *b, double *q, int64_t n) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    q[i] = div_ok<480>(b[i]) && num_ok<480>(a[i]) ? quot(a[i], recip(b[i])) : a[i] / b[i];
 }
 
 // the six NIM coefficients of one direction (gminus = gplus = 1) for n
@@ -3229,6 +3307,24 @@ __device__ __forceinline__ TDir<Ar<R>> T_direction(Ar<R> u, Ar<R> k, Ar<R> gminu
     t.p = (A[5] - V(1)) * q;
   } else {
     nim_direction<V>(u, k, gminus, gplus, v_limit, A);
+    if constexpr (std::is_same<R, double>::value) {
+      // the seven quotients over A5 share its reciprocal (nim_div.cuh); the
+      // halves are exact
+      const Recip q = recip(A[4]);
+      const double n0 = A[0] * A[5], n1 = A[1] * A[5], n5 = A[5] - 1.;
+      if (div_ok<400>(A[4]) && num_ok<400>(n0) && num_ok<400>(A[0]) && num_ok<400>(n1) && num_ok<400>(A[1]) &&
+          num_ok<400>(A[5]) && num_ok<400>(n5)) {
+        t.G1 = A[2] - quot(n0, q);
+        t.G3 = 0.5 * quot(A[0], q);
+        const double a1 = quot(A[1], q);
+        t.H2 = A[3] - a1 + quot(n1, q);
+        t.H4 = 0.5 * a1;
+        t.r = quot(1., q);
+        t.m = -quot(A[5], q);
+        t.p = quot(n5, q);
+        return t;
+      }
+    }
     t.G1 = A[2] - (A[0] * A[5] / A[4]);
     t.G3 = A[0] / (V(2.) * A[4]);
     t.H2 = A[3] - A[1] / A[4] + A[1] * A[5] / A[4];

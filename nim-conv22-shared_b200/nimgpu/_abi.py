@@ -224,6 +224,8 @@ def gpu_lib() -> C.CDLL:
         lib.nim_gpu_profile_name.restype = C.c_char_p
         lib.nim_gpu_selftest_exp.argtypes = [C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_int64]
         lib.nim_gpu_selftest_exp.restype = C.c_int
+        lib.nim_gpu_selftest_quot.argtypes = [C.POINTER(C.c_double)] * 3 + [C.c_int64]
+        lib.nim_gpu_selftest_quot.restype = C.c_int
         lib.nim_gpu_selftest_nim_coef.argtypes = [C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_int64,
                                                   C.c_int32, C.c_double, C.POINTER(C.c_double)]
         lib.nim_gpu_selftest_nim_coef.restype = C.c_int
