@@ -81,15 +81,15 @@ KERNEL_BYTES_PER_CELL = {
     "k_p_src": 8 * 39,      # faces u,v,w,T,p (15) area,normal,vol (13) G,g^ij (9); write dila,Rp (2)
     "k_p_srcN": 8 * 39,     # the float mirror's form: four cells a thread (same words)
     "k_T_cellN": 8 * 51,    # the float mirror's form of k_T_cell (same words)
-    "k_p_faceN": 8 * 52,    # the float mirror's form of k_p_face (same words)
+    "k_p_faceN": 8 * 26,    # k_p_face on cell groups (same words; the float mirror reads AA's 27 distinct words, 8 * 40)
     "k_T_faceN": 8 * 26,    # the float mirror's form of k_T_face (same words)
     "k_vel_faceN": 8 * 45,  # the float mirror's form of k_vel_face (same words)
-    "k_p_face": 8 * 52,     # faces p (3) Rp (1) AA used (39) dg (6); write faces p (3)
+    "k_p_face": 8 * 26,     # faces p (3) Rp (1) pressure NIM constants (7) gfd (6) dg (6); write faces p (3)
     "k_T_cell": 8 * 51,     # cells+old u,v,w (6) xi (9) g^ij (9) gfd (6) faces T (3) G (3) T,T_old (2); write T, MT_F terms (13)
     "k_T_face": 8 * 26,     # faces T (3) T,T_old (2) MT_F terms (12) dg (6); write faces T (3)
     # the reference-order sweeps (--schedule reference), in place
     "k_seq_vel": 8 * 59,    # cells+old u,v,w (6) faces u,v,w (9) M_F4 (8) R sums (3) M_F1..3 (15) dg (6); write cells, faces (12)
-    "k_seq_p": 8 * 52,      # faces p (3) R_p (1) AA used (39) dg (6); write faces p (3)
+    "k_seq_p": 8 * 26,      # faces p (3) R_p (1) pressure NIM constants (7) gfd (6) dg (6); write faces p (3)
     "k_T_coef": 8 * 45,     # cells+old u,v,w (6) xi (9) g^ij diagonal (3) gfd (6); write MT_F, MT_F4 terms (21)
     "k_T_cell(src)": 8 * 30,  # MT_F4 terms (9) faces T (3) G (3) g^ij (6); write MT_F4, R_D_T (9)
     "k_seq_T": 8 * 36,      # T,T_old (2) faces T (3) MT_F4 (8) R_D_T (1) MT_F terms (12) dg (6); write T, faces (4)
@@ -98,7 +98,7 @@ KERNEL_BYTES_PER_CELL = {
 # dram__bytes_write.sum, one --set full capture each); traffic grows with the
 # cells, so roofline.traffic scales these to the run's mesh
 NCU_DRAM_BYTES_PER_CELL = {
-    "k_vel_cell": 425.2, "k_p_src": 324.4, "k_p_face": 420.2, "k_vel_face_tile": 361.4, "k_vel_face": 343.1, "k_vel_cell2": 441.0,
+    "k_vel_cell": 425.2, "k_p_src": 324.4, "k_vel_face_tile": 361.4, "k_vel_face": 343.1, "k_vel_cell2": 441.0,
 }
 NCU_CAPTURE = {k: "128x128x96" for k in NCU_DRAM_BYTES_PER_CELL}
 for _k in ("k_vel_face", "k_vel_cell2"):

@@ -1122,6 +1122,7 @@ static int create_impl(const nim_mesh_desc *m, const nim_params *p, nim_ctx *x, 
   TRY(dalloc(x, &g.tang, 3 * NF));
   TRY(dalloc(x, &g.bitang, 3 * NF));
   TRY(dalloc(x, &g.AA, 45 * Nc));
+  TRY(dalloc(x, &g.pc, 7 * Nc));
   TRY(dalloc(x, &g.bcpts, 5 * NB));
   TRY(dalloc(x, &g.bca, 5 * NB));
   TRY(dalloc(x, &g.bcap, 8 * NB));

@@ -84,6 +84,8 @@ struct GeoT {
   R *bcval;   // [4][NBF]  Dirichlet face values of u, v, w, T
   R *rvol;    // [Nc]      1/vol, formed once at init in the storage type's own
               //           division (null in the dual copy, whose kernels divide)
+  R *pc;      // [7][Nc]   CC(1..3), HH(1..3), Det of the pressure NIM constants
+              //           (FP64 only: p_face_coef forms AA from them)
 };
 using Geo = GeoT<double>;
 
@@ -474,6 +476,11 @@ __global__ void __launch_bounds__(BLK) k_pressure_coeffs(Dims d, Geo g, double r
   const size_t Nc = d.Nc;
   const PConst P = pconst(g, Nc, c, rho);
   auto gfa = [&](int a, int b, int f, int cell) { return g.gf[(size_t)(a - 1 + 3 * (b - 1) + 9 * (f - 1)) * Nc + cell]; };
+  for (int dd = 0; dd < 3; ++dd) {
+    g.pc[(size_t)dd * Nc + c] = P.CC[dd];
+    g.pc[(size_t)(3 + dd) * Nc + c] = P.HH[dd];
+  }
+  g.pc[(size_t)6 * Nc + c] = P.Det;
   double A[15];
   // +r face
   for (int n = 0; n < 15; ++n) A[n] = 0.;
@@ -2900,32 +2907,96 @@ __host__ __device__ constexpr int p_term(int dd, int t) {
   }
 }
 
+// The coefficients of the pressure update of a +xi_dd face between a cell
+// and its +xi_dd neighbour (AA_px/py/pz, nim.f90:616-678).  Of the 15 stored
+// per direction nine are distinct: a cell's two faces of a transverse
+// direction share theirs, and AA(12), AA(14) are AA(13), AA(15) negated.
+//   m, mq    on the far faces 2dd-1 of the cell and 2dd of the neighbour
+//   a1, a1q  on the tr1(dd) faces of the cell and of the neighbour
+//   a2, a2q  on their tr2(dd) faces
+//   diag     on the face itself;  b, bq on R_p of the cell and the neighbour
+template <class V>
+struct PFaceCoef {
+  V m, a1, a2, mq, a1q, a2q, diag, b, bq;
+  // the coefficient on face fpos of the cell (cell 1) or the neighbour (2)
+  __device__ __forceinline__ V at(int dd, int fpos, int cell) const {
+    const int e = (fpos + 1) / 2;
+    if (cell == 1) return e == dd ? m : e == tr1(dd) ? a1 : a2;
+    return e == dd ? mq : e == tr1(dd) ? a1q : a2q;
+  }
+};
+// AA slot (1-based) of m, a1, a2, mq, a1q, a2q, diag, b, bq for direction dd
+__host__ __device__ constexpr int p_slot(int dd, int n) {
+  switch (10 * dd + n) {
+    case 10: return 1; case 11: return 4; case 12: return 8; case 13: return 3; case 14: return 6; case 15: return 10; case 16: return 2;
+    case 20: return 5; case 21: return 1; case 22: return 8; case 23: return 7; case 24: return 3; case 25: return 10; case 26: return 6;
+    case 30: return 9; case 31: return 1; case 32: return 5; case 33: return 11; case 34: return 3; case 35: return 7; case 36: return 10;
+    default: return n == 7 ? 13 : 15;
+  }
+}
+// FP64: the same values formed from the two cells' NIM constants (CC of the
+// transverse directions, HH, Det at u = 0, where EE = FF = Det/2, II = GG =
+// 1/2 and JJ = -HH) and face metrics gg (face 2dd of the cell), g2 (face
+// 2dd-1 of the neighbour), by nim.f90's products in its order: 13 words a
+// cell are read for the three directions instead of AA's 27 distinct ones
+// (39 as stored).  128x128x96: k_p_faceN<double, 2> 112 -> 106 us (416 ->
+// 208 bytes a cell: byte-bound before, now by the latency of its gathers),
+// k_p_faceN<float, 4> from the 27 distinct words 62 -> 52 us; k_p_face at
+// 131x97x83 129 -> 96 us.  The float mirror keeps AA: products formed in
+// float would round otherwise.
+template <class V>
+__device__ __forceinline__ PFaceCoef<V> p_face_form(V c1, V c2, V h, V det, V gg, V q1, V q2, V hq, V detq, V g2) {
+  PFaceCoef<V> k;
+  const V E = V(0.5) * det, Eq = V(0.5) * detq;
+  const V t = (c1 + c2) * E * h, tq = (q1 + q2) * Eq * hq;
+  k.m = -(V(0.5) + t) * gg;
+  k.mq = -(V(0.5) + tq) * g2;
+  k.diag = (V(0.5) - t) * gg + (V(0.5) - tq) * g2;
+  k.a1 = c2 * E * h * gg;
+  k.a2 = c1 * E * h * gg;
+  k.a1q = q2 * Eq * hq * g2;
+  k.a2q = q1 * Eq * hq * g2;
+  k.b = -(c1 * c2 * det * h * gg);
+  k.bq = -(q1 * q2 * detq * hq * g2);
+  return k;
+}
+template <class R>
+__device__ __forceinline__ PFaceCoef<Ar<R>> p_face_coef(const GeoT<R> &g, int Nc, int c, int cn, int dd) {
+  if constexpr (std::is_same<R, double>::value) {
+    const double *C1 = g.pc + (tr1(dd) - 1) * Nc, *C2 = g.pc + (tr2(dd) - 1) * Nc, *H = g.pc + (2 + dd) * Nc;
+    const double *D = g.pc + 6 * Nc, *G = g.gfd + 2 * (dd - 1) * Nc;
+    return p_face_form<double>(C1[c], C2[c], H[c], D[c], G[Nc + c], C1[cn], C2[cn], H[cn], D[cn], G[cn]);
+  } else {
+    const R *A = g.AA + 15 * (dd - 1) * Nc + c;
+    auto ld = [&](int n) { return (Ar<R>)A[(p_slot(dd, n) - 1) * Nc]; };
+    return {ld(0), ld(1), ld(2), ld(3), ld(4), ld(5), ld(6), ld(7), ld(8)};
+  }
+}
+
 // ---- integrate_pressure_field_i for the +xi_dd face of cell x
 // (nse.f90:1091-1289): the new value from the pressures pr
 template <class Ld, class R>
 __device__ __forceinline__ Ar<R> p_face_value(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P,
                                               const R *pr, const Cell &x, int dd) {
   using V = Ar<R>;
-  const size_t Nc = d.Nc;
-  const int c = x.c;
-  const int diag = (dd == 1) ? 2 : (dd == 2) ? 6 : 10;
+  const int Nc = d.Nc, c = x.c;
   const Cell n2 = x.nb(d, 2 * dd);
-  const R *A = g.AA + (size_t)15 * (dd - 1) * Nc;
-  const V B1 = (F.Rp[c]) * A[12 * Nc + c];
-  const V B2 = (F.Rp[n2.c]) * A[14 * Nc + c];
+  const PFaceCoef<V> K = p_face_coef(g, Nc, c, n2.c, dd);
+  const V B1 = (F.Rp[c]) * K.b;
+  const V B2 = (F.Rp[n2.c]) * K.bq;
   const V B3 = (g.dg[(2 * (dd - 1)) * Nc + c]) * tangential<Ld>(d, pr, x, 2 * dd, tr1(dd));
   const V B4 = (g.dg[(2 * (dd - 1) + 1) * Nc + c]) * tangential<Ld>(d, pr, x, 2 * dd, tr2(dd));
   V s = 0.0;
 #pragma unroll
   for (int t = 0; t < 10; ++t) {
-    const int pt = p_term(dd, t), coef = pt & 15, fpos = (pt >> 4) & 7, cell = pt >> 7;
+    const int pt = p_term(dd, t), fpos = (pt >> 4) & 7, cell = pt >> 7;
     const Cell &cl = (cell == 1) ? x : n2;
-    const V term = A[(size_t)(coef - 1) * Nc + c] * Ld::ld(pr, cl.face(d, fpos));
+    const V term = K.at(dd, fpos, cell) * Ld::ld(pr, cl.face(d, fpos));
     s = (t == 0) ? -term : s - term;
   }
   const int fo = x.face(d, 2 * dd);
   const V w = V(P.w_p);
-  return (1 - w) * Ld::ld(pr, fo) + w / (A[(size_t)(diag - 1) * Nc + c]) * (s + B1 + B2 + B3 + B4);
+  return (1 - w) * Ld::ld(pr, fo) + w / K.diag * (s + B1 + B2 + B3 + B4);
 }
 
 // ---- integrate_velocity_field_i for the +xi_dd face of cell x, one
@@ -3092,23 +3163,68 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoT<R> &g, co
       on[5][NP - 1] = pr[d.offZ + cw];
       on[6][NP - 1] = pr[d.offZ + cw + pl];
     }
-    const R *A = g.AA + (size_t)15 * (dd - 1) * Nc;
-    constexpr int diag = (dd == 1) ? 2 : (dd == 2) ? 6 : 10;
-    // the ten off-diagonal terms, in source order
-    V s[NP];
+    // the coefficients (p_face_coef) and the ten off-diagonal terms, in
+    // source order
+    V s[NP], fb[NP], fbq[NP], fd[NP];
+    {
+      PFaceCoef<V> K[NP];
+      if constexpr (std::is_same<R, double>::value) {
+        // a row of per-cell words at the cells and at their +neighbours
+        auto both = [&](const R *row, R (&v)[NP], R (&vn)[NP]) {
+          ldN<R, NP>(row, c, v);
+          if (dd == 2) {
 #pragma unroll
-    for (int t = 0; t < 10; ++t) {
-      const int pt = p_term(dd, t), coef = pt & 15, fpos = (pt >> 4) & 7, cell = pt >> 7;
-      R a[NP];
-      ldN<R, NP>(A + (size_t)(coef - 1) * Nc, c, a);
+            for (int p = 0; p + 1 < NP; ++p) vn[p] = v[p + 1];
+            vn[NP - 1] = row[c - i + ipn];
+          } else {
+            ldN<R, NP>(row, c + (dd == 1 ? NT : pl), vn);
+          }
+        };
+        constexpr int e1 = (dd == 1) ? 2 : 1, e2 = (dd == 3) ? 2 : 3;
+        R c1[NP], c2[NP], h[NP], dt[NP], gg[NP], q1[NP], q2[NP], hq[NP], dq[NP], g2[NP];
+        both(g.pc + (e1 - 1) * Nc, c1, q1);
+        both(g.pc + (e2 - 1) * Nc, c2, q2);
+        both(g.pc + (2 + dd) * Nc, h, hq);
+        both(g.pc + 6 * Nc, dt, dq);
+        ldN<R, NP>(g.gfd + (2 * (dd - 1) + 1) * Nc, c, gg);
+        const R *gl = g.gfd + 2 * (dd - 1) * Nc;
+        if (dd == 2) {
+#pragma unroll
+          for (int p = 0; p + 1 < NP; ++p) g2[p] = gl[c + p + 1];
+          g2[NP - 1] = gl[c - i + ipn];
+        } else {
+          ldN<R, NP>(gl, c + (dd == 1 ? NT : pl), g2);
+        }
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+          K[p] = p_face_form<V>(c1[p], c2[p], h[p], dt[p], gg[p], q1[p], q2[p], hq[p], dq[p], g2[p]);
+      } else {
+        const R *A = g.AA + 15 * (dd - 1) * Nc;
+        R a[9][NP];
+#pragma unroll
+        for (int n = 0; n < 9; ++n) ldN<R, NP>(A + (p_slot(dd, n) - 1) * Nc, c, a[n]);
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+          K[p] = {a[0][p], a[1][p], a[2][p], a[3][p], a[4][p], a[5][p], a[6][p], a[7][p], a[8][p]};
+      }
+#pragma unroll
+      for (int t = 0; t < 10; ++t) {
+        const int pt = p_term(dd, t), fpos = (pt >> 4) & 7, cell = pt >> 7;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          const V term = K[p].at(dd, fpos, cell) * (V)((cell == 1) ? ox[fpos][p] : on[fpos][p]);
+          s[p] = (t == 0) ? -term : s[p] - term;
+        }
+      }
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
-        const V term = a[p] * (V)((cell == 1) ? ox[fpos][p] : on[fpos][p]);
-        s[p] = (t == 0) ? -term : s[p] - term;
+        fb[p] = K[p].b;
+        fbq[p] = K[p].bq;
+        fd[p] = K[p].diag;
       }
     }
     // R_p of the cells and of their +neighbours
-    R rp[NP], rn[NP], a12[NP], a14[NP], ad[NP], dg0[NP], dg1[NP];
+    R rp[NP], rn[NP], dg0[NP], dg1[NP];
     ldN<R, NP>(F.Rp, c, rp);
     if (dd == 2) {
 #pragma unroll
@@ -3117,9 +3233,6 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoT<R> &g, co
     } else {
       ldN<R, NP>(F.Rp, c + (dd == 1 ? NT : pl), rn);
     }
-    ldN<R, NP>(A + 12 * (size_t)Nc, c, a12);
-    ldN<R, NP>(A + 14 * (size_t)Nc, c, a14);
-    ldN<R, NP>(A + (size_t)(diag - 1) * Nc, c, ad);
     ldN<R, NP>(g.dg + (size_t)(2 * (dd - 1)) * Nc, c, dg0);
     ldN<R, NP>(g.dg + (size_t)(2 * (dd - 1) + 1) * Nc, c, dg1);
     // tangential derivatives of face 2dd along tr1(dd) and tr2(dd)
@@ -3190,12 +3303,12 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoT<R> &g, co
     R out[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      const V B1 = (rp[p]) * a12[p];
-      const V B2 = (rn[p]) * a14[p];
+      const V B1 = (rp[p]) * fb[p];
+      const V B2 = (rn[p]) * fbq[p];
       const V B3 = (dg0[p]) * t1[p];
       const V B4 = (dg1[p]) * t2[p];
       const V old = ox[2 * dd][p];
-      const V nw = stored<R>((1 - w) * old + w / (ad[p]) * (s[p] + B1 + B2 + B3 + B4));
+      const V nw = stored<R>((1 - w) * old + w / (fd[p]) * (s[p] + B1 + B2 + B3 + B4));
       out[p] = (R)nw;
       e[0] = nmax(e[0], errv(nw, old, first));
     }
