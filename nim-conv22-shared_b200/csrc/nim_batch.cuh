@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(BLK) kb_zero_flux(BatchArgs A) {
 template <class R, int W>
 __global__ void __launch_bounds__(CB3, wider(minb<R>(TCELL_MINB, TCELL_MINB_F), W)) kb_T_cell(BatchArgs A) {
   batch_items<BS_T_CELL, R, FlatBlock>(A, [&](const BatchInst<R> &I, FlatBlock b) {
-    T_cell_body<false, R>(I.d, I.g, I.F, I.P, I.ctl, b);
+    T_cell_body<R>(I.d, I.g, I.F, I.P, I.ctl, b);
   });
 }
 template <class R, int W>
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(BLK) kg_zero_flux(const __grid_constant__ Batc
 }
 template <class R>
 __global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) kg_T_cell(const __grid_constant__ BatchGroup<R> L) {
-  group_item<R, FlatBlock>(L, [&](const BatchInst<R> &I, FlatBlock b) { T_cell_body<false, R>(I.d, I.g, I.F, I.P, I.ctl, b); });
+  group_item<R, FlatBlock>(L, [&](const BatchInst<R> &I, FlatBlock b) { T_cell_body<R>(I.d, I.g, I.F, I.P, I.ctl, b); });
 }
 template <class R>
 __global__ void __launch_bounds__(BLK, minb<R>(4, TFACE_MINB_F)) kg_T_face(const __grid_constant__ BatchGroup<R> L) {

@@ -89,9 +89,9 @@ struct nim_ctx {
   int kernels_per_iter = 0;
   // reference-order schedule
   bool seq = false;
-  int *order = nullptr, *lstart = nullptr;  // cells level by level, level starts
-  int nlev = 0;
-  int *border = nullptr, *blev = nullptr, *wlev = nullptr;  // wall faces, levels, per-wall level ranges
+  SeqTab seqt{};
+  bool seq_grid = false;                     // levels wider than a block's share: cooperative grids
+  int seq_threads = 0, wall_threads = 0;     // block sizes of the one-block sweeps
   int coop_vel = 0, coop_p = 0, coop_T = 0;  // cooperative grid sizes
   // nim_gpu_profile_iterations: while set, every kernel launch of an
   // iteration is followed by an event and its name
@@ -357,14 +357,7 @@ int launch_vel(nim_ctx *x, cudaStream_t s, const GeoT<DualD> &g, const FieldsT<D
 
 template <typename K>
 int launch_coop(K kern, int blocks, dim3 block, nim_ctx *x) {
-  Dims d = x->d;
-  Geo g = x->g;
-  Fields F = x->F;
-  Phys P = x->phys;
-  Ctrl *ctl = x->ctl;
-  const int *order = x->order, *lstart = x->lstart;
-  int nlev = x->nlev;
-  void *args[] = {&d, &g, &F, &P, &ctl, &order, &lstart, &nlev};
+  void *args[] = {&x->d, &x->g, &x->F, &x->phys, &x->ctl, &x->seqt};
   CK(cudaLaunchCooperativeKernel((const void *)kern, dim3(blocks), block, args, 0, x->stream));
   return NIM_OK;
 }
@@ -374,22 +367,33 @@ int launch_coop(K kern, int blocks, dim3 block, nim_ctx *x) {
 int launch_iteration_seq(nim_ctx *x) {
   const Dims &d = x->d;
   cudaStream_t s = x->stream;
-  if (x->phys.formulation == 1) {
+  const SeqTab &S = x->seqt;
+  const bool one = x->phys.formulation == 1, grid_form = x->seq_grid;
+  const int nt = x->seq_threads;
+  const bool wide = nt > SEQ_TPB;
+  if (one)
     k_vel_cell<true, 1><<<x->g3, dim3(CB, 3), 0, s>>>(d, x->g, x->F, x->phys, x->ctl);
-    TRY(mark(x, "k_vel_cell(src)"));
-    TRY(launch_coop(k_seq_vel<1>, x->coop_vel, dim3(CB, 3), x));
-  } else {
+  else
     k_vel_cell<true, 2><<<x->g3, dim3(CB, 3), 0, s>>>(d, x->g, x->F, x->phys, x->ctl);
-    TRY(mark(x, "k_vel_cell(src)"));
-    TRY(launch_coop(k_seq_vel<2>, x->coop_vel, dim3(CB, 3), x));
-  }
+  TRY(mark(x, "k_vel_cell(src)"));
+  if (grid_form)
+    TRY(one ? launch_coop(k_seq_vel<1, true, CB3>, x->coop_vel, dim3(CB, 3), x)
+            : launch_coop(k_seq_vel<2, true, CB3>, x->coop_vel, dim3(CB, 3), x));
+  else if (one)
+    (wide ? k_seq_vel<1, false, SEQ_TPB_WIDE> : k_seq_vel<1, false, SEQ_TPB>)<<<3, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+  else
+    (wide ? k_seq_vel<2, false, SEQ_TPB_WIDE> : k_seq_vel<2, false, SEQ_TPB>)<<<3, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   TRY(mark(x, "k_seq_vel"));
   k_p_src<<<x->g3, dim3(CB, 3), 0, s>>>(d, x->g, x->F, x->phys, x->ctl);
   TRY(mark(x, "k_p_src"));
-  k_seq_pbc<<<2, BLK, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, x->border, x->blev, x->wlev, 0);
-  k_seq_pbc<<<2, BLK, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, x->border, x->blev, x->wlev, 2);
+  k_p_bc_fixed<<<x->nblk_b, BLK, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+  k_seq_pbc<<<2, x->wall_threads, 0, s>>>(d, x->F, x->phys, x->ctl, S, 0);
+  k_seq_pbc<<<2, x->wall_threads, 0, s>>>(d, x->F, x->phys, x->ctl, S, 2);
   TRY(mark(x, "k_seq_pbc"));
-  TRY(launch_coop(k_seq_p, x->coop_p, dim3(BLK), x));
+  if (grid_form)
+    TRY(launch_coop(k_seq_p<true, BLK>, x->coop_p, dim3(BLK), x));
+  else
+    (wide ? k_seq_p<false, SEQ_TPB_WIDE> : k_seq_p<false, SEQ_TPB>)<<<1, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   TRY(mark(x, "k_seq_p"));
   if (x->phys.dpdx_tolerance) {
     k_p_dpdx<<<x->nblk_c, BLK, 0, s>>>(d, x->g, x->F, x->ctl);
@@ -399,15 +403,42 @@ int launch_iteration_seq(nim_ctx *x) {
   TRY(mark(x, "k_zero_flux"));
   k_T_coef<<<dim3(3, x->nblk_c), BLK, 0, s>>>(d, x->g, x->F, x->phys, x->ctl);
   TRY(mark(x, "k_T_coef"));
-  k_T_cell<true><<<x->g3, dim3(CB, 3), 0, s>>>(d, x->g, x->F, x->phys, x->ctl);
+  k_T_src<<<x->nblk_c, BLK, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   TRY(mark(x, "k_T_cell(src)"));
-  TRY(launch_coop(k_seq_T, x->coop_T, dim3(BLK), x));
+  if (grid_form)
+    TRY(launch_coop(k_seq_T<true, BLK>, x->coop_T, dim3(BLK), x));
+  else
+    (wide ? k_seq_T<false, SEQ_TPB_WIDE> : k_seq_T<false, SEQ_TPB>)<<<1, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   TRY(mark(x, "k_seq_T"));
   k_iter_end<<<1, 1, 0, s>>>(x->ctl, x->phys, 0);
   TRY(mark(x, "k_iter_end"));
   CK(cudaGetLastError());
-  x->kernels_per_iter = x->phys.dpdx_tolerance ? 12 : 11;
+  x->kernels_per_iter = x->phys.dpdx_tolerance ? 14 : 13;
   x->launches += x->kernels_per_iter;
+  return NIM_OK;
+}
+
+// a step's velocity constants in level order
+int seq_pack_velocity(nim_ctx *x) {
+  const SeqTab &S = x->seqt;
+  const int Nc = x->d.Nc;
+  const bool one = x->phys.formulation == 1;
+  const double *src[2] = {one ? x->F.AT : x->F.MF4, one ? x->F.AAv : x->F.MF};
+  const int rows[2] = {one ? 9 : 8, one ? 45 : 15};
+  k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(src[0], S.vel, S.order, rows[0], Nc);
+  k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(src[1], S.vel + (size_t)rows[0] * Nc, S.order, rows[1], Nc);
+  CK(cudaGetLastError());
+  x->launches += 2;
+  return NIM_OK;
+}
+// what stays as it is after init: the metric differences, the pressure
+// constants and the wall faces' stencils
+int seq_pack_geometry(nim_ctx *x) {
+  const SeqTab &S = x->seqt;
+  k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(x->g.dg, S.dg, S.order, 6, x->d.Nc);
+  k_seq_pack_p<<<x->nblk_c, BLK, 0, x->stream>>>(x->d, x->g, x->phys, S);
+  k_seq_pack_wall<<<x->nblk_b, BLK, 0, x->stream>>>(x->d, S);
+  CK(cudaGetLastError());
   return NIM_OK;
 }
 
@@ -479,7 +510,7 @@ int launch_temperature(nim_ctx *x, cudaStream_t s, const GeoT<R> &g, const Field
       return NIM_OK;
     }
   }
-  k_T_cell<false><<<x->g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+  k_T_cell<<<x->g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
   TRY(mark(x, "k_T_cell"));
   k_T_face<<<x->g8, BLK, 0, s>>>(d, g, F, x->phys, x->ctl);
   TRY(mark(x, "k_T_face"));
@@ -810,15 +841,15 @@ static int noalloc_setup(int device) {
 // numbers (the argument is in nim_kernels.cuh).  Wall faces, in BC-list
 // order bottom, top, inner, outer: level i + 2j on bottom and top, i + 2k on
 // inner and outer.  Also the sweep buffers and the cooperative grid sizes.
+constexpr int kSeqBlock = 1024;  // widest level swept by one block
 static int setup_levels(nim_ctx *x) {
   const Dims &d = x->d;
   const size_t Nc = d.Nc;
-  TRY(dalloc(x, &x->F.MTF4, 8 * Nc));
   TRY(dalloc(x, &x->F.MT4, 9 * Nc));
-  TRY(dalloc(x, &x->F.RDT, Nc));
   // counting sort of the cells by level
   const int nlev = (d.NT - 1) + 2 * (d.NR - 1) + 3 * (d.NZ - 1) + 1;
-  std::vector<int> lstart(nlev + 1, 0), order(Nc), fill;
+  std::vector<int> lstart(nlev + 1, 0), fill;
+  std::vector<int4> order(Nc);
   for (int c = 0; c < d.Nc; ++c) {
     const Cell q = Cell::of(d, c);
     ++lstart[q.i + 2 * q.j + 3 * q.k + 1];
@@ -831,7 +862,7 @@ static int setup_levels(nim_ctx *x) {
   fill.assign(lstart.begin(), lstart.end() - 1);
   for (int c = 0; c < d.Nc; ++c) {
     const Cell q = Cell::of(d, c);
-    order[fill[q.i + 2 * q.j + 3 * q.k]++] = c;
+    order[fill[q.i + 2 * q.j + 3 * q.k]++] = make_int4(c, q.j, q.k, 0);
   }
   // wall faces: per wall, counting sort by the in-wall level
   const int nb1 = d.NT * d.NR, nb3 = d.NT * d.NZ;
@@ -849,17 +880,33 @@ static int setup_levels(nim_ctx *x) {
     q += wn[w];
     wlev.push_back((int)blev.size() - 1);
   }
-  x->nlev = nlev;
-  TRY(dalloc(x, &x->order, Nc));
-  TRY(dalloc(x, &x->lstart, (size_t)nlev + 1));
-  TRY(dalloc(x, &x->border, (size_t)d.NBF));
-  TRY(dalloc(x, &x->blev, blev.size()));
-  TRY(dalloc(x, &x->wlev, wlev.size()));
-  CK(cudaMemcpy(x->order, order.data(), sizeof(int) * Nc, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(x->lstart, lstart.data(), sizeof(int) * (nlev + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(x->border, border.data(), sizeof(int) * d.NBF, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(x->blev, blev.data(), sizeof(int) * blev.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(x->wlev, wlev.data(), sizeof(int) * wlev.size(), cudaMemcpyHostToDevice));
+  SeqTab &S = x->seqt;
+  S.nlev = nlev;
+  TRY(dalloc(x, &S.order, Nc));
+  TRY(dalloc(x, &S.lstart, (size_t)nlev + 1));
+  TRY(dalloc(x, &S.border, (size_t)d.NBF));
+  TRY(dalloc(x, &S.blev, blev.size()));
+  TRY(dalloc(x, &S.wlev, wlev.size()));
+  TRY(dalloc(x, &S.dg, 6 * Nc));
+  TRY(dalloc(x, &S.vel, (x->phys.formulation == 1 ? 54 : 23) * Nc));
+  TRY(dalloc(x, &S.prs, 3 * kSeqP * Nc));
+  TRY(dalloc(x, &S.tmp, kSeqT * Nc));
+  TRY(dalloc(x, &S.wall, kSeqW * (size_t)d.NBF));
+  TRY(dalloc(x, &S.wface, kSeqI * (size_t)d.NBF));
+  CK(cudaMemcpy(S.order, order.data(), sizeof(int4) * Nc, cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(S.lstart, lstart.data(), sizeof(int) * (nlev + 1), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(S.border, border.data(), sizeof(int) * d.NBF, cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(S.blev, blev.data(), sizeof(int) * blev.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(S.wlev, wlev.data(), sizeof(int) * wlev.size(), cudaMemcpyHostToDevice));
+  // block sizes: whole warps for the widest level, at most SEQ_TPB_WIDE (a level
+  // up to kSeqBlock wide then takes that many turns), or a cooperative grid
+  auto warps = [](int n, int most) { return std::min(most, (n + 31) / 32 * 32); };
+  int wmax = 1;
+  for (size_t L = 0; L + 1 < blev.size(); ++L) wmax = std::max(wmax, blev[L + 1] - blev[L]);
+  x->seq_threads = warps(maxlev, SEQ_TPB_WIDE);
+  x->wall_threads = warps(wmax, BLK);
+  x->seq_grid = maxlev > kSeqBlock;
+  if (!x->seq_grid) return NIM_OK;
   // cooperative grids: no more blocks than the widest level needs, and no
   // more than can be resident at once (cudaLaunchCooperativeKernel rejects
   // a larger grid rather than running it)
@@ -870,13 +917,13 @@ static int setup_levels(nim_ctx *x) {
   const int want = std::max(1, (maxlev + BLK - 1) / BLK);
   int per = 0;
   if (x->phys.formulation == 1)
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_vel<1>, CB3, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_vel<1, true, CB3>, CB3, 0));
   else
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_vel<2>, CB3, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_vel<2, true, CB3>, CB3, 0));
   x->coop_vel = std::max(1, std::min((maxlev + CB - 1) / CB, per * sms));
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_p, BLK, 0));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_p<true, BLK>, BLK, 0));
   x->coop_p = std::max(1, std::min(want, per * sms));
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_T, BLK, 0));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_T<true, BLK>, BLK, 0));
   x->coop_T = std::max(1, std::min(want, per * sms));
   if (x->coop_vel < 1 || x->coop_p < 1 || x->coop_T < 1) return NIM_ERR_CUDA;
   return NIM_OK;
@@ -1288,6 +1335,7 @@ extern "C" int nim_gpu_init(nim_ctx *x) {
   k_wall_floor<<<x->nblk_b, BLK, 0, s>>>(d, x->g, x->ctl);
   CK(cudaGetLastError());
   if (x->mixed) TRY(mirror_geometry(x));
+  if (x->seq) TRY(seq_pack_geometry(x));
   CK(cudaStreamSynchronize(s));
   x->TI = x->params.DT;  // nse.f90:31
   x->STEP = 1;           // nse.f90:32
@@ -1313,6 +1361,7 @@ extern "C" int nim_gpu_begin_step(nim_ctx *x) {
   CK(cudaGetLastError());
   x->launches += 3;
   if (x->mixed) TRY(mirror_step_coefficients(x));
+  if (x->seq) TRY(seq_pack_velocity(x));
   x->in_step = true;
   return NIM_OK;
 }

@@ -102,10 +102,8 @@ struct FieldsT {
   R *MTF;     // [12][Nc]  the cell's own terms of MT_F1..3 (TDir): G1, G3, H2, H4 of direction d at 4(d-1)
   R *MT4;     // [9][Nc]   its terms of MT_F4 (TDir): r, m, p of direction d at 3(d-1) (reference order only)
   R *dpd;     // [3][Nc]   dpdx_old, dpdy_old, dpdz_old
-  // reference-order schedule: sources stored before the ordered sweeps
+  // reference-order schedule and formulation 1: sources stored before the sweeps
   R *Bv;      // [3][Nc]   R_C + R_D + R_B of u, v, w
-  R *MTF4;    // [8][Nc]   MT_F4
-  R *RDT;     // [Nc]      R_D_T
   // formulation 1 (nim_formulation = 1)
   R *N1;      // [22][Nc]  CC, EE, FF, GG, HH, II, JJ (3 each), Det (per step)
   R *AT;      // [9][Nc]   a_t
@@ -183,6 +181,9 @@ struct Ctrl {
 constexpr int kLowpStall = 8;
 
 constexpr int BLK = 256;
+// most threads of a reference-order sweep in one block: 256 keep a cell's
+// values in registers (255 a thread), 512 (128 a thread) serve wider levels
+constexpr int SEQ_TPB = 256, SEQ_TPB_WIDE = 512;
 constexpr int VC2_MINB = 3;  // resident blocks per SM asked of k_vel_cell2 (56 registers)
 // resident blocks per SM the float instantiations of the pass kernels ask
 // for: computing in float they need about half the FP64 registers
@@ -204,7 +205,7 @@ constexpr int CB3 = 3 * CB;        // threads per block
 // ------------------------------------------------------------ reductions
 // Max of non-negative doubles through their bit patterns (IEEE order equals
 // integer order for x >= 0; NaN sorts above +Inf and is caught as non-finite).
-// NT = threads in the block (flattened).  Call red_init() first (it holds
+// NT = threads in the block (flattened; 0: read from the launch).  Call red_init() first (it holds
 // the only barrier); block_max() is barrier-free: warps fold their maxima
 // into shared memory with atomics and the last warp to finish publishes the
 // block's maxima with one global atomic each.
@@ -240,7 +241,7 @@ __device__ __forceinline__ void block_max(BlockRed &r, const double (&v)[N], uns
       if (b[n]) atomicMax(&r.m[n], b[n]);
     __threadfence_block();
     const unsigned int done = atomicAdd(&r.count, 1u);
-    if (done == NT / 32 - 1) {
+    if (done == (NT ? NT : blockDim.x * blockDim.y) / 32 - 1) {
       __threadfence_block();
 #pragma unroll
       for (int n = 0; n < N; ++n) {
@@ -2806,18 +2807,16 @@ __global__ void __launch_bounds__(CB3, PSN_MINB) k_p_srcN(Dims d, GeoT<R> g, Fie
   p_srcN_body<R, NP>(d, g, F, P, ctl, LaunchBlock{});
 }
 
-// ---- apply_pressure_bc for wall face b (bc.f90:148-339): the new value
-// from the pressures pr, the new velocities fu/fv/fwv and the temperatures fT
-template <class Ld, class R>
-__device__ __forceinline__ Ar<R> p_bc_value(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P,
-                                            const R *pr, const R *fu, const R *fv, const R *fwv, const R *fT,
-                                            int b) {
+// ---- apply_pressure_bc for wall face b (bc.f90:148-339).  p_bc_fixed: the
+// terms that no wall pressure enters, from the new velocities fu/fv/fwv, R_p
+// and the temperatures fT: B1 and the body of the momentum balance.
+template <class R>
+__device__ __forceinline__ void p_bc_fixed(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P,
+                                           const R *fu, const R *fv, const R *fwv, const R *fT, int b,
+                                           const BFace &B, Ar<R> &B1, Ar<R> &body) {
   using V = Ar<R>;
   const int NF = d.NF, NB = d.NBF;
-  const BFace B = bface(d, b);
-  const Cell M1 = B.cell;
-  const int pos = B.pos;
-  const int fw0 = M1.face(d, pos);
+  const int fw0 = B.cell.face(d, B.pos);
   const V n[3] = {g.normal[fw0], g.normal[NF + fw0], g.normal[2 * NF + fw0]};
   const V bvec[3] = {V(0), V(0), -(V(P.g_beta) * (fT[fw0]))};
   const V b_n = dot3(bvec, n);
@@ -2830,11 +2829,26 @@ __device__ __forceinline__ Ar<R> p_bc_value(const Dims &d, const GeoT<R> &g, con
   const R *a = g.bca;
   const V d2udn2 = -(a[b] * vn[1]) - a[NB + b] * vn[2] - a[2 * NB + b] * vn[3] - a[3 * NB + b] * vn[4] -
                         a[4 * NB + b] * vn[5];
+  B1 = g.bcap[7 * NB + b] * (F.Rp[B.cell.c]);
+  body = pv<V>(P.nu, P.d_nu) * V(P.rho) * d2udn2 - b_n * V(P.rho);
+}
+// the new value from the pressures pr
+template <class Ld, class R>
+__device__ __forceinline__ Ar<R> p_bc_value(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P,
+                                            const R *pr, const R *fu, const R *fv, const R *fwv, const R *fT,
+                                            int b) {
+  using V = Ar<R>;
+  const int NB = d.NBF;
+  const BFace B = bface(d, b);
+  const Cell M1 = B.cell;
+  const int pos = B.pos;
+  const int fw0 = M1.face(d, pos);
+  V B1, body;
+  p_bc_fixed(d, g, F, P, fu, fv, fwv, fT, b, B, B1, body);
   const int dd = (pos + 1) / 2;
   const V B2 = tangential<Ld>(d, pr, M1, pos, tr1(dd)) * g.bcg[b];
   const V B3 = tangential<Ld>(d, pr, M1, pos, tr2(dd)) * g.bcg[NB + b];
   const R *ap = g.bcap;
-  const V B1 = ap[7 * NB + b] * (F.Rp[M1.c]);
   V s = 0.0;
   bool firstterm = true;
   for (int k = 1; k <= 6; ++k) {
@@ -2844,8 +2858,7 @@ __device__ __forceinline__ Ar<R> p_bc_value(const Dims &d, const GeoT<R> &g, con
     firstterm = false;
   }
   const V w = V(P.w_p2);
-  return (1 - w) * Ld::ld(pr, fw0) +
-         w / (ap[(pos - 1) * NB + b]) * (s + B1 - B2 - B3 + (pv<V>(P.nu, P.d_nu) * V(P.rho) * d2udn2 - b_n * V(P.rho)));
+  return (1 - w) * Ld::ld(pr, fw0) + w / (ap[(pos - 1) * NB + b]) * (s + B1 - B2 - B3 + body);
 }
 
 // ---- K4: apply_pressure_bc, every wall face from the values before the pass
@@ -3515,9 +3528,7 @@ __global__ void __launch_bounds__(BLK, 4) k_T_coef(Dims d, GeoT<R> g, FieldsT<R>
 // MT_A (18 words) and MT_F (15) written and read through memory by a kernel
 // of their own it was 952.  128x128x96: FP64 T_coef + T_cell 305 -> 289 us,
 // float (k_T_cellN) 128 -> 91 us, and k_T_faceN 51 -> 45 us.
-// SRC_ONLY (reference-order schedule): the constants are k_T_coef's; store
-// MT_F4 and R_D_T and leave the update to k_seq_T.
-template <bool SRC_ONLY, class R, class BI>
+template <class R, class BI>
 __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   using V = Ar<R>;
   if (ctl->done) return;
@@ -3539,10 +3550,7 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, con
   cell_faces(d, x, f);
   if (active) by_dir(threadIdx.y, [&](auto D) {
     constexpr int dd = decltype(D)::value, y = dd - 1;
-    if (SRC_ONLY) {
-      const R *q = F.MT4 + 3 * y * Nc;
-      for (int n = 0; n < 3; ++n) sF[y][n][tx] = q[n * Nc + c];
-    } else {
+    {
       const TDir<V> t = T_direction_of(g, F, P, Nc, c, dd);
       R *row = F.MTF + 4 * y * Nc;
       row[c] = t.G1;
@@ -3580,21 +3588,16 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, con
     const R *gij = g.gij;
     const V RDT = pv<V>(P.alpha, P.d_alpha) * (sG[tx] - gij[3 * Nc + c] * pxy - gij[1 * Nc + c] * pyx - gij[6 * Nc + c] * pxz -
                                   gij[2 * Nc + c] * pzx - gij[7 * Nc + c] * pyz - gij[5 * Nc + c] * pzy);
-    if (SRC_ONLY) {
-      for (int k = 0; k < 8; ++k) F.MTF4[(size_t)k * Nc + c] = F4[k];
-      F.RDT[c] = RDT;
-    } else {
-      const V cold = F.c[3][c];
-      const V nw = stored<R>(cell_update(T, f, cold, F.co[3][c], (RDT + V(0.)), F4, V(P.w[3])));
-      F.c[3][c] = nw;
-      e[0] = errv(nw, cold, first);
-    }
+    const V cold = F.c[3][c];
+    const V nw = stored<R>(cell_update(T, f, cold, F.co[3][c], (RDT + V(0.)), F4, V(P.w[3])));
+    F.c[3][c] = nw;
+    e[0] = errv(nw, cold, first);
   }
-  if (!SRC_ONLY && d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 4);
+  if (d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 4);
 }
-template <bool SRC_ONLY, class R>
+template <class R>
 __global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) k_T_cell(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  T_cell_body<SRC_ONLY, R>(d, g, F, P, ctl, LaunchBlock{});
+  T_cell_body<R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
 // ---- K7b, NP cells per thread (the float mirror's parallel passes,
@@ -4209,149 +4212,461 @@ __global__ void __launch_bounds__(BLK) k_convert(CvtList L) {
 // iterates exactly.  order[] lists the cells level by level, lstart[] the
 // level boundaries.
 
-// velocity sweep (integrate_velocity_field_formulation2_i, nse.f90:831-1006;
-// FORM 1: integrate_velocity_field_i, nse.f90:330-828).  Block (CB, 3):
-// threadIdx.y = component; the three components of a cell touch disjoint
-// data, so they run side by side.
-template <int FORM>
-__global__ void __launch_bounds__(CB3) k_seq_vel(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl,
-                                                 const int *__restrict__ order, const int *__restrict__ lstart,
-                                                 int nlev) {
+//
+// A level is a chain: barrier, the loads of what the last level wrote, the
+// update, its stores.  So the sweeps load everything a cell's update reads
+// up front, side by side (the updates of its own three faces reach the later
+// ones in registers), read the coefficients coalesced from copies in level
+// order (SeqTab), and look up the next level's cells before the barrier.
+// Levels that fit a block run in one block per swept field, whose barrier is
+// the SM's own and whose loads hit its L1; wider ones on a cooperative grid
+// (the three velocity components side by side), which reads through L2.
+// Time of a pass with dependent loads and a grid barrier a level before, and
+// now: 36x6x12 (66 cells wide) 1891 -> 486 us, 24x24x16 formulation 1 (168)
+// 3882 -> 939 us, 48x48x32 (672) 10.3 -> 5.0 ms, 128x128x96 (grid) 35.2 ->
+// 20.6 ms.  What is left of a level is its gathers: the cells of a level lie
+// on different lines of the swept arrays.
+
+// tables of the reference-order schedule
+struct SeqTab {
+  int4 *order;          // cells level by level: cell number, j, k
+  int *lstart;          // level starts
+  int nlev;
+  int *border, *blev, *wlev;  // wall faces, levels, per-wall level ranges
+  // rows in level order, [row][Nc]: the face-metric differences dg (6); the
+  // velocity constants of a step (formulation 2: M_F4 (8), M_F1..3 (15);
+  // 1: a_t (9), AA_v (45)); the pressure constants (kSeqP a direction); the
+  // temperature constants and R_D_T of a pass (kSeqT)
+  double *dg, *vel, *prs, *tmp;
+  // in border order: the faces a wall face's update reads and the
+  // constants of apply_pressure_bc in this pass
+  int *wface;    // [kSeqI][NBF]
+  double *wall;  // [kSeqW][NBF]
+};
+constexpr int kSeqI = 11;  // the face, its cell's other five, two stencils (a, b) along the wall, wall-end flags
+constexpr int kSeqP = 9;   // m, a1, a2, mq, a1q, a2q, w/diag, b, bq of one direction
+constexpr int kSeqT = 24;  // w/MT_F4(0), MT_F4(1..7), (w/MT_F(0), MT_F(1..4)) x 3, R_D_T
+constexpr int kSeqW = 10;  // w/ap(pos), B1, body, the two bcg, the five ap of the other faces
+
+// dst[row][q] = src[row][order[q]]: rows of a per-cell array into level order
+__global__ void __launch_bounds__(BLK) k_seq_pack(const double *__restrict__ src, double *__restrict__ dst,
+                                                  const int4 *__restrict__ order, int rows, int Nc) {
+  const int q = blockIdx.x * BLK + threadIdx.x;
+  if (q >= Nc) return;
+  const int c = order[q].x;
+  for (int r = 0; r < rows; ++r) dst[(size_t)r * Nc + q] = src[(size_t)r * Nc + c];
+}
+// the pressure sweep's constants in level order, once at init
+__global__ void __launch_bounds__(BLK) k_seq_pack_p(Dims d, Geo g, Phys P, SeqTab S) {
+  const int q = blockIdx.x * BLK + threadIdx.x, Nc = d.Nc;
+  if (q >= Nc) return;
+  const Cell x = Cell::of(d, S.order[q].x);
+  for (int dd = 1; dd <= 3; ++dd) {
+    if (!x.has_nb(d, 2 * dd)) continue;
+    const PFaceCoef<double> K = p_face_coef(g, Nc, x.c, x.nb(d, 2 * dd).c, dd);
+    const double v[kSeqP] = {K.m, K.a1, K.a2, K.mq, K.a1q, K.a2q, P.w_p / K.diag, K.b, K.bq};
+    for (int n = 0; n < kSeqP; ++n) S.prs[(size_t)(kSeqP * (dd - 1) + n) * Nc + q] = v[n];
+  }
+}
+// calculate_R_D_T (nse.f90:2000-2134) and the temperature sweep's constants
+// of this pass (from k_T_coef's terms), in level order
+__global__ void __launch_bounds__(BLK) k_T_src(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
+  if (ctl->done) return;
+  const int q = blockIdx.x * BLK + threadIdx.x, Nc = d.Nc;
+  if (q >= Nc) return;
+  const int c = S.order[q].x;
+  const Cell x = Cell::of(d, c);
+  int f[7];
+  cell_faces(d, x, f);
+  const double w = P.w[3];
+  double r[3], m[3], p[3], F4[8];
+  for (int n = 0; n < 3; ++n) {
+    r[n] = F.MT4[3 * n * Nc + c];
+    m[n] = F.MT4[(3 * n + 1) * Nc + c];
+    p[n] = F.MT4[(3 * n + 2) * Nc + c];
+  }
+  T_form_F4(r, m, p, P.DT, F4);
+  double *o = S.tmp + q;
+  o[0] = w / F4[0];
+  for (int k = 1; k < 8; ++k) o[k * Nc] = F4[k];
+  for (int dd = 1; dd <= 3; ++dd) {
+    if (!x.has_nb(d, 2 * dd)) continue;
+    double Fd[5];
+    T_form_Fd(F, Nc, c, x.nb(d, 2 * dd).c, dd, Fd);
+    double *of = o + (8 + 5 * (dd - 1)) * Nc;
+    of[0] = w / Fd[0];
+    for (int k = 1; k < 5; ++k) of[k * Nc] = Fd[k];
+  }
+  const double *T = F.f[4] + (size_t)parity(ctl) * d.NF;
+  o[23 * Nc] = P.alpha * diffusion_source(d, g, T, x, f);
+}
+
+// a cell of a level with its index steps to the +r, +theta, +z neighbours (0
+// where there is none: the loads then stay on the cell and are not used)
+struct SeqCell {
+  int c, i, j, k;
+  int f[7];         // its faces
+  int st, ip2;      // step to the +theta neighbour, theta index past it
+  bool has[4];      // has[dd]: a neighbour across +xi_dd
+  __device__ __forceinline__ SeqCell() {}
+  __device__ __forceinline__ SeqCell(const Dims &d, const int4 o) : c(o.x), j(o.y), k(o.z) {
+    i = c - d.NT * (j + d.NR * k);
+    st = (i == d.NT - 1) ? 1 - d.NT : 1;
+    const int ip = i + st;
+    ip2 = (ip == d.NT - 1) ? 0 : ip + 1;
+    f[1] = c + d.NT * k;
+    f[2] = f[1] + d.NT;
+    f[3] = d.offT + c;
+    f[4] = f[3] + st;
+    f[5] = d.offZ + c;
+    f[6] = f[5] + d.plane;
+    has[1] = j < d.NR - 1;
+    has[2] = true;
+    has[3] = k < d.NZ - 1;
+  }
+  __device__ __forceinline__ int nb(const Dims &d, int dd) const {  // cell index of the +xi_dd neighbour
+    return c + (dd == 1 ? (has[1] ? d.NT : 0) : dd == 2 ? st : (has[3] ? d.plane : 0));
+  }
+};
+// the faces of the cell (x) and of its +r, +theta, +z neighbours (r, t, z):
+// what its own three +xi face updates read (x[2] = r[1], x[4] = t[3],
+// x[6] = z[5]); no branches, so every load is in flight at once
+struct Hood {
+  double x[7], r[7], t[7], z[7];
+  __device__ __forceinline__ const double *of(int dd) const { return dd == 1 ? r : dd == 2 ? t : z; }
+};
+template <class Ld>
+__device__ __forceinline__ void load_hood(const Dims &d, const double *fr, const SeqCell &x, Hood &h) {
+  const int up = x.has[1] ? d.NT : 0, zr = x.has[3] ? d.NT * (d.NR + 1) : 0, zc = x.has[3] ? d.plane : 0;
+#pragma unroll
+  for (int k = 1; k <= 6; ++k) h.x[k] = Ld::ld(fr, x.f[k]);
+#pragma unroll
+  for (int k = 2; k <= 6; ++k) h.r[k] = Ld::ld(fr, x.f[k] + up);
+  h.t[1] = Ld::ld(fr, x.f[1] + x.st);
+  h.t[2] = Ld::ld(fr, x.f[2] + x.st);
+  h.t[4] = Ld::ld(fr, x.f[3] - x.i + x.ip2);
+  h.t[5] = Ld::ld(fr, x.f[5] + x.st);
+  h.t[6] = Ld::ld(fr, x.f[6] + x.st);
+  h.z[1] = Ld::ld(fr, x.f[1] + zr);
+  h.z[2] = Ld::ld(fr, x.f[2] + zr);
+  h.z[3] = Ld::ld(fr, x.f[3] + zc);
+  h.z[4] = Ld::ld(fr, x.f[4] + zc);
+  h.z[6] = Ld::ld(fr, x.f[6] + zc);
+}
+// tangential() of the faces 2, 4, 6 along their two transverse directions
+// (t[dd][0]: tr1(dd), t[dd][1]: tr2(dd)), the wall side chosen by index
+struct Tang {
+  double a[4][2], b[4][2];
+};
+template <class Ld>
+__device__ __forceinline__ void load_tang(const Dims &d, const double *fr, const SeqCell &x, const Hood &h, Tang &t) {
+  const bool rlo = x.j == 0, rhi = x.j == d.NR - 1, zlo = x.k == 0, zhi = x.k == d.NZ - 1;
+  const int ra = rlo ? 1 : -1, rb = rlo ? 2 : rhi ? -2 : 1, za = zlo ? 1 : -1, zb = zlo ? 2 : zhi ? -2 : 1;
+  const int im = (x.i == 0) ? d.NT - 1 : -1, zr = d.NT * (d.NR + 1);
+  t.a[1][0] = Ld::ld(fr, x.f[2] + im);  // face 2 along theta: always centred
+  t.b[1][0] = h.t[2];
+  t.a[1][1] = Ld::ld(fr, x.f[2] + za * zr);
+  t.b[1][1] = Ld::ld(fr, x.f[2] + zb * zr);
+  t.a[2][0] = Ld::ld(fr, x.f[4] + ra * d.NT);
+  t.b[2][0] = Ld::ld(fr, x.f[4] + rb * d.NT);
+  t.a[2][1] = Ld::ld(fr, x.f[4] + za * d.plane);
+  t.b[2][1] = Ld::ld(fr, x.f[4] + zb * d.plane);
+  t.a[3][0] = Ld::ld(fr, x.f[6] + ra * d.NT);
+  t.b[3][0] = Ld::ld(fr, x.f[6] + rb * d.NT);
+  t.a[3][1] = Ld::ld(fr, x.f[6] + im);  // face 6 along theta
+  t.b[3][1] = h.t[6];
+}
+__device__ __forceinline__ double tang_of(const Dims &d, const SeqCell &x, const Tang &t, int dd, int n, double v0) {
+  const int e = n == 0 ? tr1(dd) : tr2(dd);
+  const bool lo = (e == 1 && x.j == 0) || (e == 3 && x.k == 0);
+  const bool hi = (e == 1 && x.j == d.NR - 1) || (e == 3 && x.k == d.NZ - 1);
+  const double va = t.a[dd][n], vb = t.b[dd][n];
+  return lo ? (-(3 * v0) + 4 * va - vb) / 4. : hi ? (3 * v0 - 4 * va + vb) / 4. : (vb - va) / 4.;
+}
+// stores of the ordered sweeps: plain within a block, in program order and
+// uncached (volatile) where other SMs read
+template <class Ld>
+__device__ __forceinline__ void st_seq(double *p, size_t i, double v) {
+  if (std::is_same<Ld, LdCoh>::value)
+    st_coh(p, i, v);
+  else
+    p[i] = v;
+}
+
+// The walk over the levels.  Sweep::fixed(q, x, st) loads into registers what
+// the sweep itself does not change (coefficients, in level order) and
+// Sweep::update(x, st) does the rest; the next level's cell index, and then
+// its fixed values, are fetched before the barrier that opens it.  GRID: all
+// blocks of a cooperative launch share a level; else the block has it alone.
+template <bool GRID, class Sweep>
+__device__ __forceinline__ void walk_levels(const Dims &d, const SeqTab &S, int tid, int nth, Sweep &sw) {
   namespace cg = cooperative_groups;
-  cg::grid_group grid = cg::this_grid();
+  const int4 *__restrict__ order = S.order;
+  const int *__restrict__ lstart = S.lstart;  // two entries past the end repeat it
+  int lo = 0, hi = lstart[1], hi1 = lstart[2];
+  bool on = tid < hi, on1 = hi + tid < hi1;
+  SeqCell x(d, order[on ? tid : 0]);
+  int4 o1 = order[on1 ? hi + tid : 0];
+  typename Sweep::Fixed st;
+  if (on) sw.fixed(tid, x, st);
+  for (int L = 0; L < S.nlev; ++L) {
+    if (on) {
+      sw.update(x, st);
+      for (int q = lo + tid + nth; q < hi; q += nth) {
+        const SeqCell y(d, order[q]);
+        typename Sweep::Fixed s2;
+        sw.fixed(q, y, s2);
+        sw.update(y, s2);
+      }
+    }
+    lo = hi;
+    hi = hi1;
+    hi1 = lstart[min(L + 3, S.nlev)];
+    on = on1;
+    x = SeqCell(d, o1);
+    if (on) sw.fixed(lo + tid, x, st);
+    on1 = hi + tid < hi1;
+    o1 = order[on1 ? hi + tid : 0];
+    if (GRID)
+      cg::this_grid().sync();
+    else
+      __syncthreads();
+  }
+}
+
+// velocity sweep of one component (integrate_velocity_field_formulation2_i,
+// nse.f90:831-1006; FORM 1: integrate_velocity_field_i, nse.f90:330-828)
+template <int FORM, class Ld>
+struct SeqVel {
+  const Dims &d;
+  const SeqTab &S;
+  double *fr, *cv;
+  const double *co, *Bq;
+  double w, DT, ev;
+  bool first;
+  struct Fixed {
+    double a[FORM == 1 ? 54 : 23], dg[6], B[4], oc[4];
+  };
+  __device__ __forceinline__ void fixed(int q, const SeqCell &x, Fixed &s) const {
+    const int Nc = d.Nc;
+#pragma unroll
+    for (int n = 0; n < (FORM == 1 ? 54 : 23); ++n) s.a[n] = S.vel[n * Nc + q];
+#pragma unroll
+    for (int n = 0; n < 6; ++n) s.dg[n] = S.dg[n * Nc + q];
+    s.B[0] = Bq[x.c];
+    s.oc[0] = co[x.c];
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd) {
+      s.oc[dd] = co[x.nb(d, dd)];
+      if (FORM == 1) s.B[dd] = Bq[x.nb(d, dd)];
+    }
+  }
+  __device__ __forceinline__ void update(const SeqCell &x, const Fixed &s) {
+    Hood h;
+    Tang t;
+    load_hood<Ld>(d, fr, x, h);
+    if (FORM == 1) load_tang<Ld>(d, fr, x, h, t);
+    const double cold = Ld::ld(cv, x.c);
+    double c2[4], nw, nf[4];
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd) c2[dd] = Ld::ld(cv, x.nb(d, dd));
+    if constexpr (FORM == 1) {
+      const double Bij = s.a[6] * s.B[0];
+      nw = (1 - w) * cold + w * (-(s.a[0] * h.x[1]) - s.a[1] * h.x[2] - s.a[2] * h.x[3] - s.a[3] * h.x[4] -
+                                 s.a[4] * h.x[5] - s.a[5] * h.x[6] - s.a[7] * s.oc[0] - Bij) /
+                                (s.a[8]);
+#pragma unroll
+      for (int dd = 1; dd <= 3; ++dd) {
+        const double *A = s.a + 9 + 15 * (dd - 1), *hn = h.of(dd);
+        const double B1 = s.B[0] * A[12] * 2 * DT;
+        const double B2 = s.B[dd] * A[14] * 2 * DT;
+        const double B3 = s.dg[2 * (dd - 1)] * tang_of(d, x, t, dd, 0, h.x[2 * dd]);
+        const double B4 = s.dg[2 * (dd - 1) + 1] * tang_of(d, x, t, dd, 1, h.x[2 * dd]);
+        double sum = 0.;
+#pragma unroll
+        for (int n = 0; n < 10; ++n) {
+          const int pt = p_term(dd, n), coef = pt & 15, fpos = (pt >> 4) & 7, cell = pt >> 7;
+          const double term = A[coef - 1] * (cell == 1 ? h.x[fpos] : hn[fpos]);
+          sum = (n == 0) ? -term : sum - term;
+        }
+        sum = sum - A[11] * (nw - s.oc[0]) - A[13] * (c2[dd] - s.oc[dd]);
+        constexpr int diag[4] = {0, 2, 6, 10};
+        nf[dd] = (1 - w) * h.x[2 * dd] + w / (A[diag[dd] - 1]) * (sum + B1 + B2 + B3 + B4);
+        if (x.has[dd]) {
+          ev = nmax(ev, errv(nf[dd], h.x[2 * dd], first));
+          h.x[2 * dd] = nf[dd];
+        }
+      }
+    } else {
+      nw = (1 - w) * cold + (w / s.a[0]) * (+s.a[1] * s.oc[0] + s.a[2] * h.x[1] + s.a[3] * h.x[2] + s.a[4] * h.x[3] +
+                                            s.a[5] * h.x[4] + s.a[6] * h.x[5] + s.a[7] * h.x[6] + s.B[0]);
+#pragma unroll
+      for (int dd = 1; dd <= 3; ++dd) {
+        const double *hn = h.of(dd);
+        nf[dd] = face_update_vals<double>([&](int pos) { return h.x[pos]; }, [&](int pos) { return hn[pos]; }, nw,
+                                          c2[dd], s.oc[0], s.oc[dd], s.a + 8 + 5 * (dd - 1), s.dg[2 * (dd - 1)],
+                                          s.dg[2 * (dd - 1) + 1], dd, w);
+        if (x.has[dd]) {
+          ev = nmax(ev, errv(nf[dd], h.x[2 * dd], first));
+          h.x[2 * dd] = nf[dd];
+        }
+      }
+    }
+    ev = nmax(ev, errv(nw, cold, first));
+    st_seq<Ld>(cv, x.c, nw);
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd)
+      if (x.has[dd]) st_seq<Ld>(fr, x.f[2 * dd], nf[dd]);
+  }
+};
+// The three components of a cell touch disjoint data: GRID blocks (CB, 3)
+// run them side by side (threadIdx.y), without GRID each has a block.
+template <int FORM, bool GRID, int TPB>
+__global__ void __launch_bounds__(TPB) k_seq_vel(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<3>(red);
-  const int par = parity(ctl);
-  const bool first = ctl->first;
-  const size_t Nc = d.Nc, NF = d.NF;
-  const int v = threadIdx.y;
+  const int par = parity(ctl), v = GRID ? threadIdx.y : blockIdx.x;
+  SeqVel<FORM, typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{
+      d, S, F.f[v] + (size_t)par * d.NF, F.c[v], F.co[v], F.Bv + (size_t)v * d.Nc, P.w[v], P.DT, 0., ctl->first != 0};
+  walk_levels<GRID>(d, S, GRID ? blockIdx.x * CB + threadIdx.x : threadIdx.x, GRID ? gridDim.x * CB : blockDim.x, sw);
   double e[3] = {0., 0., 0.};
-  const int tid = blockIdx.x * CB + threadIdx.x, nth = gridDim.x * CB;
-  double *fr = F.f[v] + par * NF;
-  double *cv = F.c[v];
-  const double *co = F.co[v];
-  for (int L = 0; L < nlev; ++L) {
-    for (int q = lstart[L] + tid; q < lstart[L + 1]; q += nth) {
-      const int c = order[q];
-      const Cell x = Cell::of(d, c);
-      int f[7];
-      cell_faces(d, x, f);
-      const double cold = LdCoh::ld(cv, c);
-      double nw;
-      if (FORM == 1) {
-        double at[9];
-        for (int k = 0; k < 9; ++k) at[k] = F.AT[(size_t)k * Nc + c];
-        nw = cell_update_f1<LdCoh>(fr, f, cold, co[c], F.Bv[(size_t)v * Nc + c], at, P.w[v]);
-      } else {
-        double F4[8];
-        for (int k = 0; k < 8; ++k) F4[k] = F.MF4[(size_t)k * Nc + c];
-        nw = cell_update<LdCoh>(fr, f, cold, co[c], F.Bv[(size_t)v * Nc + c], F4, P.w[v]);
-      }
-      st_coh(cv, c, nw);
-      e[v] = nmax(e[v], errv(nw, cold, first));
-#pragma unroll
-      for (int dd = 1; dd <= 3; ++dd) {
-        if (!x.has_nb(d, 2 * dd)) continue;
-        const Cell x2 = x.nb(d, 2 * dd);
-        const int fo = x.face(d, 2 * dd);
-        const double old = LdCoh::ld(fr, fo);
-        double nf;
-        if (FORM == 1) {
-          nf = v1_face_value<LdCoh>(d, g, F, P, fr, cv, co, F.Bv + (size_t)v * Nc, x, dd, P.w[v]);
-        } else {
-          double Fd[5];
-          for (int k = 0; k < 5; ++k) Fd[k] = F.MF[(size_t)(5 * (dd - 1) + k) * Nc + c];
-          nf = face_update_cv<LdCoh>(d, fr, nw, LdCoh::ld(cv, x2.c), co, Fd, g.dg[(2 * (dd - 1)) * Nc + c],
-                                     g.dg[(2 * (dd - 1) + 1) * Nc + c], dd, x, x2, P.w[v]);
-        }
-        st_coh(fr, fo, nf);
-        e[v] = nmax(e[v], errv(nf, old, first));
-      }
-    }
-    grid.sync();
-  }
-  block_max<3, CB3>(red, e, ctl->err[par]);
+  e[v] = sw.ev;
+  block_max<3, 0>(red, e, ctl->err[par]);
 }
 
 // pressure sweep (integrate_pressure_field_i, nse.f90:1091-1289)
-__global__ void __launch_bounds__(BLK) k_seq_p(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl,
-                                               const int *__restrict__ order, const int *__restrict__ lstart,
-                                               int nlev) {
-  namespace cg = cooperative_groups;
-  cg::grid_group grid = cg::this_grid();
+template <class Ld>
+struct SeqP {
+  const Dims &d;
+  const SeqTab &S;
+  double *pr;
+  const double *Rp;
+  double w, ev;
+  bool first;
+  struct Fixed {
+    double k[4][7], B1[4], B2[4], dg[6];
+  };
+  __device__ __forceinline__ void fixed(int q, const SeqCell &x, Fixed &s) const {
+    const int Nc = d.Nc;
+    const double rp = Rp[x.c];
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd) {
+      const double *A = S.prs + kSeqP * (dd - 1) * Nc + q;
+#pragma unroll
+      for (int n = 0; n < 7; ++n) s.k[dd][n] = A[n * Nc];
+      s.B1[dd] = rp * A[7 * Nc];
+      s.B2[dd] = Rp[x.nb(d, dd)] * A[8 * Nc];
+    }
+#pragma unroll
+    for (int n = 0; n < 6; ++n) s.dg[n] = S.dg[n * Nc + q];
+  }
+  __device__ __forceinline__ void update(const SeqCell &x, const Fixed &s) {
+    Hood h;
+    Tang t;
+    load_hood<Ld>(d, pr, x, h);
+    load_tang<Ld>(d, pr, x, h, t);
+    double nf[4];
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd) {
+      const double *hn = h.of(dd), *k = s.k[dd];
+      const PFaceCoef<double> K = {k[0], k[1], k[2], k[3], k[4], k[5], 0., 0., 0.};
+      const double B3 = s.dg[2 * (dd - 1)] * tang_of(d, x, t, dd, 0, h.x[2 * dd]);
+      const double B4 = s.dg[2 * (dd - 1) + 1] * tang_of(d, x, t, dd, 1, h.x[2 * dd]);
+      double sum = 0.;
+#pragma unroll
+      for (int n = 0; n < 10; ++n) {
+        const int pt = p_term(dd, n), fpos = (pt >> 4) & 7, cell = pt >> 7;
+        const double term = K.at(dd, fpos, cell) * (cell == 1 ? h.x[fpos] : hn[fpos]);
+        sum = (n == 0) ? -term : sum - term;
+      }
+      nf[dd] = (1 - w) * h.x[2 * dd] + k[6] * (sum + s.B1[dd] + s.B2[dd] + B3 + B4);
+      if (x.has[dd]) {
+        ev = nmax(ev, errv(nf[dd], h.x[2 * dd], first));
+        h.x[2 * dd] = nf[dd];
+      }
+    }
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd)
+      if (x.has[dd]) st_seq<Ld>(pr, x.f[2 * dd], nf[dd]);
+  }
+};
+template <bool GRID, int TPB>
+__global__ void __launch_bounds__(TPB) k_seq_p(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
   const int par = parity(ctl);
-  const bool first = ctl->first;
-  const size_t NF = d.NF;
-  double e[1] = {0.};
-  double *pr = F.f[3] + par * NF;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  for (int L = 0; L < nlev; ++L) {
-    for (int q = lstart[L] + tid; q < lstart[L + 1]; q += nth) {
-      const Cell x = Cell::of(d, order[q]);
-#pragma unroll
-      for (int dd = 1; dd <= 3; ++dd) {
-        if (!x.has_nb(d, 2 * dd)) continue;
-        const int fo = x.face(d, 2 * dd);
-        const double old = LdCoh::ld(pr, fo);
-        const double nw = p_face_value<LdCoh>(d, g, F, P, pr, x, dd);
-        st_coh(pr, fo, nw);
-        e[0] = nmax(e[0], errv(nw, old, first));
-      }
-    }
-    grid.sync();
-  }
-  block_max<1>(red, e, ctl->err[par] + 3);
+  SeqP<typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{d, S, F.f[3] + (size_t)par * d.NF, F.Rp, P.w_p, 0.,
+                                                                   ctl->first != 0};
+  walk_levels<GRID>(d, S, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sw);
+  const double e[1] = {sw.ev};
+  block_max<1, 0>(red, e, ctl->err[par] + 3);
 }
 
 // temperature sweep (integrate_temperature_field_formulation2_i, nse.f90:1009-1089)
-__global__ void __launch_bounds__(BLK) k_seq_T(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl,
-                                               const int *__restrict__ order, const int *__restrict__ lstart,
-                                               int nlev) {
-  namespace cg = cooperative_groups;
-  cg::grid_group grid = cg::this_grid();
+template <class Ld>
+struct SeqT {
+  const Dims &d;
+  const SeqTab &S;
+  double *T, *cv;
+  const double *co;
+  double w, ev;
+  bool first;
+  struct Fixed {
+    double a[kSeqT], dg[6], oc[4];
+  };
+  __device__ __forceinline__ void fixed(int q, const SeqCell &x, Fixed &s) const {
+    const int Nc = d.Nc;
+#pragma unroll
+    for (int n = 0; n < kSeqT; ++n) s.a[n] = S.tmp[n * Nc + q];
+#pragma unroll
+    for (int n = 0; n < 6; ++n) s.dg[n] = S.dg[n * Nc + q];
+    s.oc[0] = co[x.c];
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd) s.oc[dd] = co[x.nb(d, dd)];
+  }
+  __device__ __forceinline__ void update(const SeqCell &x, const Fixed &s) {
+    Hood h;
+    load_hood<Ld>(d, T, x, h);
+    const double cold = Ld::ld(cv, x.c);
+    double c2[4], nf[4];
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd) c2[dd] = Ld::ld(cv, x.nb(d, dd));
+    const double nw = (1 - w) * cold + s.a[0] * (+s.a[1] * s.oc[0] + s.a[2] * h.x[1] + s.a[3] * h.x[2] +
+                                                 s.a[4] * h.x[3] + s.a[5] * h.x[4] + s.a[6] * h.x[5] +
+                                                 s.a[7] * h.x[6] + (s.a[23] + 0.));
+    ev = nmax(ev, errv(nw, cold, first));
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd) {
+      const double *Fd = s.a + 8 + 5 * (dd - 1), *hn = h.of(dd);
+      const int e1 = tr1(dd), e2 = tr2(dd);
+      const double B3 = s.dg[2 * (dd - 1)] * (h.x[2 * e1] - h.x[2 * e1 - 1] + hn[2 * e1] - hn[2 * e1 - 1]) / 4.0;
+      const double B4 = s.dg[2 * (dd - 1) + 1] * (h.x[2 * e2] - h.x[2 * e2 - 1] + hn[2 * e2] - hn[2 * e2 - 1]) / 4.0;
+      nf[dd] = (1 - w) * h.x[2 * dd] + Fd[0] * (+Fd[1] * h.x[2 * dd - 1] + Fd[2] * hn[2 * dd] +
+                                                Fd[3] * (nw + s.oc[0]) + Fd[4] * (c2[dd] + s.oc[dd]) - B3 - B4);
+      if (x.has[dd]) {
+        ev = nmax(ev, errv(nf[dd], h.x[2 * dd], first));
+        h.x[2 * dd] = nf[dd];
+      }
+    }
+    st_seq<Ld>(cv, x.c, nw);
+#pragma unroll
+    for (int dd = 1; dd <= 3; ++dd)
+      if (x.has[dd]) st_seq<Ld>(T, x.f[2 * dd], nf[dd]);
+  }
+};
+template <bool GRID, int TPB>
+__global__ void __launch_bounds__(TPB) k_seq_T(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
   const int par = parity(ctl);
-  const bool first = ctl->first;
-  const size_t Nc = d.Nc, NF = d.NF;
-  double e[1] = {0.};
-  double *T = F.f[4] + par * NF;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  for (int L = 0; L < nlev; ++L) {
-    for (int q = lstart[L] + tid; q < lstart[L + 1]; q += nth) {
-      const int c = order[q];
-      const Cell x = Cell::of(d, c);
-      int f[7];
-      cell_faces(d, x, f);
-      double F4[8];
-      for (int k = 0; k < 8; ++k) F4[k] = F.MTF4[(size_t)k * Nc + c];
-      const double cold = LdCoh::ld(F.c[3], c);
-      const double nw = cell_update<LdCoh>(T, f, cold, F.co[3][c], (F.RDT[c] + 0.), F4, P.w[3]);
-      st_coh(F.c[3], c, nw);
-      e[0] = nmax(e[0], errv(nw, cold, first));
-#pragma unroll
-      for (int dd = 1; dd <= 3; ++dd) {
-        if (!x.has_nb(d, 2 * dd)) continue;
-        const Cell x2 = x.nb(d, 2 * dd);
-        double Fd[5];
-        T_form_Fd(F, (int)Nc, c, x2.c, dd, Fd);
-        const int fo = x.face(d, 2 * dd);
-        const double old = LdCoh::ld(T, fo);
-        const double nwf = face_update_cv<LdCoh>(d, T, nw, LdCoh::ld(F.c[3], x2.c), F.co[3], Fd,
-                                                g.dg[(2 * (dd - 1)) * Nc + c], g.dg[(2 * (dd - 1) + 1) * Nc + c], dd,
-                                                x, x2, P.w[3]);
-        st_coh(T, fo, nwf);
-        e[0] = nmax(e[0], errv(nwf, old, first));
-      }
-    }
-    grid.sync();
-  }
-  block_max<1>(red, e, ctl->err[par] + 4);
+  SeqT<typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{
+      d, S, F.f[4] + (size_t)par * d.NF, F.c[3], F.co[3], P.w[3], 0., ctl->first != 0};
+  walk_levels<GRID>(d, S, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sw);
+  const double e[1] = {sw.ev};
+  block_max<1, 0>(red, e, ctl->err[par] + 4);
 }
 
 // apply_pressure_bc in the reference's BC-list order (bc.f90:148-340).  Within
@@ -4360,33 +4675,117 @@ __global__ void __launch_bounds__(BLK) k_seq_T(Dims d, Geo g, Fields F, Phys P, 
 // order; bottom and top do not read each other, inner and outer read bottom
 // and top only, so one block per wall runs {bottom, top} and then
 // {inner, outer}.  border[] lists BC-list indices wall by wall and level by
-// level; wlev[w] .. wlev[w+1] are wall w's entries of blev[].
-__global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl,
-                                                 const int *__restrict__ border, const int *__restrict__ blev,
-                                                 const int *__restrict__ wlev, int wall0) {
+// level; wlev[w] .. wlev[w+1] are wall w's entries of blev[].  What no wall
+// pressure enters is formed for all faces at once by k_p_bc_fixed.
+// the stencil of every wall face, once at init: flags bit m set where the
+// stencil along the m-th transverse direction starts at a low wall end, bit
+// 2 + m at a high one
+__global__ void __launch_bounds__(BLK) k_seq_pack_wall(Dims d, SeqTab S) {
+  const int q = blockIdx.x * BLK + threadIdx.x, NB = d.NBF;
+  if (q >= NB) return;
+  const BFace B = bface(d, S.border[q]);
+  const Cell &x = B.cell;
+  const int pos = B.pos, dd = (pos + 1) / 2;
+  int *o = S.wface + q;
+  o[0] = x.face(d, pos);
+  int n = 1, flags = 0;
+  for (int k = 1; k <= 6; ++k)
+    if (k != pos) o[n++ * NB] = x.face(d, k);
+  for (int m = 0; m < 2; ++m) {
+    const int e = m == 0 ? tr1(dd) : tr2(dd);
+    const bool lo = !x.has_nb(d, 2 * e - 1), hi = !x.has_nb(d, 2 * e);
+    const Cell p1 = x.nb(d, lo ? 2 * e : 2 * e - 1);
+    const Cell p2 = lo ? p1.nb(d, 2 * e) : hi ? p1.nb(d, 2 * e - 1) : x.nb(d, 2 * e);
+    o[(6 + m) * NB] = p1.face(d, pos);
+    o[(8 + m) * NB] = p2.face(d, pos);
+    flags |= (lo ? 1 : 0) << m | (hi ? 4 : 0) << m;
+  }
+  o[10 * NB] = flags;
+}
+__global__ void __launch_bounds__(BLK) k_p_bc_fixed(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
+  if (ctl->done) return;
+  const int q = blockIdx.x * BLK + threadIdx.x, NB = d.NBF;
+  if (q >= NB) return;
+  const int b = S.border[q];
+  const BFace B = bface(d, b);
+  const size_t NF = d.NF;
+  const int par = parity(ctl), nh = newhalf(ctl);
+  double B1, body;
+  p_bc_fixed(d, g, F, P, F.f[0] + nh * NF, F.f[1] + nh * NF, F.f[2] + nh * NF, F.f[4] + par * NF, b, B, B1, body);
+  double *o = S.wall + q;
+  o[0] = P.w_p2 / (g.bcap[(B.pos - 1) * NB + b]);
+  o[NB] = B1;
+  o[2 * NB] = body;
+  o[3 * NB] = g.bcg[b];
+  o[4 * NB] = g.bcg[NB + b];
+  int n = 5;
+  for (int k = 1; k <= 6; ++k)
+    if (k != B.pos) o[n++ * NB] = g.bcap[(k - 1) * NB + b];
+}
+__global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl *ctl, SeqTab S, int wall0) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
-  const int par = parity(ctl), nh = newhalf(ctl);
+  const int par = parity(ctl), NB = d.NBF;
   const bool first = ctl->first;
-  const size_t NF = d.NF;
   double e[1] = {0.};
-  double *pr = F.f[3] + par * NF;
-  const int w = wall0 + blockIdx.x;
-  for (int L = wlev[w]; L < wlev[w + 1]; ++L) {
-    for (int q = blev[L] + threadIdx.x; q < blev[L + 1]; q += blockDim.x) {
-      const int b = border[q];
-      const BFace B = bface(d, b);
-      const int fw0 = B.cell.face(d, B.pos);
-      const double old = LdCoh::ld(pr, fw0);
-      const double nw = p_bc_value<LdCoh>(d, g, F, P, pr, F.f[0] + nh * NF, F.f[1] + nh * NF, F.f[2] + nh * NF,
-                                            F.f[4] + par * NF, b);
-      st_coh(pr, fw0, nw);
-      e[0] = nmax(e[0], errv(nw, old, first));
+  double *pr = F.f[3] + (size_t)par * d.NF;
+  const int *__restrict__ blev = S.blev;
+  const double w = P.w_p2;
+  const int wl = wall0 + blockIdx.x, L0 = S.wlev[wl], L1 = S.wlev[wl + 1], tid = threadIdx.x;
+  struct Face {
+    int i[kSeqI];
+    double o[kSeqW];
+  };
+  auto look = [&](int q, Face &y) {
+#pragma unroll
+    for (int r = 0; r < kSeqI; ++r) y.i[r] = S.wface[r * NB + q];
+#pragma unroll
+    for (int r = 0; r < kSeqW; ++r) y.o[r] = S.wall[r * NB + q];
+  };
+  auto update = [&](const Face &y) {
+    const double old = pr[y.i[0]];
+    double v[5], va[2], vb[2], t[2];
+#pragma unroll
+    for (int n = 0; n < 5; ++n) v[n] = pr[y.i[1 + n]];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      va[m] = pr[y.i[6 + m]];
+      vb[m] = pr[y.i[8 + m]];
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const bool lo = (y.i[10] >> m) & 1, hi = (y.i[10] >> (2 + m)) & 1;
+      t[m] = lo ? (-(3 * old) + 4 * va[m] - vb[m]) / 4. : hi ? (3 * old - 4 * va[m] + vb[m]) / 4. : (vb[m] - va[m]) / 4.;
+    }
+    double s = -(y.o[5] * v[0]);
+#pragma unroll
+    for (int n = 1; n < 5; ++n) s = s - y.o[5 + n] * v[n];
+    const double B2 = t[0] * y.o[3], B3 = t[1] * y.o[4];
+    const double nw = (1 - w) * old + y.o[0] * (s + y.o[1] - B2 - B3 + y.o[2]);
+    pr[y.i[0]] = nw;
+    e[0] = nmax(e[0], errv(nw, old, first));
+  };
+  int lo = blev[L0], hi = blev[L0 + 1];
+  Face y;
+  if (lo + tid < hi) look(lo + tid, y);
+  for (int L = L0; L < L1; ++L) {
+    if (lo + tid < hi) {
+      update(y);
+      for (int q = lo + tid + blockDim.x; q < hi; q += blockDim.x) {
+        Face z;
+        look(q, z);
+        update(z);
+      }
+    }
+    if (L + 1 < L1) {  // the next level's face, before the barrier
+      lo = hi;
+      hi = blev[L + 2];
+      if (lo + tid < hi) look(lo + tid, y);
     }
     __syncthreads();
   }
-  block_max<1>(red, e, ctl->err[par] + 3);
+  block_max<1, 0>(red, e, ctl->err[par] + 3);
 }
 
 // ====================================================== end of integrate
