@@ -37,6 +37,20 @@ __host__ __device__ __forceinline__ DualD operator/(const DualD &a, const DualD 
   const double q = a.v / b.v;
   return DualD(q, (a.t - q * b.t) / b.v);
 }
+// With a plain number (a constant, a parameter, a geometry value: derivative
+// zero) the terms that carry its derivative drop out, which changes no bit of
+// what is left.
+__host__ __device__ __forceinline__ DualD operator+(const DualD &a, double b) { return DualD(a.v + b, a.t); }
+__host__ __device__ __forceinline__ DualD operator+(double a, const DualD &b) { return DualD(a + b.v, b.t); }
+__host__ __device__ __forceinline__ DualD operator-(const DualD &a, double b) { return DualD(a.v - b, a.t); }
+__host__ __device__ __forceinline__ DualD operator-(double a, const DualD &b) { return DualD(a - b.v, -b.t); }
+__host__ __device__ __forceinline__ DualD operator*(const DualD &a, double b) { return DualD(a.v * b, a.t * b); }
+__host__ __device__ __forceinline__ DualD operator*(double a, const DualD &b) { return DualD(a * b.v, a * b.t); }
+__host__ __device__ __forceinline__ DualD operator/(const DualD &a, double b) { return DualD(a.v / b, a.t / b); }
+__host__ __device__ __forceinline__ DualD operator/(double a, const DualD &b) {
+  const double q = a / b.v;
+  return DualD(q, -(q * b.t) / b.v);
+}
 __host__ __device__ __forceinline__ bool operator<(const DualD &a, const DualD &b) { return a.v < b.v; }
 __host__ __device__ __forceinline__ bool operator>(const DualD &a, const DualD &b) { return a.v > b.v; }
 __host__ __device__ __forceinline__ bool operator<=(const DualD &a, const DualD &b) { return a.v <= b.v; }

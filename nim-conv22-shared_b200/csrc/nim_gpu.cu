@@ -123,10 +123,9 @@ struct nim_ctx {
   int graph32_iters = 0;
   int phase = 0;
   int last_lowp = 0, last_hi = 0;
-  // tangent-linear state (nim_gpu_tangent_*): dual copies of the geometry
-  // and of the iterate, their own control block and step counter
+  // tangent-linear state (nim_gpu_tangent_*): a dual copy of the iterate,
+  // its own control block and step counter
   bool dual_alloc = false, dual_ready = false;
-  GeoT<DualD> gD{};
   FieldsT<DualD> FD{};
   Ctrl *ctlD = nullptr;
   int32_t dual_STEP = 0;
@@ -292,7 +291,7 @@ int mark(nim_ctx *x, const char *name) {
 // the velocity sources + cell kernel and the face kernel of the context's
 // formulation (parallel schedule), over arrays of storage type R
 template <class R>
-int launch_vel(nim_ctx *x, cudaStream_t s, const GeoT<R> &g, const FieldsT<R> &F) {
+int launch_vel(nim_ctx *x, cudaStream_t s, const GeoOf<R> &g, const FieldsT<R> &F) {
   const Dims &d = x->d;
   if (x->phys.formulation == 1) {
     k_vel_cell<false, 1><<<x->g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
@@ -347,7 +346,7 @@ int launch_vel(nim_ctx *x, cudaStream_t s, const GeoT<R> &g, const FieldsT<R> &F
   return NIM_OK;
 }
 // the tangent-linear state (formulation 2): the gather forms of both sweeps
-int launch_vel(nim_ctx *x, cudaStream_t s, const GeoT<DualD> &g, const FieldsT<DualD> &F) {
+int launch_vel(nim_ctx *x, cudaStream_t s, const Geo &g, const FieldsT<DualD> &F) {
   k_vel_cell<false, 2><<<x->g3, dim3(CB, 3), 0, s>>>(x->d, g, F, x->phys, x->ctl);
   TRY(mark(x, "k_vel_cell"));
   k_vel_face<<<x->g3, dim3(CB, 3), 0, s>>>(x->d, g, F, x->phys, x->ctl);
@@ -444,7 +443,7 @@ int seq_pack_geometry(nim_ctx *x) {
 
 // the pressure part of a parallel pass (nse.f90:150-156)
 template <class R>
-int launch_pressure(nim_ctx *x, cudaStream_t s, const GeoT<R> &g, const FieldsT<R> &F) {
+int launch_pressure(nim_ctx *x, cudaStream_t s, const GeoOf<R> &g, const FieldsT<R> &F) {
   const Dims &d = x->d;
   const dim3 g3 = x->g3;
   // the float mirror sweeps four theta-adjacent cells a thread (n_theta % 4
@@ -496,7 +495,7 @@ int launch_pressure(nim_ctx *x, cudaStream_t s, const GeoT<R> &g, const FieldsT<
 
 // the temperature part of a parallel pass (nse.f90:157-162)
 template <class R>
-int launch_temperature(nim_ctx *x, cudaStream_t s, const GeoT<R> &g, const FieldsT<R> &F) {
+int launch_temperature(nim_ctx *x, cudaStream_t s, const GeoOf<R> &g, const FieldsT<R> &F) {
   const Dims &d = x->d;
   k_zero_flux<<<grid(2 * d.plane), BLK, 0, s>>>(d, g, F, x->ctl);
   TRY(mark(x, "k_zero_flux"));
@@ -519,7 +518,7 @@ int launch_temperature(nim_ctx *x, cudaStream_t s, const GeoT<R> &g, const Field
 
 // one pass of the parallel schedule over arrays of storage type R
 template <class R>
-int launch_parallel(nim_ctx *x, const GeoT<R> &g, const FieldsT<R> &F, int lowp) {
+int launch_parallel(nim_ctx *x, const GeoOf<R> &g, const FieldsT<R> &F, int lowp) {
   cudaStream_t s = x->stream;
   TRY(launch_vel(x, s, g, F));
   TRY(launch_pressure(x, s, g, F));
@@ -970,7 +969,7 @@ static bool encode_map(CUtensorMap *map, const R *base, int rank, const uint64_t
 }
 
 template <class R>
-static bool encode_vel_face_maps(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, VelFaceMaps &M) {
+static bool encode_vel_face_maps(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, VelFaceMaps &M) {
   const uint64_t NT = d.NT, NR = d.NR, NZ = d.NZ, NF = d.NF, Nc = d.Nc;
   bool ok = true;
   for (int q = 0; q < 3; ++q) {
@@ -2787,23 +2786,7 @@ namespace {
 
 int dual_alloc(nim_ctx *x) {
   const Dims &d = x->d;
-  const size_t Nc = d.Nc, NF = d.NF, NB = d.NBF;
-  GeoT<DualD> &h = x->gD;
-  TRY(dalloc(x, &h.vol, Nc));
-  TRY(dalloc(x, &h.G, 3 * Nc));
-  TRY(dalloc(x, &h.gij, 9 * Nc));
-  TRY(dalloc(x, &h.xi, 9 * Nc));
-  TRY(dalloc(x, &h.gfd, 6 * Nc));
-  TRY(dalloc(x, &h.dg, 6 * Nc));
-  TRY(dalloc(x, &h.area, NF));
-  TRY(dalloc(x, &h.normal, 3 * NF));
-  TRY(dalloc(x, &h.AA, 45 * Nc));
-  h.bcpts = x->g.bcpts;  // integer: shared with the FP64 side
-  TRY(dalloc(x, &h.bca, 5 * NB));
-  TRY(dalloc(x, &h.bcap, 8 * NB));
-  TRY(dalloc(x, &h.bcg, 2 * NB));
-  TRY(dalloc(x, &h.zf, 4 * NB));
-  TRY(dalloc(x, &h.nuw, 4 * NB));
+  const size_t Nc = d.Nc, NF = d.NF;
   FieldsT<DualD> &H = x->FD;
   for (int q = 0; q < 5; ++q) TRY(dalloc(x, &H.f[q], 2 * NF));
   for (int q = 0; q < 4; ++q) {
@@ -2826,28 +2809,10 @@ int dual_alloc(nim_ctx *x) {
   return NIM_OK;
 }
 
-// the FP64 geometry and iterate into the dual arrays, derivatives zero
+// the FP64 iterate into the dual arrays, derivatives zero
 int dual_copy(nim_ctx *x) {
   const Dims &d = x->d;
-  const size_t Nc = d.Nc, NF = d.NF, NB = d.NBF;
-  const Geo &g = x->g;
-  GeoT<DualD> &h = x->gD;
-  Cvt c;
-  c.add(g.vol, h.vol, Nc);
-  c.add(g.G, h.G, 3 * Nc);
-  c.add(g.gij, h.gij, 9 * Nc);
-  c.add(g.xi, h.xi, 9 * Nc);
-  c.add(g.gfd, h.gfd, 6 * Nc);
-  c.add(g.dg, h.dg, 6 * Nc);
-  c.add(g.area, h.area, NF);
-  c.add(g.normal, h.normal, 3 * NF);
-  c.add(g.AA, h.AA, 45 * Nc);
-  c.add(g.bca, h.bca, 5 * NB);
-  c.add(g.bcap, h.bcap, 8 * NB);
-  c.add(g.bcg, h.bcg, 2 * NB);
-  c.add(g.zf, h.zf, 4 * NB);
-  c.add(g.nuw, h.nuw, 4 * NB);
-  TRY((run_cvt<double, DualD>(x, c)));
+  const size_t Nc = d.Nc, NF = d.NF;
   const Fields &F = x->F;
   FieldsT<DualD> &H = x->FD;
   Cvt s;
@@ -2932,12 +2897,12 @@ int dual_step(nim_ctx *x, nim_step_stats *s, double *dnu2) {
   cudaStream_t st = x->stream;
   DualCtl use(x);
   k_step_reset<<<1, 1, 0, st>>>(x->ctl);
-  k_vel_coef_A<<<x->nblk_c, BLK, 0, st>>>(d, x->gD, x->FD, x->phys);
+  k_vel_coef_A<<<x->nblk_c, BLK, 0, st>>>(d, x->g, x->FD, x->phys);
   k_vel_coef_F<<<x->nblk_c, BLK, 0, st>>>(d, x->FD, x->phys);
   CK(cudaGetLastError());
   x->launches += 3;
   for (;;) {
-    for (int k = 0; k < 8; ++k) TRY(launch_parallel(x, x->gD, x->FD, 0));
+    for (int k = 0; k < 8; ++k) TRY(launch_parallel(x, x->g, x->FD, 0));
     TRY(read_ctrl(x));
     if (x->ctl_host->done) break;
     if (x->ctl_host->step_iters >= kDualCap) {
@@ -2946,7 +2911,7 @@ int dual_step(nim_ctx *x, nim_step_stats *s, double *dnu2) {
     }
   }
   const int status = x->ctl_host->status;
-  k_after_integrate<<<x->nblk_c, BLK, 0, st>>>(d, x->gD, x->FD, x->phys, x->ctl, x->nblk_c);
+  k_after_integrate<<<x->nblk_c, BLK, 0, st>>>(d, x->g, x->FD, x->phys, x->ctl, x->nblk_c);
   k_finish_sum<<<1, BLK, 0, st>>>(x->F.part, x->nblk_c, 1, x->sums);
   CK(cudaGetLastError());
   x->launches += 2;
@@ -2963,7 +2928,7 @@ int dual_step(nim_ctx *x, nim_step_stats *s, double *dnu2) {
   if (status != NIM_OK) return status;
   const int nr = 2 * d.NT * d.NZ, gn = grid(nr);
   k_update_time<<<x->nblk_c, BLK, 0, st>>>(d, x->FD, x->ctl);
-  k_nusselt<<<gn, BLK, 0, st>>>(d, x->gD, x->FD, x->ctl, gn);
+  k_nusselt<<<gn, BLK, 0, st>>>(d, x->g, x->FD, x->ctl, gn);
   k_finish_sum<<<1, BLK, 0, st>>>(x->F.part, gn, 8, x->sums);
   CK(cudaGetLastError());
   x->launches += 3;

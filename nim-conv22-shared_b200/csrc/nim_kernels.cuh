@@ -55,6 +55,18 @@ struct ArithOf<DualD> {
 };
 template <class R>
 using Ar = typename ArithOf<R>::type;
+// Type of what carries no derivative beside values of type V: constants,
+// parameters, geometry.
+template <class V>
+struct PlainOf {
+  using type = V;
+};
+template <>
+struct PlainOf<DualD> {
+  using type = double;
+};
+template <class V>
+using Kc = typename PlainOf<V>::type;
 
 // ------------------------------------------------------------ device state
 // Geometry and field arrays, by storage type R: double for the FP64 path;
@@ -83,11 +95,15 @@ struct GeoT {
   R *nuw;     // [4][NBF]  find_Nu2 weights (A, B, C, D) for r walls
   R *bcval;   // [4][NBF]  Dirichlet face values of u, v, w, T
   R *rvol;    // [Nc]      1/vol, formed once at init in the storage type's own
-              //           division (null in the dual copy, whose kernels divide)
+              //           division
   R *pc;      // [7][Nc]   CC(1..3), HH(1..3), Det of the pressure NIM constants
               //           (FP64 only: p_face_coef forms AA from them)
 };
 using Geo = GeoT<double>;
+// the geometry kernels over arrays of storage type R read: the tangent-linear
+// state moves over the FP64 geometry itself (its derivatives are zero)
+template <class R>
+using GeoOf = GeoT<Kc<R>>;
 
 template <class R>
 struct FieldsT {
@@ -140,16 +156,6 @@ template <class V>
 __device__ __forceinline__ V pv(double v, double t) {
   return ParOf<V>::get(v, t);
 }
-// 1/vol of cell c: the stored reciprocal (the same IEEE division in the
-// storage type, formed once at init), or the division itself for the dual
-// copy
-template <class R>
-__device__ __forceinline__ Ar<R> inv_vol(const GeoT<R> &g, int c) {
-  if constexpr (std::is_same<R, double>::value || std::is_same<R, float>::value)
-    return g.rvol[c];
-  else
-    return Ar<R>(1.) / g.vol[c];
-}
 
 // Control block in device memory; k_iter_end is its only writer during an
 // iteration, the host reads it between batches.
@@ -194,9 +200,12 @@ constexpr int TCN_MINB = 2;  // k_T_cellN (four float cells a thread)
 constexpr int PFN_MINB = 2;  // k_p_faceN (four float or two FP64 faces a thread)
 constexpr int TFN_MINB = 2;  // k_T_faceN (four float faces a thread)
 constexpr int VFN_MINB = 2;  // k_vel_faceN (four float faces a thread)
+// Dual values take two words each: two blocks (80 registers) for every kernel
+// (a pass at 64x64x48: the FP64 bounds 432 us, one block 436, two 346, three
+// 358).
 template <class R>
 constexpr int minb(int fp64, int fp32) {
-  return sizeof(R) == 8 ? fp64 : fp32;
+  return sizeof(R) == 8 ? fp64 : sizeof(R) == 4 ? fp32 : 2;
 }
 // kernels that spread one cell over three threads (component or direction)
 constexpr int CB = 128;            // cells per block
@@ -701,36 +710,36 @@ __global__ void k_apply_dirichlet(Dims d, Geo g, Fields F) {
 // NIM coefficients of one direction for contravariant speed u and
 // diffusivity k: M_A(d,1:6) / MT_A(d,1:6) (nim.f90:181-287, 354-460).
 template <class V>
-__device__ __forceinline__ void nim_direction_general(V u, V k, V gminus, V gplus, double v_limit, V A[6]) {
-  const V a = V(1.);
+__device__ __forceinline__ void nim_direction_general(V u, V k, Kc<V> gminus, Kc<V> gplus, double v_limit, V A[6]) {
+  const V a = Kc<V>(1.);
   const V Re = 2 * a * u / k;
   if (fabs(Re) > v_limit) {
     const V e = nim_exp(Re);
-    A[0] = (2 * a / (k * (V(1.) / e - V(1.))) + V(1.) / u) * gplus;
-    A[1] = (-(2 * a / (k * (V(1.) - e))) - V(1.) / u) * gminus;
-    A[2] = (u / (k * (V(1.) / e - V(1.)))) * gplus;
-    A[3] = (u / (k * (V(1.) - e))) * gminus;
+    A[0] = (2 * a / (k * (Kc<V>(1.) / e - Kc<V>(1.))) + Kc<V>(1.) / u) * gplus;
+    A[1] = (-(2 * a / (k * (Kc<V>(1.) - e))) - Kc<V>(1.) / u) * gminus;
+    A[2] = (u / (k * (Kc<V>(1.) / e - Kc<V>(1.)))) * gplus;
+    A[3] = (u / (k * (Kc<V>(1.) - e))) * gminus;
     if (Re > 0) {
-      A[4] = (-k + (a * u * (V(1.) / e + V(1.)) / (-(V(1.) / e) + V(1.)))) / (u * u);
-      A[5] = V(1.) / (-(V(1.) / e) + V(1.)) - V(1.) / (Re);
+      A[4] = (-k + (a * u * (Kc<V>(1.) / e + Kc<V>(1.)) / (-(Kc<V>(1.) / e) + Kc<V>(1.)))) / (u * u);
+      A[5] = Kc<V>(1.) / (-(Kc<V>(1.) / e) + Kc<V>(1.)) - Kc<V>(1.) / (Re);
     } else {
-      A[4] = (-k + (a * u * (V(1.) + e) / (-V(1.) + e))) / (u * u);
-      A[5] = e / (-V(1.) + e) - V(1.) / (Re);
+      A[4] = (-k + (a * u * (Kc<V>(1.) + e) / (-Kc<V>(1.) + e))) / (u * u);
+      A[5] = e / (-Kc<V>(1.) + e) - Kc<V>(1.) / (Re);
     }
   } else {
     const PwT<V> U(u), K(k);
-    A[0] = (-(a / k) - (u) / (V(3.) * K[2]) + (U[3]) / (V(45.) * K[4]) - (2 * U[5]) / (V(945.) * K[6]) +
-            -((U[7]) / (V(4725.) * K[8])) - (2 * U[9]) / (V(93555.) * K[10])) * gplus;
-    A[1] = (-(a / k) + (u) / (V(3.) * K[2]) - (U[3]) / (V(45.) * K[4]) + (2 * U[5]) / (V(945.) * K[6]) -
-            -((U[7]) / (V(4725.) * K[8])) + (2 * U[9]) / (V(93555.) * K[10])) * gminus;
-    A[2] = (-(1 / (V(2.) * a)) - u / (V(2.) * k) - (U[2]) / (V(6.) * K[2]) + (U[4]) / (V(90.) * K[4]) -
-            -((U[6]) / (V(945.) * K[6])) + (U[8]) / (V(9450.) * K[8]) - (U[10]) / (V(93555.) * K[10])) * gplus;
-    A[3] = (-(1 / (V(2.) * a)) + u / (V(2.) * k) - (U[2]) / (V(6.) * K[2]) + (U[4]) / (V(90.) * K[4]) -
-            -((U[6]) / (V(945.) * K[6])) + (U[8]) / (V(9450.) * K[8]) - (U[10]) / (V(93555.) * K[10])) * gminus;
-    A[4] = V(1.) / (V(3.) * k) - (U[2]) / (V(45.) * K[3]) + (2 * U[4]) / (V(945.) * K[5]) - -((U[6]) / (V(4725.) * K[7])) +
-           (2 * U[8]) / (V(93555.) * K[9]) - -((1382 * U[10]) / (V(6.38512875e8) * K[11]));
-    A[5] = V(0.5) + (u) / (V(6.) * k) - (U[3]) / (V(90.) * K[3]) + (U[5]) / (V(945.) * K[5]) - -((U[7]) / (V(9450.) * K[7])) +
-           (U[9]) / (V(93555.) * K[9]);
+    A[0] = (-(a / k) - (u) / (Kc<V>(3.) * K[2]) + (U[3]) / (Kc<V>(45.) * K[4]) - (2 * U[5]) / (Kc<V>(945.) * K[6]) +
+            -((U[7]) / (Kc<V>(4725.) * K[8])) - (2 * U[9]) / (Kc<V>(93555.) * K[10])) * gplus;
+    A[1] = (-(a / k) + (u) / (Kc<V>(3.) * K[2]) - (U[3]) / (Kc<V>(45.) * K[4]) + (2 * U[5]) / (Kc<V>(945.) * K[6]) -
+            -((U[7]) / (Kc<V>(4725.) * K[8])) + (2 * U[9]) / (Kc<V>(93555.) * K[10])) * gminus;
+    A[2] = (-(1 / (Kc<V>(2.) * a)) - u / (Kc<V>(2.) * k) - (U[2]) / (Kc<V>(6.) * K[2]) + (U[4]) / (Kc<V>(90.) * K[4]) -
+            -((U[6]) / (Kc<V>(945.) * K[6])) + (U[8]) / (Kc<V>(9450.) * K[8]) - (U[10]) / (Kc<V>(93555.) * K[10])) * gplus;
+    A[3] = (-(1 / (Kc<V>(2.) * a)) + u / (Kc<V>(2.) * k) - (U[2]) / (Kc<V>(6.) * K[2]) + (U[4]) / (Kc<V>(90.) * K[4]) -
+            -((U[6]) / (Kc<V>(945.) * K[6])) + (U[8]) / (Kc<V>(9450.) * K[8]) - (U[10]) / (Kc<V>(93555.) * K[10])) * gminus;
+    A[4] = Kc<V>(1.) / (Kc<V>(3.) * k) - (U[2]) / (Kc<V>(45.) * K[3]) + (2 * U[4]) / (Kc<V>(945.) * K[5]) - -((U[6]) / (Kc<V>(4725.) * K[7])) +
+           (2 * U[8]) / (Kc<V>(93555.) * K[9]) - -((1382 * U[10]) / (Kc<V>(6.38512875e8) * K[11]));
+    A[5] = Kc<V>(0.5) + (u) / (Kc<V>(6.) * k) - (U[3]) / (Kc<V>(90.) * K[3]) + (U[5]) / (Kc<V>(945.) * K[5]) - -((U[7]) / (Kc<V>(9450.) * K[7])) +
+           (U[9]) / (Kc<V>(93555.) * K[9]);
   }
 }
 
@@ -749,9 +758,9 @@ __device__ __noinline__ void nim_direction_slow(double u, double k, double gminu
 // before; 150x101x77 237 -> 170 us.  And the series stops at the last term that can
 // change its sum: for |Re| <= 0.01, i.e. x = |u/k| <= 0.005, a term below a
 // quarter ulp of the partial sum it is added to leaves it as it is, which
-// holds from x^7/4725 (1.7e-20 of A(1), A(2)), x^6/945 (1.65e-17 against
-// sums of 0.5 whose half spacing is at least 2.7e-17, A(3), A(4)),
-// 3 x^6/4725 (1e-17 of A(5)) and x^7/9450 (8.3e-21 against 0.5, A(6)) on.
+// holds from x^7/4725 (1.7e-20 of Kc<A>(1), Kc<A>(2)), x^6/945 (1.65e-17 against
+// sums of 0.5 whose half spacing is at least 2.7e-17, Kc<A>(3), Kc<A>(4)),
+// 3 x^6/4725 (1e-17 of Kc<A>(5)) and x^7/9450 (8.3e-21 against 0.5, Kc<A>(6)) on.
 __device__ __forceinline__ void nim_direction_fast(double u, double k, double gminus, double gplus, double v_limit,
                                                    double A[6]) {
   const Recip rk = recip(k);
@@ -798,7 +807,7 @@ __device__ __forceinline__ void nim_direction_fast(double u, double k, double gm
   if (!ok) nim_direction_slow(u, k, gminus, gplus, v_limit, A);
 }
 template <class V>
-__device__ __forceinline__ void nim_direction(V u, V k, V gminus, V gplus, double v_limit, V A[6]) {
+__device__ __forceinline__ void nim_direction(V u, V k, Kc<V> gminus, Kc<V> gplus, double v_limit, V A[6]) {
   if constexpr (std::is_same<V, double>::value)
     nim_direction_fast(u, k, gminus, gplus, v_limit, A);
   else
@@ -882,14 +891,14 @@ __global__ void k_nim_coef_selftest(const double *u, const double *k, double *A,
 }
 
 // contravariant component dd (1..3) of a Cartesian velocity in cell c
-template <class R>
-__device__ __forceinline__ Ar<R> contravariant(const R *xi, int Nc, int c, int dd, Ar<R> u, Ar<R> v, Ar<R> w) {
+template <class R, class V>
+__device__ __forceinline__ V contravariant(const R *xi, int Nc, int c, int dd, V u, V v, V w) {
   return u * xi[(dd - 1 + 0) * Nc + c] + v * xi[(dd - 1 + 3) * Nc + c] + w * xi[(dd - 1 + 6) * Nc + c];
 }
 
 // calculate_velocity_nim_constants_formulation2, first pass (nim.f90:165-289)
 template <class R>
-__global__ void __launch_bounds__(BLK) k_vel_coef_A(Dims d, GeoT<R> g, FieldsT<R> F, Phys P) {
+__global__ void __launch_bounds__(BLK) k_vel_coef_A(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P) {
   using V = Ar<R>;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.Nc) return;
@@ -907,23 +916,23 @@ __global__ void __launch_bounds__(BLK) k_vel_coef_A(Dims d, GeoT<R> g, FieldsT<R
 // M_F4 and M_F1..3 from M_A (nim.f90:293-328); also used for the
 // temperature's MT_F (nim.f90:466-500).
 template <class V>
-__device__ __forceinline__ void form_F4(const V A[3][6], V DT, V F4[8]) {
-  F4[1] = V(0.5) * (V(1.) / A[0][4] + V(1.) / A[1][4] + V(1.) / A[2][4] - V(1.) / DT);
+__device__ __forceinline__ void form_F4(const V A[3][6], Kc<V> DT, V F4[8]) {
+  F4[1] = Kc<V>(0.5) * (Kc<V>(1.) / A[0][4] + Kc<V>(1.) / A[1][4] + Kc<V>(1.) / A[2][4] - Kc<V>(1.) / DT);
   F4[2] = -(A[0][5] / A[0][4]);
-  F4[3] = (A[0][5] - V(1.)) / A[0][4];
+  F4[3] = (A[0][5] - Kc<V>(1.)) / A[0][4];
   F4[4] = -(A[1][5] / A[1][4]);
-  F4[5] = (A[1][5] - V(1.)) / A[1][4];
+  F4[5] = (A[1][5] - Kc<V>(1.)) / A[1][4];
   F4[6] = -(A[2][5] / A[2][4]);
-  F4[7] = (A[2][5] - V(1.)) / A[2][4];
+  F4[7] = (A[2][5] - Kc<V>(1.)) / A[2][4];
   F4[0] = F4[1] + F4[2] + F4[3] + F4[4] + F4[5] + F4[6] + F4[7];
 }
 template <class V>
 __device__ __forceinline__ void form_Fd(const V Ai[6], const V A2[6], V G[5]) {
   G[1] = Ai[2] - (Ai[0] * Ai[5] / Ai[4]);
   G[2] = A2[3] - A2[1] / A2[4] + A2[1] * A2[5] / A2[4];
-  G[3] = Ai[0] / (V(2.) * Ai[4]);
-  G[4] = A2[1] / (V(2.) * A2[4]);
-  G[0] = G[1] + G[2] + V(2.) * G[3] + V(2.) * G[4];
+  G[3] = Ai[0] / (Kc<V>(2.) * Ai[4]);
+  G[4] = A2[1] / (Kc<V>(2.) * A2[4]);
+  G[0] = G[1] + G[2] + Kc<V>(2.) * G[3] + Kc<V>(2.) * G[4];
 }
 
 template <class R>
@@ -1184,7 +1193,7 @@ __device__ __forceinline__ void by_dir(int y, Fn &&fn) {
 // Green-Gauss derivative dphi_dx2/dy2/dz2 (nse.f90:2866-2903), component cc
 // in the value type V of phi (the kernel's arithmetic type)
 template <class R, class V>
-__device__ __forceinline__ V green_gauss(const GeoT<R> &g, size_t NF, V invV, const V phi[7], const int f[7], int cc) {
+__device__ __forceinline__ V green_gauss(const GeoT<R> &g, size_t NF, Kc<V> invV, const V phi[7], const int f[7], int cc) {
   const R *A = g.area, *n = g.normal + cc * NF;
   return invV * (phi[2] * A[f[2]] * (n[f[2]]) - phi[1] * A[f[1]] * (n[f[1]]) + phi[4] * A[f[4]] * (n[f[4]]) -
                  phi[3] * A[f[3]] * (n[f[3]]) + phi[6] * A[f[6]] * (n[f[6]]) - phi[5] * A[f[5]] * (n[f[5]]));
@@ -1200,32 +1209,32 @@ __device__ __forceinline__ Ar<R> tangential(const Dims &d, const R *__restrict__
   const bool lo = !x.has_nb(d, 2 * e - 1), hi = !x.has_nb(d, 2 * e);
   if (lo) {
     const Cell m2 = x.nb(d, 2 * e), m3 = m2.nb(d, 2 * e);
-    return (-(3 * Ld::ld(phi, x.face(d, fpos))) + 4 * Ld::ld(phi, m2.face(d, fpos)) - Ld::ld(phi, m3.face(d, fpos))) / A(4);
+    return (-(3 * Ld::ld(phi, x.face(d, fpos))) + 4 * Ld::ld(phi, m2.face(d, fpos)) - Ld::ld(phi, m3.face(d, fpos))) / Kc<A>(4);
   } else if (hi) {
     const Cell m1 = x.nb(d, 2 * e - 1), m3 = m1.nb(d, 2 * e - 1);
-    return (3 * Ld::ld(phi, x.face(d, fpos)) - 4 * Ld::ld(phi, m1.face(d, fpos)) + Ld::ld(phi, m3.face(d, fpos))) / A(4);
+    return (3 * Ld::ld(phi, x.face(d, fpos)) - 4 * Ld::ld(phi, m1.face(d, fpos)) + Ld::ld(phi, m3.face(d, fpos))) / Kc<A>(4);
   }
-  return (Ld::ld(phi, x.nb(d, 2 * e).face(d, fpos)) - Ld::ld(phi, x.nb(d, 2 * e - 1).face(d, fpos))) / A(4);
+  return (Ld::ld(phi, x.nb(d, 2 * e).face(d, fpos)) - Ld::ld(phi, x.nb(d, 2 * e - 1).face(d, fpos))) / Kc<A>(4);
 }
 
 // G_i d_i phi - g^ij d_ij phi of calculate_R_D2 / R_D_p2 / R_D_T
 // (nse.f90:1852-1859, 1995-1996, 2132-2133), before the coefficient.
 template <class R>
-__device__ __forceinline__ Ar<R> diffusion_source(const Dims &d, const GeoT<R> &g, const R *__restrict__ phi,
+__device__ __forceinline__ Ar<R> diffusion_source(const Dims &d, const GeoOf<R> &g, const R *__restrict__ phi,
                                                   const Cell &x, const int f[7]) {
   using V = Ar<R>;
   const size_t Nc = d.Nc;
   const int c = x.c;
-  const V pxy = V(0.5) * (tangential(d, phi, x, 2, 2) - tangential(d, phi, x, 1, 2));
-  const V pzy = V(0.5) * (tangential(d, phi, x, 6, 2) - tangential(d, phi, x, 5, 2));
-  const V pyx = V(0.5) * (tangential(d, phi, x, 4, 1) - tangential(d, phi, x, 3, 1));
-  const V pzx = V(0.5) * (tangential(d, phi, x, 6, 1) - tangential(d, phi, x, 5, 1));
-  const V pxz = V(0.5) * (tangential(d, phi, x, 2, 3) - tangential(d, phi, x, 1, 3));
-  const V pyz = V(0.5) * (tangential(d, phi, x, 4, 3) - tangential(d, phi, x, 3, 3));
-  const V px = (phi[f[2]] - phi[f[1]]) / V(2.);
-  const V py = (phi[f[4]] - phi[f[3]]) / V(2.);
-  const V pz = (phi[f[6]] - phi[f[5]]) / V(2.);
-  const R *G = g.G, *gij = g.gij;
+  const V pxy = Kc<V>(0.5) * (tangential(d, phi, x, 2, 2) - tangential(d, phi, x, 1, 2));
+  const V pzy = Kc<V>(0.5) * (tangential(d, phi, x, 6, 2) - tangential(d, phi, x, 5, 2));
+  const V pyx = Kc<V>(0.5) * (tangential(d, phi, x, 4, 1) - tangential(d, phi, x, 3, 1));
+  const V pzx = Kc<V>(0.5) * (tangential(d, phi, x, 6, 1) - tangential(d, phi, x, 5, 1));
+  const V pxz = Kc<V>(0.5) * (tangential(d, phi, x, 2, 3) - tangential(d, phi, x, 1, 3));
+  const V pyz = Kc<V>(0.5) * (tangential(d, phi, x, 4, 3) - tangential(d, phi, x, 3, 3));
+  const V px = (phi[f[2]] - phi[f[1]]) / Kc<V>(2.);
+  const V py = (phi[f[4]] - phi[f[3]]) / Kc<V>(2.);
+  const V pz = (phi[f[6]] - phi[f[5]]) / Kc<V>(2.);
+  const Kc<R> *G = g.G, *gij = g.gij;
   return (G[c] * px + G[Nc + c] * py + G[2 * Nc + c] * pz - gij[3 * Nc + c] * pxy - gij[1 * Nc + c] * pyx -
           gij[6 * Nc + c] * pxz - gij[2 * Nc + c] * pzx - gij[7 * Nc + c] * pyz - gij[5 * Nc + c] * pzy);
 }
@@ -1242,7 +1251,7 @@ __device__ __forceinline__ void cell_faces(const Dims &d, const Cell &x, int f[7
 // Cell-average update (nse.f90:840-848; T: 1018-1026)
 template <class Ld = LdPlain, class R>
 __device__ __forceinline__ Ar<R> cell_update(const R *__restrict__ fr, const int f[7], Ar<R> c, Ar<R> cold,
-                                             Ar<R> B, const Ar<R> F4[8], Ar<R> w) {
+                                             Ar<R> B, const Ar<R> F4[8], Kc<Ar<R>> w) {
   return (1 - w) * c +
          (w / F4[0]) * (+F4[1] * cold + F4[2] * Ld::ld(fr, f[1]) + F4[3] * Ld::ld(fr, f[2]) +
                         F4[4] * Ld::ld(fr, f[3]) + F4[5] * Ld::ld(fr, f[4]) + F4[6] * Ld::ld(fr, f[5]) +
@@ -1253,11 +1262,11 @@ __device__ __forceinline__ Ar<R> cell_update(const R *__restrict__ fr, const int
 // fx(pos) of cell x and fx2(pos) of its +xi_d neighbour x2, their cell
 // values cx, cx2 and old cell values ox, ox2
 template <class V, class FX, class FX2>
-__device__ __forceinline__ V face_update_vals(FX &&fx, FX2 &&fx2, V cx, V cx2, V ox, V ox2, const V Fd[5], V dg0,
-                                              V dg1, int dd, V w) {
+__device__ __forceinline__ V face_update_vals(FX &&fx, FX2 &&fx2, V cx, V cx2, V ox, V ox2, const V Fd[5], Kc<V> dg0,
+                                              Kc<V> dg1, int dd, Kc<V> w) {
   const int e1 = tr1(dd), e2 = tr2(dd);
-  const V B3 = (dg0) * (fx(2 * e1) - fx(2 * e1 - 1) + fx2(2 * e1) - fx2(2 * e1 - 1)) / V(4.0);
-  const V B4 = (dg1) * (fx(2 * e2) - fx(2 * e2 - 1) + fx2(2 * e2) - fx2(2 * e2 - 1)) / V(4.0);
+  const V B3 = (dg0) * (fx(2 * e1) - fx(2 * e1 - 1) + fx2(2 * e1) - fx2(2 * e1 - 1)) / Kc<V>(4.0);
+  const V B4 = (dg1) * (fx(2 * e2) - fx(2 * e2 - 1) + fx2(2 * e2) - fx2(2 * e2 - 1)) / Kc<V>(4.0);
   return (1 - w) * fx(2 * dd) +
          (w / Fd[0]) * (+Fd[1] * fx(2 * dd - 1) + Fd[2] * fx2(2 * dd) + Fd[3] * (cx + ox) + Fd[4] * (cx2 + ox2) -
                         B3 - B4);
@@ -1265,16 +1274,16 @@ __device__ __forceinline__ V face_update_vals(FX &&fx, FX2 &&fx2, V cx, V cx2, V
 // the same from the face array fr; cx, cx2 the cell values of x and x2
 template <class Ld = LdPlain, class R>
 __device__ __forceinline__ Ar<R> face_update_cv(const Dims &d, const R *__restrict__ fr, Ar<R> cx, Ar<R> cx2,
-                                                const R *__restrict__ co, const Ar<R> Fd[5], Ar<R> dg0, Ar<R> dg1,
-                                                int dd, const Cell &x, const Cell &x2, Ar<R> w) {
+                                                const R *__restrict__ co, const Ar<R> Fd[5], Kc<Ar<R>> dg0, Kc<Ar<R>> dg1,
+                                                int dd, const Cell &x, const Cell &x2, Kc<Ar<R>> w) {
   return face_update_vals<Ar<R>>([&](int pos) { return Ld::ld(fr, x.face(d, pos)); },
                                  [&](int pos) { return Ld::ld(fr, x2.face(d, pos)); }, cx, cx2, (Ar<R>)co[x.c],
                                  (Ar<R>)co[x2.c], Fd, dg0, dg1, dd, w);
 }
 template <class Ld = LdPlain, class R>
 __device__ __forceinline__ Ar<R> face_update(const Dims &d, const R *__restrict__ fr, const R *__restrict__ cv,
-                                             const R *__restrict__ co, const Ar<R> Fd[5], Ar<R> dg0, Ar<R> dg1,
-                                             int dd, const Cell &x, const Cell &x2, Ar<R> w) {
+                                             const R *__restrict__ co, const Ar<R> Fd[5], Kc<Ar<R>> dg0, Kc<Ar<R>> dg1,
+                                             int dd, const Cell &x, const Cell &x2, Kc<Ar<R>> w) {
   return face_update_cv<Ld>(d, fr, Ld::ld(cv, x.c), Ld::ld(cv, x2.c), co, Fd, dg0, dg1, dd, x, x2, w);
 }
 
@@ -1430,7 +1439,7 @@ __device__ __forceinline__ bool patch_cell(const Dims &d, Cell &x, const FlatBlo
 // field_i (nse.f90:341-378); the R sums are stored too, for the face sweep
 // reads them at both cells of a face.
 template <bool SRC_ONLY, int FORM, class R, class BI>
-__device__ __forceinline__ void vel_cell_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void vel_cell_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -1449,12 +1458,12 @@ __device__ __forceinline__ void vel_cell_body(const Dims &d, const GeoT<R> &g, c
     const R *fp = F.f[3] + par * NF;
     V pf[7];
     for (int k = 1; k <= 6; ++k) pf[k] = fp[f[k]];
-    const V invV = inv_vol(g, c);
-    const V base = (q == 2) ? -(V(P.g_beta) * V(0.5) * (F.c[3][c] + F.co[3][c])) : V(0.);
-    const V RB = base + V(P.inv_rho) * green_gauss(g, NF, invV, pf, f, q);
+    const Kc<V> invV = g.rvol[c];
+    const V base = (q == 2) ? -(Kc<V>(P.g_beta) * Kc<V>(0.5) * (F.c[3][c] + F.co[3][c])) : Kc<V>(0.);
+    const V RB = base + Kc<V>(P.inv_rho) * green_gauss(g, NF, invV, pf, f, q);
     const R *fr = F.f[q] + par * NF;
     const V RD = pv<V>(P.inv_Re, P.d_inv_Re) * diffusion_source(d, g, fr, x, f);
-    const V B = (V(0.) + RD + RB);
+    const V B = (Kc<V>(0.) + RD + RB);
     if (SRC_ONLY || FORM == 1) F.Bv[(size_t)q * Nc + c] = B;
     if (!SRC_ONLY) {
       const V cold = F.c[q][c];
@@ -1462,11 +1471,11 @@ __device__ __forceinline__ void vel_cell_body(const Dims &d, const GeoT<R> &g, c
       if (FORM == 1) {
         V at[9];
         for (int k = 0; k < 9; ++k) at[k] = F.AT[(size_t)k * Nc + c];
-        nw = stored<R>(cell_update_f1(fr, f, cold, F.co[q][c], B, at, V(P.w[q])));
+        nw = stored<R>(cell_update_f1(fr, f, cold, F.co[q][c], B, at, Kc<V>(P.w[q])));
       } else {
         V F4[8];
         for (int k = 0; k < 8; ++k) F4[k] = F.MF4[(size_t)k * Nc + c];
-        nw = stored<R>(cell_update(fr, f, cold, F.co[q][c], B, F4, V(P.w[q])));
+        nw = stored<R>(cell_update(fr, f, cold, F.co[q][c], B, F4, Kc<V>(P.w[q])));
       }
       F.c[q][c] = nw;
       e[q] = errv(nw, cold, first);
@@ -1476,7 +1485,7 @@ __device__ __forceinline__ void vel_cell_body(const Dims &d, const GeoT<R> &g, c
   if (!SRC_ONLY && d.owns(blockIdx.z)) block_max<3, CB3>(red, e, ctl->err[par]);
 }
 template <bool SRC_ONLY, int FORM, class R>
-__global__ void __launch_bounds__(CB3, 3) k_vel_cell(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, minb<R>(3, 3)) k_vel_cell(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   vel_cell_body<SRC_ONLY, FORM, R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
@@ -1511,9 +1520,9 @@ __device__ __forceinline__ void ld2(const R *__restrict__ p, int i, R &a, R &b) 
 // along +e, vm1 / vm2 along -e (only those the branch reads are used)
 template <class V>
 __device__ __forceinline__ V tang_vals(bool lo, bool hi, V v0, V vp1, V vp2, V vm1, V vm2) {
-  if (lo) return (-(3 * v0) + 4 * vp1 - vp2) / V(4.);
-  if (hi) return (3 * v0 - 4 * vm1 + vm2) / V(4.);
-  return (vp1 - vm1) / V(4.);
+  if (lo) return (-(3 * v0) + 4 * vp1 - vp2) / Kc<V>(4.);
+  if (hi) return (3 * v0 - 4 * vm1 + vm2) / Kc<V>(4.);
+  return (vp1 - vm1) / Kc<V>(4.);
 }
 
 // Index arithmetic here is 32-bit (its largest offset is 9 x the cell count;
@@ -1524,7 +1533,7 @@ __device__ __forceinline__ V tang_vals(bool lo, bool hi, V v0, V vp1, V vp2, V v
 // separate instantiation: at this kernel's register bound the test alone
 // costs spills)
 template <class R, bool SLAB = false, class BI = LaunchBlock>
-__device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -1557,7 +1566,7 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
     // RB = base + 1/rho * green_gauss (component q): the sum term by term in
     // source order (faces 2, 1, 4, 3, 6, 5) for both cells
     const R *pp = F.f[3] + par * NF, *nq = g.normal + q * NF;
-    V gs0 = V(0.), gs1 = V(0.);
+    V gs0 = Kc<V>(0.), gs1 = Kc<V>(0.);
     {
       const int order[6] = {2, 1, 4, 3, 6, 5};
       // face 3 of both cells, loaded with face 4's turn: the pair's second
@@ -1598,17 +1607,17 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
     {
       R v0, v1;
       ld2(g.vol, c, v0, v1);
-      V base0 = V(0.), base1 = V(0.);
+      V base0 = Kc<V>(0.), base1 = Kc<V>(0.);
       if (q == 2) {
         R t0, t1, o0, o1;
         ld2(F.c[3], c, t0, t1);
         ld2(F.co[3], c, o0, o1);
-        base0 = -(V(P.g_beta) * V(0.5) * (t0 + o0));
-        base1 = -(V(P.g_beta) * V(0.5) * (t1 + o1));
+        base0 = -(Kc<V>(P.g_beta) * Kc<V>(0.5) * (t0 + o0));
+        base1 = -(Kc<V>(P.g_beta) * Kc<V>(0.5) * (t1 + o1));
       }
-      const V invV0 = V(1.) / v0, invV1 = V(1.) / v1;
-      RB0 = base0 + V(P.inv_rho) * (invV0 * gs0);
-      RB1 = base1 + V(P.inv_rho) * (invV1 * gs1);
+      const V invV0 = Kc<V>(1.) / v0, invV1 = Kc<V>(1.) / v1;
+      RB0 = base0 + Kc<V>(P.inv_rho) * (invV0 * gs0);
+      RB1 = base1 + Kc<V>(P.inv_rho) * (invV1 * gs1);
     }
     // own faces of component q (stored values)
     const R *fr = F.f[q] + par * NF;
@@ -1619,8 +1628,8 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
     o1[4] = fr[f4b];
     // rows / planes a and b: the -e,+e neighbours (centred), +1,+2 (lo) or -1,-2 (hi)
     auto along = [&](bool lo, bool hi, V v0, V va, V vb) {
-      return lo ? tang_vals(true, false, v0, va, vb, V(0.), V(0.))
-                : hi ? tang_vals(false, true, v0, V(0.), V(0.), va, vb) : tang_vals(false, false, v0, vb, V(0.), va, V(0.));
+      return lo ? tang_vals(true, false, v0, va, vb, Kc<V>(0.), Kc<V>(0.))
+                : hi ? tang_vals(false, true, v0, Kc<V>(0.), Kc<V>(0.), va, vb) : tang_vals(false, false, v0, vb, Kc<V>(0.), va, Kc<V>(0.));
     };
     // R_D: G_i d_i phi - g^ij d_ij phi, term by term in source order; each
     // cross derivative is formed for both cells right before its term
@@ -1630,9 +1639,9 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
     const int ka = zlo ? k + 1 : k - 1, kb = zlo ? k + 2 : (zhi ? k - 2 : k + 1);
     V s0, s1;
     {
-      const V px0 = (o0[2] - o0[1]) / V(2.), px1 = (o1[2] - o1[1]) / V(2.);
-      const V py0 = (o0[4] - o0[3]) / V(2.), py1 = (o1[4] - o1[3]) / V(2.);
-      const V pz0 = (o0[6] - o0[5]) / V(2.), pz1 = (o1[6] - o1[5]) / V(2.);
+      const V px0 = (o0[2] - o0[1]) / Kc<V>(2.), px1 = (o1[2] - o1[1]) / Kc<V>(2.);
+      const V py0 = (o0[4] - o0[3]) / Kc<V>(2.), py1 = (o1[4] - o1[3]) / Kc<V>(2.);
+      const V pz0 = (o0[6] - o0[5]) / Kc<V>(2.), pz1 = (o1[6] - o1[5]) / Kc<V>(2.);
       R a0, a1;
       ld2(g.G, c, a0, a1);
       s0 = a0 * px0;
@@ -1654,8 +1663,8 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
       const int rrow = NT * (j + (NR + 1) * k);
       const V r_m1 = fr[rrow + im1], r_p2 = fr[rrow + ip2];
       const V r1_m1 = fr[rrow + NT + im1], r1_p2 = fr[rrow + NT + ip2];
-      term(3, V(0.5) * (((V)o1[2] - r1_m1) / V(4.) - ((V)o1[1] - r_m1) / V(4.)),
-           V(0.5) * ((r1_p2 - (V)o0[2]) / V(4.) - (r_p2 - (V)o0[1]) / V(4.)));
+      term(3, Kc<V>(0.5) * (((V)o1[2] - r1_m1) / Kc<V>(4.) - ((V)o1[1] - r_m1) / Kc<V>(4.)),
+           Kc<V>(0.5) * ((r1_p2 - (V)o0[2]) / Kc<V>(4.) - (r_p2 - (V)o0[1]) / Kc<V>(4.)));
     }
     {  // pyx: theta faces of rows a, b
       const int tra = d.offT + NT * (ra + NR * k), trb = d.offT + NT * (rb + NR * k);
@@ -1663,8 +1672,8 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
       ld2(fr, tra + i, a0, a1);
       ld2(fr, trb + i, b0, b1);
       const R a2 = fr[tra + ip2], b2 = fr[trb + ip2];
-      term(1, V(0.5) * (along(rlo, rhi, o0[4], a1, b1) - along(rlo, rhi, o0[3], a0, b0)),
-           V(0.5) * (along(rlo, rhi, o1[4], a2, b2) - along(rlo, rhi, o1[3], a1, b1)));
+      term(1, Kc<V>(0.5) * (along(rlo, rhi, o0[4], a1, b1) - along(rlo, rhi, o0[3], a0, b0)),
+           Kc<V>(0.5) * (along(rlo, rhi, o1[4], a2, b2) - along(rlo, rhi, o1[3], a1, b1)));
     }
     {  // pxz: r faces (rows j, j+1) of planes a, b
       const int rka = NT * (j + (NR + 1) * ka), rkb = NT * (j + (NR + 1) * kb);
@@ -1673,8 +1682,8 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
       ld2(fr, rkb + i, pb0, pb1);
       ld2(fr, rka + NT + i, pA0, pA1);
       ld2(fr, rkb + NT + i, pB0, pB1);
-      term(6, V(0.5) * (along(zlo, zhi, o0[2], pA0, pB0) - along(zlo, zhi, o0[1], pa0, pb0)),
-           V(0.5) * (along(zlo, zhi, o1[2], pA1, pB1) - along(zlo, zhi, o1[1], pa1, pb1)));
+      term(6, Kc<V>(0.5) * (along(zlo, zhi, o0[2], pA0, pB0) - along(zlo, zhi, o0[1], pa0, pb0)),
+           Kc<V>(0.5) * (along(zlo, zhi, o1[2], pA1, pB1) - along(zlo, zhi, o1[1], pa1, pb1)));
     }
     {  // pzx: z faces (levels k, k+1) of rows a, b
       const int zra = d.offZ + NT * (ra + NR * k), zrb = d.offZ + NT * (rb + NR * k);
@@ -1683,8 +1692,8 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
       ld2(fr, zrb + i, zb0, zb1);
       ld2(fr, zra + pl + i, zA0, zA1);
       ld2(fr, zrb + pl + i, zB0, zB1);
-      term(2, V(0.5) * (along(rlo, rhi, o0[6], zA0, zB0) - along(rlo, rhi, o0[5], za0, zb0)),
-           V(0.5) * (along(rlo, rhi, o1[6], zA1, zB1) - along(rlo, rhi, o1[5], za1, zb1)));
+      term(2, Kc<V>(0.5) * (along(rlo, rhi, o0[6], zA0, zB0) - along(rlo, rhi, o0[5], za0, zb0)),
+           Kc<V>(0.5) * (along(rlo, rhi, o1[6], zA1, zB1) - along(rlo, rhi, o1[5], za1, zb1)));
     }
     {  // pyz: theta faces of planes a, b
       const int tka = d.offT + NT * (j + NR * ka), tkb = d.offT + NT * (j + NR * kb);
@@ -1692,23 +1701,23 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
       ld2(fr, tka + i, a0, a1);
       ld2(fr, tkb + i, b0, b1);
       const R a2 = fr[tka + ip2], b2 = fr[tkb + ip2];
-      term(7, V(0.5) * (along(zlo, zhi, o0[4], a1, b1) - along(zlo, zhi, o0[3], a0, b0)),
-           V(0.5) * (along(zlo, zhi, o1[4], a2, b2) - along(zlo, zhi, o1[3], a1, b1)));
+      term(7, Kc<V>(0.5) * (along(zlo, zhi, o0[4], a1, b1) - along(zlo, zhi, o0[3], a0, b0)),
+           Kc<V>(0.5) * (along(zlo, zhi, o1[4], a2, b2) - along(zlo, zhi, o1[3], a1, b1)));
     }
     {  // pzy: z faces (levels k, k+1) at theta i-1, i+2
       const int zlev = d.offZ + NT * (j + NR * k);
       const V z_m1 = fr[zlev + im1], z_p2 = fr[zlev + ip2];
       const V z1_m1 = fr[zlev + pl + im1], z1_p2 = fr[zlev + pl + ip2];
-      term(5, V(0.5) * (((V)o1[6] - z1_m1) / V(4.) - ((V)o1[5] - z_m1) / V(4.)),
-           V(0.5) * ((z1_p2 - (V)o0[6]) / V(4.) - (z_p2 - (V)o0[5]) / V(4.)));
+      term(5, Kc<V>(0.5) * (((V)o1[6] - z1_m1) / Kc<V>(4.) - ((V)o1[5] - z_m1) / Kc<V>(4.)),
+           Kc<V>(0.5) * ((z1_p2 - (V)o0[6]) / Kc<V>(4.) - (z_p2 - (V)o0[5]) / Kc<V>(4.)));
     }
     const V RD0 = pv<V>(P.inv_Re, P.d_inv_Re) * s0, RD1 = pv<V>(P.inv_Re, P.d_inv_Re) * s1;
-    const V B0 = (V(0.) + RD0 + RB0), B1 = (V(0.) + RD1 + RB1);
+    const V B0 = (Kc<V>(0.) + RD0 + RB0), B1 = (Kc<V>(0.) + RD1 + RB1);
     // cell update (cell_update), term by term
     R cv0, cv1, co0, co1, a0, a1;
     ld2(F.c[q], c, cv0, cv1);
     ld2(F.co[q], c, co0, co1);
-    const V w = V(P.w[q]);
+    const Kc<V> w = Kc<V>(P.w[q]);
     ld2(F.MF4, c, a0, a1);
     const V F40 = a0, F41 = a1;
     ld2(F.MF4 + Nc, c, a0, a1);
@@ -1730,7 +1739,7 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoT<R> &g, 
   if (!SLAB || d.owns(k)) block_max<3, CB3>(red, e, ctl->err[par]);
 }
 template <class R, bool SLAB = false>
-__global__ void __launch_bounds__(CB3, minb<R>(VC2_MINB, VC2_MINB_F)) k_vel_cell2(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, minb<R>(VC2_MINB, VC2_MINB_F)) k_vel_cell2(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   vel_cell2_body<R, SLAB>(d, g, F, P, ctl, LaunchBlock{});
 }
 
@@ -1774,7 +1783,7 @@ __device__ __forceinline__ void stN(R *__restrict__ p, int i, const R (&v)[NP]) 
 }
 
 template <class R, int NP, bool SLAB = false>
-__global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -1830,16 +1839,16 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
       ldN<R, NP>(g.vol, c, vol);
       V base[NP];
 #pragma unroll
-      for (int p = 0; p < NP; ++p) base[p] = V(0.);
+      for (int p = 0; p < NP; ++p) base[p] = Kc<V>(0.);
       if (q == 2) {
         R t[NP], o[NP];
         ldN<R, NP>(F.c[3], c, t);
         ldN<R, NP>(F.co[3], c, o);
 #pragma unroll
-        for (int p = 0; p < NP; ++p) base[p] = -(V(P.g_beta) * V(0.5) * (t[p] + o[p]));
+        for (int p = 0; p < NP; ++p) base[p] = -(Kc<V>(P.g_beta) * Kc<V>(0.5) * (t[p] + o[p]));
       }
 #pragma unroll
-      for (int p = 0; p < NP; ++p) RB[p] = base[p] + V(P.inv_rho) * ((V(1.) / vol[p]) * gs[p]);
+      for (int p = 0; p < NP; ++p) RB[p] = base[p] + Kc<V>(P.inv_rho) * ((Kc<V>(1.) / vol[p]) * gs[p]);
     }
     // own faces of component q (stored values)
     const R *fr = F.f[q] + par * NF;
@@ -1847,8 +1856,8 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
 #pragma unroll
     for (int m = 1; m <= 6; ++m) faceN(fr, m, o[m]);
     auto along = [&](bool lo, bool hi, V v0, V va, V vb) {
-      return lo ? tang_vals(true, false, v0, va, vb, V(0.), V(0.))
-                : hi ? tang_vals(false, true, v0, V(0.), V(0.), va, vb) : tang_vals(false, false, v0, vb, V(0.), va, V(0.));
+      return lo ? tang_vals(true, false, v0, va, vb, Kc<V>(0.), Kc<V>(0.))
+                : hi ? tang_vals(false, true, v0, Kc<V>(0.), Kc<V>(0.), va, vb) : tang_vals(false, false, v0, vb, Kc<V>(0.), va, Kc<V>(0.));
     };
     const bool rlo = (j == 0), rhi = (j == NR - 1);
     const int ra = rlo ? j + 1 : j - 1, rb = rlo ? j + 2 : (rhi ? j - 2 : j + 1);
@@ -1859,13 +1868,13 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
       R a[NP];
       ldN<R, NP>(g.G, c, a);
 #pragma unroll
-      for (int p = 0; p < NP; ++p) s[p] = a[p] * ((o[2][p] - o[1][p]) / V(2.));
+      for (int p = 0; p < NP; ++p) s[p] = a[p] * ((o[2][p] - o[1][p]) / Kc<V>(2.));
       ldN<R, NP>(g.G + Nc, c, a);
 #pragma unroll
-      for (int p = 0; p < NP; ++p) s[p] = s[p] + a[p] * ((o[4][p] - o[3][p]) / V(2.));
+      for (int p = 0; p < NP; ++p) s[p] = s[p] + a[p] * ((o[4][p] - o[3][p]) / Kc<V>(2.));
       ldN<R, NP>(g.G + 2 * Nc, c, a);
 #pragma unroll
-      for (int p = 0; p < NP; ++p) s[p] = s[p] + a[p] * ((o[6][p] - o[5][p]) / V(2.));
+      for (int p = 0; p < NP; ++p) s[p] = s[p] + a[p] * ((o[6][p] - o[5][p]) / Kc<V>(2.));
     }
     auto term = [&](int slot, const V (&dv)[NP]) {
       R a[NP];
@@ -1882,7 +1891,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
       for (int p = 0; p < NP; ++p) {
         const V up2 = (p + 1 < NP) ? (V)o[2][p + 1] : r1_pn, um2 = (p > 0) ? (V)o[2][p - 1] : r1_m1;
         const V up1 = (p + 1 < NP) ? (V)o[1][p + 1] : r_pn, um1 = (p > 0) ? (V)o[1][p - 1] : r_m1;
-        dv[p] = V(0.5) * ((up2 - um2) / V(4.) - (up1 - um1) / V(4.));
+        dv[p] = Kc<V>(0.5) * ((up2 - um2) / Kc<V>(4.) - (up1 - um1) / Kc<V>(4.));
       }
       term(3, dv);
     }
@@ -1903,7 +1912,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
       V dv[NP];
 #pragma unroll
       for (int p = 0; p < NP; ++p)
-        dv[p] = V(0.5) * (along(rlo, rhi, o[4][p], av[p + 1], bv[p + 1]) - along(rlo, rhi, o[3][p], av[p], bv[p]));
+        dv[p] = Kc<V>(0.5) * (along(rlo, rhi, o[4][p], av[p + 1], bv[p + 1]) - along(rlo, rhi, o[3][p], av[p], bv[p]));
       term(1, dv);
     }
     {  // pxz: r faces (rows j, j+1) of planes a, b
@@ -1916,7 +1925,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
       V dv[NP];
 #pragma unroll
       for (int p = 0; p < NP; ++p)
-        dv[p] = V(0.5) * (along(zlo, zhi, o[2][p], pA[p], pB[p]) - along(zlo, zhi, o[1][p], pa[p], pb[p]));
+        dv[p] = Kc<V>(0.5) * (along(zlo, zhi, o[2][p], pA[p], pB[p]) - along(zlo, zhi, o[1][p], pa[p], pb[p]));
       term(6, dv);
     }
     {  // pzx: z faces (levels k, k+1) of rows a, b
@@ -1929,7 +1938,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
       V dv[NP];
 #pragma unroll
       for (int p = 0; p < NP; ++p)
-        dv[p] = V(0.5) * (along(rlo, rhi, o[6][p], zA[p], zB[p]) - along(rlo, rhi, o[5][p], za[p], zb[p]));
+        dv[p] = Kc<V>(0.5) * (along(rlo, rhi, o[6][p], zA[p], zB[p]) - along(rlo, rhi, o[5][p], za[p], zb[p]));
       term(2, dv);
     }
     {  // pyz: theta faces of planes a, b
@@ -1949,7 +1958,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
       V dv[NP];
 #pragma unroll
       for (int p = 0; p < NP; ++p)
-        dv[p] = V(0.5) * (along(zlo, zhi, o[4][p], av[p + 1], bv[p + 1]) - along(zlo, zhi, o[3][p], av[p], bv[p]));
+        dv[p] = Kc<V>(0.5) * (along(zlo, zhi, o[4][p], av[p + 1], bv[p + 1]) - along(zlo, zhi, o[3][p], av[p], bv[p]));
       term(7, dv);
     }
     {  // pzy: z faces (levels k, k+1) at theta i-1 .. i+NP
@@ -1961,7 +1970,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
       for (int p = 0; p < NP; ++p) {
         const V up6 = (p + 1 < NP) ? (V)o[6][p + 1] : z1_pn, um6 = (p > 0) ? (V)o[6][p - 1] : z1_m1;
         const V up5 = (p + 1 < NP) ? (V)o[5][p + 1] : z_pn, um5 = (p > 0) ? (V)o[5][p - 1] : z_m1;
-        dv[p] = V(0.5) * ((up6 - um6) / V(4.) - (up5 - um5) / V(4.));
+        dv[p] = Kc<V>(0.5) * ((up6 - um6) / Kc<V>(4.) - (up5 - um5) / Kc<V>(4.));
       }
       term(5, dv);
     }
@@ -1969,7 +1978,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
     R cv[NP], co[NP], a[NP], F40[NP];
     ldN<R, NP>(F.c[q], c, cv);
     ldN<R, NP>(F.co[q], c, co);
-    const V w = V(P.w[q]);
+    const Kc<V> w = Kc<V>(P.w[q]);
     ldN<R, NP>(F.MF4, c, F40);
     ldN<R, NP>(F.MF4 + Nc, c, a);
     V u[NP];
@@ -1984,7 +1993,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
     R out[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      const V B = (V(0.) + pv<V>(P.inv_Re, P.d_inv_Re) * s[p] + RB[p]);
+      const V B = (Kc<V>(0.) + pv<V>(P.inv_Re, P.d_inv_Re) * s[p] + RB[p]);
       const V nw = stored<R>((1 - w) * (V)cv[p] + (w / F40[p]) * (u[p] + B));
       out[p] = (R)nw;
       e[q] = nmax(e[q], errv(nw, cv[p], first));
@@ -1997,7 +2006,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoT<R> g, 
 // ---- K2: +xi face updates of u, v, w (nse.f90:878-1005).
 // Block (CB, 3): threadIdx.y = direction.
 template <class R, class BI>
-__device__ __forceinline__ void vel_face_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void vel_face_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -2016,12 +2025,12 @@ __device__ __forceinline__ void vel_face_body(const Dims &d, const GeoT<R> &g, c
       const Cell x2 = x.nb(d, 2 * dd);
       V Fd[5];
       for (int k = 0; k < 5; ++k) Fd[k] = F.MF[(size_t)(5 * (dd - 1) + k) * Nc + c];
-      const V dg0 = g.dg[(2 * (dd - 1)) * Nc + c], dg1 = g.dg[(2 * (dd - 1) + 1) * Nc + c];
+      const Kc<V> dg0 = g.dg[(2 * (dd - 1)) * Nc + c], dg1 = g.dg[(2 * (dd - 1) + 1) * Nc + c];
       const int fo = x.face(d, 2 * dd);
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const R *fr = F.f[q] + par * NF;
-        const V nw = stored<R>(face_update(d, fr, F.c[q], F.co[q], Fd, dg0, dg1, dd, x, x2, V(P.w[q])));
+        const V nw = stored<R>(face_update(d, fr, F.c[q], F.co[q], Fd, dg0, dg1, dd, x, x2, Kc<V>(P.w[q])));
         F.f[q][(1 - par) * NF + fo] = nw;
         e[q] = errv(nw, fr[fo], first);
       }
@@ -2030,7 +2039,7 @@ __device__ __forceinline__ void vel_face_body(const Dims &d, const GeoT<R> &g, c
   if (d.owns(blockIdx.z)) block_max<3, CB3>(red, e, ctl->err[par]);
 }
 template <class R>
-__global__ void __launch_bounds__(CB3, 3) k_vel_face(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, minb<R>(3, 3)) k_vel_face(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   vel_face_body<R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
@@ -2162,7 +2171,7 @@ __device__ __forceinline__ bool vt_seam(const Dims &d, const FieldsT<R> &F, int 
 // SLAB: a z-slab context, whose maxima skip the planes a neighbour owns
 template <class R, bool SLAB = false>
 __global__ void __launch_bounds__(3 * VT_T, minb<R>(VT_MINB, VT_MINB_F))
-    k_vel_face_tile(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl, int kc, const __grid_constant__ VelFaceMaps M) {
+    k_vel_face_tile(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl, int kc, const __grid_constant__ VelFaceMaps M) {
   using V = Ar<R>;
   using L = VtLayout<R>;
   if (ctl->done) return;
@@ -2260,7 +2269,7 @@ __global__ void __launch_bounds__(3 * VT_T, minb<R>(VT_MINB, VT_MINB_F))
           const R *cq0 = P0 + q * L::Q + L::RF + 2 * L::C5, *cq2 = Q0 + q * L::Q + L::RF + 2 * L::C5;
           const V nw = stored<R>(face_update_vals(
               fx, fx2, cq0[jj * L::W + ii], cq2[(jj + dj) * L::W + ii + di], cq0[L::C5 + jj * L::W + ii],
-              cq2[L::C5 + (jj + dj) * L::W + ii + di], Fd, dg0, dg1, dd, V(P.w[q])));
+              cq2[L::C5 + (jj + dj) * L::W + ii + di], Fd, dg0, dg1, dd, Kc<V>(P.w[q])));
           F.f[q][(1 - par) * NF + fo] = nw;
           if (!SLAB || d.owns(k)) e[q] = nmax(e[q], errv(nw, fx(2 * dd), first));
         }
@@ -2388,7 +2397,7 @@ __device__ __forceinline__ bool ct_seam(const Dims &d, const FieldsT<R> &F, int 
 
 template <class R>
 __global__ void __launch_bounds__(3 * CT_T, CT_MINB)
-    k_vel_cell_tile(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl, int kc, const __grid_constant__ VelCellMaps M) {
+    k_vel_cell_tile(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl, int kc, const __grid_constant__ VelCellMaps M) {
   using V = Ar<R>;
   using L = CtLayout<R>;
   if (ctl->done) return;
@@ -2455,9 +2464,9 @@ __global__ void __launch_bounds__(3 * CT_T, CT_MINB)
       const R *fp = F.f[3] + par * NF;
       V pf[7];
       for (int m = 1; m <= 6; ++m) pf[m] = fp[f[m]];
-      const V invV = V(1.) / g.vol[c];
-      const V base = (q == 2) ? -(V(P.g_beta) * V(0.5) * (F.c[3][c] + F.co[3][c])) : V(0.);
-      const V RB = base + V(P.inv_rho) * green_gauss(g, NF, invV, pf, f, q);
+      const Kc<V> invV = Kc<V>(1.) / g.vol[c];
+      const V base = (q == 2) ? -(Kc<V>(P.g_beta) * Kc<V>(0.5) * (F.c[3][c] + F.co[3][c])) : Kc<V>(0.);
+      const V RB = base + Kc<V>(P.inv_rho) * green_gauss(g, NF, invV, pf, f, q);
       // face pos of the cell (di, dj, dk) away, component q, from the ring
       auto fv = [&](int pos, int di, int dj, int dk) -> V {
         const int pb = k + dk + (pos == 6 ? 1 : 0) - P0;
@@ -2475,28 +2484,28 @@ __global__ void __launch_bounds__(3 * CT_T, CT_MINB)
       auto tng = [&](int pos, int e) -> V {
         auto at = [&](int s) { return fv(pos, e == 2 ? s : 0, e == 1 ? s : 0, e == 3 ? s : 0); };
         const bool lo = !x.has_nb(d, 2 * e - 1), hi = !x.has_nb(d, 2 * e);
-        if (lo) return (-(3 * at(0)) + 4 * at(1) - at(2)) / V(4.);
-        if (hi) return (3 * at(0) - 4 * at(-1) + at(-2)) / V(4.);
-        return (at(1) - at(-1)) / V(4.);
+        if (lo) return (-(3 * at(0)) + 4 * at(1) - at(2)) / Kc<V>(4.);
+        if (hi) return (3 * at(0) - 4 * at(-1) + at(-2)) / Kc<V>(4.);
+        return (at(1) - at(-1)) / Kc<V>(4.);
       };
-      const V pxy = V(0.5) * (tng(2, 2) - tng(1, 2));
-      const V pzy = V(0.5) * (tng(6, 2) - tng(5, 2));
-      const V pyx = V(0.5) * (tng(4, 1) - tng(3, 1));
-      const V pzx = V(0.5) * (tng(6, 1) - tng(5, 1));
-      const V pxz = V(0.5) * (tng(2, 3) - tng(1, 3));
-      const V pyz = V(0.5) * (tng(4, 3) - tng(3, 3));
+      const V pxy = Kc<V>(0.5) * (tng(2, 2) - tng(1, 2));
+      const V pzy = Kc<V>(0.5) * (tng(6, 2) - tng(5, 2));
+      const V pyx = Kc<V>(0.5) * (tng(4, 1) - tng(3, 1));
+      const V pzx = Kc<V>(0.5) * (tng(6, 1) - tng(5, 1));
+      const V pxz = Kc<V>(0.5) * (tng(2, 3) - tng(1, 3));
+      const V pyz = Kc<V>(0.5) * (tng(4, 3) - tng(3, 3));
       R fr[7];  // the stored values: the differences below are taken in R, as in diffusion_source
       for (int m = 1; m <= 6; ++m) fr[m] = (R)fv(m, 0, 0, 0);
-      const V px = (fr[2] - fr[1]) / V(2.);
-      const V py = (fr[4] - fr[3]) / V(2.);
-      const V pz = (fr[6] - fr[5]) / V(2.);
-      const R *G = g.G, *gij = g.gij;
+      const V px = (fr[2] - fr[1]) / Kc<V>(2.);
+      const V py = (fr[4] - fr[3]) / Kc<V>(2.);
+      const V pz = (fr[6] - fr[5]) / Kc<V>(2.);
+      const Kc<R> *G = g.G, *gij = g.gij;
       const V RD =
           pv<V>(P.inv_Re, P.d_inv_Re) * (G[c] * px + G[Nc + c] * py + G[2 * Nc + c] * pz - gij[3 * Nc + c] * pxy -
                       gij[1 * Nc + c] * pyx - gij[6 * Nc + c] * pxz - gij[2 * Nc + c] * pzx - gij[7 * Nc + c] * pyz -
                       gij[5 * Nc + c] * pzy);
-      const V B = (V(0.) + RD + RB);
-      const V cv = F.c[q][c], cold = F.co[q][c], w = V(P.w[q]);
+      const V B = (Kc<V>(0.) + RD + RB);
+      const V cv = F.c[q][c], cold = F.co[q][c], w = Kc<V>(P.w[q]);
       V F4[8];
       for (int m = 0; m < 8; ++m) F4[m] = F.MF4[(size_t)m * Nc + c];
       const V nw = stored<R>((1 - w) * cv + (w / F4[0]) * (+F4[1] * cold + F4[2] * fr[1] + F4[3] * fr[2] +
@@ -2526,7 +2535,7 @@ __global__ void __launch_bounds__(3 * CT_T, CT_MINB)
 // velocity component y and two of the six cross derivatives of p (y = 1 also
 // d(bz)/dz); thread 0 combines them in the reference's order.
 template <class R, class BI>
-__device__ __forceinline__ void p_src_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void p_src_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   if (ctl->done) return;
   using A = Ar<R>;
   __shared__ A sh[3][3][CB];  // gradients of u, v, w
@@ -2544,7 +2553,7 @@ __device__ __forceinline__ void p_src_body(const Dims &d, const GeoT<R> &g, cons
     cell_faces(d, x, f);
     by_dir(threadIdx.y, [&](auto Q) {
       constexpr int q = decltype(Q)::value - 1;
-      const A invV = inv_vol(g, c);
+      const Kc<A> invV = g.rvol[c];
       const R *fq = F.f[q] + newhalf(ctl) * NF;
       A vf[7];
       for (int k = 1; k <= 6; ++k) vf[k] = fq[f[k]];
@@ -2553,15 +2562,15 @@ __device__ __forceinline__ void p_src_body(const Dims &d, const GeoT<R> &g, cons
       if (q == 1) {
         const R *fT = F.f[4] + par * NF;
         A bzf[7];
-        for (int k = 1; k <= 6; ++k) bzf[k] = -(A(P.g_beta) * (fT[f[k]]));
+        for (int k = 1; k <= 6; ++k) bzf[k] = -(Kc<A>(P.g_beta) * (fT[f[k]]));
         sbz[tx] = green_gauss(g, NF, invV, bzf, f, 2);
       }
       // y=0 pxy,pzy  y=1 pyx,pzx  y=2 pxz,pyz (calculate_R_D_p2 order)
       constexpr int e2 = (q == 0) ? 2 : (q == 1) ? 1 : 3;
       constexpr int fa = (q == 1) ? 4 : 2, fb = (q == 1) ? 3 : 1;
-      sX[q][0][tx] = A(0.5) * (tangential(d, fp, x, fa, e2) - tangential(d, fp, x, fb, e2));
-      sX[q][1][tx] = (q == 2) ? A(0.5) * (tangential(d, fp, x, 4, 3) - tangential(d, fp, x, 3, 3))
-                              : A(0.5) * (tangential(d, fp, x, 6, e2) - tangential(d, fp, x, 5, e2));
+      sX[q][0][tx] = Kc<A>(0.5) * (tangential(d, fp, x, fa, e2) - tangential(d, fp, x, fb, e2));
+      sX[q][1][tx] = (q == 2) ? Kc<A>(0.5) * (tangential(d, fp, x, 4, 3) - tangential(d, fp, x, 3, 3))
+                              : Kc<A>(0.5) * (tangential(d, fp, x, 6, e2) - tangential(d, fp, x, 5, e2));
     });
   }
   __syncthreads();
@@ -2573,21 +2582,21 @@ __device__ __forceinline__ void p_src_body(const Dims &d, const GeoT<R> &g, cons
     const A Dila = du_dx + dv_dy + dw_dz;
     F.dila[c] = Dila;
     const A RBp = -(du_dx * du_dx + dv_dy * dv_dy + dw_dz * dw_dz) -
-                  A(2) * (du_dy * dv_dx + dv_dz * dw_dy + dw_dx * du_dz) - dbz_dz + Dila / (2 * A(P.DT));
+                  Kc<A>(2) * (du_dy * dv_dx + dv_dz * dw_dy + dw_dx * du_dz) - dbz_dz + Dila / (2 * Kc<A>(P.DT));
     const A pxy = sX[0][0][tx], pzy = sX[0][1][tx], pyx = sX[1][0][tx], pzx = sX[1][1][tx];
     const A pxz = sX[2][0][tx], pyz = sX[2][1][tx];
-    const A px = (fp[f[2]] - fp[f[1]]) / A(2);
-    const A py = (fp[f[4]] - fp[f[3]]) / A(2);
-    const A pz = (fp[f[6]] - fp[f[5]]) / A(2);
-    const R *Gv = g.G, *gij = g.gij;
-    const A RDp = A(P.inv_rho) * (Gv[c] * px + Gv[Nc + c] * py + Gv[2 * Nc + c] * pz - gij[3 * Nc + c] * pxy -
+    const A px = (fp[f[2]] - fp[f[1]]) / Kc<A>(2);
+    const A py = (fp[f[4]] - fp[f[3]]) / Kc<A>(2);
+    const A pz = (fp[f[6]] - fp[f[5]]) / Kc<A>(2);
+    const Kc<R> *Gv = g.G, *gij = g.gij;
+    const A RDp = Kc<A>(P.inv_rho) * (Gv[c] * px + Gv[Nc + c] * py + Gv[2 * Nc + c] * pz - gij[3 * Nc + c] * pxy -
                                     gij[1 * Nc + c] * pyx - gij[6 * Nc + c] * pxz - gij[2 * Nc + c] * pzx -
                                     gij[7 * Nc + c] * pyz - gij[5 * Nc + c] * pzy);
     F.Rp[c] = RDp + RBp;
   }
 }
 template <class R>
-__global__ void __launch_bounds__(CB3, minb<R>(4, PSRC_MINB_F)) k_p_src(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, minb<R>(4, PSRC_MINB_F)) k_p_src(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   p_src_body<R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
@@ -2599,7 +2608,7 @@ __global__ void __launch_bounds__(CB3, minb<R>(4, PSRC_MINB_F)) k_p_src(Dims d, 
 // cross derivatives of p for the NP cells; thread 0 combines them in the
 // reference's order.  Each cell's arithmetic is k_p_src's.
 template <class R, int NP, class BI>
-__device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ V sh[3][3][CB * NP];  // gradients of u, v, w
@@ -2630,8 +2639,8 @@ __device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoT<R> &g, con
   };
   const R *fp = F.f[3] + par * NF;
   auto along = [&](bool lo, bool hi, V v0, V va, V vb) {
-    return lo ? tang_vals(true, false, v0, va, vb, V(0.), V(0.))
-              : hi ? tang_vals(false, true, v0, V(0.), V(0.), va, vb) : tang_vals(false, false, v0, vb, V(0.), va, V(0.));
+    return lo ? tang_vals(true, false, v0, va, vb, Kc<V>(0.), Kc<V>(0.))
+              : hi ? tang_vals(false, true, v0, Kc<V>(0.), Kc<V>(0.), va, vb) : tang_vals(false, false, v0, vb, Kc<V>(0.), va, Kc<V>(0.));
   };
   if (active) by_dir(threadIdx.y, [&](auto Q) {
     constexpr int q = decltype(Q)::value - 1;
@@ -2703,10 +2712,10 @@ __device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoT<R> &g, con
       for (int p = 0; p < NP; ++p) {
         const V up2 = (p + 1 < NP) ? (V)o[2][p + 1] : r1_pn, um2 = (p > 0) ? (V)o[2][p - 1] : r1_m1;
         const V up1 = (p + 1 < NP) ? (V)o[1][p + 1] : r_pn, um1 = (p > 0) ? (V)o[1][p - 1] : r_m1;
-        sX[0][0][tx * NP + p] = V(0.5) * ((up2 - um2) / V(4.) - (up1 - um1) / V(4.));
+        sX[0][0][tx * NP + p] = Kc<V>(0.5) * ((up2 - um2) / Kc<V>(4.) - (up1 - um1) / Kc<V>(4.));
         const V up6 = (p + 1 < NP) ? (V)o[6][p + 1] : z1_pn, um6 = (p > 0) ? (V)o[6][p - 1] : z1_m1;
         const V up5 = (p + 1 < NP) ? (V)o[5][p + 1] : z_pn, um5 = (p > 0) ? (V)o[5][p - 1] : z_m1;
-        sX[0][1][tx * NP + p] = V(0.5) * ((up6 - um6) / V(4.) - (up5 - um5) / V(4.));
+        sX[0][1][tx * NP + p] = Kc<V>(0.5) * ((up6 - um6) / Kc<V>(4.) - (up5 - um5) / Kc<V>(4.));
       }
     } else if (q == 1) {  // pyx (theta faces along r), pzx (z faces along r)
       const int tra = d.offT + NT * (ra + NR * k), trb = d.offT + NT * (rb + NR * k);
@@ -2731,9 +2740,9 @@ __device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoT<R> &g, con
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         sX[1][0][tx * NP + p] =
-            V(0.5) * (along(rlo, rhi, o[4][p], av[p + 1], bv[p + 1]) - along(rlo, rhi, o[3][p], av[p], bv[p]));
+            Kc<V>(0.5) * (along(rlo, rhi, o[4][p], av[p + 1], bv[p + 1]) - along(rlo, rhi, o[3][p], av[p], bv[p]));
         sX[1][1][tx * NP + p] =
-            V(0.5) * (along(rlo, rhi, o[6][p], zA[p], zB[p]) - along(rlo, rhi, o[5][p], za[p], zb[p]));
+            Kc<V>(0.5) * (along(rlo, rhi, o[6][p], zA[p], zB[p]) - along(rlo, rhi, o[5][p], za[p], zb[p]));
       }
     } else {  // pxz (r faces along z), pyz (theta faces along z)
       const int rka = NT * (j + (NR + 1) * ka), rkb = NT * (j + (NR + 1) * kb);
@@ -2758,9 +2767,9 @@ __device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoT<R> &g, con
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         sX[2][0][tx * NP + p] =
-            V(0.5) * (along(zlo, zhi, o[2][p], pA[p], pB[p]) - along(zlo, zhi, o[1][p], pa[p], pb[p]));
+            Kc<V>(0.5) * (along(zlo, zhi, o[2][p], pA[p], pB[p]) - along(zlo, zhi, o[1][p], pa[p], pb[p]));
         sX[2][1][tx * NP + p] =
-            V(0.5) * (along(zlo, zhi, o[4][p], av[p + 1], bv[p + 1]) - along(zlo, zhi, o[3][p], av[p], bv[p]));
+            Kc<V>(0.5) * (along(zlo, zhi, o[4][p], av[p + 1], bv[p + 1]) - along(zlo, zhi, o[3][p], av[p], bv[p]));
       }
     }
   });
@@ -2788,13 +2797,13 @@ __device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoT<R> &g, con
       const V Dila = du_dx + dv_dy + dw_dz;
       dila[p] = Dila;
       const V RBp = -(du_dx * du_dx + dv_dy * dv_dy + dw_dz * dw_dz) -
-                    V(2) * (du_dy * dv_dx + dv_dz * dw_dy + dw_dx * du_dz) - dbz_dz + Dila / (2 * V(P.DT));
+                    Kc<V>(2) * (du_dy * dv_dx + dv_dz * dw_dy + dw_dx * du_dz) - dbz_dz + Dila / (2 * Kc<V>(P.DT));
       const V pxy = sX[0][0][e], pzy = sX[0][1][e], pyx = sX[1][0][e], pzx = sX[1][1][e];
       const V pxz = sX[2][0][e], pyz = sX[2][1][e];
-      const V px = (o[2][p] - o[1][p]) / V(2);
-      const V py = (o[4][p] - o[3][p]) / V(2);
-      const V pz = (o[6][p] - o[5][p]) / V(2);
-      const V RDp = V(P.inv_rho) * (G0[p] * px + G1[p] * py + G2[p] * pz - gs[0][p] * pxy - gs[1][p] * pyx -
+      const V px = (o[2][p] - o[1][p]) / Kc<V>(2);
+      const V py = (o[4][p] - o[3][p]) / Kc<V>(2);
+      const V pz = (o[6][p] - o[5][p]) / Kc<V>(2);
+      const V RDp = Kc<V>(P.inv_rho) * (G0[p] * px + G1[p] * py + G2[p] * pz - gs[0][p] * pxy - gs[1][p] * pyx -
                                     gs[2][p] * pxz - gs[3][p] * pzx - gs[4][p] * pyz - gs[5][p] * pzy);
       rp[p] = RDp + RBp;
     }
@@ -2803,7 +2812,7 @@ __device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoT<R> &g, con
   }
 }
 template <class R, int NP>
-__global__ void __launch_bounds__(CB3, PSN_MINB) k_p_srcN(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, PSN_MINB) k_p_srcN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   p_srcN_body<R, NP>(d, g, F, P, ctl, LaunchBlock{});
 }
 
@@ -2811,14 +2820,14 @@ __global__ void __launch_bounds__(CB3, PSN_MINB) k_p_srcN(Dims d, GeoT<R> g, Fie
 // terms that no wall pressure enters, from the new velocities fu/fv/fwv, R_p
 // and the temperatures fT: B1 and the body of the momentum balance.
 template <class R>
-__device__ __forceinline__ void p_bc_fixed(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P,
+__device__ __forceinline__ void p_bc_fixed(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P,
                                            const R *fu, const R *fv, const R *fwv, const R *fT, int b,
                                            const BFace &B, Ar<R> &B1, Ar<R> &body) {
   using V = Ar<R>;
   const int NF = d.NF, NB = d.NBF;
   const int fw0 = B.cell.face(d, B.pos);
-  const V n[3] = {g.normal[fw0], g.normal[NF + fw0], g.normal[2 * NF + fw0]};
-  const V bvec[3] = {V(0), V(0), -(V(P.g_beta) * (fT[fw0]))};
+  const Kc<V> n[3] = {g.normal[fw0], g.normal[NF + fw0], g.normal[2 * NF + fw0]};
+  const V bvec[3] = {Kc<V>(0), Kc<V>(0), -(Kc<V>(P.g_beta) * (fT[fw0]))};
   const V b_n = dot3(bvec, n);
   V vn[6];
   for (int j = 1; j <= 5; ++j) {
@@ -2826,15 +2835,15 @@ __device__ __forceinline__ void p_bc_fixed(const Dims &d, const GeoT<R> &g, cons
     const V v[3] = {fu[pt], fv[pt], fwv[pt]};
     vn[j] = dot3(v, n);
   }
-  const R *a = g.bca;
+  const Kc<R> *a = g.bca;
   const V d2udn2 = -(a[b] * vn[1]) - a[NB + b] * vn[2] - a[2 * NB + b] * vn[3] - a[3 * NB + b] * vn[4] -
                         a[4 * NB + b] * vn[5];
   B1 = g.bcap[7 * NB + b] * (F.Rp[B.cell.c]);
-  body = pv<V>(P.nu, P.d_nu) * V(P.rho) * d2udn2 - b_n * V(P.rho);
+  body = pv<V>(P.nu, P.d_nu) * Kc<V>(P.rho) * d2udn2 - b_n * Kc<V>(P.rho);
 }
 // the new value from the pressures pr
 template <class Ld, class R>
-__device__ __forceinline__ Ar<R> p_bc_value(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P,
+__device__ __forceinline__ Ar<R> p_bc_value(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P,
                                             const R *pr, const R *fu, const R *fv, const R *fwv, const R *fT,
                                             int b) {
   using V = Ar<R>;
@@ -2848,7 +2857,7 @@ __device__ __forceinline__ Ar<R> p_bc_value(const Dims &d, const GeoT<R> &g, con
   const int dd = (pos + 1) / 2;
   const V B2 = tangential<Ld>(d, pr, M1, pos, tr1(dd)) * g.bcg[b];
   const V B3 = tangential<Ld>(d, pr, M1, pos, tr2(dd)) * g.bcg[NB + b];
-  const R *ap = g.bcap;
+  const Kc<R> *ap = g.bcap;
   V s = 0.0;
   bool firstterm = true;
   for (int k = 1; k <= 6; ++k) {
@@ -2863,7 +2872,7 @@ __device__ __forceinline__ Ar<R> p_bc_value(const Dims &d, const GeoT<R> &g, con
 
 // ---- K4: apply_pressure_bc, every wall face from the values before the pass
 template <class R, class BI>
-__device__ __forceinline__ void p_bc_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void p_bc_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
@@ -2884,7 +2893,7 @@ __device__ __forceinline__ void p_bc_body(const Dims &d, const GeoT<R> &g, const
   block_max<1>(red, e, ctl->err[par] + 3);
 }
 template <class R>
-__global__ void __launch_bounds__(BLK) k_p_bc(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(BLK) k_p_bc(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   p_bc_body<R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
@@ -2960,11 +2969,11 @@ __host__ __device__ constexpr int p_slot(int dd, int n) {
 template <class V>
 __device__ __forceinline__ PFaceCoef<V> p_face_form(V c1, V c2, V h, V det, V gg, V q1, V q2, V hq, V detq, V g2) {
   PFaceCoef<V> k;
-  const V E = V(0.5) * det, Eq = V(0.5) * detq;
+  const V E = Kc<V>(0.5) * det, Eq = Kc<V>(0.5) * detq;
   const V t = (c1 + c2) * E * h, tq = (q1 + q2) * Eq * hq;
-  k.m = -(V(0.5) + t) * gg;
-  k.mq = -(V(0.5) + tq) * g2;
-  k.diag = (V(0.5) - t) * gg + (V(0.5) - tq) * g2;
+  k.m = -(Kc<V>(0.5) + t) * gg;
+  k.mq = -(Kc<V>(0.5) + tq) * g2;
+  k.diag = (Kc<V>(0.5) - t) * gg + (Kc<V>(0.5) - tq) * g2;
   k.a1 = c2 * E * h * gg;
   k.a2 = c1 * E * h * gg;
   k.a1q = q2 * Eq * hq * g2;
@@ -2989,12 +2998,12 @@ __device__ __forceinline__ PFaceCoef<Ar<R>> p_face_coef(const GeoT<R> &g, int Nc
 // ---- integrate_pressure_field_i for the +xi_dd face of cell x
 // (nse.f90:1091-1289): the new value from the pressures pr
 template <class Ld, class R>
-__device__ __forceinline__ Ar<R> p_face_value(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P,
+__device__ __forceinline__ Ar<R> p_face_value(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P,
                                               const R *pr, const Cell &x, int dd) {
   using V = Ar<R>;
   const int Nc = d.Nc, c = x.c;
   const Cell n2 = x.nb(d, 2 * dd);
-  const PFaceCoef<V> K = p_face_coef(g, Nc, c, n2.c, dd);
+  const PFaceCoef<Kc<V>> K = p_face_coef(g, Nc, c, n2.c, dd);
   const V B1 = (F.Rp[c]) * K.b;
   const V B2 = (F.Rp[n2.c]) * K.bq;
   const V B3 = (g.dg[(2 * (dd - 1)) * Nc + c]) * tangential<Ld>(d, pr, x, 2 * dd, tr1(dd));
@@ -3008,7 +3017,7 @@ __device__ __forceinline__ Ar<R> p_face_value(const Dims &d, const GeoT<R> &g, c
     s = (t == 0) ? -term : s - term;
   }
   const int fo = x.face(d, 2 * dd);
-  const V w = V(P.w_p);
+  const Kc<V> w = Kc<V>(P.w_p);
   return (1 - w) * Ld::ld(pr, fo) + w / K.diag * (s + B1 + B2 + B3 + B4);
 }
 
@@ -3018,7 +3027,7 @@ __device__ __forceinline__ Ar<R> p_face_value(const Dims &d, const GeoT<R> &g, c
 // tangential cross terms (the centred B3/B4 the source forms first are
 // overwritten before use).  fr faces, cv / co cells and old cells.
 template <class Ld, class R>
-__device__ __forceinline__ Ar<R> v1_face_value(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P,
+__device__ __forceinline__ Ar<R> v1_face_value(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P,
                                                const R *fr, const R *cv, const R *co, const R *Bq, const Cell &x,
                                                int dd, Ar<R> w) {
   using V = Ar<R>;
@@ -3026,11 +3035,11 @@ __device__ __forceinline__ Ar<R> v1_face_value(const Dims &d, const GeoT<R> &g, 
   const int c = x.c;
   const Cell n2 = x.nb(d, 2 * dd);
   const R *A = F.AAv + (size_t)15 * (dd - 1) * Nc;
-  const V B1 = Bq[c] * A[12 * Nc + c] * 2 * V(P.DT);
-  const V B2 = Bq[n2.c] * A[14 * Nc + c] * 2 * V(P.DT);
+  const V B1 = Bq[c] * A[12 * Nc + c] * 2 * Kc<V>(P.DT);
+  const V B2 = Bq[n2.c] * A[14 * Nc + c] * 2 * Kc<V>(P.DT);
   const V B3 = (g.dg[(2 * (dd - 1)) * Nc + c]) * tangential<Ld>(d, fr, x, 2 * dd, tr1(dd));
   const V B4 = (g.dg[(2 * (dd - 1) + 1) * Nc + c]) * tangential<Ld>(d, fr, x, 2 * dd, tr2(dd));
-  V s = V(0.0);
+  V s = Kc<V>(0.0);
 #pragma unroll
   for (int t = 0; t < 10; ++t) {
     const int pt = p_term(dd, t), coef = pt & 15, fpos = (pt >> 4) & 7, cell = pt >> 7;
@@ -3046,7 +3055,7 @@ __device__ __forceinline__ Ar<R> v1_face_value(const Dims &d, const GeoT<R> &g, 
 // ---- K2 of formulation 1: +xi face updates of u, v, w (nse.f90:378-826),
 // cur -> next.  Block (CB, 3): threadIdx.y = direction.
 template <class R>
-__global__ void __launch_bounds__(CB3, 2) k_vel1_face(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, 2) k_vel1_face(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -3066,7 +3075,7 @@ __global__ void __launch_bounds__(CB3, 2) k_vel1_face(Dims d, GeoT<R> g, FieldsT
       for (int q = 0; q < 3; ++q) {
         const R *fr = F.f[q] + par * NF;
         const V nw = stored<R>(
-            v1_face_value<LdPlain>(d, g, F, P, fr, F.c[q], F.co[q], F.Bv + (size_t)q * Nc, x, dd, V(P.w[q])));
+            v1_face_value<LdPlain>(d, g, F, P, fr, F.c[q], F.co[q], F.Bv + (size_t)q * Nc, x, dd, Kc<V>(P.w[q])));
         F.f[q][(1 - par) * NF + fo] = nw;
         e[q] = errv(nw, fr[fo], first);
       }
@@ -3078,7 +3087,7 @@ __global__ void __launch_bounds__(CB3, 2) k_vel1_face(Dims d, GeoT<R> g, FieldsT
 // ---- K5: integrate_pressure_field_i, cur -> next.
 // Block (CB, 3): threadIdx.y = direction.
 template <class R, class BI>
-__device__ __forceinline__ void p_face_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void p_face_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
@@ -3102,7 +3111,7 @@ __device__ __forceinline__ void p_face_body(const Dims &d, const GeoT<R> &g, con
   if (d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 3);
 }
 template <class R>
-__global__ void __launch_bounds__(CB3, minb<R>(5, PFACE_MINB_F)) k_p_face(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, minb<R>(5, PFACE_MINB_F)) k_p_face(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   p_face_body<R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
@@ -3116,14 +3125,13 @@ __global__ void __launch_bounds__(CB3, minb<R>(5, PFACE_MINB_F)) k_p_face(Dims d
 // (they start one cell off the vector boundary).  Each face's arithmetic is
 // p_face_value's.
 template <class R, int NP, class BI>
-__device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
   const int par = parity(ctl);
   const bool first = ctl->first;
-  const int tx = threadIdx.x;
   int i, j;
   group_cell<NP>(d, blockIdx, i, j);
   const int k = blockIdx.z;
@@ -3255,8 +3263,8 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoT<R> &g, co
     const bool zlo = (k == 0), zhi = (k == d.NZ - 1);
     const int ka = zlo ? k + 1 : k - 1, kb = zlo ? k + 2 : (zhi ? k - 2 : k + 1);
     auto along = [&](bool lo, bool hi, V v0, V va, V vb) {
-      return lo ? tang_vals(true, false, v0, va, vb, V(0.), V(0.))
-                : hi ? tang_vals(false, true, v0, V(0.), V(0.), va, vb) : tang_vals(false, false, v0, vb, V(0.), va, V(0.));
+      return lo ? tang_vals(true, false, v0, va, vb, Kc<V>(0.), Kc<V>(0.))
+                : hi ? tang_vals(false, true, v0, Kc<V>(0.), Kc<V>(0.), va, vb) : tang_vals(false, false, v0, vb, Kc<V>(0.), va, Kc<V>(0.));
     };
     if (dd == 1) {  // face 2 (r faces of row j+1): along theta (centred), along z
       const int rrow = NT * (j + 1 + (NR + 1) * k);
@@ -3267,7 +3275,7 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoT<R> &g, co
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         const V up = (p + 1 < NP) ? (V)ox[2][p + 1] : pn, um = (p > 0) ? (V)ox[2][p - 1] : m1;
-        t1[p] = (up - um) / V(4.);
+        t1[p] = (up - um) / Kc<V>(4.);
         t2[p] = along(zlo, zhi, ox[2][p], za[p], zb[p]);
       }
     } else if (dd == 2) {  // face 4 (theta faces at i+1 ..): along r, along z
@@ -3309,10 +3317,10 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoT<R> &g, co
       for (int p = 0; p < NP; ++p) {
         t1[p] = along(rlo, rhi, ox[6][p], za[p], zb[p]);
         const V up = (p + 1 < NP) ? (V)ox[6][p + 1] : pn, um = (p > 0) ? (V)ox[6][p - 1] : m1;
-        t2[p] = (up - um) / V(4.);
+        t2[p] = (up - um) / Kc<V>(4.);
       }
     }
-    const V w = V(P.w_p);
+    const Kc<V> w = Kc<V>(P.w_p);
     R out[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
@@ -3338,13 +3346,13 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoT<R> &g, co
   if (d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 3);
 }
 template <class R, int NP>
-__global__ void __launch_bounds__(CB3, PFN_MINB) k_p_faceN(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, PFN_MINB) k_p_faceN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   p_faceN_body<R, NP>(d, g, F, P, ctl, LaunchBlock{});
 }
 
 // ---- K5b (is_dpdx_tolerance): cell pressure gradients (nse.f90:292-307)
 template <class R, class BI>
-__device__ __forceinline__ void p_dpdx_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void p_dpdx_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
@@ -3358,9 +3366,9 @@ __device__ __forceinline__ void p_dpdx_body(const Dims &d, const GeoT<R> &g, con
     cell_faces(d, x, f);
     const R *p = F.f[3] + newhalf(ctl) * NF;
     using V = Ar<R>;
-    const V v[3] = {stored<R>((p[f[2]] - p[f[1]]) / V(2.) * g.xi[0 * Nc + c]),
-                    stored<R>((p[f[4]] - p[f[3]]) / V(2.) * g.xi[4 * Nc + c]),
-                    stored<R>((p[f[6]] - p[f[5]]) / V(2.) * g.xi[8 * Nc + c])};
+    const V v[3] = {stored<R>((p[f[2]] - p[f[1]]) / Kc<V>(2.) * g.xi[0 * Nc + c]),
+                    stored<R>((p[f[4]] - p[f[3]]) / Kc<V>(2.) * g.xi[4 * Nc + c]),
+                    stored<R>((p[f[6]] - p[f[5]]) / Kc<V>(2.) * g.xi[8 * Nc + c])};
     for (int q = 0; q < 3; ++q) {
       if (d.owns(x.k)) e[0] = nmax(e[0], fabs(val(v[q]) - val(F.dpd[q * Nc + c])));
       F.dpd[q * Nc + c] = v[q];
@@ -3369,13 +3377,13 @@ __device__ __forceinline__ void p_dpdx_body(const Dims &d, const GeoT<R> &g, con
   block_max<1>(red, e, ctl->err[par] + 5);
 }
 template <class R>
-__global__ void __launch_bounds__(BLK) k_p_dpdx(Dims d, GeoT<R> g, FieldsT<R> F, Ctrl *ctl) {
+__global__ void __launch_bounds__(BLK) k_p_dpdx(Dims d, GeoOf<R> g, FieldsT<R> F, Ctrl *ctl) {
   p_dpdx_body<R>(d, g, F, ctl, LaunchBlock{});
 }
 
 // ---- K6: apply_zero_flux (bc.f90:345-390) on the z walls, in place
 template <class R, class BI>
-__device__ __forceinline__ void zero_flux_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void zero_flux_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
@@ -3398,7 +3406,7 @@ __device__ __forceinline__ void zero_flux_body(const Dims &d, const GeoT<R> &g, 
   block_max<1>(red, e, ctl->err[par] + 4);
 }
 template <class R>
-__global__ void __launch_bounds__(BLK) k_zero_flux(Dims d, GeoT<R> g, FieldsT<R> F, Ctrl *ctl) {
+__global__ void __launch_bounds__(BLK) k_zero_flux(Dims d, GeoOf<R> g, FieldsT<R> F, Ctrl *ctl) {
   zero_flux_body<R>(d, g, F, ctl, LaunchBlock{});
 }
 
@@ -3417,20 +3425,20 @@ struct TDir {
   V G1, G3, H2, H4, r, m, p;
 };
 template <class R>
-__device__ __forceinline__ TDir<Ar<R>> T_direction(Ar<R> u, Ar<R> k, Ar<R> gminus, Ar<R> gplus, double v_limit) {
+__device__ __forceinline__ TDir<Ar<R>> T_direction(Ar<R> u, Ar<R> k, Kc<Ar<R>> gminus, Kc<Ar<R>> gplus, double v_limit) {
   using V = Ar<R>;
   TDir<V> t;
   V A[6];
   if constexpr (std::is_same<R, float>::value) {
     nim_direction_f32(u, k, gminus, gplus, A);
-    const V q = V(1) / A[4];  // A5 = 4h/k > 0: every division by it a multiplication
+    const V q = Kc<V>(1) / A[4];  // A5 = 4h/k > 0: every division by it a multiplication
     t.G1 = A[2] - A[0] * A[5] * q;
-    t.G3 = V(0.5) * A[0] * q;
+    t.G3 = Kc<V>(0.5) * A[0] * q;
     t.H2 = A[3] - A[1] * q + A[1] * A[5] * q;
-    t.H4 = V(0.5) * A[1] * q;
+    t.H4 = Kc<V>(0.5) * A[1] * q;
     t.r = q;
     t.m = -(A[5] * q);
-    t.p = (A[5] - V(1)) * q;
+    t.p = (A[5] - Kc<V>(1)) * q;
   } else {
     nim_direction<V>(u, k, gminus, gplus, v_limit, A);
     if constexpr (std::is_same<R, double>::value) {
@@ -3452,31 +3460,31 @@ __device__ __forceinline__ TDir<Ar<R>> T_direction(Ar<R> u, Ar<R> k, Ar<R> gminu
       }
     }
     t.G1 = A[2] - (A[0] * A[5] / A[4]);
-    t.G3 = A[0] / (V(2.) * A[4]);
+    t.G3 = A[0] / (Kc<V>(2.) * A[4]);
     t.H2 = A[3] - A[1] / A[4] + A[1] * A[5] / A[4];
-    t.H4 = A[1] / (V(2.) * A[4]);
-    t.r = V(1.) / A[4];
+    t.H4 = A[1] / (Kc<V>(2.) * A[4]);
+    t.r = Kc<V>(1.) / A[4];
     t.m = -(A[5] / A[4]);
-    t.p = (A[5] - V(1.)) / A[4];
+    t.p = (A[5] - Kc<V>(1.)) / A[4];
   }
   return t;
 }
 // direction dd (1..3) of cell c, from the cell velocities of this pass
 template <class R>
-__device__ __forceinline__ TDir<Ar<R>> T_direction_of(const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, int Nc,
+__device__ __forceinline__ TDir<Ar<R>> T_direction_of(const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, int Nc,
                                                       int c, int dd) {
   using V = Ar<R>;
-  const V ut = V(0.5) * (F.c[0][c] + F.co[0][c]);
-  const V vt = V(0.5) * (F.c[1][c] + F.co[1][c]);
-  const V wt = V(0.5) * (F.c[2][c] + F.co[2][c]);
+  const V ut = Kc<V>(0.5) * (F.c[0][c] + F.co[0][c]);
+  const V vt = Kc<V>(0.5) * (F.c[1][c] + F.co[1][c]);
+  const V wt = Kc<V>(0.5) * (F.c[2][c] + F.co[2][c]);
   const V u = contravariant(g.xi, Nc, c, dd, ut, vt, wt);
   return T_direction<R>(u, g.gij[(dd - 1 + 3 * (dd - 1)) * Nc + c] * pv<V>(P.alpha, P.d_alpha),
                         g.gfd[(2 * (dd - 1)) * Nc + c], g.gfd[(2 * (dd - 1) + 1) * Nc + c], P.v_limit);
 }
 // MT_F4 (nim.f90:466-475) from the three directions' terms
 template <class V>
-__device__ __forceinline__ void T_form_F4(const V r[3], const V m[3], const V p[3], V DT, V F4[8]) {
-  F4[1] = V(0.5) * (r[0] + r[1] + r[2] - V(1.) / DT);
+__device__ __forceinline__ void T_form_F4(const V r[3], const V m[3], const V p[3], Kc<V> DT, V F4[8]) {
+  F4[1] = Kc<V>(0.5) * (r[0] + r[1] + r[2] - Kc<V>(1.) / DT);
   F4[2] = m[0];
   F4[3] = p[0];
   F4[4] = m[1];
@@ -3494,14 +3502,14 @@ __device__ __forceinline__ void T_form_Fd(const FieldsT<R> &F, int Nc, int c, in
   Fd[3] = row[Nc + c];
   Fd[2] = row[2 * Nc + c2];
   Fd[4] = row[3 * Nc + c2];
-  Fd[0] = Fd[1] + Fd[2] + V(2.) * Fd[3] + V(2.) * Fd[4];
+  Fd[0] = Fd[1] + Fd[2] + Kc<V>(2.) * Fd[3] + Kc<V>(2.) * Fd[4];
 }
 
 // The reference order's temperature constants: the TDir terms of every cell
 // and direction stored for k_T_cell(src) and the ordered sweep.
 // Grid (3, ceil(Nc/BLK)): blockIdx.x is the direction.
 template <class R>
-__global__ void __launch_bounds__(BLK, 4) k_T_coef(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(BLK, 4) k_T_coef(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   if (ctl->done) return;
   const int c = blockIdx.y * BLK + threadIdx.x;
   if (c >= d.Nc) return;
@@ -3529,7 +3537,7 @@ __global__ void __launch_bounds__(BLK, 4) k_T_coef(Dims d, GeoT<R> g, FieldsT<R>
 // of their own it was 952.  128x128x96: FP64 T_coef + T_cell 305 -> 289 us,
 // float (k_T_cellN) 128 -> 91 us, and k_T_faceN 51 -> 45 us.
 template <class R, class BI>
-__device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void T_cell_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -3564,13 +3572,13 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, con
     // cross derivatives of calculate_R_D_T: y=0 pxy,pzy  y=1 pyx,pzx  y=2 pxz,pyz
     constexpr int e2 = (y == 0) ? 2 : (y == 1) ? 1 : 3;
     constexpr int fa = (y == 1) ? 4 : 2, fb = (y == 1) ? 3 : 1;
-    sX[y][0][tx] = V(0.5) * (tangential(d, T, x, (y == 2) ? 2 : fa, e2) - tangential(d, T, x, (y == 2) ? 1 : fb, e2));
-    sX[y][1][tx] = (y == 2) ? V(0.5) * (tangential(d, T, x, 4, 3) - tangential(d, T, x, 3, 3))
-                            : V(0.5) * (tangential(d, T, x, 6, e2) - tangential(d, T, x, 5, e2));
+    sX[y][0][tx] = Kc<V>(0.5) * (tangential(d, T, x, (y == 2) ? 2 : fa, e2) - tangential(d, T, x, (y == 2) ? 1 : fb, e2));
+    sX[y][1][tx] = (y == 2) ? Kc<V>(0.5) * (tangential(d, T, x, 4, 3) - tangential(d, T, x, 3, 3))
+                            : Kc<V>(0.5) * (tangential(d, T, x, 6, e2) - tangential(d, T, x, 5, e2));
     if (y == 2) {  // the leading G_i d_i T terms of R_D_T, in source order
-      const V px = (T[f[2]] - T[f[1]]) / V(2.);
-      const V py = (T[f[4]] - T[f[3]]) / V(2.);
-      const V pz = (T[f[6]] - T[f[5]]) / V(2.);
+      const V px = (T[f[2]] - T[f[1]]) / Kc<V>(2.);
+      const V py = (T[f[4]] - T[f[3]]) / Kc<V>(2.);
+      const V pz = (T[f[6]] - T[f[5]]) / Kc<V>(2.);
       sG[tx] = g.G[c] * px + g.G[Nc + c] * py + g.G[2 * Nc + c] * pz;
     }
   });
@@ -3582,21 +3590,21 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoT<R> &g, con
       m[n] = sF[n][1][tx];
       p[n] = sF[n][2][tx];
     }
-    T_form_F4(r, m, p, V(P.DT), F4);
+    T_form_F4(r, m, p, Kc<V>(P.DT), F4);
     const V pxy = sX[0][0][tx], pzy = sX[0][1][tx], pyx = sX[1][0][tx], pzx = sX[1][1][tx];
     const V pxz = sX[2][0][tx], pyz = sX[2][1][tx];
-    const R *gij = g.gij;
+    const Kc<R> *gij = g.gij;
     const V RDT = pv<V>(P.alpha, P.d_alpha) * (sG[tx] - gij[3 * Nc + c] * pxy - gij[1 * Nc + c] * pyx - gij[6 * Nc + c] * pxz -
                                   gij[2 * Nc + c] * pzx - gij[7 * Nc + c] * pyz - gij[5 * Nc + c] * pzy);
     const V cold = F.c[3][c];
-    const V nw = stored<R>(cell_update(T, f, cold, F.co[3][c], (RDT + V(0.)), F4, V(P.w[3])));
+    const V nw = stored<R>(cell_update(T, f, cold, F.co[3][c], (RDT + Kc<V>(0.)), F4, Kc<V>(P.w[3])));
     F.c[3][c] = nw;
     e[0] = errv(nw, cold, first);
   }
   if (d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 4);
 }
 template <class R>
-__global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) k_T_cell(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) k_T_cell(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   T_cell_body<R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
@@ -3607,7 +3615,7 @@ __global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) k_T_ce
 // thread 2 also the G_i d_i T prefix; thread 0 assembles MT_F4, R_D_T and
 // the cell update.  Each cell's arithmetic is k_T_cell's.
 template <class R, int NP>
-__global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -3641,8 +3649,8 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
   };
   const R *T = F.f[4] + par * NF;
   auto along = [&](bool lo, bool hi, V v0, V va, V vb) {
-    return lo ? tang_vals(true, false, v0, va, vb, V(0.), V(0.))
-              : hi ? tang_vals(false, true, v0, V(0.), V(0.), va, vb) : tang_vals(false, false, v0, vb, V(0.), va, V(0.));
+    return lo ? tang_vals(true, false, v0, va, vb, Kc<V>(0.), Kc<V>(0.))
+              : hi ? tang_vals(false, true, v0, Kc<V>(0.), Kc<V>(0.), va, vb) : tang_vals(false, false, v0, vb, Kc<V>(0.), va, Kc<V>(0.));
   };
   double e[1] = {0.};
   if (active) by_dir(threadIdx.y, [&](auto D) {
@@ -3659,7 +3667,7 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
           ldN<R, NP>(xd + 3 * q * Nc, c, xi);
 #pragma unroll
           for (int p = 0; p < NP; ++p) {
-            const V tp = (V(0.5) * (a[p] + b[p])) * xi[p];
+            const V tp = (Kc<V>(0.5) * (a[p] + b[p])) * xi[p];
             u[p] = (q == 0) ? tp : u[p] + tp;
           }
         }
@@ -3699,10 +3707,10 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
       for (int p = 0; p < NP; ++p) {
         const V up2 = (p + 1 < NP) ? (V)o[2][p + 1] : r1_pn, um2 = (p > 0) ? (V)o[2][p - 1] : r1_m1;
         const V up1 = (p + 1 < NP) ? (V)o[1][p + 1] : r_pn, um1 = (p > 0) ? (V)o[1][p - 1] : r_m1;
-        sX[0][0][tx * NP + p] = V(0.5) * ((up2 - um2) / V(4.) - (up1 - um1) / V(4.));
+        sX[0][0][tx * NP + p] = Kc<V>(0.5) * ((up2 - um2) / Kc<V>(4.) - (up1 - um1) / Kc<V>(4.));
         const V up6 = (p + 1 < NP) ? (V)o[6][p + 1] : z1_pn, um6 = (p > 0) ? (V)o[6][p - 1] : z1_m1;
         const V up5 = (p + 1 < NP) ? (V)o[5][p + 1] : z_pn, um5 = (p > 0) ? (V)o[5][p - 1] : z_m1;
-        sX[0][1][tx * NP + p] = V(0.5) * ((up6 - um6) / V(4.) - (up5 - um5) / V(4.));
+        sX[0][1][tx * NP + p] = Kc<V>(0.5) * ((up6 - um6) / Kc<V>(4.) - (up5 - um5) / Kc<V>(4.));
       }
     } else if (y == 1) {
       const int tra = d.offT + NT * (ra + NR * k), trb = d.offT + NT * (rb + NR * k);
@@ -3727,9 +3735,9 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         sX[1][0][tx * NP + p] =
-            V(0.5) * (along(rlo, rhi, o[4][p], av[p + 1], bv[p + 1]) - along(rlo, rhi, o[3][p], av[p], bv[p]));
+            Kc<V>(0.5) * (along(rlo, rhi, o[4][p], av[p + 1], bv[p + 1]) - along(rlo, rhi, o[3][p], av[p], bv[p]));
         sX[1][1][tx * NP + p] =
-            V(0.5) * (along(rlo, rhi, o[6][p], zA[p], zB[p]) - along(rlo, rhi, o[5][p], za[p], zb[p]));
+            Kc<V>(0.5) * (along(rlo, rhi, o[6][p], zA[p], zB[p]) - along(rlo, rhi, o[5][p], za[p], zb[p]));
       }
     } else {
       const int rka = NT * (j + (NR + 1) * ka), rkb = NT * (j + (NR + 1) * kb);
@@ -3758,13 +3766,13 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         sX[2][0][tx * NP + p] =
-            V(0.5) * (along(zlo, zhi, o[2][p], pA[p], pB[p]) - along(zlo, zhi, o[1][p], pa[p], pb[p]));
+            Kc<V>(0.5) * (along(zlo, zhi, o[2][p], pA[p], pB[p]) - along(zlo, zhi, o[1][p], pa[p], pb[p]));
         sX[2][1][tx * NP + p] =
-            V(0.5) * (along(zlo, zhi, o[4][p], av[p + 1], bv[p + 1]) - along(zlo, zhi, o[3][p], av[p], bv[p]));
+            Kc<V>(0.5) * (along(zlo, zhi, o[4][p], av[p + 1], bv[p + 1]) - along(zlo, zhi, o[3][p], av[p], bv[p]));
         // the leading G_i d_i T terms of R_D_T, in source order
-        const V px = (o[2][p] - o[1][p]) / V(2.);
-        const V py = (o[4][p] - o[3][p]) / V(2.);
-        const V pz = (o[6][p] - o[5][p]) / V(2.);
+        const V px = (o[2][p] - o[1][p]) / Kc<V>(2.);
+        const V py = (o[4][p] - o[3][p]) / Kc<V>(2.);
+        const V pz = (o[6][p] - o[5][p]) / Kc<V>(2.);
         sG[tx * NP + p] = G0[p] * px + G1[p] * py + G2[p] * pz;
       }
     }
@@ -3781,7 +3789,7 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
     R cur[NP], old[NP], out[NP];
     ldN<R, NP>(F.c[3], c, cur);
     ldN<R, NP>(F.co[3], c, old);
-    const V w = V(P.w[3]);
+    const Kc<V> w = Kc<V>(P.w[3]);
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const int e2 = tx * NP + p;
@@ -3791,7 +3799,7 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
         m[q] = sF[q][1][e2];
         q3[q] = sF[q][2][e2];
       }
-      T_form_F4(r, m, q3, V(P.DT), F4);
+      T_form_F4(r, m, q3, Kc<V>(P.DT), F4);
       const V pxy = sX[0][0][e2], pzy = sX[0][1][e2], pyx = sX[1][0][e2], pzx = sX[1][1][e2];
       const V pxz = sX[2][0][e2], pyz = sX[2][1][e2];
       const V RDT = pv<V>(P.alpha, P.d_alpha) * (sG[e2] - gs[0][p] * pxy - gs[1][p] * pyx - gs[2][p] * pxz -
@@ -3801,7 +3809,7 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
       const V nw = stored<R>((1 - w) * c0 + (w / F4[0]) * (+F4[1] * (V)old[p] + F4[2] * (V)o[1][p] +
                                                             F4[3] * (V)o[2][p] + F4[4] * (V)o[3][p] +
                                                             F4[5] * (V)o[4][p] + F4[6] * (V)o[5][p] +
-                                                            F4[7] * (V)o[6][p] + (RDT + V(0.))));
+                                                            F4[7] * (V)o[6][p] + (RDT + Kc<V>(0.))));
       out[p] = (R)nw;
       e[0] = nmax(e[0], errv(nw, c0, first));
     }
@@ -3813,7 +3821,7 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoT<R> g, Fi
 // ---- K8: +xi face updates of T (nse.f90:1033-1088), cur -> next; the z-wall
 // values set by apply_zero_flux travel to the next half too
 template <class R, class BI>
-__device__ __forceinline__ void T_face_body(const Dims &d, const GeoT<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+__device__ __forceinline__ void T_face_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -3835,7 +3843,7 @@ __device__ __forceinline__ void T_face_body(const Dims &d, const GeoT<R> &g, con
       T_form_Fd(F, Nc, c, x2.c, dd, Fd);
       const int fo = x.face(d, 2 * dd);
       const V nw = stored<R>(face_update(d, T, F.c[3], F.co[3], Fd, g.dg[(2 * (dd - 1)) * Nc + c],
-                                              g.dg[(2 * (dd - 1) + 1) * Nc + c], dd, x, x2, V(P.w[3])));
+                                              g.dg[(2 * (dd - 1) + 1) * Nc + c], dd, x, x2, Kc<V>(P.w[3])));
       Tn[fo] = nw;
       e[0] = nmax(e[0], errv(nw, T[fo], first));
     }
@@ -3845,7 +3853,7 @@ __device__ __forceinline__ void T_face_body(const Dims &d, const GeoT<R> &g, con
   if (d.owns(blockIdx.z)) block_max<1>(red, e, ctl->err[par] + 4);
 }
 template <class R>
-__global__ void __launch_bounds__(BLK, minb<R>(4, TFACE_MINB_F)) k_T_face(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(BLK, minb<R>(4, TFACE_MINB_F)) k_T_face(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   T_face_body<R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
@@ -3918,8 +3926,8 @@ __device__ __forceinline__ double face_updateN(const Dims &d, int i, int j, int 
   R out[NP];
 #pragma unroll
   for (int p = 0; p < NP; ++p) {
-    const V B3 = (dg0[p]) * ((V)ox[2 * e1][p] - ox[2 * e1 - 1][p] + on[2 * e1][p] - on[2 * e1 - 1][p]) / V(4.0);
-    const V B4 = (dg1[p]) * ((V)ox[2 * e2][p] - ox[2 * e2 - 1][p] + on[2 * e2][p] - on[2 * e2 - 1][p]) / V(4.0);
+    const V B3 = (dg0[p]) * ((V)ox[2 * e1][p] - ox[2 * e1 - 1][p] + on[2 * e1][p] - on[2 * e1 - 1][p]) / Kc<V>(4.0);
+    const V B4 = (dg1[p]) * ((V)ox[2 * e2][p] - ox[2 * e2 - 1][p] + on[2 * e2][p] - on[2 * e2 - 1][p]) / Kc<V>(4.0);
     const V old = ox[2 * dd][p];
     const V nw = stored<R>((1 - w) * old + (w / Fd[0][p]) * (+Fd[1][p] * (V)ox[2 * dd - 1][p] +
                                                                Fd[2][p] * (V)on[2 * dd][p] +
@@ -3944,7 +3952,7 @@ __device__ __forceinline__ double face_updateN(const Dims &d, int i, int j, int 
 // +theta neighbours as k_p_faceN forms them) and carries the z-wall values
 // to the next half (thread 2).  Each face's arithmetic is face_update's.
 template <class R, int NP>
-__global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   using V = Ar<R>;
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -4044,17 +4052,17 @@ __global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoT<R> g, Fi
         ldN<R, NP>(row + 3 * Nc, c + (dd == 1 ? NT : pl), Fd[4]);
       }
 #pragma unroll
-      for (int p = 0; p < NP; ++p) Fd[0][p] = (V)Fd[1][p] + Fd[2][p] + V(2) * Fd[3][p] + V(2) * Fd[4][p];
+      for (int p = 0; p < NP; ++p) Fd[0][p] = (V)Fd[1][p] + Fd[2][p] + Kc<V>(2) * Fd[3][p] + Kc<V>(2) * Fd[4][p];
     }
     ldN<R, NP>(g.dg + (size_t)(2 * (dd - 1)) * Nc, c, dg0);
     ldN<R, NP>(g.dg + (size_t)(2 * (dd - 1) + 1) * Nc, c, dg1);
     constexpr int e1 = (dd == 1) ? 2 : 1, e2 = (dd == 3) ? 2 : 3;  // tr1(dd), tr2(dd)
-    const V w = V(P.w[3]);
+    const Kc<V> w = Kc<V>(P.w[3]);
     R out[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      const V B3 = (dg0[p]) * ((V)ox[2 * e1][p] - ox[2 * e1 - 1][p] + on[2 * e1][p] - on[2 * e1 - 1][p]) / V(4.0);
-      const V B4 = (dg1[p]) * ((V)ox[2 * e2][p] - ox[2 * e2 - 1][p] + on[2 * e2][p] - on[2 * e2 - 1][p]) / V(4.0);
+      const V B3 = (dg0[p]) * ((V)ox[2 * e1][p] - ox[2 * e1 - 1][p] + on[2 * e1][p] - on[2 * e1 - 1][p]) / Kc<V>(4.0);
+      const V B4 = (dg1[p]) * ((V)ox[2 * e2][p] - ox[2 * e2 - 1][p] + on[2 * e2][p] - on[2 * e2 - 1][p]) / Kc<V>(4.0);
       const V old = ox[2 * dd][p];
       const V nw = stored<R>((1 - w) * old + (w / Fd[0][p]) * (+Fd[1][p] * (V)ox[2 * dd - 1][p] +
                                                                  Fd[2][p] * (V)on[2 * dd][p] +
@@ -4079,7 +4087,7 @@ __global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoT<R> g, Fi
 // cells, block (CB, 3): thread y updates the +xi face of direction y+1 of
 // the NP cells for each component (face_updateN), as k_vel_face.
 template <class R, int NP>
-__global__ void __launch_bounds__(CB3, VFN_MINB) k_vel_faceN(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+__global__ void __launch_bounds__(CB3, VFN_MINB) k_vel_faceN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<3>(red);
@@ -4793,7 +4801,7 @@ __global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl 
 // (the dual instantiation: the maxima and the sum of squares of the values;
 // meshes_dila with its derivative)
 template <class R>
-__global__ void __launch_bounds__(BLK) k_after_integrate(Dims d, GeoT<R> g, FieldsT<R> F, Phys P, Ctrl *ctl,
+__global__ void __launch_bounds__(BLK) k_after_integrate(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl,
                                                          int nblk) {
   using V = Ar<R>;
   __shared__ BlockRed red;
@@ -4817,7 +4825,7 @@ __global__ void __launch_bounds__(BLK) k_after_integrate(Dims d, GeoT<R> g, Fiel
       vf[k] = F.f[1][par * NF + f[k]];
       wf[k] = F.f[2][par * NF + f[k]];
     }
-    const V invV = V(1.) / g.vol[c];
+    const Kc<V> invV = Kc<V>(1.) / g.vol[c];
     const V Dila = green_gauss(g, NF, invV, uf, f, 0) + green_gauss(g, NF, invV, vf, f, 1) +
                    green_gauss(g, NF, invV, wf, f, 2);
     F.dila[c] = Dila;
@@ -4854,13 +4862,13 @@ __global__ void __launch_bounds__(BLK) k_update_time(Dims d, FieldsT<R> F, Ctrl 
   if (c >= d.Nc) return;
   const Cell x = Cell::of(d, c);
   for (int q = 0; q < 4; ++q) {
-    F.ct[q][c] = (F.co[q][c] + F.c[q][c]) / V(2.);
+    F.ct[q][c] = (F.co[q][c] + F.c[q][c]) / Kc<V>(2.);
     F.co[q][c] = F.c[q][c];
   }
   int f[7];
   cell_faces(d, x, f);
   const R *p = F.f[3] + par * (size_t)d.NF;
-  F.mp[c] = (p[f[1]] + p[f[2]] + p[f[3]] + p[f[4]] + p[f[5]] + p[f[6]]) / V(6.0);
+  F.mp[c] = (p[f[1]] + p[f[2]] + p[f[3]] + p[f[4]] + p[f[5]] + p[f[6]]) / Kc<V>(6.0);
   F.dila_old[c] = F.dila[c];
 }
 
@@ -4869,7 +4877,7 @@ __global__ void __launch_bounds__(BLK) k_update_time(Dims d, FieldsT<R> F, Ctrl 
 // (the dual instantiation sums the four values, then their derivatives:
 // eight partial sums)
 template <class R>
-__global__ void __launch_bounds__(BLK) k_nusselt(Dims d, GeoT<R> g, FieldsT<R> F, Ctrl *ctl, int nblk) {
+__global__ void __launch_bounds__(BLK) k_nusselt(Dims d, GeoOf<R> g, FieldsT<R> F, Ctrl *ctl, int nblk) {
   using V = Ar<R>;
   const int par = parity(ctl);
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -4882,12 +4890,12 @@ __global__ void __launch_bounds__(BLK) k_nusselt(Dims d, GeoT<R> g, FieldsT<R> F
     const int in = (B.pos == 1) ? 2 : 1;
     const Cell c2 = B.cell.nb(d, in), c3 = c2.nb(d, in);
     const R *T = F.f[4] + par * NF;
-    const R *w = g.nuw;
+    const Kc<R> *w = g.nuw;
     const int f1 = B.cell.face(d, B.pos);
     const V inner = -((w[b]) * T[f1]) + w[NB + b] * T[B.cell.face(d, in)] - w[2 * NB + b] * T[c2.face(d, in)] +
                     w[3 * NB + b] * T[c3.face(d, in)];
     const V dTdx = (B.pos == 1) ? -(inner) : inner;
-    const V A = g.area[f1];
+    const Kc<V> A = g.area[f1];
     if (B.pos == 1) {
       s[2] = A * dTdx;
       s[3] = A;
