@@ -29,12 +29,10 @@ enum BatchSlot {
   BS_VEL_FACE,   // k_vel_face (FlatBlock)
   BS_P_SRC2,     // k_p_srcN<double, 2> (FlatBlock)
   BS_P_SRC,      // k_p_src (FlatBlock)
-  BS_P_BC,       // k_p_bc
-  BS_P_BC_COPY,  // k_p_bc_copy
+  BS_WALLS,      // k_walls
   BS_P_FACE2,    // k_p_faceN<double, 2> (FlatBlock)
   BS_P_FACE,     // k_p_face (FlatBlock)
   BS_P_DPDX,     // k_p_dpdx (is_dpdx_tolerance)
-  BS_ZERO_FLUX,  // k_zero_flux
   BS_T_CELL,     // k_T_cell (FlatBlock)
   BS_T_FACE,     // k_T_face (FlatBlock)
   BS_COUNT
@@ -222,15 +220,9 @@ __global__ void __launch_bounds__(CB3, wider(minb<R>(4, PSRC_MINB_F), W)) kb_p_s
   });
 }
 template <class R, int W>
-__global__ void __launch_bounds__(BLK) kb_p_bc(BatchArgs A) {
-  batch_items<BS_P_BC, R>(A, [&](const BatchInst<R> &I, BatchBlock b) {
-    p_bc_body<R>(I.d, I.g, I.F, I.P, I.ctl, b);
-  });
-}
-template <class R, int W>
-__global__ void __launch_bounds__(BLK) kb_p_bc_copy(BatchArgs A) {
-  batch_items<BS_P_BC_COPY, R>(A, [&](const BatchInst<R> &I, BatchBlock b) {
-    p_bc_copy_body<R>(I.d, I.F, I.ctl, b);
+__global__ void __launch_bounds__(BLK) kb_walls(BatchArgs A) {
+  batch_items<BS_WALLS, R>(A, [&](const BatchInst<R> &I, BatchBlock b) {
+    walls_body<R>(I.d, I.g, I.F, I.P, I.ctl, b);
   });
 }
 template <int W>
@@ -249,12 +241,6 @@ template <class R, int W>
 __global__ void __launch_bounds__(BLK) kb_p_dpdx(BatchArgs A) {
   batch_items<BS_P_DPDX, R>(A, [&](const BatchInst<R> &I, BatchBlock b) {
     p_dpdx_body<R>(I.d, I.g, I.F, I.ctl, b);
-  });
-}
-template <class R, int W>
-__global__ void __launch_bounds__(BLK) kb_zero_flux(BatchArgs A) {
-  batch_items<BS_ZERO_FLUX, R>(A, [&](const BatchInst<R> &I, BatchBlock b) {
-    zero_flux_body<R>(I.d, I.g, I.F, I.ctl, b);
   });
 }
 template <class R, int W>
@@ -331,12 +317,8 @@ __global__ void __launch_bounds__(CB3, minb<R>(4, PSRC_MINB_F)) kg_p_src(const _
   group_item<R, FlatBlock>(L, [&](const BatchInst<R> &I, FlatBlock b) { p_src_body<R>(I.d, I.g, I.F, I.P, I.ctl, b); });
 }
 template <class R>
-__global__ void __launch_bounds__(BLK) kg_p_bc(const __grid_constant__ BatchGroup<R> L) {
-  group_item<R, BatchBlock>(L, [&](const BatchInst<R> &I, BatchBlock b) { p_bc_body<R>(I.d, I.g, I.F, I.P, I.ctl, b); });
-}
-template <class R>
-__global__ void __launch_bounds__(BLK) kg_p_bc_copy(const __grid_constant__ BatchGroup<R> L) {
-  group_item<R, BatchBlock>(L, [&](const BatchInst<R> &I, BatchBlock b) { p_bc_copy_body<R>(I.d, I.F, I.ctl, b); });
+__global__ void __launch_bounds__(BLK) kg_walls(const __grid_constant__ BatchGroup<R> L) {
+  group_item<R, BatchBlock>(L, [&](const BatchInst<R> &I, BatchBlock b) { walls_body<R>(I.d, I.g, I.F, I.P, I.ctl, b); });
 }
 __global__ void __launch_bounds__(CB3, PFN_MINB) kg_p_face2(const __grid_constant__ BatchGroup<double> L) {
   group_item<double, FlatBlock>(L, [&](const BatchInst<double> &I, FlatBlock b) { p_faceN_body<double, 2>(I.d, I.g, I.F, I.P, I.ctl, b); });
@@ -348,10 +330,6 @@ __global__ void __launch_bounds__(CB3, minb<R>(5, PFACE_MINB_F)) kg_p_face(const
 template <class R>
 __global__ void __launch_bounds__(BLK) kg_p_dpdx(const __grid_constant__ BatchGroup<R> L) {
   group_item<R, BatchBlock>(L, [&](const BatchInst<R> &I, BatchBlock b) { p_dpdx_body<R>(I.d, I.g, I.F, I.ctl, b); });
-}
-template <class R>
-__global__ void __launch_bounds__(BLK) kg_zero_flux(const __grid_constant__ BatchGroup<R> L) {
-  group_item<R, BatchBlock>(L, [&](const BatchInst<R> &I, BatchBlock b) { zero_flux_body<R>(I.d, I.g, I.F, I.ctl, b); });
 }
 template <class R>
 __global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) kg_T_cell(const __grid_constant__ BatchGroup<R> L) {

@@ -74,7 +74,12 @@ struct nim_ctx {
   double *scratch = nullptr; // gather/scatter staging [54*Nc or 3*NF]
   double *sums = nullptr;    // [8] outputs of k_finish_sum
   int nblk_c = 0, nblk_b = 0, nblk_c3 = 0;
-  dim3 g3{1, 1, 1}, g8{1, 1, 1};  // patch grids: 32x4 (x3 threads) and 32x8 cells
+  dim3 g3{1, 1, 1};  // patch grid: 32x4 cells (x3 threads)
+  // grids of the sweeps with one cell (128 or 256 a block), two and four cells
+  // a thread: patches of the (theta, r) plane, or runs of it in cell order
+  // where patches would leave too many lanes idle (flat)
+  dim3 s1{1, 1, 1}, s1w{1, 1, 1}, s2{1, 1, 1}, s4{1, 1, 1};
+  bool flat1 = false, flat2 = false, flat4 = false;
   std::vector<void *> allocs;
   cudaGraphExec_t graph = nullptr;
   int graph_iters = 0;
@@ -293,63 +298,67 @@ int mark(nim_ctx *x, const char *name) {
 template <class R>
 int launch_vel(nim_ctx *x, cudaStream_t s, const GeoOf<R> &g, const FieldsT<R> &F) {
   const Dims &d = x->d;
-  if (x->phys.formulation == 1) {
-    k_vel_cell<false, 1><<<x->g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+  const dim3 t3(CB, 3);
+  const Phys &P = x->phys;
+  Ctrl *ctl = x->ctl;
+  if (P.formulation == 1) {
+    k_vel_cell<false, 1><<<x->g3, t3, 0, s>>>(d, g, F, P, ctl);
     TRY(mark(x, "k_vel_cell"));
-    k_vel1_face<<<x->g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+    k_vel1_face<<<x->g3, t3, 0, s>>>(d, g, F, P, ctl);
     TRY(mark(x, "k_vel1_face"));
+    return NIM_OK;
+  }
+  if (x->cell_tile) {
+    const dim3 gt((d.NT + 31) / 32, (d.NR + CT_R - 1) / CT_R, (d.NZ + x->tile_kc - 1) / x->tile_kc);
+    const VelCellMaps &M = std::is_same<R, double>::value ? x->cmap64 : x->cmap32;
+    k_vel_cell_tile<R><<<gt, dim3(CT_T, 3), CtLayout<R>::bytes, s>>>(d, g, F, P, ctl, x->tile_kc, M);
+    TRY(mark(x, "k_vel_cell_tile"));
+  } else if (std::is_same<R, float>::value && x->cell_quad) {
+    if constexpr (std::is_same<R, float>::value) {
+      if (x->flat4)
+        k_vel_cellN<R, 4, false, true><<<x->s4, t3, 0, s>>>(d, g, F, P, ctl);
+      else
+        k_vel_cellN<R, 4><<<x->s4, t3, 0, s>>>(d, g, F, P, ctl);
+      TRY(mark(x, "k_vel_cellN"));
+    }
+  } else if (x->cell_pair) {
+    if (x->slab_count)
+      (x->flat2 ? k_vel_cell2<R, true, true> : k_vel_cell2<R, true, false>)<<<x->s2, t3, 0, s>>>(d, g, F, P, ctl);
+    else
+      (x->flat2 ? k_vel_cell2<R, false, true> : k_vel_cell2<R, false, false>)<<<x->s2, t3, 0, s>>>(d, g, F, P, ctl);
+    TRY(mark(x, "k_vel_cell2"));
   } else {
-    if (x->cell_tile) {
-      const dim3 gt((d.NT + 31) / 32, (d.NR + CT_R - 1) / CT_R, (d.NZ + x->tile_kc - 1) / x->tile_kc);
-      const VelCellMaps &M = std::is_same<R, double>::value ? x->cmap64 : x->cmap32;
-      k_vel_cell_tile<R><<<gt, dim3(CT_T, 3), CtLayout<R>::bytes, s>>>(d, g, F, x->phys, x->ctl, x->tile_kc, M);
-      TRY(mark(x, "k_vel_cell_tile"));
-    } else if (std::is_same<R, float>::value && x->cell_quad) {
-      if constexpr (std::is_same<R, float>::value) {
-        const dim3 gq((d.NT + 127) / 128, (d.NR + 3) / 4, d.NZ);
-        if (x->slab_count)
-          k_vel_cellN<R, 4, true><<<gq, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
-        else
-          k_vel_cellN<R, 4><<<gq, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
-        TRY(mark(x, "k_vel_cellN"));
-      }
-    } else if (x->cell_pair) {
-      const dim3 gp((d.NT + 63) / 64, (d.NR + 3) / 4, d.NZ);
-      if (x->slab_count)
-        k_vel_cell2<R, true><<<gp, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+    (x->flat1 ? k_vel_cell<false, 2, true, R> : k_vel_cell<false, 2, false, R>)<<<x->s1, t3, 0, s>>>(d, g, F, P, ctl);
+    TRY(mark(x, "k_vel_cell"));
+  }
+  if (std::is_same<R, float>::value && x->face_quad) {
+    if constexpr (std::is_same<R, float>::value) {  // the float mirror, four cells a thread
+      if (x->flat4)
+        k_vel_faceN<R, 4, true><<<x->s4, t3, 0, s>>>(d, g, F, P, ctl);
       else
-        k_vel_cell2<R><<<gp, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
-      TRY(mark(x, "k_vel_cell2"));
-    } else {
-      k_vel_cell<false, 2><<<x->g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
-      TRY(mark(x, "k_vel_cell"));
+        k_vel_faceN<R, 4><<<x->s4, t3, 0, s>>>(d, g, F, P, ctl);
+      TRY(mark(x, "k_vel_faceN"));
     }
-    if (std::is_same<R, float>::value && x->face_quad) {
-      if constexpr (std::is_same<R, float>::value) {  // the float mirror, four cells a thread
-        const dim3 gq((d.NT + 127) / 128, (d.NR + 3) / 4, d.NZ);
-        k_vel_faceN<R, 4><<<gq, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
-        TRY(mark(x, "k_vel_faceN"));
-      }
-    } else if (x->bulk) {
-      const dim3 gt((d.NT + 31) / 32, (d.NR + VT_R - 1) / VT_R, (d.NZ + x->tile_kc - 1) / x->tile_kc);
-      const VelFaceMaps &M = std::is_same<R, double>::value ? x->vmap64 : x->vmap32;
-      if (x->slab_count)
-        k_vel_face_tile<R, true><<<gt, dim3(VT_T, 3), VtLayout<R>::bytes, s>>>(d, g, F, x->phys, x->ctl, x->tile_kc, M);
-      else
-        k_vel_face_tile<R><<<gt, dim3(VT_T, 3), VtLayout<R>::bytes, s>>>(d, g, F, x->phys, x->ctl, x->tile_kc, M);
-      TRY(mark(x, "k_vel_face_tile"));
-    } else {
-      k_vel_face<<<x->g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
-      TRY(mark(x, "k_vel_face"));
-    }
+  } else if (x->bulk) {
+    const dim3 gt((d.NT + 31) / 32, (d.NR + VT_R - 1) / VT_R, (d.NZ + x->tile_kc - 1) / x->tile_kc);
+    const VelFaceMaps &M = std::is_same<R, double>::value ? x->vmap64 : x->vmap32;
+    if (x->slab_count)
+      k_vel_face_tile<R, true><<<gt, dim3(VT_T, 3), VtLayout<R>::bytes, s>>>(d, g, F, P, ctl, x->tile_kc, M);
+    else
+      k_vel_face_tile<R><<<gt, dim3(VT_T, 3), VtLayout<R>::bytes, s>>>(d, g, F, P, ctl, x->tile_kc, M);
+    TRY(mark(x, "k_vel_face_tile"));
+  } else {
+    (x->flat1 ? k_vel_face<true, R> : k_vel_face<false, R>)<<<x->s1, t3, 0, s>>>(d, g, F, P, ctl);
+    TRY(mark(x, "k_vel_face"));
   }
   return NIM_OK;
 }
 // the tangent-linear state (formulation 2): the gather forms of both sweeps
 int launch_vel(nim_ctx *x, cudaStream_t s, const Geo &g, const FieldsT<DualD> &F) {
-  k_vel_cell<false, 2><<<x->g3, dim3(CB, 3), 0, s>>>(x->d, g, F, x->phys, x->ctl);
+  const dim3 t3(CB, 3);
+  (x->flat1 ? k_vel_cell<false, 2, true, DualD> : k_vel_cell<false, 2, false, DualD>)<<<x->s1, t3, 0, s>>>(x->d, g, F, x->phys, x->ctl);
   TRY(mark(x, "k_vel_cell"));
-  k_vel_face<<<x->g3, dim3(CB, 3), 0, s>>>(x->d, g, F, x->phys, x->ctl);
+  (x->flat1 ? k_vel_face<true, DualD> : k_vel_face<false, DualD>)<<<x->s1, t3, 0, s>>>(x->d, g, F, x->phys, x->ctl);
   TRY(mark(x, "k_vel_face"));
   return NIM_OK;
 }
@@ -445,49 +454,48 @@ int seq_pack_geometry(nim_ctx *x) {
 template <class R>
 int launch_pressure(nim_ctx *x, cudaStream_t s, const GeoOf<R> &g, const FieldsT<R> &F) {
   const Dims &d = x->d;
-  const dim3 g3 = x->g3;
+  const dim3 t3(CB, 3);
+  const Phys &P = x->phys;
+  Ctrl *ctl = x->ctl;
   // the float mirror sweeps four theta-adjacent cells a thread (n_theta % 4
   // == 0), the FP64 path two (n_theta even: double2 loads; measured at C2,
   // k_p_face 154 -> 113 us, k_p_src 160 -> 159 us; the temperature and
   // velocity sweeps stay one cell a thread, their pair forms were slower)
   const bool quad = std::is_same<R, float>::value && x->cell_quad;
   const bool pair = std::is_same<R, double>::value && x->press_pair;
-  const dim3 gq((d.NT + 127) / 128, (d.NR + 3) / 4, d.NZ);
-  const dim3 gp((d.NT + 63) / 64, (d.NR + 3) / 4, d.NZ);
   if (quad) {
     if constexpr (std::is_same<R, float>::value) {
-      k_p_srcN<R, 4><<<gq, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+      (x->flat4 ? k_p_srcN<R, 4, true> : k_p_srcN<R, 4, false>)<<<x->s4, t3, 0, s>>>(d, g, F, P, ctl);
       TRY(mark(x, "k_p_srcN"));
     }
   } else if (pair) {
     if constexpr (std::is_same<R, double>::value) {
-      k_p_srcN<R, 2><<<gp, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+      (x->flat2 ? k_p_srcN<R, 2, true> : k_p_srcN<R, 2, false>)<<<x->s2, t3, 0, s>>>(d, g, F, P, ctl);
       TRY(mark(x, "k_p_srcN"));
     }
   } else {
-    k_p_src<<<g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+    (x->flat1 ? k_p_src<true, R> : k_p_src<false, R>)<<<x->s1, t3, 0, s>>>(d, g, F, P, ctl);
     TRY(mark(x, "k_p_src"));
   }
-  k_p_bc<<<x->nblk_b, BLK, 0, s>>>(d, g, F, x->phys, x->ctl);
-  TRY(mark(x, "k_p_bc"));
-  k_p_bc_copy<<<x->nblk_b, BLK, 0, s>>>(d, F, x->ctl);
-  TRY(mark(x, "k_p_bc_copy"));
+  // apply_pressure_bc, and the temperature's apply_zero_flux beside it
+  k_walls<<<grid(d.NBF + 2 * d.plane), BLK, 0, s>>>(d, g, F, P, ctl);
+  TRY(mark(x, "k_walls"));
   if (quad) {
     if constexpr (std::is_same<R, float>::value) {
-      k_p_faceN<R, 4><<<gq, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+      (x->flat4 ? k_p_faceN<R, 4, true> : k_p_faceN<R, 4, false>)<<<x->s4, t3, 0, s>>>(d, g, F, P, ctl);
       TRY(mark(x, "k_p_faceN"));
     }
   } else if (pair) {
     if constexpr (std::is_same<R, double>::value) {
-      k_p_faceN<R, 2><<<gp, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+      (x->flat2 ? k_p_faceN<R, 2, true> : k_p_faceN<R, 2, false>)<<<x->s2, t3, 0, s>>>(d, g, F, P, ctl);
       TRY(mark(x, "k_p_faceN"));
     }
   } else {
-    k_p_face<<<g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+    (x->flat1 ? k_p_face<true, R> : k_p_face<false, R>)<<<x->s1, t3, 0, s>>>(d, g, F, P, ctl);
     TRY(mark(x, "k_p_face"));
   }
-  if (x->phys.dpdx_tolerance) {
-    k_p_dpdx<<<x->nblk_c, BLK, 0, s>>>(d, g, F, x->ctl);
+  if (P.dpdx_tolerance) {
+    k_p_dpdx<<<x->nblk_c, BLK, 0, s>>>(d, g, F, ctl);
     TRY(mark(x, "k_p_dpdx"));
   }
   return NIM_OK;
@@ -497,21 +505,19 @@ int launch_pressure(nim_ctx *x, cudaStream_t s, const GeoOf<R> &g, const FieldsT
 template <class R>
 int launch_temperature(nim_ctx *x, cudaStream_t s, const GeoOf<R> &g, const FieldsT<R> &F) {
   const Dims &d = x->d;
-  k_zero_flux<<<grid(2 * d.plane), BLK, 0, s>>>(d, g, F, x->ctl);
-  TRY(mark(x, "k_zero_flux"));
+  const dim3 t3(CB, 3);
   if constexpr (std::is_same<R, float>::value) {
     if (x->cell_quad) {  // the float mirror: four theta-adjacent cells a thread
-      const dim3 gq((d.NT + 127) / 128, (d.NR + 3) / 4, d.NZ);
-      k_T_cellN<R, 4><<<gq, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+      (x->flat4 ? k_T_cellN<R, 4, true> : k_T_cellN<R, 4, false>)<<<x->s4, t3, 0, s>>>(d, g, F, x->phys, x->ctl);
       TRY(mark(x, "k_T_cellN"));
-      k_T_faceN<R, 4><<<gq, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+      (x->flat4 ? k_T_faceN<R, 4, true> : k_T_faceN<R, 4, false>)<<<x->s4, t3, 0, s>>>(d, g, F, x->phys, x->ctl);
       TRY(mark(x, "k_T_faceN"));
       return NIM_OK;
     }
   }
-  k_T_cell<<<x->g3, dim3(CB, 3), 0, s>>>(d, g, F, x->phys, x->ctl);
+  (x->flat1 ? k_T_cell<true, R> : k_T_cell<false, R>)<<<x->s1, t3, 0, s>>>(d, g, F, x->phys, x->ctl);
   TRY(mark(x, "k_T_cell"));
-  k_T_face<<<x->g8, BLK, 0, s>>>(d, g, F, x->phys, x->ctl);
+  (x->flat1 ? k_T_face<true, R> : k_T_face<false, R>)<<<x->s1w, BLK, 0, s>>>(d, g, F, x->phys, x->ctl);
   TRY(mark(x, "k_T_face"));
   return NIM_OK;
 }
@@ -526,7 +532,7 @@ int launch_parallel(nim_ctx *x, const GeoOf<R> &g, const FieldsT<R> &F, int lowp
   k_iter_end<<<1, 1, 0, s>>>(x->ctl, x->phys, lowp);
   TRY(mark(x, "k_iter_end"));
   CK(cudaGetLastError());
-  x->kernels_per_iter = x->phys.dpdx_tolerance ? 11 : 10;
+  x->kernels_per_iter = x->phys.dpdx_tolerance ? 9 : 8;
   x->launches += x->kernels_per_iter;
   return NIM_OK;
 }
@@ -1107,6 +1113,12 @@ extern "C" int nim_slab_halo(int32_t n_theta, int32_t n_r, int32_t n_z, int32_t 
 
 // slab: null for the whole mesh, else {nslab, s}: the context holds z-slab s
 // of nslab (nim_slab_layout) with its halo planes
+// share of busy threads below which a sweep runs in cell order.  Both sides,
+// us a pass of FP64: 131x97x83 (0.81 busy) 843 patches, 744 runs; 150x101x77
+// (pairs 0.77, one cell 0.91: runs for the pairs only) 820, 792; 72x72x54
+// (0.75) 261, 220; 128x128x96 (1.0) 890, 959: a patch keeps the r neighbours
+// of its cells in the block's cache lines.
+constexpr double kFlatBelow = 0.9;
 static int create_impl(const nim_mesh_desc *m, const nim_params *p, nim_ctx *x, const int32_t *slab = nullptr) {
   CK(cudaGetDevice(&x->device));
   TRY(noalloc_setup(x->device));
@@ -1151,7 +1163,22 @@ static int create_impl(const nim_mesh_desc *m, const nim_params *p, nim_ctx *x, 
   x->nblk_b = grid(d.NBF);
   x->nblk_c3 = (d.Nc + CB - 1) / CB;
   x->g3 = dim3((d.NT + 31) / 32, (d.NR + 3) / 4, d.NZ);
-  x->g8 = dim3((d.NT + 31) / 32, (d.NR + 7) / 8, d.NZ);
+  // NP cells a thread: patches of 32 NP cells by four rows (eight in blocks
+  // of 256), or runs of the plane where the patches' threads would be idle
+  // for more than a tenth (theta remainders of a warp, row remainders)
+  auto sweep = [&](int np, int rows, bool &flat) {
+    const int groups = d.NT / np, bx = (groups + 31) / 32, by = (d.NR + rows - 1) / rows;
+    const double busy = (double)groups * d.NR / ((double)bx * 32 * by * rows);
+    flat = d.NT % np == 0 && busy < kFlatBelow;
+    return flat ? dim3((groups * d.NR + 32 * rows - 1) / (32 * rows), 1, d.NZ) : dim3((d.NT + 32 * np - 1) / (32 * np), by, d.NZ);
+  };
+  bool wide = false;
+  x->s1 = sweep(1, 4, x->flat1);
+  x->s1w = sweep(1, 8, wide);
+  if (wide != x->flat1)  // one choice for the one-cell sweeps
+    x->s1w = x->flat1 ? dim3((d.plane + BLK - 1) / BLK, 1, d.NZ) : dim3((d.NT + 31) / 32, (d.NR + 7) / 8, d.NZ);
+  x->s2 = sweep(2, 4, x->flat2);
+  x->s4 = sweep(4, 4, x->flat4);
   const size_t Nc = d.Nc, NF = d.NF, NB = d.NBF;
   Geo &g = x->g;
   TRY(dalloc(x, &g.vol, Nc));
@@ -1739,11 +1766,9 @@ int fused_occupancy(FusedBatch &B, int sms) {
     TRY(persistent_blocks(kb_p_face2<W>, CB3, sms, b[BS_P_FACE2]));
   }
   TRY(persistent_blocks(kb_p_src<R, W>, CB3, sms, b[BS_P_SRC]));
-  TRY(persistent_blocks(kb_p_bc<R, W>, BLK, sms, b[BS_P_BC]));
-  TRY(persistent_blocks(kb_p_bc_copy<R, W>, BLK, sms, b[BS_P_BC_COPY]));
+  TRY(persistent_blocks(kb_walls<R, W>, BLK, sms, b[BS_WALLS]));
   TRY(persistent_blocks(kb_p_face<R, W>, CB3, sms, b[BS_P_FACE]));
   TRY(persistent_blocks(kb_p_dpdx<R, W>, BLK, sms, b[BS_P_DPDX]));
-  TRY(persistent_blocks(kb_zero_flux<R, W>, BLK, sms, b[BS_ZERO_FLUX]));
   TRY(persistent_blocks(kb_T_cell<R, W>, CB3, sms, b[BS_T_CELL]));
   TRY(persistent_blocks(kb_T_face<R, W>, BLK, sms, b[BS_T_FACE]));
   return NIM_OK;
@@ -1765,14 +1790,12 @@ int fused_slots(FusedBatch &B) {
     if (u[BS_P_SRC2]) kb_p_src2<W><<<b[BS_P_SRC2], t3, 0, s>>>(A);
   }
   if (u[BS_P_SRC]) kb_p_src<R, W><<<b[BS_P_SRC], t3, 0, s>>>(A);
-  if (u[BS_P_BC]) kb_p_bc<R, W><<<b[BS_P_BC], BLK, 0, s>>>(A);
-  if (u[BS_P_BC_COPY]) kb_p_bc_copy<R, W><<<b[BS_P_BC_COPY], BLK, 0, s>>>(A);
+  if (u[BS_WALLS]) kb_walls<R, W><<<b[BS_WALLS], BLK, 0, s>>>(A);
   if constexpr (ph == 1) {
     if (u[BS_P_FACE2]) kb_p_face2<W><<<b[BS_P_FACE2], t3, 0, s>>>(A);
   }
   if (u[BS_P_FACE]) kb_p_face<R, W><<<b[BS_P_FACE], t3, 0, s>>>(A);
   if (u[BS_P_DPDX]) kb_p_dpdx<R, W><<<b[BS_P_DPDX], BLK, 0, s>>>(A);
-  if (u[BS_ZERO_FLUX]) kb_zero_flux<R, W><<<b[BS_ZERO_FLUX], BLK, 0, s>>>(A);
   if (u[BS_T_CELL]) kb_T_cell<R, W><<<b[BS_T_CELL], t3, 0, s>>>(A);
   if (u[BS_T_FACE]) kb_T_face<R, W><<<b[BS_T_FACE], BLK, 0, s>>>(A);
   CK(cudaGetLastError());
@@ -1793,11 +1816,9 @@ void group_launch(int slot, const BatchGroup<R> &L, cudaStream_t s) {
     case BS_VEL_CELL: kg_vel_cell<R><<<nb, t3, 0, s>>>(L); break;
     case BS_VEL_FACE: kg_vel_face<R><<<nb, t3, 0, s>>>(L); break;
     case BS_P_SRC: kg_p_src<R><<<nb, t3, 0, s>>>(L); break;
-    case BS_P_BC: kg_p_bc<R><<<nb, BLK, 0, s>>>(L); break;
-    case BS_P_BC_COPY: kg_p_bc_copy<R><<<nb, BLK, 0, s>>>(L); break;
+    case BS_WALLS: kg_walls<R><<<nb, BLK, 0, s>>>(L); break;
     case BS_P_FACE: kg_p_face<R><<<nb, t3, 0, s>>>(L); break;
     case BS_P_DPDX: kg_p_dpdx<R><<<nb, BLK, 0, s>>>(L); break;
-    case BS_ZERO_FLUX: kg_zero_flux<R><<<nb, BLK, 0, s>>>(L); break;
     case BS_T_CELL: kg_T_cell<R><<<nb, t3, 0, s>>>(L); break;
     case BS_T_FACE: kg_T_face<R><<<nb, BLK, 0, s>>>(L); break;
     default:
@@ -1937,7 +1958,6 @@ int fused_setup(FusedBatch &B, int32_t n, nim_ctx *const *ctx) {
     const BatchGrid f3{(unsigned)((d.plane + CB - 1) / CB), 1u, (unsigned)d.NZ};
     const BatchGrid f8{(unsigned)((d.plane + BLK - 1) / BLK), 1u, (unsigned)d.NZ};
     const BatchGrid f3p{(unsigned)((d.plane / 2 + CB - 1) / CB), 1u, (unsigned)d.NZ};  // pairs of cells
-    const BatchGrid gb{(unsigned)x->nblk_b, 1u, 1u};
     for (int ph = 0; ph < 2; ++ph) {
       if (ph == 0 && !B.mixed) continue;
       BatchGrid *G = &grids[((size_t)ph * n + i) * BS_COUNT];
@@ -1960,10 +1980,8 @@ int fused_setup(FusedBatch &B, int32_t n, nim_ctx *const *ctx) {
         G[BS_P_SRC] = f3;
         G[BS_P_FACE] = f3;
       }
-      G[BS_P_BC] = gb;
-      G[BS_P_BC_COPY] = gb;
+      G[BS_WALLS] = BatchGrid{(unsigned)grid(d.NBF + 2 * d.plane), 1u, 1u};
       if (x->phys.dpdx_tolerance) G[BS_P_DPDX] = BatchGrid{(unsigned)x->nblk_c, 1u, 1u};
-      G[BS_ZERO_FLUX] = BatchGrid{(unsigned)grid(2 * d.plane), 1u, 1u};
       G[BS_T_CELL] = f3;
       G[BS_T_FACE] = f8;
       for (int q = 0; q < BS_COUNT; ++q) B.use[ph][q] = B.use[ph][q] || G[q].x > 0;

@@ -15,10 +15,8 @@
 //                (k_vel_face_tile on large meshes: the same sweep with its
 //                operands staged in shared memory by TMA boxes)
 //   k_p_src      calculate_R_b_p + calculate_R_D_p2           (-> Rp, dila)
-//   k_p_bc       apply_pressure_bc                            (cur -> next, walls)
-//   k_p_bc_copy  new wall values into cur
+//   k_walls      apply_pressure_bc and apply_zero_flux        (cur -> next, walls)
 //   k_p_face     integrate_pressure_field_i                   (cur -> next)
-//   k_zero_flux  apply_zero_flux                              (in place, cur)
 //   k_T_cell     calculate_temperature_nim_constants_formulation2 +
 //                calculate_R_D_T + cell-average update of T   (in place)
 //   k_T_face     +xi face updates of T                        (cur -> next)
@@ -1271,15 +1269,20 @@ __device__ __forceinline__ V face_update_vals(FX &&fx, FX2 &&fx2, V cx, V cx2, V
          (w / Fd[0]) * (+Fd[1] * fx(2 * dd - 1) + Fd[2] * fx2(2 * dd) + Fd[3] * (cx + ox) + Fd[4] * (cx2 + ox2) -
                         B3 - B4);
 }
-// the same from the arrays: faces fr, cells cv, old cells co
+// the same from the arrays: faces fr, cells cv, old cells co; z-wall faces
+// dN elements on (zwall)
+__device__ __forceinline__ int zwall(const Dims &d, const Cell &x, int pos, int dN) {
+  return (pos == 5 && x.k == 0) || (pos == 6 && x.k == d.NZ - 1) ? dN : 0;
+}
 template <class R>
 __device__ __forceinline__ Ar<R> face_update(const Dims &d, const R *__restrict__ fr, const R *__restrict__ cv,
                                              const R *__restrict__ co, const Ar<R> Fd[5], Kc<Ar<R>> dg0, Kc<Ar<R>> dg1,
-                                             int dd, const Cell &x, const Cell &x2, Kc<Ar<R>> w) {
-  return face_update_vals<Ar<R>>([&](int pos) -> Ar<R> { return fr[x.face(d, pos)]; },
-                                 [&](int pos) -> Ar<R> { return fr[x2.face(d, pos)]; }, (Ar<R>)cv[x.c], (Ar<R>)cv[x2.c],
-                                 (Ar<R>)co[x.c], (Ar<R>)co[x2.c], Fd, dg0, dg1, dd, w);
+                                             int dd, const Cell &x, const Cell &x2, Kc<Ar<R>> w, int dN = 0) {
+  return face_update_vals<Ar<R>>([&](int pos) -> Ar<R> { return fr[x.face(d, pos) + zwall(d, x, pos, dN)]; },
+                                 [&](int pos) -> Ar<R> { return fr[x2.face(d, pos) + zwall(d, x2, pos, dN)]; },
+                                 (Ar<R>)cv[x.c], (Ar<R>)cv[x2.c], (Ar<R>)co[x.c], (Ar<R>)co[x2.c], Fd, dg0, dg1, dd, w);
 }
+
 // Formulation 1 cell update of one velocity component (integrate_velocity_
 // field_i, nse.f90:341-352); Rs = R_C + R_D + R_B of the cell, at = a_t(1:9).
 template <class Ld = LdPlain, class R>
@@ -1368,7 +1371,7 @@ struct LaunchBlock {
 struct BatchBlock {
   unsigned x, y, z;
 };
-// A block of a fused batch launch over cells in cell order: x numbers the
+// A block of a launch over cells in cell order: x numbers the
 // runs of blockDim.x consecutive cells of plane z (y unused).  Every lane
 // has a cell whatever n_theta is, where the 32-wide theta patches of
 // patch_cell leave lanes idle on narrow meshes (n_theta = 40: 5 of 8 warps'
@@ -1376,6 +1379,61 @@ struct BatchBlock {
 struct FlatBlock {
   unsigned x, y, z;
 };
+// a launch's own blocks, over patches or (FLAT) in cell order: grid
+// (runs of a plane, 1, NZ)
+template <bool FLAT>
+__device__ __forceinline__ auto launch_block() {
+  if constexpr (FLAT)
+    return FlatBlock{::blockIdx.x, 0u, ::blockIdx.z};
+  else
+    return LaunchBlock{};
+}
+
+// What a pass kernel's body takes from the launch it runs in, and where its
+// change maxima go.  LaunchPass: the body is the launch.  It returns at once
+// when the step's loop has stopped, reads the parity itself, and the block's
+// maxima go to the control block.
+struct LaunchPass {
+  Ctrl *ctl;
+  int par, nh;
+  bool first;
+  __device__ __forceinline__ static BlockRed &shared() {
+    __shared__ BlockRed red;
+    return red;
+  }
+  // N maxima (0: the body has none); false: the loop has stopped
+  template <int N>
+  __device__ __forceinline__ bool begin(Ctrl *c) {
+    ctl = c;
+    if (c->done) return false;
+    if (N) red_init<N>(shared());
+    par = parity(c);
+    nh = newhalf(c);
+    first = c->first;
+    return true;
+  }
+  template <int NT, int N>
+  __device__ __forceinline__ void end(const double (&e)[N], int slot) {
+    block_max<N, NT>(shared(), e, ctl->err[par] + slot);
+  }
+};
+// a body inside another body: the outer one's parity, maxima of slots 3 and 4
+struct InPass {
+  int par, nh;
+  bool first;
+  double m[2];
+  template <int N>
+  __device__ __forceinline__ bool begin(Ctrl *) { return true; }
+  template <int NT, int N>
+  __device__ __forceinline__ void end(const double (&e)[N], int slot) { m[slot - 3] = e[0]; }
+};
+// one index per thread: a launch over blockDim.x-wide blocks, or given
+struct LinIndex {
+  int i;
+};
+template <class BI>
+__device__ __forceinline__ int lin_index(const BI b) { return b.x * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ int lin_index(const LinIndex b) { return b.i; }
 
 __device__ __forceinline__ double errv(double nw, double old, bool first) { return fabs(nw - (first ? 0.0 : old)); }
 __device__ __forceinline__ double errv(const DualD &nw, const DualD &old, bool first) {
@@ -1410,7 +1468,7 @@ __device__ __forceinline__ void group_cell(const Dims &d, const BI bi, int &i, i
 }
 template <int NP>
 __device__ __forceinline__ void group_cell(const Dims &d, const FlatBlock bi, int &i, int &j) {
-  const int t = (int)bi.x * CB + (int)threadIdx.x, per = d.NT / NP;  // group of plane z
+  const int t = (int)bi.x * (int)blockDim.x + (int)threadIdx.x, per = d.NT / NP;  // group of plane z
   j = t / per;
   i = NP * (t - j * per);
 }
@@ -1431,14 +1489,12 @@ __device__ __forceinline__ bool patch_cell(const Dims &d, Cell &x, const FlatBlo
 // FORM 1 (nim_formulation = 1): the a_t cell update of integrate_velocity_
 // field_i (nse.f90:341-378); the R sums are stored too, for the face sweep
 // reads them at both cells of a face.
-template <bool SRC_ONLY, int FORM, class R, class BI>
-__device__ __forceinline__ void vel_cell_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+template <bool SRC_ONLY, int FORM, class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void vel_cell_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
   using V = Ar<R>;
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<3>(red);
-  const int par = parity(ctl);
-  const bool first = ctl->first;
+  if (!ps.template begin<3>(ctl)) return;
+  const int par = ps.par;
+  const bool first = ps.first;
   const int q = threadIdx.y;
   Cell x;
   const bool act = patch_cell(d, x, blockIdx);
@@ -1475,11 +1531,11 @@ __device__ __forceinline__ void vel_cell_body(const Dims &d, const GeoOf<R> &g, 
     }
   }
   // blocks of one z plane: a plane another slab owns adds nothing
-  if (!SRC_ONLY && d.owns(blockIdx.z)) block_max<3, CB3>(red, e, ctl->err[par]);
+  if (!SRC_ONLY && d.owns(blockIdx.z)) ps.template end<CB3>(e, 0);
 }
-template <bool SRC_ONLY, int FORM, class R>
+template <bool SRC_ONLY, int FORM, bool FLAT = false, class R>
 __global__ void __launch_bounds__(CB3, minb<R>(3, 3)) k_vel_cell(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  vel_cell_body<SRC_ONLY, FORM, R>(d, g, F, P, ctl, LaunchBlock{});
+  vel_cell_body<SRC_ONLY, FORM, R>(d, g, F, P, ctl, launch_block<FLAT>());
 }
 
 // ---- K1, vectorised form (parallel schedule, formulation 2): k_vel_cell
@@ -1525,14 +1581,12 @@ __device__ __forceinline__ V tang_vals(bool lo, bool hi, V v0, V vp1, V vp2, V v
 // SLAB: a z-slab context, whose maxima skip the planes a neighbour owns (a
 // separate instantiation: at this kernel's register bound the test alone
 // costs spills)
-template <class R, bool SLAB = false, class BI = LaunchBlock>
-__device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+template <class R, bool SLAB = false, class BI = LaunchBlock, class PS = LaunchPass>
+__device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
   using V = Ar<R>;
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<3>(red);
-  const int par = parity(ctl);
-  const bool first = ctl->first;
+  if (!ps.template begin<3>(ctl)) return;
+  const int par = ps.par;
+  const bool first = ps.first;
   const int q = threadIdx.y;
   int i = blockIdx.x * 64 + 2 * (threadIdx.x & 31);
   int j = blockIdx.y * (CB / 32) + (threadIdx.x >> 5);
@@ -1729,11 +1783,11 @@ __device__ __forceinline__ void vel_cell2_body(const Dims &d, const GeoOf<R> &g,
     *reinterpret_cast<typename Pair2<R>::T *>(F.c[q] + c) = out;
     e[q] = nmax(errv(nw0, cv0, first), errv(nw1, cv1, first));
   }
-  if (!SLAB || d.owns(k)) block_max<3, CB3>(red, e, ctl->err[par]);
+  if (!SLAB || d.owns(k)) ps.template end<CB3>(e, 0);
 }
-template <class R, bool SLAB = false>
+template <class R, bool SLAB = false, bool FLAT = false>
 __global__ void __launch_bounds__(CB3, minb<R>(VC2_MINB, VC2_MINB_F)) k_vel_cell2(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  vel_cell2_body<R, SLAB>(d, g, F, P, ctl, LaunchBlock{});
+  vel_cell2_body<R, SLAB>(d, g, F, P, ctl, launch_block<FLAT>());
 }
 
 // ---- K1, NP cells per thread: k_vel_cell2's sweep over NP theta-adjacent
@@ -1775,7 +1829,7 @@ __device__ __forceinline__ void stN(R *__restrict__ p, int i, const R (&v)[NP]) 
   *reinterpret_cast<typename VecN<R, NP>::T *>(p + i) = t;
 }
 
-template <class R, int NP, bool SLAB = false>
+template <class R, int NP, bool SLAB = false, bool FLAT = false>
 __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   using V = Ar<R>;
   if (ctl->done) return;
@@ -1784,8 +1838,8 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoOf<R> g,
   const int par = parity(ctl);
   const bool first = ctl->first;
   const int q = threadIdx.y;
-  const int i = blockIdx.x * (32 * NP) + NP * (threadIdx.x & 31);
-  const int j = blockIdx.y * (CB / 32) + (threadIdx.x >> 5);
+  int i, j;
+  group_cell<NP>(d, launch_block<FLAT>(), i, j);
   const int k = blockIdx.z;
   double e[3] = {0., 0., 0.};
   if (i < d.NT && j < d.NR) {
@@ -1998,14 +2052,12 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoOf<R> g,
 
 // ---- K2: +xi face updates of u, v, w (nse.f90:878-1005).
 // Block (CB, 3): threadIdx.y = direction.
-template <class R, class BI>
-__device__ __forceinline__ void vel_face_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+template <class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void vel_face_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
   using V = Ar<R>;
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<3>(red);
-  const int par = parity(ctl);
-  const bool first = ctl->first;
+  if (!ps.template begin<3>(ctl)) return;
+  const int par = ps.par;
+  const bool first = ps.first;
   Cell x;
   const bool act = patch_cell(d, x, blockIdx);
   const int c = x.c;
@@ -2029,11 +2081,11 @@ __device__ __forceinline__ void vel_face_body(const Dims &d, const GeoOf<R> &g, 
       }
     });
   }
-  if (d.owns(blockIdx.z)) block_max<3, CB3>(red, e, ctl->err[par]);
+  if (d.owns(blockIdx.z)) ps.template end<CB3>(e, 0);
 }
-template <class R>
+template <bool FLAT = false, class R>
 __global__ void __launch_bounds__(CB3, minb<R>(3, 3)) k_vel_face(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  vel_face_body<R>(d, g, F, P, ctl, LaunchBlock{});
+  vel_face_body<R>(d, g, F, P, ctl, launch_block<FLAT>());
 }
 
 // ---- K2, z-marching form: the same face updates, one block per patch of
@@ -2527,14 +2579,14 @@ __global__ void __launch_bounds__(3 * CT_T, CT_MINB)
 // calculate_R_D_p2 1863-1997).  Block (CB, 3): thread y forms the gradient of
 // velocity component y and two of the six cross derivatives of p (y = 1 also
 // d(bz)/dz); thread 0 combines them in the reference's order.
-template <class R, class BI>
-__device__ __forceinline__ void p_src_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
-  if (ctl->done) return;
+template <class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void p_src_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
+  if (!ps.template begin<0>(ctl)) return;
   using A = Ar<R>;
   __shared__ A sh[3][3][CB];  // gradients of u, v, w
   __shared__ A sX[3][2][CB];  // cross derivatives of p
   __shared__ A sbz[CB];
-  const int par = parity(ctl);
+  const int par = ps.par;
   const int q = threadIdx.y, tx = threadIdx.x;
   Cell x;
   const bool active = patch_cell(d, x, blockIdx);
@@ -2547,7 +2599,7 @@ __device__ __forceinline__ void p_src_body(const Dims &d, const GeoOf<R> &g, con
     by_dir(threadIdx.y, [&](auto Q) {
       constexpr int q = decltype(Q)::value - 1;
       const Kc<A> invV = g.rvol[c];
-      const R *fq = F.f[q] + newhalf(ctl) * NF;
+      const R *fq = F.f[q] + ps.nh * NF;
       A vf[7];
       for (int k = 1; k <= 6; ++k) vf[k] = fq[f[k]];
 #pragma unroll
@@ -2588,9 +2640,9 @@ __device__ __forceinline__ void p_src_body(const Dims &d, const GeoOf<R> &g, con
     F.Rp[c] = RDp + RBp;
   }
 }
-template <class R>
+template <bool FLAT = false, class R>
 __global__ void __launch_bounds__(CB3, minb<R>(4, PSRC_MINB_F)) k_p_src(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  p_src_body<R>(d, g, F, P, ctl, LaunchBlock{});
+  p_src_body<R>(d, g, F, P, ctl, launch_block<FLAT>());
 }
 
 // ---- K3, NP cells per thread (the float mirror with NP = 4, the FP64 path
@@ -2600,14 +2652,14 @@ __global__ void __launch_bounds__(CB3, minb<R>(4, PSRC_MINB_F)) k_p_src(Dims d, 
 // gradients of velocity component y (y = 1 also d(bz)/dz) and two of the six
 // cross derivatives of p for the NP cells; thread 0 combines them in the
 // reference's order.  Each cell's arithmetic is k_p_src's.
-template <class R, int NP, class BI>
-__device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+template <class R, int NP, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
   using V = Ar<R>;
-  if (ctl->done) return;
+  if (!ps.template begin<0>(ctl)) return;
   __shared__ V sh[3][3][CB * NP];  // gradients of u, v, w
   __shared__ V sX[3][2][CB * NP];  // cross derivatives of p
   __shared__ V sbz[CB * NP];
-  const int par = parity(ctl);
+  const int par = ps.par;
   const int tx = threadIdx.x;
   int i, j;
   group_cell<NP>(d, blockIdx, i, j);
@@ -2662,7 +2714,7 @@ __device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoOf<R> &g, co
       for (int p = 0; p < NP; ++p) out[p] = invV[p] * out[p];
     };
     {
-      const R *fq = F.f[q] + newhalf(ctl) * NF;
+      const R *fq = F.f[q] + ps.nh * NF;
       R vf[7][NP];
 #pragma unroll
       for (int m = 1; m <= 6; ++m) faceN(fq, m, vf[m]);
@@ -2804,9 +2856,9 @@ __device__ __forceinline__ void p_srcN_body(const Dims &d, const GeoOf<R> &g, co
     stN<R, NP>(F.Rp, c, rp);
   }
 }
-template <class R, int NP>
+template <class R, int NP, bool FLAT = false>
 __global__ void __launch_bounds__(CB3, PSN_MINB) k_p_srcN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  p_srcN_body<R, NP>(d, g, F, P, ctl, LaunchBlock{});
+  p_srcN_body<R, NP>(d, g, F, P, ctl, launch_block<FLAT>());
 }
 
 // ---- apply_pressure_bc for wall face b (bc.f90:148-339).  p_bc_fixed: the
@@ -2864,14 +2916,14 @@ __device__ __forceinline__ Ar<R> p_bc_value(const Dims &d, const GeoOf<R> &g, co
 }
 
 // ---- K4: apply_pressure_bc, every wall face from the values before the pass
-template <class R, class BI>
-__device__ __forceinline__ void p_bc_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<1>(red);
-  const int par = parity(ctl), nh = newhalf(ctl);
-  const bool first = ctl->first;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+// (the current half) into the next half, which is where the rest of the pass
+// reads the walls (p_face_value; at +-(1 - 2 par) NF from the current half)
+template <class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void p_bc_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
+  if (!ps.template begin<1>(ctl)) return;
+  const int par = ps.par, nh = ps.nh;
+  const bool first = ps.first;
+  const int b = lin_index(blockIdx);
   double e[1] = {0.};
   if (b < d.NBF) {
     const int NF = d.NF;
@@ -2883,26 +2935,11 @@ __device__ __forceinline__ void p_bc_body(const Dims &d, const GeoOf<R> &g, cons
     F.f[3][(1 - par) * NF + fw0] = nw;
     e[0] = d.owns(B.cell.k) ? errv(nw, pr[fw0], first) : 0.;
   }
-  block_max<1>(red, e, ctl->err[par] + 3);
+  ps.template end<BLK>(e, 3);
 }
 template <class R>
 __global__ void __launch_bounds__(BLK) k_p_bc(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   p_bc_body<R>(d, g, F, P, ctl, LaunchBlock{});
-}
-
-template <class R, class BI>
-__device__ __forceinline__ void p_bc_copy_body(const Dims &d, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx) {
-  if (ctl->done) return;
-  const int par = parity(ctl);
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= d.NBF) return;
-  const BFace B = bface(d, b);
-  const int f = B.cell.face(d, B.pos);
-  F.f[3][par * d.NF + f] = F.f[3][(1 - par) * d.NF + f];
-}
-template <class R>
-__global__ void k_p_bc_copy(Dims d, FieldsT<R> F, Ctrl *ctl) {
-  p_bc_copy_body<R>(d, F, ctl, LaunchBlock{});
 }
 
 // (coefficient, face, cell) of the ten off-diagonal terms of the pressure
@@ -2989,10 +3026,11 @@ __device__ __forceinline__ PFaceCoef<Ar<R>> p_face_coef(const GeoT<R> &g, int Nc
 }
 
 // ---- integrate_pressure_field_i for the +xi_dd face of cell x
-// (nse.f90:1091-1289): the new value from the pressures pr
+// (nse.f90:1091-1289): the new value from the pressures pr, wall faces dN
+// elements on
 template <class Ld, class R>
 __device__ __forceinline__ Ar<R> p_face_value(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P,
-                                              const R *pr, const Cell &x, int dd) {
+                                              const R *pr, const Cell &x, int dd, int dN) {
   using V = Ar<R>;
   const int Nc = d.Nc, c = x.c;
   const Cell n2 = x.nb(d, 2 * dd);
@@ -3006,7 +3044,7 @@ __device__ __forceinline__ Ar<R> p_face_value(const Dims &d, const GeoOf<R> &g, 
   for (int t = 0; t < 10; ++t) {
     const int pt = p_term(dd, t), fpos = (pt >> 4) & 7, cell = pt >> 7;
     const Cell &cl = (cell == 1) ? x : n2;
-    const V term = K.at(dd, fpos, cell) * Ld::ld(pr, cl.face(d, fpos));
+    const V term = K.at(dd, fpos, cell) * Ld::ld(pr, cl.face(d, fpos) + (cl.has_nb(d, fpos) ? 0 : dN));
     s = (t == 0) ? -term : s - term;
   }
   const int fo = x.face(d, 2 * dd);
@@ -3079,13 +3117,11 @@ __global__ void __launch_bounds__(CB3, 2) k_vel1_face(Dims d, GeoOf<R> g, Fields
 
 // ---- K5: integrate_pressure_field_i, cur -> next.
 // Block (CB, 3): threadIdx.y = direction.
-template <class R, class BI>
-__device__ __forceinline__ void p_face_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<1>(red);
-  const int par = parity(ctl);
-  const bool first = ctl->first;
+template <class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void p_face_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
+  if (!ps.template begin<1>(ctl)) return;
+  const int par = ps.par;
+  const bool first = ps.first;
   Cell x;
   const bool act = patch_cell(d, x, blockIdx);
   double e[1] = {0.};
@@ -3095,17 +3131,17 @@ __device__ __forceinline__ void p_face_body(const Dims &d, const GeoOf<R> &g, co
       if (!x.has_nb(d, 2 * dd)) return;
       const size_t NF = d.NF;
       const R *pr = F.f[3] + par * NF;
-      const Ar<R> nw = stored<R>(p_face_value<LdPlain>(d, g, F, P, pr, x, dd));
+      const Ar<R> nw = stored<R>(p_face_value<LdPlain>(d, g, F, P, pr, x, dd, (1 - 2 * par) * d.NF));
       const int fo = x.face(d, 2 * dd);
       F.f[3][(1 - par) * NF + fo] = nw;
       e[0] = errv(nw, pr[fo], first);
     });
   }
-  if (d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 3);
+  if (d.owns(blockIdx.z)) ps.template end<CB3>(e, 3);
 }
-template <class R>
+template <bool FLAT = false, class R>
 __global__ void __launch_bounds__(CB3, minb<R>(5, PFACE_MINB_F)) k_p_face(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  p_face_body<R>(d, g, F, P, ctl, LaunchBlock{});
+  p_face_body<R>(d, g, F, P, ctl, launch_block<FLAT>());
 }
 
 // ---- K5, NP cells per thread (the float mirror with NP = 4, the FP64 path
@@ -3117,14 +3153,12 @@ __global__ void __launch_bounds__(CB3, minb<R>(5, PFACE_MINB_F)) k_p_face(Dims d
 // the metric differences; the theta faces' new values are stored one by one
 // (they start one cell off the vector boundary).  Each face's arithmetic is
 // p_face_value's.
-template <class R, int NP, class BI>
-__device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+template <class R, int NP, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
   using V = Ar<R>;
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<1>(red);
-  const int par = parity(ctl);
-  const bool first = ctl->first;
+  if (!ps.template begin<1>(ctl)) return;
+  const int par = ps.par;
+  const bool first = ps.first;
   int i, j;
   group_cell<NP>(d, blockIdx, i, j);
   const int k = blockIdx.z;
@@ -3136,12 +3170,13 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoOf<R> &g, c
     const int c = i + NT * (j + NR * k);
     const int im1 = (i == 0) ? NT - 1 : i - 1, ipn = (i + NP >= NT) ? i + NP - NT : i + NP;
     const R *pr = F.f[3] + par * NF;
+    const int dN = (1 - 2 * par) * NF;  // to the wall faces' new values
     // faces 1..6 of the NP cells starting at (i, jj, kk) (face 4: the +theta
     // face of cell p is the -theta face of cell p+1)
     auto group = [&](int jj, int kk, R (&v)[7][NP]) {
       const int cc = i + NT * (jj + NR * kk), ff = cc + NT * kk;
-      ldN<R, NP>(pr, ff, v[1]);
-      ldN<R, NP>(pr, ff + NT, v[2]);
+      ldN<R, NP>(pr, ff + (jj == 0 ? dN : 0), v[1]);
+      ldN<R, NP>(pr, ff + NT + (jj == NR - 1 ? dN : 0), v[2]);
       R t[NP];
       ldN<R, NP>(pr, d.offT + cc, t);
 #pragma unroll
@@ -3149,8 +3184,8 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoOf<R> &g, c
 #pragma unroll
       for (int p = 0; p + 1 < NP; ++p) v[4][p] = t[p + 1];
       v[4][NP - 1] = pr[d.offT + cc - i + ipn];
-      ldN<R, NP>(pr, d.offZ + cc, v[5]);
-      ldN<R, NP>(pr, d.offZ + cc + pl, v[6]);
+      ldN<R, NP>(pr, d.offZ + cc + (kk == 0 ? dN : 0), v[5]);
+      ldN<R, NP>(pr, d.offZ + cc + pl + (kk == d.NZ - 1 ? dN : 0), v[6]);
     };
     R ox[7][NP], on[7][NP];
     group(j, k, ox);
@@ -3171,11 +3206,11 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoOf<R> &g, c
       }
 #pragma unroll
       for (int p = 0; p < NP; ++p) on[3][p] = ox[4][p];
-      on[1][NP - 1] = pr[cw + NT * k];
-      on[2][NP - 1] = pr[cw + NT * k + NT];
+      on[1][NP - 1] = pr[cw + NT * k + (j == 0 ? dN : 0)];
+      on[2][NP - 1] = pr[cw + NT * k + NT + (j == NR - 1 ? dN : 0)];
       on[4][NP - 1] = pr[d.offT + cw - ipn + iw];
-      on[5][NP - 1] = pr[d.offZ + cw];
-      on[6][NP - 1] = pr[d.offZ + cw + pl];
+      on[5][NP - 1] = pr[d.offZ + cw + (k == 0 ? dN : 0)];
+      on[6][NP - 1] = pr[d.offZ + cw + pl + (k == d.NZ - 1 ? dN : 0)];
     }
     // the coefficients (p_face_coef) and the ten off-diagonal terms, in
     // source order
@@ -3336,28 +3371,26 @@ __device__ __forceinline__ void p_faceN_body(const Dims &d, const GeoOf<R> &g, c
       stN<R, NP>(dst, dd == 1 ? f1 + NT : d.offZ + c + pl, out);
     }
   });
-  if (d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 3);
+  if (d.owns(blockIdx.z)) ps.template end<CB3>(e, 3);
 }
-template <class R, int NP>
+template <class R, int NP, bool FLAT = false>
 __global__ void __launch_bounds__(CB3, PFN_MINB) k_p_faceN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  p_faceN_body<R, NP>(d, g, F, P, ctl, LaunchBlock{});
+  p_faceN_body<R, NP>(d, g, F, P, ctl, launch_block<FLAT>());
 }
 
 // ---- K5b (is_dpdx_tolerance): cell pressure gradients (nse.f90:292-307)
-template <class R, class BI>
-__device__ __forceinline__ void p_dpdx_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx) {
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<1>(red);
-  const int par = parity(ctl);
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+template <class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void p_dpdx_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
+  if (!ps.template begin<1>(ctl)) return;
+  const int par = ps.par;
+  const int c = lin_index(blockIdx);
   double e[1] = {0.};
   if (c < d.Nc) {
     const Cell x = Cell::of(d, c);
     const size_t Nc = d.Nc, NF = d.NF;
     int f[7];
     cell_faces(d, x, f);
-    const R *p = F.f[3] + newhalf(ctl) * NF;
+    const R *p = F.f[3] + ps.nh * NF;
     using V = Ar<R>;
     const V v[3] = {stored<R>((p[f[2]] - p[f[1]]) / Kc<V>(2.) * g.xi[0 * Nc + c]),
                     stored<R>((p[f[4]] - p[f[3]]) / Kc<V>(2.) * g.xi[4 * Nc + c]),
@@ -3367,40 +3400,56 @@ __device__ __forceinline__ void p_dpdx_body(const Dims &d, const GeoOf<R> &g, co
       F.dpd[q * Nc + c] = v[q];
     }
   }
-  block_max<1>(red, e, ctl->err[par] + 5);
+  ps.template end<BLK>(e, 5);
 }
 template <class R>
 __global__ void __launch_bounds__(BLK) k_p_dpdx(Dims d, GeoOf<R> g, FieldsT<R> F, Ctrl *ctl) {
   p_dpdx_body<R>(d, g, F, ctl, LaunchBlock{});
 }
 
-// ---- K6: apply_zero_flux (bc.f90:345-390) on the z walls, in place
-template <class R, class BI>
-__device__ __forceinline__ void zero_flux_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx) {
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<1>(red);
-  const int par = parity(ctl);
-  const bool first = ctl->first;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+// ---- K6: apply_zero_flux (bc.f90:345-390) on the z walls, into the next half
+// (the rest of the pass reads the z walls there; one half: in place)
+template <class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void zero_flux_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
+  if (!ps.template begin<1>(ctl)) return;
+  const int par = ps.par, nh = ps.nh;
+  const bool first = ps.first;
+  const int b = lin_index(blockIdx);
   double e[1] = {0.};
   if (b < 2 * d.plane) {
     const int NF = d.NF, NB = d.NBF;
     const BFace B = bface(d, b);
     const int in = (B.pos == 5) ? 6 : 5;
     const Cell c2 = B.cell.nb(d, in), c3 = c2.nb(d, in);
-    R *T = F.f[4] + par * NF;
+    const R *T = F.f[4] + par * NF;
     const int f1 = B.cell.face(d, B.pos);
     const Ar<R> nw = stored<R>((+g.zf[NB + b] * T[B.cell.face(d, in)] - g.zf[2 * NB + b] * T[c2.face(d, in)] +
                                 g.zf[3 * NB + b] * T[c3.face(d, in)]) / g.zf[b]);
     e[0] = d.owns(B.cell.k) ? errv(nw, T[f1], first) : 0.;
-    T[f1] = nw;
+    F.f[4][nh * NF + f1] = nw;
   }
-  block_max<1>(red, e, ctl->err[par] + 4);
+  ps.template end<BLK>(e, 4);
 }
 template <class R>
 __global__ void __launch_bounds__(BLK) k_zero_flux(Dims d, GeoOf<R> g, FieldsT<R> F, Ctrl *ctl) {
   zero_flux_body<R>(d, g, F, ctl, LaunchBlock{});
+}
+
+// ---- K4 + K6 in one launch: neither reads what the other writes
+template <class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void walls_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
+  if (!ps.template begin<2>(ctl)) return;
+  const int i = lin_index(blockIdx);
+  InPass in{ps.par, ps.nh, ps.first, {0., 0.}};
+  if (i < d.NBF)
+    p_bc_body<R>(d, g, F, P, ctl, LinIndex{i}, in);
+  else
+    zero_flux_body<R>(d, g, F, ctl, LinIndex{i - d.NBF}, in);
+  ps.template end<BLK>(in.m, 3);
+}
+template <class R>
+__global__ void __launch_bounds__(BLK) k_walls(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
+  walls_body<R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
 // ---- K7: calculate_temperature_nim_constants_formulation2 (nim.f90:334-500)
@@ -3529,17 +3578,15 @@ __global__ void __launch_bounds__(BLK, 4) k_T_coef(Dims d, GeoOf<R> g, FieldsT<R
 // MT_A (18 words) and MT_F (15) written and read through memory by a kernel
 // of their own it was 952.  128x128x96: FP64 T_coef + T_cell 305 -> 289 us,
 // float (k_T_cellN) 128 -> 91 us, and k_T_faceN 51 -> 45 us.
-template <class R, class BI>
-__device__ __forceinline__ void T_cell_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+template <class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void T_cell_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
   using V = Ar<R>;
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<1>(red);
+  if (!ps.template begin<1>(ctl)) return;
   __shared__ V sX[3][2][CB];   // cross derivatives
   __shared__ V sF[3][3][CB];   // r, m, p of MT_F4 by direction
   __shared__ V sG[CB];         // G1 dT/dx + G2 dT/dy + G3 dT/dz, by thread 2
-  const int par = parity(ctl);
-  const bool first = ctl->first;
+  const int par = ps.par;
+  const bool first = ps.first;
   const int tx = threadIdx.x;
   Cell x;
   const bool active = patch_cell(d, x, blockIdx);
@@ -3547,8 +3594,12 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoOf<R> &g, co
   double e[1] = {0.};
   const int Nc = d.Nc, NF = d.NF;
   const R *T = F.f[4] + par * NF;
+  // the z walls' new values, dN elements on
+  const int dN = (ps.nh - par) * NF, d5 = zwall(d, x, 5, dN), d6 = zwall(d, x, 6, dN);
   int f[7];
   cell_faces(d, x, f);
+  f[5] += d5;
+  f[6] += d6;
   if (active) by_dir(threadIdx.y, [&](auto D) {
     constexpr int dd = decltype(D)::value, y = dd - 1;
     {
@@ -3567,7 +3618,7 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoOf<R> &g, co
     constexpr int fa = (y == 1) ? 4 : 2, fb = (y == 1) ? 3 : 1;
     sX[y][0][tx] = Kc<V>(0.5) * (tangential(d, T, x, (y == 2) ? 2 : fa, e2) - tangential(d, T, x, (y == 2) ? 1 : fb, e2));
     sX[y][1][tx] = (y == 2) ? Kc<V>(0.5) * (tangential(d, T, x, 4, 3) - tangential(d, T, x, 3, 3))
-                            : Kc<V>(0.5) * (tangential(d, T, x, 6, e2) - tangential(d, T, x, 5, e2));
+                            : Kc<V>(0.5) * (tangential(d, T + d6, x, 6, e2) - tangential(d, T + d5, x, 5, e2));
     if (y == 2) {  // the leading G_i d_i T terms of R_D_T, in source order
       const V px = (T[f[2]] - T[f[1]]) / Kc<V>(2.);
       const V py = (T[f[4]] - T[f[3]]) / Kc<V>(2.);
@@ -3594,11 +3645,11 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoOf<R> &g, co
     F.c[3][c] = nw;
     e[0] = errv(nw, cold, first);
   }
-  if (d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 4);
+  if (d.owns(blockIdx.z)) ps.template end<CB3>(e, 4);
 }
-template <class R>
+template <bool FLAT = false, class R>
 __global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) k_T_cell(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  T_cell_body<R>(d, g, F, P, ctl, LaunchBlock{});
+  T_cell_body<R>(d, g, F, P, ctl, launch_block<FLAT>());
 }
 
 // ---- K7b, NP cells per thread (the float mirror's parallel passes,
@@ -3607,7 +3658,7 @@ __global__ void __launch_bounds__(CB3, minb<R>(TCELL_MINB, TCELL_MINB_F)) k_T_ce
 // constants of direction y+1 and two of the six cross derivatives of T;
 // thread 2 also the G_i d_i T prefix; thread 0 assembles MT_F4, R_D_T and
 // the cell update.  Each cell's arithmetic is k_T_cell's.
-template <class R, int NP>
+template <class R, int NP, bool FLAT = false>
 __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   using V = Ar<R>;
   if (ctl->done) return;
@@ -3619,15 +3670,17 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoOf<R> g, F
   const int par = parity(ctl);
   const bool first = ctl->first;
   const int tx = threadIdx.x;
-  const int i = blockIdx.x * (32 * NP) + NP * (tx & 31);
-  const int j = blockIdx.y * (CB / 32) + (tx >> 5);
+  int i, j;
+  group_cell<NP>(d, launch_block<FLAT>(), i, j);
   const int k = blockIdx.z;
   const bool active = i < d.NT && j < d.NR;
   const int Nc = d.Nc, NF = d.NF, NT = d.NT, NR = d.NR, pl = d.plane;
   const int c = i + NT * (j + NR * k);
   const int im1 = (i == 0) ? NT - 1 : i - 1, ipn = (i + NP >= NT) ? i + NP - NT : i + NP;
   const int f1 = c + NT * k;
-  const int fi[7] = {0, f1, f1 + NT, d.offT + c, d.offT + c + 1, d.offZ + c, d.offZ + c + pl};
+  const int dN = (1 - 2 * par) * NF;  // to the z walls' new values
+  const int d5 = k == 0 ? dN : 0, d6 = k == d.NZ - 1 ? dN : 0;
+  const int fi[7] = {0, f1, f1 + NT, d.offT + c, d.offT + c + 1, d.offZ + c + d5, d.offZ + c + pl + d6};
   const int f4b = d.offT + c - i + ipn;
   auto faceN = [&](const R *a, int m, R (&v)[NP]) {
     if (m == 4) {
@@ -3695,7 +3748,8 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoOf<R> g, F
     if (y == 0) {
       const int rrow = NT * (j + (NR + 1) * k), zlev = d.offZ + NT * (j + NR * k);
       const V r_m1 = T[rrow + im1], r_pn = T[rrow + ipn], r1_m1 = T[rrow + NT + im1], r1_pn = T[rrow + NT + ipn];
-      const V z_m1 = T[zlev + im1], z_pn = T[zlev + ipn], z1_m1 = T[zlev + pl + im1], z1_pn = T[zlev + pl + ipn];
+      const V z_m1 = T[zlev + d5 + im1], z_pn = T[zlev + d5 + ipn];
+      const V z1_m1 = T[zlev + pl + d6 + im1], z1_pn = T[zlev + pl + d6 + ipn];
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         const V up2 = (p + 1 < NP) ? (V)o[2][p + 1] : r1_pn, um2 = (p > 0) ? (V)o[2][p - 1] : r1_m1;
@@ -3721,10 +3775,10 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoOf<R> g, F
         bv[NP] = T[trb + ipn];
       }
       R za[NP], zb[NP], zA[NP], zB[NP];
-      ldN<R, NP>(T, zra + i, za);
-      ldN<R, NP>(T, zrb + i, zb);
-      ldN<R, NP>(T, zra + pl + i, zA);
-      ldN<R, NP>(T, zrb + pl + i, zB);
+      ldN<R, NP>(T, zra + d5 + i, za);
+      ldN<R, NP>(T, zrb + d5 + i, zb);
+      ldN<R, NP>(T, zra + pl + d6 + i, zA);
+      ldN<R, NP>(T, zrb + pl + d6 + i, zB);
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         sX[1][0][tx * NP + p] =
@@ -3811,16 +3865,14 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoOf<R> g, F
   if (d.owns(blockIdx.z)) block_max<1, CB3>(red, e, ctl->err[par] + 4);
 }
 
-// ---- K8: +xi face updates of T (nse.f90:1033-1088), cur -> next; the z-wall
-// values set by apply_zero_flux travel to the next half too
-template <class R, class BI>
-__device__ __forceinline__ void T_face_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx) {
+// ---- K8: +xi face updates of T (nse.f90:1033-1088), cur -> next (the z walls
+// read, and staying, in the next half)
+template <class R, class BI, class PS = LaunchPass>
+__device__ __forceinline__ void T_face_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
   using V = Ar<R>;
-  if (ctl->done) return;
-  __shared__ BlockRed red;
-  red_init<1>(red);
-  const int par = parity(ctl);
-  const bool first = ctl->first;
+  if (!ps.template begin<1>(ctl)) return;
+  const int par = ps.par;
+  const bool first = ps.first;
   Cell x;
   const bool act = patch_cell(d, x, blockIdx);
   const int c = x.c;
@@ -3836,18 +3888,17 @@ __device__ __forceinline__ void T_face_body(const Dims &d, const GeoOf<R> &g, co
       T_form_Fd(F, Nc, c, x2.c, dd, Fd);
       const int fo = x.face(d, 2 * dd);
       const V nw = stored<R>(face_update(d, T, F.c[3], F.co[3], Fd, g.dg[(2 * (dd - 1)) * Nc + c],
-                                              g.dg[(2 * (dd - 1) + 1) * Nc + c], dd, x, x2, Kc<V>(P.w[3])));
+                                              g.dg[(2 * (dd - 1) + 1) * Nc + c], dd, x, x2, Kc<V>(P.w[3]),
+                                              (1 - 2 * par) * NF));
       Tn[fo] = nw;
       e[0] = nmax(e[0], errv(nw, T[fo], first));
     }
-    if (x.k == 0) Tn[x.face(d, 5)] = T[x.face(d, 5)];
-    if (x.k == d.NZ - 1) Tn[x.face(d, 6)] = T[x.face(d, 6)];
   }
-  if (d.owns(blockIdx.z)) block_max<1>(red, e, ctl->err[par] + 4);
+  if (d.owns(blockIdx.z)) ps.template end<BLK>(e, 4);
 }
-template <class R>
+template <bool FLAT = false, class R>
 __global__ void __launch_bounds__(BLK, minb<R>(4, TFACE_MINB_F)) k_T_face(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  T_face_body<R>(d, g, F, P, ctl, LaunchBlock{});
+  T_face_body<R>(d, g, F, P, ctl, launch_block<FLAT>());
 }
 
 // The +xi_dd face updates of one field (faces fr of the current half, new
@@ -3942,9 +3993,9 @@ __device__ __forceinline__ double face_updateN(const Dims &d, int i, int j, int 
 // ---- K8, NP cells per thread (the float mirror, n_theta % NP == 0):
 // k_T_face over NP theta-adjacent cells, block (CB, 3): thread y updates the
 // +xi face of direction y+1 of the NP cells from NP-wide vector loads (the
-// +theta neighbours as k_p_faceN forms them) and carries the z-wall values
-// to the next half (thread 2).  Each face's arithmetic is face_update's.
-template <class R, int NP>
+// +theta neighbours as k_p_faceN forms them).  Each face's arithmetic is
+// face_update's.
+template <class R, int NP, bool FLAT = false>
 __global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   using V = Ar<R>;
   if (ctl->done) return;
@@ -3953,8 +4004,8 @@ __global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoOf<R> g, F
   const int par = parity(ctl);
   const bool first = ctl->first;
   const int tx = threadIdx.x;
-  const int i = blockIdx.x * (32 * NP) + NP * (tx & 31);
-  const int j = blockIdx.y * (CB / 32) + (tx >> 5);
+  int i, j;
+  group_cell<NP>(d, launch_block<FLAT>(), i, j);
   const int k = blockIdx.z;
   double e[1] = {0.};
   if (i < d.NT && j < d.NR) by_dir(threadIdx.y, [&](auto D) {
@@ -3964,17 +4015,7 @@ __global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoOf<R> g, F
     const int ipn = (i + NP >= NT) ? i + NP - NT : i + NP;
     const R *T = F.f[4] + par * NF;
     R *Tn = F.f[4] + (1 - par) * NF;
-    if (dd == 3) {  // the z-wall values set by apply_zero_flux travel to the next half
-      R t[NP];
-      if (k == 0) {
-        ldN<R, NP>(T, d.offZ + c, t);
-        stN<R, NP>(Tn, d.offZ + c, t);
-      }
-      if (k == d.NZ - 1) {
-        ldN<R, NP>(T, d.offZ + c + pl, t);
-        stN<R, NP>(Tn, d.offZ + c + pl, t);
-      }
-    }
+    const int dN = (1 - 2 * par) * NF;  // to the z walls' new values
     if ((dd == 1 && j == NR - 1) || (dd == 3 && k == d.NZ - 1)) return;  // a wall face
     auto group = [&](int jj, int kk, R (&v)[7][NP]) {
       const int cc = i + NT * (jj + NR * kk), ff = cc + NT * kk;
@@ -3987,8 +4028,8 @@ __global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoOf<R> g, F
 #pragma unroll
       for (int p = 0; p + 1 < NP; ++p) v[4][p] = t[p + 1];
       v[4][NP - 1] = T[d.offT + cc - i + ipn];
-      ldN<R, NP>(T, d.offZ + cc, v[5]);
-      ldN<R, NP>(T, d.offZ + cc + pl, v[6]);
+      ldN<R, NP>(T, d.offZ + cc + (kk == 0 ? dN : 0), v[5]);
+      ldN<R, NP>(T, d.offZ + cc + pl + (kk == d.NZ - 1 ? dN : 0), v[6]);
     };
     R ox[7][NP], on[7][NP], cx[NP], cxo[NP], cn[NP], cno[NP];
     group(j, k, ox);
@@ -4019,8 +4060,8 @@ __global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoOf<R> g, F
       on[1][NP - 1] = T[cw + NT * k];
       on[2][NP - 1] = T[cw + NT * k + NT];
       on[4][NP - 1] = T[d.offT + cw - ipn + iw];
-      on[5][NP - 1] = T[d.offZ + cw];
-      on[6][NP - 1] = T[d.offZ + cw + pl];
+      on[5][NP - 1] = T[d.offZ + cw + (k == 0 ? dN : 0)];
+      on[6][NP - 1] = T[d.offZ + cw + pl + (k == d.NZ - 1 ? dN : 0)];
       cn[NP - 1] = F.c[3][cw];
       cno[NP - 1] = F.co[3][cw];
     }
@@ -4079,7 +4120,7 @@ __global__ void __launch_bounds__(CB3, TFN_MINB) k_T_faceN(Dims d, GeoOf<R> g, F
 // +xi face updates of u, v, w (nse.f90:878-1005) over NP theta-adjacent
 // cells, block (CB, 3): thread y updates the +xi face of direction y+1 of
 // the NP cells for each component (face_updateN), as k_vel_face.
-template <class R, int NP>
+template <class R, int NP, bool FLAT = false>
 __global__ void __launch_bounds__(CB3, VFN_MINB) k_vel_faceN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   if (ctl->done) return;
   __shared__ BlockRed red;
@@ -4087,8 +4128,8 @@ __global__ void __launch_bounds__(CB3, VFN_MINB) k_vel_faceN(Dims d, GeoOf<R> g,
   const int par = parity(ctl);
   const bool first = ctl->first;
   const int tx = threadIdx.x;
-  const int i = blockIdx.x * (32 * NP) + NP * (tx & 31);
-  const int j = blockIdx.y * (CB / 32) + (tx >> 5);
+  int i, j;
+  group_cell<NP>(d, launch_block<FLAT>(), i, j);
   const int k = blockIdx.z;
   double e[3] = {0., 0., 0.};
   if (i < d.NT && j < d.NR) by_dir(threadIdx.y, [&](auto D) {
