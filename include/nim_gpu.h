@@ -205,7 +205,10 @@ void nim_params_reference(nim_params *p);
    cell pairs with paired loads when n_theta is even, else one cell per
    thread; NIM_CELL_SWEEP=gather forces the one-cell form, =tile a
    TMA-staged form under the face sweep's n_theta conditions (not faster at
-   the benchmark sizes, so off by default).  All forms give identical
+   the benchmark sizes, so off by default).  The inner loop of a small mesh
+   (formulation 2, parallel schedule) runs as one cooperative launch instead
+   of a graph of launches; NIM_PASS_LOOP=on or =off overrides, and naming a
+   form of a sweep as above asks for launches.  All forms give identical
    results. */
 int nim_gpu_create(const nim_mesh_desc *mesh, const nim_params *params,
                    nim_ctx **out);

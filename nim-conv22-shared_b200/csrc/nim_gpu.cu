@@ -122,6 +122,12 @@ struct nim_ctx {
   bool face_quad = false;  // and its face sweep of u, v, w as k_vel_faceN
   bool press_pair = false; // the FP64 pressure sweeps two cells a thread (k_p_srcN, k_p_faceN)
   VelCellMaps cmap64{}, cmap32{};
+  // k_pass_loop: a small mesh's inner loop as one cooperative launch, block
+  // (loop_bx, 3); off while the context advances in a batch (the enclosures
+  // share the GPU)
+  bool loop = false, in_batch = false, loop_pair = false;
+  int loop_bx = 0, loop_blocks = 0;
+  unsigned *loop_bar = nullptr;
   GeoT<float> g32{};
   FieldsT<float> F32{};
   cudaGraphExec_t graph32 = nullptr;
@@ -542,6 +548,65 @@ int launch_parallel(nim_ctx *x, const GeoOf<R> &g, const FieldsT<R> &F, int lowp
 int launch_iteration(nim_ctx *x, bool lowp = false, bool stall_rule = true) {
   if (x->seq) return launch_iteration_seq(x);
   return lowp ? launch_parallel(x, x->g32, x->F32, stall_rule ? 1 : 0) : launch_parallel(x, x->g, x->F, 0);
+}
+
+// up to kLoopPasses passes in one cooperative launch (k_pass_loop)
+constexpr int kLoopPasses = 256;
+constexpr int kLoopCells = 120000, kLoopCellsFlat = 400000;  // most cells of the loop form
+template <class R>
+const void *pass_loop_kernel(bool pair) {
+  return pair ? (const void *)k_pass_loop<R, true> : (const void *)k_pass_loop<R, false>;
+}
+template <class R>
+int launch_loop(nim_ctx *x, GeoT<R> g, FieldsT<R> F, int lowp) {
+  int passes = kLoopPasses;
+  void *args[] = {&x->d, &g, &F, &x->phys, &x->ctl, &x->loop_bar, &passes, &lowp};
+  CK(cudaMemsetAsync(x->loop_bar, 0, sizeof(unsigned), x->stream));
+  CK(cudaLaunchCooperativeKernel(pass_loop_kernel<R>(x->loop_pair), dim3(x->loop_blocks), dim3(x->loop_bx, 3), args, 0,
+                                 x->stream));
+  x->launches += 1;
+  return NIM_OK;
+}
+// Whether the loop form runs (k_pass_loop has both sides' times: up to
+// kLoopCells cells, and further where the launches' sweeps run in cell order
+// too, which costs them what the loop pays anyway), and its blocks: the
+// narrowest block (32, 64 or 128 cells by 3) whose grid over the widest part
+// is resident at once, so that the work spreads over as many SMs as there
+// are, else 128.  NIM_PASS_LOOP=on or =off in the environment overrides;
+// naming a form of a sweep (NIM_CELL_SWEEP, NIM_FACE_SWEEP) asks for launches.
+int choose_loop(nim_ctx *x) {
+  auto env = [](const char *n) {
+    const char *v = std::getenv(n);
+    return std::string(v ? v : "");
+  };
+  const std::string force = env("NIM_PASS_LOOP");
+  const Dims &d = x->d;
+  const int most = !x->mixed && (x->flat1 || x->flat2) ? kLoopCellsFlat : kLoopCells;
+  x->loop = !x->seq && x->phys.formulation == 2 && !x->slab_count && !x->cell_tile && force != "off" &&
+            (force == "on" || (d.Nc <= most && env("NIM_CELL_SWEEP").empty() && env("NIM_FACE_SWEEP").empty()));
+  if (!x->loop) return NIM_OK;
+  int sms = 0, coop = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, x->device));
+  CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, x->device));
+  auto items = [&](int bx) { return ((d.plane + bx - 1) / bx) * d.NZ; };
+  for (int bx = 32; bx <= CB; bx *= 2) {
+    int per = 1 << 20;
+    for (int form = 0; form < 4; ++form) {  // precision, pair: one choice for both
+      if (!x->mixed && form >= 2) break;
+      int nb = 0;
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+          &nb, form >= 2 ? pass_loop_kernel<float>(form & 1) : pass_loop_kernel<double>(form & 1), 3 * bx, 0));
+      per = std::min(per, nb);
+    }
+    x->loop_bx = bx;
+    x->loop_blocks = std::min(items(bx), per * sms);
+    if (items(bx) <= per * sms) break;
+  }
+  // two cells a thread in the velocity cell sweep once one cell a thread
+  // would take several turns
+  x->loop_pair = x->cell_pair && items(x->loop_bx) > x->loop_blocks;
+  if (!coop || x->loop_blocks < 1) x->loop = false;
+  return NIM_OK;
 }
 
 int build_graph(nim_ctx *x, int iters, bool lowp = false) {
@@ -1258,6 +1323,7 @@ static int create_impl(const nim_mesh_desc *m, const nim_params *p, nim_ctx *x, 
   }
   TRY(dalloc(x, &F.part, 8 * (size_t)std::max(x->nblk_c, grid(2 * d.NT * d.NZ))));
   TRY(dalloc(x, &x->ctl, 1));
+  TRY(dalloc(x, &x->loop_bar, 1));
   TRY(dalloc(x, &x->node_xyz, 3 * (size_t)nnode));
   TRY(dalloc(x, &x->bcv, 25));
   TRY(dalloc(x, &x->perm, NF));
@@ -1289,6 +1355,7 @@ static int create_impl(const nim_mesh_desc *m, const nim_params *p, nim_ctx *x, 
     }
   }
   if (x->seq) TRY(setup_levels(x));
+  TRY(choose_loop(x));
   CK(cudaMemcpyAsync(x->node_xyz, node_xyz, 3 * sizeof(double) * nnode, cudaMemcpyHostToDevice, x->stream));
   double bcv[25];
   for (int f = 0; f < 5; ++f)
@@ -1440,6 +1507,11 @@ int ctrl_async(nim_ctx *x) {
 
 int iterations_launch(nim_ctx *x, int batches) {
   const int G = x->graph_G;
+  if (x->loop && !x->in_batch) {
+    TRY(x->phase == 1 ? launch_loop<float>(x, x->g32, x->F32, 1) : launch_loop<double>(x, x->g, x->F, 0));
+    x->run.launched += kLoopPasses;
+    return ctrl_async(x);
+  }
   if (x->seq) {
     for (int k = 0; k < batches * G; ++k) TRY(launch_iteration(x));
   } else {
@@ -1466,8 +1538,9 @@ int after_loop_start(nim_ctx *x) {
 // integrate_nse, first batch: launch ahead by the previous step's count
 int integrate_start(nim_ctx *x) {
   const int G = x->graph_G;
-  if (!x->seq && (!x->graph || x->graph_iters != G)) TRY(build_graph(x, G));
-  if (x->mixed && (!x->graph32 || x->graph32_iters != G)) TRY(build_graph(x, G, true));
+  const bool graphs = !x->seq && (!x->loop || x->in_batch);
+  if (graphs && (!x->graph || x->graph_iters != G)) TRY(build_graph(x, G));
+  if (graphs && x->mixed && (!x->graph32 || x->graph32_iters != G)) TRY(build_graph(x, G, true));
   // with max_iters <= 0 the device never stops on its own; bound the host loop
   x->run.cap = (x->params.max_iters > 0) ? (long long)x->params.max_iters + 2 * G : 100000000LL;
   x->run.launched = 0;
@@ -1632,6 +1705,19 @@ extern "C" int nim_gpu_step(nim_ctx *x, int32_t nsteps, nim_step_stats *per, int
 // context's stream fed, polling their events instead of waiting on any, so
 // the kernels of all instances share the GPU.  Per instance the calls and
 // their order are exactly nim_gpu_step's.
+namespace {
+// while several contexts share the GPU, none takes all of it (k_pass_loop)
+struct InBatch {
+  int n;
+  nim_ctx *const *ctx;
+  InBatch(int n_, nim_ctx *const *c) : n(n_), ctx(c) {
+    for (int i = 0; i < n; ++i) ctx[i]->in_batch = n > 1;
+  }
+  ~InBatch() {
+    for (int i = 0; i < n; ++i) ctx[i]->in_batch = false;
+  }
+};
+}  // namespace
 extern "C" int nim_batch_step(int32_t n, nim_ctx *const *ctx, int32_t nsteps, nim_step_stats *per, int32_t *done) {
   if (n <= 0 || !ctx || nsteps < 0) return NIM_ERR_BAD_ARG;
   for (int32_t i = 0; i < n; ++i) {
@@ -1644,6 +1730,7 @@ extern "C" int nim_batch_step(int32_t n, nim_ctx *const *ctx, int32_t nsteps, ni
   if (done)
     for (int32_t i = 0; i < n; ++i) done[i] = 0;
   if (nsteps == 0) return NIM_OK;
+  const InBatch share(n, ctx);
   CK(cudaSetDevice(ctx[0]->device));
   enum { ITER, AFTER, END, FINISHED };
   std::vector<int> phase(n, ITER), k(n, 0);

@@ -185,6 +185,7 @@ struct Ctrl {
 constexpr int kLowpStall = 8;
 
 constexpr int BLK = 256;
+constexpr int LOOP_MINB = 2;  // resident blocks per SM of k_pass_loop at its widest (384 threads, 80 registers)
 // most threads of a reference-order sweep in one block: 256 keep a cell's
 // values in registers (255 a thread), 512 (128 a thread) serve wider levels
 constexpr int SEQ_TPB = 256, SEQ_TPB_WIDE = 512;
@@ -1392,7 +1393,9 @@ __device__ __forceinline__ auto launch_block() {
 // What a pass kernel's body takes from the launch it runs in, and where its
 // change maxima go.  LaunchPass: the body is the launch.  It returns at once
 // when the step's loop has stopped, reads the parity itself, and the block's
-// maxima go to the control block.
+// maxima go to the control block.  LoopPass (k_pass_loop): the body is a
+// phase of a persistent loop, which holds the parity and keeps each thread's
+// maxima to the end of the pass.
 struct LaunchPass {
   Ctrl *ctl;
   int par, nh;
@@ -1416,6 +1419,16 @@ struct LaunchPass {
   __device__ __forceinline__ void end(const double (&e)[N], int slot) {
     block_max<N, NT>(shared(), e, ctl->err[par] + slot);
   }
+};
+struct LoopPass {
+  Ctrl *ctl;
+  int par, nh;
+  bool first;
+  double m[6];  // u, v, w, p, T, dpdx
+  template <int N>
+  __device__ __forceinline__ bool begin(Ctrl *) { return true; }
+  template <int NT, int N>
+  __device__ __forceinline__ void end(const double (&e)[N], int slot);
 };
 // a body inside another body: the outer one's parity, maxima of slots 3 and 4
 struct InPass {
@@ -1441,6 +1454,12 @@ __device__ __forceinline__ double errv(const DualD &nw, const DualD &old, bool f
 }
 // max that keeps a NaN (fmax would drop it and hide a blow-up)
 __device__ __forceinline__ double nmax(double a, double b) { return (b > a || b != b) ? b : a; }
+
+template <int NT, int N>
+__device__ __forceinline__ void LoopPass::end(const double (&e)[N], int slot) {
+#pragma unroll
+  for (int n = 0; n < N; ++n) m[slot + n] = nmax(m[slot + n], e[n]);
+}
 
 // Cell of this thread in a 3D launch over patches of 32 (theta) x R (r)
 // cells of one z-plane: grid (ceil(NT/32), ceil(NR/R), NZ), threadIdx.x
@@ -4221,6 +4240,167 @@ __device__ __forceinline__ void iter_end_body(Ctrl *ctl, const Phys &P, int lowp
 }
 __global__ void k_iter_end(Ctrl *ctl, Phys P, int lowp) {
   iter_end_body(ctl, P, lowp, LaunchBlock{});
+}
+
+// ---- The inner loop of a small mesh as one cooperative launch: passes until
+// the stop test holds (at most `passes`), with a grid barrier between the
+// parts of a pass instead of a launch.  On small meshes a pass is a chain of
+// ten launches of a few microseconds each (launch, parity and stop flag,
+// loads, a block's maxima); here it is five barriers: sweeps that read nothing
+// of each other's share a part, and the maxima are folded once a pass.  The parts run the plain kernels' bodies over runs of consecutive
+// cells (FlatBlock), so the results are theirs to the bit.
+//
+// Block (BX, 3), BX = 32, 64 or 128 cells (host: choose_loop), all blocks
+// resident (a cooperative launch).  What one part writes, other SMs read in
+// the next: every block adds to a counter in memory (release) and polls it
+// (then acquires), so every later load sees it (no load here takes the
+// non-coherent path: the arrays are written in this launch).  Hardware
+// barriers of one 16-block cluster were slower from the smallest mesh on (40
+// against 31 us a pass at 36x6x12): sixteen SMs are too few for the parts.
+//
+// Time of a pass as launches of a graph and as this loop: 36x6x12 43 -> 31
+// us, 45x37x29 60 -> 51, 48x48x32 76 -> 70 (mixed 50 -> 45), 64x64x48 152 ->
+// 155, 72x72x54 220 -> 208, 80x80x60 292 -> 276, 96x96x64 390 -> 412, where
+// the two-cell pressure sweeps and whole-warp patches of the launches win.
+constexpr int kBarTries = 1 << 22;  // polls of a barrier before the step ends with NIM_ERR_TIMEOUT
+struct LoopBarrier {
+  unsigned *count;   // arrivals since the launch (zeroed before it)
+  unsigned target;   // arrivals that complete the next barrier
+  __device__ __forceinline__ explicit LoopBarrier(unsigned *c) : count(c), target(gridDim.x) {}
+  // false: the wait ran out (every block leaves, the step has timed out)
+  __device__ __forceinline__ bool sync(Ctrl *ctl) {
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+      unsigned seen;
+      asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(count) : "memory");
+      int n = 0;
+      do {
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
+      } while ((int)(seen - target) < 0 && ++n < kBarTries);
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      if (n >= kBarTries) {
+        ok = false;
+        atomicCAS(&ctl->status, 0, -5);  // NIM_ERR_TIMEOUT
+        *(volatile int *)&ctl->done = 1;
+      }
+    }
+    target += gridDim.x;
+    return __syncthreads_and(ok);
+  }
+};
+// +xi_dd face updates of T, thread y = direction y+1 (T_face_body spread over
+// three threads a cell)
+template <class R, class PS>
+__device__ __forceinline__ void T_face3_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P,
+                                             const FlatBlock bi, PS &ps) {
+  using V = Ar<R>;
+  Cell x;
+  if (!patch_cell(d, x, bi)) return;
+  const int Nc = d.Nc, NF = d.NF, c = x.c;
+  const R *T = F.f[4] + ps.par * NF;
+  R *Tn = F.f[4] + (1 - ps.par) * NF;
+  double e[1] = {0.};
+  by_dir(threadIdx.y, [&](auto D) {
+    constexpr int dd = decltype(D)::value;
+    if (!x.has_nb(d, 2 * dd)) return;
+    const Cell x2 = x.nb(d, 2 * dd);
+    V Fd[5];
+    T_form_Fd(F, Nc, c, x2.c, dd, Fd);
+    const int fo = x.face(d, 2 * dd);
+    const V nw = stored<R>(face_update(d, T, F.c[3], F.co[3], Fd, g.dg[(2 * (dd - 1)) * Nc + c],
+                                       g.dg[(2 * (dd - 1) + 1) * Nc + c], dd, x, x2, Kc<V>(P.w[3]),
+                                       (1 - 2 * ps.par) * NF));
+    Tn[fo] = nw;
+    e[0] = errv(nw, T[fo], ps.first);
+  });
+  ps.template end<0>(e, 4);
+}
+// PAIR: k_vel_cell2's form of the velocity cell sweep (n_theta even)
+template <class R, bool PAIR>
+__global__ void __launch_bounds__(CB3, LOOP_MINB) k_pass_loop(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl,
+                                                              unsigned *arrivals, int passes, int lowp) {
+  const int tid = threadIdx.x + blockDim.x * threadIdx.y, nth = blockDim.x * blockDim.y;
+  const int NB = gridDim.x, b0 = blockIdx.x;
+  // items of a part: runs of blockDim.x cells, or pairs, of each plane
+  const int r1 = (d.plane + blockDim.x - 1) / blockDim.x, n1 = r1 * d.NZ;
+  const int r2 = PAIR ? (d.plane / 2 + blockDim.x - 1) / blockDim.x : r1, n2 = r2 * d.NZ;
+  auto run = [](int w, int r) { return FlatBlock{(unsigned)(w % r), 0u, (unsigned)(w / r)}; };
+  // Every block steps a copy of the control block of its own: after the last
+  // barrier of a pass all read the same maxima, so all take the same decision
+  // without another exchange; block 0 keeps the one in memory up to date.
+  __shared__ Ctrl sc;
+  __shared__ BlockRed red;
+  LoopBarrier bar(arrivals);
+  if (tid == 0) sc = *ctl;
+  __syncthreads();
+  for (int n = 0; n < passes && !sc.done; ++n) {
+    LoopPass ps;
+    ps.ctl = ctl;
+    ps.par = sc.iter & sc.pmask;
+    ps.nh = sc.pmask ? 1 - ps.par : ps.par;
+    ps.first = sc.first;
+    for (int q = 0; q < 6; ++q) ps.m[q] = 0.;
+    // u, v, w of the cells; the z walls of T
+    for (int w = b0; w < n2; w += NB) {
+      if constexpr (PAIR)
+        vel_cell2_body<R, false>(d, g, F, P, ctl, run(w, r2), ps);
+      else
+        vel_cell_body<false, 2, R>(d, g, F, P, ctl, run(w, r1), ps);
+    }
+    for (int i = (NB - 1 - b0) * nth + tid; i < 2 * d.plane; i += NB * nth)
+      zero_flux_body<R>(d, g, F, ctl, LinIndex{i}, ps);
+    if (!bar.sync(ctl)) return;
+    // the faces of u, v, w; T of the cells (which reads the cells' u, v, w)
+    for (int w = b0; w < 2 * n1; w += NB) {
+      if (w < n1) {
+        T_cell_body<R>(d, g, F, P, ctl, run(w, r1), ps);
+        __syncthreads();
+      } else {
+        vel_face_body<R>(d, g, F, P, ctl, run(w - n1, r1), ps);
+      }
+    }
+    if (!bar.sync(ctl)) return;
+    // the pressure sources (with the old T of the faces); T of the faces
+    for (int w = b0; w < 2 * n1; w += NB) {
+      if (w < n1) {
+        p_src_body<R>(d, g, F, P, ctl, run(w, r1), ps);
+        __syncthreads();
+      } else {
+        T_face3_body<R>(d, g, F, P, run(w - n1, r1), ps);
+      }
+    }
+    if (!bar.sync(ctl)) return;
+    for (int i = b0 * nth + tid; i < d.NBF; i += NB * nth) p_bc_body<R>(d, g, F, P, ctl, LinIndex{i}, ps);
+    if (!bar.sync(ctl)) return;
+    for (int w = b0; w < n1; w += NB) p_face_body<R>(d, g, F, P, ctl, run(w, r1), ps);
+    if (P.dpdx_tolerance) {
+      if (!bar.sync(ctl)) return;
+      for (int i = b0 * nth + tid; i < d.Nc; i += NB * nth) p_dpdx_body<R>(d, g, F, ctl, LinIndex{i}, ps);
+    }
+    red_init<6>(red);
+    block_max<6, 0>(red, ps.m, ctl->err[ps.par]);
+    if (!bar.sync(ctl)) return;
+    if (tid == 0) {
+      // the other slot is accumulated into again only six barriers on
+      for (int q = 0; q < 6; ++q) sc.err[ps.par][q] = __ldcg(&ctl->err[ps.par][q]);
+      iter_end_body(&sc, P, lowp, LaunchBlock{});
+      if (b0 == 0)
+        for (int q = 0; q < 8; ++q) ctl->err[1 - ps.par][q] = 0ull;
+    }
+    __syncthreads();
+  }
+  if (b0 == 0 && tid == 0) {
+    ctl->iter = sc.iter;
+    ctl->step_iters = sc.step_iters;
+    ctl->status = sc.status;
+    ctl->first = sc.first;
+    for (int q = 0; q < 5; ++q) ctl->last_err[q] = sc.last_err[q];
+    ctl->lowp_iters = sc.lowp_iters;
+    ctl->stall = sc.stall;
+    for (int q = 0; q < 5; ++q) ctl->best[q] = sc.best[q];
+    ctl->done = sc.done;
+  }
 }
 
 // start of the FP32 phase of a mixed-precision step (after k_step_reset)
