@@ -3596,7 +3596,11 @@ __global__ void __launch_bounds__(BLK, 4) k_T_coef(Dims d, GeoOf<R> g, FieldsT<R
 // here moves 616 bytes a cell in this kernel and k_T_face together; with
 // MT_A (18 words) and MT_F (15) written and read through memory by a kernel
 // of their own it was 952.  128x128x96: FP64 T_coef + T_cell 305 -> 289 us,
-// float (k_T_cellN) 128 -> 91 us, and k_T_faceN 51 -> 45 us.
+// float (k_T_cellN) 128 -> 91 us, and k_T_faceN 51 -> 45 us.  The cross
+// derivatives come first: their loads and the constants' then overlap across
+// warps instead of the gathers waiting behind the quotients (197 against 212
+// us in FP64, 88 against 96 in float; the g^ij and face products handed to
+// the direction threads instead of thread 0: 208-229 us).
 template <class R, class BI, class PS = LaunchPass>
 __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, const Phys &P, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
   using V = Ar<R>;
@@ -3621,17 +3625,6 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoOf<R> &g, co
   f[6] += d6;
   if (active) by_dir(threadIdx.y, [&](auto D) {
     constexpr int dd = decltype(D)::value, y = dd - 1;
-    {
-      const TDir<V> t = T_direction_of(g, F, P, Nc, c, dd);
-      R *row = F.MTF + 4 * y * Nc;
-      row[c] = t.G1;
-      row[Nc + c] = t.G3;
-      row[2 * Nc + c] = t.H2;
-      row[3 * Nc + c] = t.H4;
-      sF[y][0][tx] = t.r;
-      sF[y][1][tx] = t.m;
-      sF[y][2][tx] = t.p;
-    }
     // cross derivatives of calculate_R_D_T: y=0 pxy,pzy  y=1 pyx,pzx  y=2 pxz,pyz
     constexpr int e2 = (y == 0) ? 2 : (y == 1) ? 1 : 3;
     constexpr int fa = (y == 1) ? 4 : 2, fb = (y == 1) ? 3 : 1;
@@ -3643,6 +3636,17 @@ __device__ __forceinline__ void T_cell_body(const Dims &d, const GeoOf<R> &g, co
       const V py = (T[f[4]] - T[f[3]]) / Kc<V>(2.);
       const V pz = (T[f[6]] - T[f[5]]) / Kc<V>(2.);
       sG[tx] = g.G[c] * px + g.G[Nc + c] * py + g.G[2 * Nc + c] * pz;
+    }
+    {
+      const TDir<V> t = T_direction_of(g, F, P, Nc, c, dd);
+      R *row = F.MTF + 4 * y * Nc;
+      row[c] = t.G1;
+      row[Nc + c] = t.G3;
+      row[2 * Nc + c] = t.H2;
+      row[3 * Nc + c] = t.H4;
+      sF[y][0][tx] = t.r;
+      sF[y][1][tx] = t.m;
+      sF[y][2][tx] = t.p;
     }
   });
   __syncthreads();
@@ -3720,41 +3724,6 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoOf<R> g, F
   double e[1] = {0.};
   if (active) by_dir(threadIdx.y, [&](auto D) {
     constexpr int dd = decltype(D)::value, y = dd - 1;
-    {  // the NIM constants of direction dd (T_direction_of)
-      V u[NP];
-      {
-        const R *xd = g.xi + (dd - 1) * Nc;
-        R a[NP], b[NP], xi[NP];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          ldN<R, NP>(F.c[q], c, a);
-          ldN<R, NP>(F.co[q], c, b);
-          ldN<R, NP>(xd + 3 * q * Nc, c, xi);
-#pragma unroll
-          for (int p = 0; p < NP; ++p) {
-            const V tp = (Kc<V>(0.5) * (a[p] + b[p])) * xi[p];
-            u[p] = (q == 0) ? tp : u[p] + tp;
-          }
-        }
-      }
-      R kd[NP], gm[NP], gp[NP], out[4][NP];
-      ldN<R, NP>(g.gij + 4 * (dd - 1) * Nc, c, kd);
-      ldN<R, NP>(g.gfd + 2 * (dd - 1) * Nc, c, gm);
-      ldN<R, NP>(g.gfd + (2 * (dd - 1) + 1) * Nc, c, gp);
-#pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        const TDir<V> t = T_direction<R>(u[p], kd[p] * pv<V>(P.alpha, P.d_alpha), gm[p], gp[p], P.v_limit);
-        out[0][p] = t.G1;
-        out[1][p] = t.G3;
-        out[2][p] = t.H2;
-        out[3][p] = t.H4;
-        sF[y][0][tx * NP + p] = t.r;
-        sF[y][1][tx * NP + p] = t.m;
-        sF[y][2][tx * NP + p] = t.p;
-      }
-#pragma unroll
-      for (int n = 0; n < 4; ++n) stN<R, NP>(F.MTF + (4 * (dd - 1) + n) * Nc, c, out[n]);
-    }
     // T's faces of the NP cells
     R o[7][NP];
 #pragma unroll
@@ -3841,6 +3810,41 @@ __global__ void __launch_bounds__(CB3, TCN_MINB) k_T_cellN(Dims d, GeoOf<R> g, F
         const V pz = (o[6][p] - o[5][p]) / Kc<V>(2.);
         sG[tx * NP + p] = G0[p] * px + G1[p] * py + G2[p] * pz;
       }
+    }
+    {  // the NIM constants of direction dd (T_direction_of)
+      V u[NP];
+      {
+        const R *xd = g.xi + (dd - 1) * Nc;
+        R a[NP], b[NP], xi[NP];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          ldN<R, NP>(F.c[q], c, a);
+          ldN<R, NP>(F.co[q], c, b);
+          ldN<R, NP>(xd + 3 * q * Nc, c, xi);
+#pragma unroll
+          for (int p = 0; p < NP; ++p) {
+            const V tp = (Kc<V>(0.5) * (a[p] + b[p])) * xi[p];
+            u[p] = (q == 0) ? tp : u[p] + tp;
+          }
+        }
+      }
+      R kd[NP], gm[NP], gp[NP], out[4][NP];
+      ldN<R, NP>(g.gij + 4 * (dd - 1) * Nc, c, kd);
+      ldN<R, NP>(g.gfd + 2 * (dd - 1) * Nc, c, gm);
+      ldN<R, NP>(g.gfd + (2 * (dd - 1) + 1) * Nc, c, gp);
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const TDir<V> t = T_direction<R>(u[p], kd[p] * pv<V>(P.alpha, P.d_alpha), gm[p], gp[p], P.v_limit);
+        out[0][p] = t.G1;
+        out[1][p] = t.G3;
+        out[2][p] = t.H2;
+        out[3][p] = t.H4;
+        sF[y][0][tx * NP + p] = t.r;
+        sF[y][1][tx * NP + p] = t.m;
+        sF[y][2][tx * NP + p] = t.p;
+      }
+#pragma unroll
+      for (int n = 0; n < 4; ++n) stN<R, NP>(F.MTF + (4 * (dd - 1) + n) * Nc, c, out[n]);
     }
   });
   __syncthreads();
