@@ -95,7 +95,7 @@ struct nim_ctx {
   // reference-order schedule
   bool seq = false;
   SeqTab seqt{};
-  bool seq_grid = false;                     // levels wider than a block's share: cooperative grids
+  int seq_mode = 0;                          // kSeqBlock, kSeqGrid or kSeqSkew
   int seq_threads = 0, wall_threads = 0;     // block sizes of the one-block sweeps
   int coop_vel = 0, coop_p = 0, coop_T = 0;  // cooperative grid sizes
   // nim_gpu_profile_iterations: while set, every kernel launch of an
@@ -382,7 +382,7 @@ int launch_iteration_seq(nim_ctx *x) {
   const Dims &d = x->d;
   cudaStream_t s = x->stream;
   const SeqTab &S = x->seqt;
-  const bool one = x->phys.formulation == 1, grid_form = x->seq_grid;
+  const bool one = x->phys.formulation == 1, grid_form = x->seq_mode == kSeqGrid, skewed = x->seq_mode == kSeqSkew;
   const int nt = x->seq_threads;
   const bool wide = nt > SEQ_TPB;
   if (one)
@@ -390,13 +390,25 @@ int launch_iteration_seq(nim_ctx *x) {
   else
     k_vel_cell<true, 2><<<x->g3, dim3(CB, 3), 0, s>>>(d, x->g, x->F, x->phys, x->ctl);
   TRY(mark(x, "k_vel_cell(src)"));
+  // one block over wide levels works on skewed copies (SeqTab)
+  const size_t Nc = d.Nc, L = S.skew.L;
+  SkewFields sv{}, sp{}, st{};
+  for (int q = 0; q < 3; ++q)
+    sv.q[q] = SkewField{x->F.f[q], x->F.c[q], x->F.co[q], x->F.Bv + q * Nc, S.skv + (size_t)(kSkewVel * q) * L};
+  sp.q[0] = SkewField{x->F.f[3], nullptr, x->F.Rp, nullptr, S.skp};
+  st.q[0] = SkewField{x->F.f[4], x->F.c[3], x->F.co[3], nullptr, S.skt};
+  const dim3 gv(x->nblk_c, 3), g1(x->nblk_c, 1);
+  if (skewed) k_seq_skew<<<gv, BLK, 0, s>>>(d, S.skew, sv, x->ctl);
   if (grid_form)
-    TRY(one ? launch_coop(k_seq_vel<1, true, CB3>, x->coop_vel, dim3(CB, 3), x)
-            : launch_coop(k_seq_vel<2, true, CB3>, x->coop_vel, dim3(CB, 3), x));
-  else if (one)
-    (wide ? k_seq_vel<1, false, SEQ_TPB_WIDE> : k_seq_vel<1, false, SEQ_TPB>)<<<3, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+    TRY(one ? launch_coop(k_seq_vel<1, kSeqGrid, CB3>, x->coop_vel, dim3(CB, 3), x)
+            : launch_coop(k_seq_vel<2, kSeqGrid, CB3>, x->coop_vel, dim3(CB, 3), x));
+  else if (skewed && wide)
+    (one ? k_seq_vel<1, kSeqSkew, SEQ_TPB_WIDE> : k_seq_vel<2, kSeqSkew, SEQ_TPB_WIDE>)<<<3, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+  else if (skewed)
+    (one ? k_seq_vel<1, kSeqSkew, SEQ_TPB> : k_seq_vel<2, kSeqSkew, SEQ_TPB>)<<<3, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   else
-    (wide ? k_seq_vel<2, false, SEQ_TPB_WIDE> : k_seq_vel<2, false, SEQ_TPB>)<<<3, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+    (one ? k_seq_vel<1, kSeqBlock, SEQ_TPB> : k_seq_vel<2, kSeqBlock, SEQ_TPB>)<<<3, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+  if (skewed) k_seq_unskew<<<gv, BLK, 0, s>>>(d, S.skew, sv, x->ctl);
   TRY(mark(x, "k_seq_vel"));
   k_p_src<<<x->g3, dim3(CB, 3), 0, s>>>(d, x->g, x->F, x->phys, x->ctl);
   TRY(mark(x, "k_p_src"));
@@ -404,10 +416,12 @@ int launch_iteration_seq(nim_ctx *x) {
   k_seq_pbc<<<2, x->wall_threads, 0, s>>>(d, x->F, x->phys, x->ctl, S, 0);
   k_seq_pbc<<<2, x->wall_threads, 0, s>>>(d, x->F, x->phys, x->ctl, S, 2);
   TRY(mark(x, "k_seq_pbc"));
+  if (skewed) k_seq_skew<<<g1, BLK, 0, s>>>(d, S.skew, sp, x->ctl);
   if (grid_form)
-    TRY(launch_coop(k_seq_p<true, BLK>, x->coop_p, dim3(BLK), x));
+    TRY(launch_coop(k_seq_p<kSeqGrid, BLK>, x->coop_p, dim3(BLK), x));
   else
-    (wide ? k_seq_p<false, SEQ_TPB_WIDE> : k_seq_p<false, SEQ_TPB>)<<<1, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+    (!skewed ? k_seq_p<kSeqBlock, SEQ_TPB> : wide ? k_seq_p<kSeqSkew, SEQ_TPB_WIDE> : k_seq_p<kSeqSkew, SEQ_TPB>)<<<1, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+  if (skewed) k_seq_unskew<<<g1, BLK, 0, s>>>(d, S.skew, sp, x->ctl);
   TRY(mark(x, "k_seq_p"));
   if (x->phys.dpdx_tolerance) {
     k_p_dpdx<<<x->nblk_c, BLK, 0, s>>>(d, x->g, x->F, x->ctl);
@@ -419,15 +433,17 @@ int launch_iteration_seq(nim_ctx *x) {
   TRY(mark(x, "k_T_coef"));
   k_T_src<<<x->nblk_c, BLK, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   TRY(mark(x, "k_T_cell(src)"));
+  if (skewed) k_seq_skew<<<g1, BLK, 0, s>>>(d, S.skew, st, x->ctl);
   if (grid_form)
-    TRY(launch_coop(k_seq_T<true, BLK>, x->coop_T, dim3(BLK), x));
+    TRY(launch_coop(k_seq_T<kSeqGrid, BLK>, x->coop_T, dim3(BLK), x));
   else
-    (wide ? k_seq_T<false, SEQ_TPB_WIDE> : k_seq_T<false, SEQ_TPB>)<<<1, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+    (!skewed ? k_seq_T<kSeqBlock, SEQ_TPB> : wide ? k_seq_T<kSeqSkew, SEQ_TPB_WIDE> : k_seq_T<kSeqSkew, SEQ_TPB>)<<<1, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+  if (skewed) k_seq_unskew<<<g1, BLK, 0, s>>>(d, S.skew, st, x->ctl);
   TRY(mark(x, "k_seq_T"));
   k_iter_end<<<1, 1, 0, s>>>(x->ctl, x->phys, 0);
   TRY(mark(x, "k_iter_end"));
   CK(cudaGetLastError());
-  x->kernels_per_iter = x->phys.dpdx_tolerance ? 14 : 13;
+  x->kernels_per_iter = (x->phys.dpdx_tolerance ? 14 : 13) + (skewed ? 6 : 0);
   x->launches += x->kernels_per_iter;
   return NIM_OK;
 }
@@ -441,8 +457,13 @@ int seq_pack_velocity(nim_ctx *x) {
   const int rows[2] = {one ? 9 : 8, one ? 45 : 15};
   k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(src[0], S.vel, S.order, rows[0], Nc);
   k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(src[1], S.vel + (size_t)rows[0] * Nc, S.order, rows[1], Nc);
+  double *quo = S.vel + (size_t)(one ? 54 : 23) * Nc;
+  const double *A = x->F.AAv, *M = x->F.MF;
+  const size_t n = Nc;
+  k_seq_pack_quo<<<x->nblk_c, BLK, 0, x->stream>>>(one ? nullptr : x->F.MF4, one ? A + n : M, one ? A + 20 * n : M + 5 * n,
+                                                   one ? A + 39 * n : M + 10 * n, quo, x->phys, S.order, Nc);
   CK(cudaGetLastError());
-  x->launches += 2;
+  x->launches += 3;
   return NIM_OK;
 }
 // what stays as it is after init: the metric differences, the pressure
@@ -911,7 +932,9 @@ static int noalloc_setup(int device) {
 // numbers (the argument is in nim_kernels.cuh).  Wall faces, in BC-list
 // order bottom, top, inner, outer: level i + 2j on bottom and top, i + 2k on
 // inner and outer.  Also the sweep buffers and the cooperative grid sizes.
-constexpr int kSeqBlock = 1024;  // widest level swept by one block
+// widest level swept by one block, and from where on it works on skewed copies
+// (measured beside the sweeps)
+constexpr int kSeqBlockMost = 1024, kSeqSkewFrom = 96;
 static int setup_levels(nim_ctx *x) {
   const Dims &d = x->d;
   const size_t Nc = d.Nc;
@@ -958,7 +981,7 @@ static int setup_levels(nim_ctx *x) {
   TRY(dalloc(x, &S.blev, blev.size()));
   TRY(dalloc(x, &S.wlev, wlev.size()));
   TRY(dalloc(x, &S.dg, 6 * Nc));
-  TRY(dalloc(x, &S.vel, (x->phys.formulation == 1 ? 54 : 23) * Nc));
+  TRY(dalloc(x, &S.vel, (x->phys.formulation == 1 ? 66 : 35) * Nc));
   TRY(dalloc(x, &S.prs, 3 * kSeqP * Nc));
   TRY(dalloc(x, &S.tmp, kSeqT * Nc));
   TRY(dalloc(x, &S.wall, kSeqW * (size_t)d.NBF));
@@ -969,14 +992,23 @@ static int setup_levels(nim_ctx *x) {
   CK(cudaMemcpy(S.blev, blev.data(), sizeof(int) * blev.size(), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(S.wlev, wlev.data(), sizeof(int) * wlev.size(), cudaMemcpyHostToDevice));
   // block sizes: whole warps for the widest level, at most SEQ_TPB_WIDE (a level
-  // up to kSeqBlock wide then takes that many turns), or a cooperative grid
+  // up to kSeqBlockMost wide then takes that many turns), or a cooperative grid
   auto warps = [](int n, int most) { return std::min(most, (n + 31) / 32 * 32); };
   int wmax = 1;
   for (size_t L = 0; L + 1 < blev.size(); ++L) wmax = std::max(wmax, blev[L + 1] - blev[L]);
   x->seq_threads = warps(maxlev, SEQ_TPB_WIDE);
   x->wall_threads = warps(wmax, BLK);
-  x->seq_grid = maxlev > kSeqBlock;
-  if (!x->seq_grid) return NIM_OK;
+  x->seq_mode = maxlev > kSeqBlockMost ? kSeqGrid : maxlev > kSeqSkewFrom ? kSeqSkew : kSeqBlock;
+  if (x->seq_mode == kSeqBlock) return NIM_OK;
+  if (x->seq_mode == kSeqSkew) {
+    S.skew.sk = d.NR + 1;
+    S.skew.st = (d.NZ + 1) * S.skew.sk;
+    S.skew.L = (nlev + 3) * S.skew.st;  // levels from -3 (the low z wall's layer)
+    TRY(dalloc(x, &S.skv, 3 * kSkewVel * (size_t)S.skew.L));
+    TRY(dalloc(x, &S.skp, kSkewP * (size_t)S.skew.L));
+    TRY(dalloc(x, &S.skt, kSkewTm * (size_t)S.skew.L));
+    return NIM_OK;
+  }
   // cooperative grids: no more blocks than the widest level needs, and no
   // more than can be resident at once (cudaLaunchCooperativeKernel rejects
   // a larger grid rather than running it)
@@ -987,13 +1019,13 @@ static int setup_levels(nim_ctx *x) {
   const int want = std::max(1, (maxlev + BLK - 1) / BLK);
   int per = 0;
   if (x->phys.formulation == 1)
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_vel<1, true, CB3>, CB3, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_vel<1, kSeqGrid, CB3>, CB3, 0));
   else
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_vel<2, true, CB3>, CB3, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_vel<2, kSeqGrid, CB3>, CB3, 0));
   x->coop_vel = std::max(1, std::min((maxlev + CB - 1) / CB, per * sms));
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_p<true, BLK>, BLK, 0));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_p<kSeqGrid, BLK>, BLK, 0));
   x->coop_p = std::max(1, std::min(want, per * sms));
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_T<true, BLK>, BLK, 0));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_seq_T<kSeqGrid, BLK>, BLK, 0));
   x->coop_T = std::max(1, std::min(want, per * sms));
   if (x->coop_vel < 1 || x->coop_p < 1 || x->coop_T < 1) return NIM_ERR_CUDA;
   return NIM_OK;

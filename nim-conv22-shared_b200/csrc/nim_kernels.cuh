@@ -4457,11 +4457,35 @@ __global__ void __launch_bounds__(BLK) k_convert(CvtList L) {
 // Levels that fit a block run in one block per swept field, whose barrier is
 // the SM's own and whose loads hit its L1; wider ones on a cooperative grid
 // (the three velocity components side by side), which reads through L2.
-// Time of a pass with dependent loads and a grid barrier a level before, and
-// now: 36x6x12 (66 cells wide) 1891 -> 486 us, 24x24x16 formulation 1 (168)
-// 3882 -> 939 us, 48x48x32 (672) 10.3 -> 5.0 ms, 128x128x96 (grid) 35.2 ->
-// 20.6 ms.  What is left of a level is its gathers: the cells of a level lie
-// on different lines of the swept arrays.
+// In one block a wide level is bound by L1 lines: its cells lie apart in the
+// fields, 32 lines a load.  From kSeqSkewFrom cells on the block therefore
+// works on skewed copies (below); a narrow level waits on latency instead,
+// neighbouring levels share the fields' lines, and the copies' six launches
+// do not come back (36x6x12, 66 wide: 443 us a pass without, 526 with;
+// 24x24x16 formulation 1, 168 wide: 896 without, 835 with).  The divisions by
+// what a step or the run keeps are done once, with the packing, and nothing
+// is computed from a level's constants before the barrier, where it would
+// wait for their loads.
+// Time of a pass with dependent loads and a grid barrier a level, then loads
+// up front in one block, and now: 36x6x12 1891 -> 486 -> 431 us, 24x24x16
+// formulation 1 3882 -> 939 -> 824 us, 48x48x32 (672 wide) 10.3 -> 5.0 ->
+// 3.5 ms, 128x128x96 (grid) 35.2 -> 20.6 -> 19.8 ms.
+
+// Skewed copies of the swept fields (one block over wide levels): cell (i, j, k) of
+// level t = i + 2j + 3k at t st + (k + 1) sk + j + 1, its +xi faces in three
+// planes of L values at the cell's place, its average and the sweep's other
+// per-cell values in planes after them.  Neighbouring cells sit at constant
+// distances, and a level's cells, which differ in (j, k) only, on adjacent
+// addresses: a gather of a warp is two or three cache lines, not 32.  Row
+// j = -1 and layer k = -1 hold the low wall faces; t is shifted by kSkewT for
+// them.
+struct Skew {
+  int st, sk, L;  // steps of t and k, values of a plane
+  __host__ __device__ int at(int i, int j, int k) const {
+    return (i + 2 * j + 3 * k + 3) * st + (k + 1) * sk + j + 1;
+  }
+};
+constexpr int kSkewVel = 6, kSkewP = 4, kSkewTm = 5;  // planes: faces (3), average, old value, R sums; R_p; average, old value
 
 // tables of the reference-order schedule
 struct SeqTab {
@@ -4471,14 +4495,22 @@ struct SeqTab {
   int *border, *blev, *wlev;  // wall faces, levels, per-wall level ranges
   // rows in level order, [row][Nc]: the face-metric differences dg (6); the
   // velocity constants of a step (formulation 2: M_F4 (8), M_F1..3 (15);
-  // 1: a_t (9), AA_v (45)); the pressure constants (kSeqP a direction); the
+  // 1: a_t (9), AA_v (45)) and the relaxation factors of u, v, w over their
+  // divisors (4 each); the pressure constants (kSeqP a direction); the
   // temperature constants and R_D_T of a pass (kSeqT)
   double *dg, *vel, *prs, *tmp;
   // in border order: the faces a wall face's update reads and the
   // constants of apply_pressure_bc in this pass
   int *wface;    // [kSeqI][NBF]
   double *wall;  // [kSeqW][NBF]
+  // skewed copies of u, v, w, of p and of T (null where the sweeps work on
+  // the fields themselves)
+  Skew skew;
+  double *skv, *skp, *skt;
 };
+// how a sweep runs: one block over the fields themselves, all blocks of a
+// cooperative launch, one block over skewed copies
+enum { kSeqBlock, kSeqGrid, kSeqSkew };
 constexpr int kSeqI = 11;  // the face, its cell's other five, two stencils (a, b) along the wall, wall-end flags
 constexpr int kSeqP = 9;   // m, a1, a2, mq, a1q, a2q, w/diag, b, bq of one direction
 constexpr int kSeqT = 24;  // w/MT_F4(0), MT_F4(1..7), (w/MT_F(0), MT_F(1..4)) x 3, R_D_T
@@ -4491,6 +4523,20 @@ __global__ void __launch_bounds__(BLK) k_seq_pack(const double *__restrict__ src
   if (q >= Nc) return;
   const int c = order[q].x;
   for (int r = 0; r < rows; ++r) dst[(size_t)r * Nc + q] = src[(size_t)r * Nc + c];
+}
+// w / div[order[q]] of the three components, for rows r of div: dst[4 v + r]
+__global__ void __launch_bounds__(BLK) k_seq_pack_quo(const double *d0, const double *d1, const double *d2,
+                                                      const double *d3, double *__restrict__ dst, Phys P,
+                                                      const int4 *__restrict__ order, int Nc) {
+  const int q = blockIdx.x * BLK + threadIdx.x;
+  if (q >= Nc) return;
+  const int c = order[q].x;
+  const double *div[4] = {d0, d1, d2, d3};
+  for (int r = 0; r < 4; ++r) {
+    if (!div[r]) continue;
+    const double v = div[r][c];
+    for (int n = 0; n < 3; ++n) dst[(size_t)(4 * n + r) * Nc + q] = P.w[n] / v;
+  }
 }
 // the pressure sweep's constants in level order, once at init
 __global__ void __launch_bounds__(BLK) k_seq_pack_p(Dims d, Geo g, Phys P, SeqTab S) {
@@ -4537,31 +4583,61 @@ __global__ void __launch_bounds__(BLK) k_T_src(Dims d, Geo g, Fields F, Phys P, 
   o[23 * Nc] = P.alpha * diffusion_source(d, g, T, x, f);
 }
 
-// a cell of a level with its index steps to the +r, +theta, +z neighbours (0
-// where there is none: the loads then stay on the cell and are not used)
+// a cell of a level: where its values are, and the index steps to those of
+// its neighbours (0 where there is none: the loads then stay on the cell and
+// are not used), in the library's layout or in a skewed copy
 struct SeqCell {
   int c, i, j, k;
-  int f[7];         // its faces
-  int st, ip2;      // step to the +theta neighbour, theta index past it
-  bool has[4];      // has[dd]: a neighbour across +xi_dd
+  int f[7];           // its faces
+  int t4;             // the +theta neighbour's +theta face
+  int tn, tp;         // steps in theta: to the next cell's r and z faces, to the one before
+  int dr, dzr, dz;    // steps in r, in z of r faces, in z of the others
+  bool has[4];        // has[dd]: a neighbour across +xi_dd
   __device__ __forceinline__ SeqCell() {}
-  __device__ __forceinline__ SeqCell(const Dims &d, const int4 o) : c(o.x), j(o.y), k(o.z) {
+  __device__ __forceinline__ SeqCell(const Dims &d, const int4 o) {
+    c = o.x;
+    j = o.y;
+    k = o.z;
     i = c - d.NT * (j + d.NR * k);
-    st = (i == d.NT - 1) ? 1 - d.NT : 1;
-    const int ip = i + st;
-    ip2 = (ip == d.NT - 1) ? 0 : ip + 1;
+    tn = (i == d.NT - 1) ? 1 - d.NT : 1;
+    tp = (i == 0) ? d.NT - 1 : -1;
+    const int ip = i + tn, ip2 = (ip == d.NT - 1) ? 0 : ip + 1;
     f[1] = c + d.NT * k;
     f[2] = f[1] + d.NT;
     f[3] = d.offT + c;
-    f[4] = f[3] + st;
+    f[4] = f[3] + tn;
     f[5] = d.offZ + c;
     f[6] = f[5] + d.plane;
+    t4 = f[3] - i + ip2;
+    dr = d.NT;
+    dzr = d.NT * (d.NR + 1);
+    dz = d.plane;
     has[1] = j < d.NR - 1;
     has[2] = true;
     has[3] = k < d.NZ - 1;
   }
-  __device__ __forceinline__ int nb(const Dims &d, int dd) const {  // cell index of the +xi_dd neighbour
-    return c + (dd == 1 ? (has[1] ? d.NT : 0) : dd == 2 ? st : (has[3] ? d.plane : 0));
+  __device__ __forceinline__ SeqCell(const Dims &d, const Skew &w, const int4 o) {
+    j = o.y;
+    k = o.z;
+    i = o.x - d.NT * (j + d.NR * k);
+    c = w.at(i, j, k);
+    tn = (i == d.NT - 1) ? (1 - d.NT) * w.st : w.st;
+    tp = (i == 0) ? (d.NT - 1) * w.st : -w.st;
+    dr = 2 * w.st + 1;
+    dzr = dz = 3 * w.st + w.sk;
+    f[2] = c;
+    f[1] = c - dr;
+    f[4] = w.L + c;
+    f[3] = f[4] + tp;
+    f[6] = 2 * w.L + c;
+    f[5] = f[6] - dz;
+    t4 = f[4] + tn;
+    has[1] = j < d.NR - 1;
+    has[2] = true;
+    has[3] = k < d.NZ - 1;
+  }
+  __device__ __forceinline__ int nb(int dd) const {  // cell index of the +xi_dd neighbour
+    return c + (dd == 1 ? (has[1] ? dr : 0) : dd == 2 ? tn : (has[3] ? dz : 0));
   }
 };
 // the faces of the cell (x) and of its +r, +theta, +z neighbours (r, t, z):
@@ -4572,17 +4648,17 @@ struct Hood {
   __device__ __forceinline__ const double *of(int dd) const { return dd == 1 ? r : dd == 2 ? t : z; }
 };
 template <class Ld>
-__device__ __forceinline__ void load_hood(const Dims &d, const double *fr, const SeqCell &x, Hood &h) {
-  const int up = x.has[1] ? d.NT : 0, zr = x.has[3] ? d.NT * (d.NR + 1) : 0, zc = x.has[3] ? d.plane : 0;
+__device__ __forceinline__ void load_hood(const double *fr, const SeqCell &x, Hood &h) {
+  const int up = x.has[1] ? x.dr : 0, zr = x.has[3] ? x.dzr : 0, zc = x.has[3] ? x.dz : 0;
 #pragma unroll
   for (int k = 1; k <= 6; ++k) h.x[k] = Ld::ld(fr, x.f[k]);
 #pragma unroll
   for (int k = 2; k <= 6; ++k) h.r[k] = Ld::ld(fr, x.f[k] + up);
-  h.t[1] = Ld::ld(fr, x.f[1] + x.st);
-  h.t[2] = Ld::ld(fr, x.f[2] + x.st);
-  h.t[4] = Ld::ld(fr, x.f[3] - x.i + x.ip2);
-  h.t[5] = Ld::ld(fr, x.f[5] + x.st);
-  h.t[6] = Ld::ld(fr, x.f[6] + x.st);
+  h.t[1] = Ld::ld(fr, x.f[1] + x.tn);
+  h.t[2] = Ld::ld(fr, x.f[2] + x.tn);
+  h.t[4] = Ld::ld(fr, x.t4);
+  h.t[5] = Ld::ld(fr, x.f[5] + x.tn);
+  h.t[6] = Ld::ld(fr, x.f[6] + x.tn);
   h.z[1] = Ld::ld(fr, x.f[1] + zr);
   h.z[2] = Ld::ld(fr, x.f[2] + zr);
   h.z[3] = Ld::ld(fr, x.f[3] + zc);
@@ -4598,18 +4674,17 @@ template <class Ld>
 __device__ __forceinline__ void load_tang(const Dims &d, const double *fr, const SeqCell &x, const Hood &h, Tang &t) {
   const bool rlo = x.j == 0, rhi = x.j == d.NR - 1, zlo = x.k == 0, zhi = x.k == d.NZ - 1;
   const int ra = rlo ? 1 : -1, rb = rlo ? 2 : rhi ? -2 : 1, za = zlo ? 1 : -1, zb = zlo ? 2 : zhi ? -2 : 1;
-  const int im = (x.i == 0) ? d.NT - 1 : -1, zr = d.NT * (d.NR + 1);
-  t.a[1][0] = Ld::ld(fr, x.f[2] + im);  // face 2 along theta: always centred
+  t.a[1][0] = Ld::ld(fr, x.f[2] + x.tp);  // face 2 along theta: always centred
   t.b[1][0] = h.t[2];
-  t.a[1][1] = Ld::ld(fr, x.f[2] + za * zr);
-  t.b[1][1] = Ld::ld(fr, x.f[2] + zb * zr);
-  t.a[2][0] = Ld::ld(fr, x.f[4] + ra * d.NT);
-  t.b[2][0] = Ld::ld(fr, x.f[4] + rb * d.NT);
-  t.a[2][1] = Ld::ld(fr, x.f[4] + za * d.plane);
-  t.b[2][1] = Ld::ld(fr, x.f[4] + zb * d.plane);
-  t.a[3][0] = Ld::ld(fr, x.f[6] + ra * d.NT);
-  t.b[3][0] = Ld::ld(fr, x.f[6] + rb * d.NT);
-  t.a[3][1] = Ld::ld(fr, x.f[6] + im);  // face 6 along theta
+  t.a[1][1] = Ld::ld(fr, x.f[2] + za * x.dzr);
+  t.b[1][1] = Ld::ld(fr, x.f[2] + zb * x.dzr);
+  t.a[2][0] = Ld::ld(fr, x.f[4] + ra * x.dr);
+  t.b[2][0] = Ld::ld(fr, x.f[4] + rb * x.dr);
+  t.a[2][1] = Ld::ld(fr, x.f[4] + za * x.dz);
+  t.b[2][1] = Ld::ld(fr, x.f[4] + zb * x.dz);
+  t.a[3][0] = Ld::ld(fr, x.f[6] + ra * x.dr);
+  t.b[3][0] = Ld::ld(fr, x.f[6] + rb * x.dr);
+  t.a[3][1] = Ld::ld(fr, x.f[6] + x.tp);  // face 6 along theta
   t.b[3][1] = h.t[6];
 }
 __device__ __forceinline__ double tang_of(const Dims &d, const SeqCell &x, const Tang &t, int dd, int n, double v0) {
@@ -4619,6 +4694,44 @@ __device__ __forceinline__ double tang_of(const Dims &d, const SeqCell &x, const
   const double va = t.a[dd][n], vb = t.b[dd][n];
   return lo ? (-(3 * v0) + 4 * va - vb) / 4. : hi ? (3 * v0 - 4 * va + vb) / 4. : (vb - va) / 4.;
 }
+// a field into its skewed planes and back: blockIdx.y numbers the fields
+struct SkewField {
+  double *f, *c;           // faces (current half), cell averages (null: none)
+  const double *c1, *c2;   // further cell values, to the planes after them
+  double *dst;
+};
+struct SkewFields {
+  SkewField q[3];
+};
+__global__ void __launch_bounds__(BLK) k_seq_skew(Dims d, Skew w, SkewFields A, const Ctrl *ctl) {
+  if (ctl->done) return;
+  const int n = blockIdx.x * BLK + threadIdx.x;
+  if (n >= d.Nc) return;
+  const SkewField &q = A.q[blockIdx.y];
+  const Cell x = Cell::of(d, n);
+  const size_t L = w.L;
+  double *o = q.dst + w.at(x.i, x.j, x.k);
+  for (int dd = 0; dd < 3; ++dd) o[dd * L] = q.f[x.face(d, 2 * dd + 2)];
+  if (x.j == 0) o[-(2 * w.st + 1)] = q.f[x.face(d, 1)];
+  if (x.k == 0) o[2 * (ptrdiff_t)L - (3 * w.st + w.sk)] = q.f[x.face(d, 5)];
+  int m = 3;
+  if (q.c) o[m++ * L] = q.c[n];
+  o[m++ * L] = q.c1[n];
+  if (q.c2) o[m * L] = q.c2[n];
+}
+__global__ void __launch_bounds__(BLK) k_seq_unskew(Dims d, Skew w, SkewFields A, const Ctrl *ctl) {
+  if (ctl->done) return;
+  const int n = blockIdx.x * BLK + threadIdx.x;
+  if (n >= d.Nc) return;
+  const SkewField &q = A.q[blockIdx.y];
+  const Cell x = Cell::of(d, n);
+  const size_t L = w.L;
+  const double *o = q.dst + w.at(x.i, x.j, x.k);
+  for (int dd = 0; dd < 3; ++dd)
+    if (x.has_nb(d, 2 * dd + 2)) q.f[x.face(d, 2 * dd + 2)] = o[dd * L];  // the sweeps write no wall face
+  if (q.c) q.c[n] = o[3 * L];
+}
+
 // stores of the ordered sweeps: plain within a block, in program order and
 // uncached (volatile) where other SMs read
 template <class Ld>
@@ -4632,16 +4745,25 @@ __device__ __forceinline__ void st_seq(double *p, size_t i, double v) {
 // The walk over the levels.  Sweep::fixed(q, x, st) loads into registers what
 // the sweep itself does not change (coefficients, in level order) and
 // Sweep::update(x, st) does the rest; the next level's cell index, and then
-// its fixed values, are fetched before the barrier that opens it.  GRID: all
+// its fixed values, are fetched before the barrier that opens it.  kSeqGrid: all
 // blocks of a cooperative launch share a level; else the block has it alone.
-template <bool GRID, class Sweep>
+template <int MODE, class Sweep>
 __device__ __forceinline__ void walk_levels(const Dims &d, const SeqTab &S, int tid, int nth, Sweep &sw) {
   namespace cg = cooperative_groups;
   const int4 *__restrict__ order = S.order;
-  const int *__restrict__ lstart = S.lstart;  // two entries past the end repeat it
-  int lo = 0, hi = lstart[1], hi1 = lstart[2];
+  const int *__restrict__ lstart = S.lstart;
+  auto cell = [&](const int4 o) {
+    if constexpr (MODE == kSeqSkew)
+      return SeqCell(d, S.skew, o);
+    else
+      return SeqCell(d, o);
+  };
+  // the ends of this level, the next one and the one after, and the next
+  // level's cell: each looked up a level before it is needed
+  auto end = [&](int L) { return lstart[min(L + 1, S.nlev)]; };
+  int lo = 0, hi = end(0), hi1 = end(1), hi2 = end(2);
   bool on = tid < hi, on1 = hi + tid < hi1;
-  SeqCell x(d, order[on ? tid : 0]);
+  SeqCell x = cell(order[on ? tid : 0]);
   int4 o1 = order[on1 ? hi + tid : 0];
   typename Sweep::Fixed st;
   if (on) sw.fixed(tid, x, st);
@@ -4649,7 +4771,7 @@ __device__ __forceinline__ void walk_levels(const Dims &d, const SeqTab &S, int 
     if (on) {
       sw.update(x, st);
       for (int q = lo + tid + nth; q < hi; q += nth) {
-        const SeqCell y(d, order[q]);
+        const SeqCell y = cell(order[q]);
         typename Sweep::Fixed s2;
         sw.fixed(q, y, s2);
         sw.update(y, s2);
@@ -4657,13 +4779,14 @@ __device__ __forceinline__ void walk_levels(const Dims &d, const SeqTab &S, int 
     }
     lo = hi;
     hi = hi1;
-    hi1 = lstart[min(L + 3, S.nlev)];
+    hi1 = hi2;
+    hi2 = end(L + 3);
     on = on1;
-    x = SeqCell(d, o1);
+    x = cell(o1);
     if (on) sw.fixed(lo + tid, x, st);
     on1 = hi + tid < hi1;
     o1 = order[on1 ? hi + tid : 0];
-    if (GRID)
+    if (MODE == kSeqGrid)
       cg::this_grid().sync();
     else
       __syncthreads();
@@ -4680,32 +4803,35 @@ struct SeqVel {
   const double *co, *Bq;
   double w, DT, ev;
   bool first;
+  const double *quo;  // [4][Nc] w over M_F4(1) and M_F(1) of the three faces (FORM 1: over AA_v's diagonals)
   struct Fixed {
-    double a[FORM == 1 ? 54 : 23], dg[6], B[4], oc[4];
+    double a[FORM == 1 ? 54 : 23], wq[4], dg[6], B[4], oc[4];
   };
   __device__ __forceinline__ void fixed(int q, const SeqCell &x, Fixed &s) const {
     const int Nc = d.Nc;
 #pragma unroll
     for (int n = 0; n < (FORM == 1 ? 54 : 23); ++n) s.a[n] = S.vel[n * Nc + q];
 #pragma unroll
+    for (int n = (FORM == 1 ? 1 : 0); n < 4; ++n) s.wq[n] = quo[n * Nc + q];
+#pragma unroll
     for (int n = 0; n < 6; ++n) s.dg[n] = S.dg[n * Nc + q];
     s.B[0] = Bq[x.c];
     s.oc[0] = co[x.c];
 #pragma unroll
     for (int dd = 1; dd <= 3; ++dd) {
-      s.oc[dd] = co[x.nb(d, dd)];
-      if (FORM == 1) s.B[dd] = Bq[x.nb(d, dd)];
+      s.oc[dd] = co[x.nb(dd)];
+      if (FORM == 1) s.B[dd] = Bq[x.nb(dd)];
     }
   }
   __device__ __forceinline__ void update(const SeqCell &x, const Fixed &s) {
     Hood h;
     Tang t;
-    load_hood<Ld>(d, fr, x, h);
+    load_hood<Ld>(fr, x, h);
     if (FORM == 1) load_tang<Ld>(d, fr, x, h, t);
     const double cold = Ld::ld(cv, x.c);
     double c2[4], nw, nf[4];
 #pragma unroll
-    for (int dd = 1; dd <= 3; ++dd) c2[dd] = Ld::ld(cv, x.nb(d, dd));
+    for (int dd = 1; dd <= 3; ++dd) c2[dd] = Ld::ld(cv, x.nb(dd));
     if constexpr (FORM == 1) {
       const double Bij = s.a[6] * s.B[0];
       nw = (1 - w) * cold + w * (-(s.a[0] * h.x[1]) - s.a[1] * h.x[2] - s.a[2] * h.x[3] - s.a[3] * h.x[4] -
@@ -4726,22 +4852,24 @@ struct SeqVel {
           sum = (n == 0) ? -term : sum - term;
         }
         sum = sum - A[11] * (nw - s.oc[0]) - A[13] * (c2[dd] - s.oc[dd]);
-        constexpr int diag[4] = {0, 2, 6, 10};
-        nf[dd] = (1 - w) * h.x[2 * dd] + w / (A[diag[dd] - 1]) * (sum + B1 + B2 + B3 + B4);
+        nf[dd] = (1 - w) * h.x[2 * dd] + s.wq[dd] * (sum + B1 + B2 + B3 + B4);
         if (x.has[dd]) {
           ev = nmax(ev, errv(nf[dd], h.x[2 * dd], first));
           h.x[2 * dd] = nf[dd];
         }
       }
     } else {
-      nw = (1 - w) * cold + (w / s.a[0]) * (+s.a[1] * s.oc[0] + s.a[2] * h.x[1] + s.a[3] * h.x[2] + s.a[4] * h.x[3] +
+      nw = (1 - w) * cold + s.wq[0] * (+s.a[1] * s.oc[0] + s.a[2] * h.x[1] + s.a[3] * h.x[2] + s.a[4] * h.x[3] +
                                             s.a[5] * h.x[4] + s.a[6] * h.x[5] + s.a[7] * h.x[6] + s.B[0]);
 #pragma unroll
       for (int dd = 1; dd <= 3; ++dd) {
         const double *hn = h.of(dd);
-        nf[dd] = face_update_vals<double>([&](int pos) { return h.x[pos]; }, [&](int pos) { return hn[pos]; }, nw,
-                                          c2[dd], s.oc[0], s.oc[dd], s.a + 8 + 5 * (dd - 1), s.dg[2 * (dd - 1)],
-                                          s.dg[2 * (dd - 1) + 1], dd, w);
+        const double *Fd = s.a + 8 + 5 * (dd - 1);
+        const int e1 = tr1(dd), e2 = tr2(dd);  // face_update_vals
+        const double B3 = s.dg[2 * (dd - 1)] * (h.x[2 * e1] - h.x[2 * e1 - 1] + hn[2 * e1] - hn[2 * e1 - 1]) / 4.0;
+        const double B4 = s.dg[2 * (dd - 1) + 1] * (h.x[2 * e2] - h.x[2 * e2 - 1] + hn[2 * e2] - hn[2 * e2 - 1]) / 4.0;
+        nf[dd] = (1 - w) * h.x[2 * dd] + s.wq[dd] * (+Fd[1] * h.x[2 * dd - 1] + Fd[2] * hn[2 * dd] +
+                                                     Fd[3] * (nw + s.oc[0]) + Fd[4] * (c2[dd] + s.oc[dd]) - B3 - B4);
         if (x.has[dd]) {
           ev = nmax(ev, errv(nf[dd], h.x[2 * dd], first));
           h.x[2 * dd] = nf[dd];
@@ -4755,17 +4883,22 @@ struct SeqVel {
       if (x.has[dd]) st_seq<Ld>(fr, x.f[2 * dd], nf[dd]);
   }
 };
-// The three components of a cell touch disjoint data: GRID blocks (CB, 3)
-// run them side by side (threadIdx.y), without GRID each has a block.
-template <int FORM, bool GRID, int TPB>
-__global__ void __launch_bounds__(TPB) k_seq_vel(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
+// The three components of a cell touch disjoint data: a grid's blocks (CB, 3)
+// run them side by side (threadIdx.y), else each has a block.
+template <int FORM, int MODE, int TPB>
+__global__ void __launch_bounds__(TPB, 1) k_seq_vel(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<3>(red);
+  constexpr bool GRID = MODE == kSeqGrid, SKEW = MODE == kSeqSkew;
   const int par = parity(ctl), v = GRID ? threadIdx.y : blockIdx.x;
+  double *b = SKEW ? S.skv + (size_t)(kSkewVel * v) * S.skew.L : nullptr;  // the component's skewed planes
+  const size_t L = S.skew.L;
   SeqVel<FORM, typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{
-      d, S, F.f[v] + (size_t)par * d.NF, F.c[v], F.co[v], F.Bv + (size_t)v * d.Nc, P.w[v], P.DT, 0., ctl->first != 0};
-  walk_levels<GRID>(d, S, GRID ? blockIdx.x * CB + threadIdx.x : threadIdx.x, GRID ? gridDim.x * CB : blockDim.x, sw);
+      d, S, SKEW ? b : F.f[v] + (size_t)par * d.NF, SKEW ? b + 3 * L : F.c[v], SKEW ? b + 4 * L : F.co[v],
+      SKEW ? b + 5 * L : F.Bv + (size_t)v * d.Nc, P.w[v], P.DT, 0., ctl->first != 0,
+      S.vel + (size_t)((FORM == 1 ? 54 : 23) + 4 * v) * d.Nc};
+  walk_levels<MODE>(d, S, GRID ? blockIdx.x * CB + threadIdx.x : threadIdx.x, GRID ? gridDim.x * CB : blockDim.x, sw);
   double e[3] = {0., 0., 0.};
   e[v] = sw.ev;
   block_max<3, 0>(red, e, ctl->err[par]);
@@ -4781,18 +4914,17 @@ struct SeqP {
   double w, ev;
   bool first;
   struct Fixed {
-    double k[4][7], B1[4], B2[4], dg[6];
+    double k[4][kSeqP], rp[4], dg[6];
   };
   __device__ __forceinline__ void fixed(int q, const SeqCell &x, Fixed &s) const {
     const int Nc = d.Nc;
-    const double rp = Rp[x.c];
+    s.rp[0] = Rp[x.c];
 #pragma unroll
     for (int dd = 1; dd <= 3; ++dd) {
       const double *A = S.prs + kSeqP * (dd - 1) * Nc + q;
 #pragma unroll
-      for (int n = 0; n < 7; ++n) s.k[dd][n] = A[n * Nc];
-      s.B1[dd] = rp * A[7 * Nc];
-      s.B2[dd] = Rp[x.nb(d, dd)] * A[8 * Nc];
+      for (int n = 0; n < kSeqP; ++n) s.k[dd][n] = A[n * Nc];
+      s.rp[dd] = Rp[x.nb(dd)];
     }
 #pragma unroll
     for (int n = 0; n < 6; ++n) s.dg[n] = S.dg[n * Nc + q];
@@ -4800,7 +4932,7 @@ struct SeqP {
   __device__ __forceinline__ void update(const SeqCell &x, const Fixed &s) {
     Hood h;
     Tang t;
-    load_hood<Ld>(d, pr, x, h);
+    load_hood<Ld>(pr, x, h);
     load_tang<Ld>(d, pr, x, h, t);
     double nf[4];
 #pragma unroll
@@ -4816,7 +4948,7 @@ struct SeqP {
         const double term = K.at(dd, fpos, cell) * (cell == 1 ? h.x[fpos] : hn[fpos]);
         sum = (n == 0) ? -term : sum - term;
       }
-      nf[dd] = (1 - w) * h.x[2 * dd] + k[6] * (sum + s.B1[dd] + s.B2[dd] + B3 + B4);
+      nf[dd] = (1 - w) * h.x[2 * dd] + k[6] * (sum + s.rp[0] * k[7] + s.rp[dd] * k[8] + B3 + B4);
       if (x.has[dd]) {
         ev = nmax(ev, errv(nf[dd], h.x[2 * dd], first));
         h.x[2 * dd] = nf[dd];
@@ -4827,15 +4959,17 @@ struct SeqP {
       if (x.has[dd]) st_seq<Ld>(pr, x.f[2 * dd], nf[dd]);
   }
 };
-template <bool GRID, int TPB>
-__global__ void __launch_bounds__(TPB) k_seq_p(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
+template <int MODE, int TPB>
+__global__ void __launch_bounds__(TPB, 1) k_seq_p(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
+  constexpr bool GRID = MODE == kSeqGrid, SKEW = MODE == kSeqSkew;
   const int par = parity(ctl);
-  SeqP<typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{d, S, F.f[3] + (size_t)par * d.NF, F.Rp, P.w_p, 0.,
-                                                                   ctl->first != 0};
-  walk_levels<GRID>(d, S, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sw);
+  SeqP<typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{
+      d, S, SKEW ? S.skp : F.f[3] + (size_t)par * d.NF, SKEW ? S.skp + 3 * (size_t)S.skew.L : F.Rp, P.w_p, 0.,
+      ctl->first != 0};
+  walk_levels<MODE>(d, S, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sw);
   const double e[1] = {sw.ev};
   block_max<1, 0>(red, e, ctl->err[par] + 3);
 }
@@ -4860,15 +4994,15 @@ struct SeqT {
     for (int n = 0; n < 6; ++n) s.dg[n] = S.dg[n * Nc + q];
     s.oc[0] = co[x.c];
 #pragma unroll
-    for (int dd = 1; dd <= 3; ++dd) s.oc[dd] = co[x.nb(d, dd)];
+    for (int dd = 1; dd <= 3; ++dd) s.oc[dd] = co[x.nb(dd)];
   }
   __device__ __forceinline__ void update(const SeqCell &x, const Fixed &s) {
     Hood h;
-    load_hood<Ld>(d, T, x, h);
+    load_hood<Ld>(T, x, h);
     const double cold = Ld::ld(cv, x.c);
     double c2[4], nf[4];
 #pragma unroll
-    for (int dd = 1; dd <= 3; ++dd) c2[dd] = Ld::ld(cv, x.nb(d, dd));
+    for (int dd = 1; dd <= 3; ++dd) c2[dd] = Ld::ld(cv, x.nb(dd));
     const double nw = (1 - w) * cold + s.a[0] * (+s.a[1] * s.oc[0] + s.a[2] * h.x[1] + s.a[3] * h.x[2] +
                                                  s.a[4] * h.x[3] + s.a[5] * h.x[4] + s.a[6] * h.x[5] +
                                                  s.a[7] * h.x[6] + (s.a[23] + 0.));
@@ -4892,15 +5026,17 @@ struct SeqT {
       if (x.has[dd]) st_seq<Ld>(T, x.f[2 * dd], nf[dd]);
   }
 };
-template <bool GRID, int TPB>
-__global__ void __launch_bounds__(TPB) k_seq_T(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
+template <int MODE, int TPB>
+__global__ void __launch_bounds__(TPB, 1) k_seq_T(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
+  constexpr bool GRID = MODE == kSeqGrid, SKEW = MODE == kSeqSkew;
   const int par = parity(ctl);
   SeqT<typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{
-      d, S, F.f[4] + (size_t)par * d.NF, F.c[3], F.co[3], P.w[3], 0., ctl->first != 0};
-  walk_levels<GRID>(d, S, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sw);
+      d, S, SKEW ? S.skt : F.f[4] + (size_t)par * d.NF, SKEW ? S.skt + 3 * (size_t)S.skew.L : F.c[3],
+      SKEW ? S.skt + 4 * (size_t)S.skew.L : F.co[3], P.w[3], 0., ctl->first != 0};
+  walk_levels<MODE>(d, S, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sw);
   const double e[1] = {sw.ev};
   block_max<1, 0>(red, e, ctl->err[par] + 4);
 }
