@@ -95,7 +95,7 @@ struct nim_ctx {
   // reference-order schedule
   bool seq = false;
   SeqTab seqt{};
-  int seq_mode = 0;                          // kSeqBlock, kSeqGrid or kSeqSkew
+  int seq_mode = 0;                          // kSeqShared, kSeqGrid or kSeqSkew
   int seq_threads = 0, wall_threads = 0;     // block sizes of the one-block sweeps
   int coop_vel = 0, coop_p = 0, coop_T = 0;  // cooperative grid sizes
   // nim_gpu_profile_iterations: while set, every kernel launch of an
@@ -385,6 +385,8 @@ int launch_iteration_seq(nim_ctx *x) {
   const bool one = x->phys.formulation == 1, grid_form = x->seq_mode == kSeqGrid, skewed = x->seq_mode == kSeqSkew;
   const int nt = x->seq_threads;
   const bool wide = nt > SEQ_TPB;
+  const bool shared = x->seq_mode == kSeqShared;
+  const size_t smf = shared ? sizeof(double) * d.NF : 0, smc = shared ? smf + sizeof(double) * d.Nc : 0;  // faces; and averages
   if (one)
     k_vel_cell<true, 1><<<x->g3, dim3(CB, 3), 0, s>>>(d, x->g, x->F, x->phys, x->ctl);
   else
@@ -407,20 +409,20 @@ int launch_iteration_seq(nim_ctx *x) {
   else if (skewed)
     (one ? k_seq_vel<1, kSeqSkew, SEQ_TPB> : k_seq_vel<2, kSeqSkew, SEQ_TPB>)<<<3, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   else
-    (one ? k_seq_vel<1, kSeqBlock, SEQ_TPB> : k_seq_vel<2, kSeqBlock, SEQ_TPB>)<<<3, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+    (one ? k_seq_vel<1, kSeqShared, SEQ_TPB> : k_seq_vel<2, kSeqShared, SEQ_TPB>)<<<3, nt, smc, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   if (skewed) k_seq_unskew<<<gv, BLK, 0, s>>>(d, S.skew, sv, x->ctl);
   TRY(mark(x, "k_seq_vel"));
   k_p_src<<<x->g3, dim3(CB, 3), 0, s>>>(d, x->g, x->F, x->phys, x->ctl);
   TRY(mark(x, "k_p_src"));
   k_p_bc_fixed<<<x->nblk_b, BLK, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
-  k_seq_pbc<<<2, x->wall_threads, 0, s>>>(d, x->F, x->phys, x->ctl, S, 0);
-  k_seq_pbc<<<2, x->wall_threads, 0, s>>>(d, x->F, x->phys, x->ctl, S, 2);
+  (shared ? k_seq_pbc<true> : k_seq_pbc<false>)<<<2, x->wall_threads, smf, s>>>(d, x->F, x->phys, x->ctl, S, 0);
+  (shared ? k_seq_pbc<true> : k_seq_pbc<false>)<<<2, x->wall_threads, smf, s>>>(d, x->F, x->phys, x->ctl, S, 2);
   TRY(mark(x, "k_seq_pbc"));
   if (skewed) k_seq_skew<<<g1, BLK, 0, s>>>(d, S.skew, sp, x->ctl);
   if (grid_form)
     TRY(launch_coop(k_seq_p<kSeqGrid, BLK>, x->coop_p, dim3(BLK), x));
   else
-    (!skewed ? k_seq_p<kSeqBlock, SEQ_TPB> : wide ? k_seq_p<kSeqSkew, SEQ_TPB_WIDE> : k_seq_p<kSeqSkew, SEQ_TPB>)<<<1, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+    (!skewed ? k_seq_p<kSeqShared, SEQ_TPB> : wide ? k_seq_p<kSeqSkew, SEQ_TPB_WIDE> : k_seq_p<kSeqSkew, SEQ_TPB>)<<<1, nt, smf, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   if (skewed) k_seq_unskew<<<g1, BLK, 0, s>>>(d, S.skew, sp, x->ctl);
   TRY(mark(x, "k_seq_p"));
   if (x->phys.dpdx_tolerance) {
@@ -437,7 +439,7 @@ int launch_iteration_seq(nim_ctx *x) {
   if (grid_form)
     TRY(launch_coop(k_seq_T<kSeqGrid, BLK>, x->coop_T, dim3(BLK), x));
   else
-    (!skewed ? k_seq_T<kSeqBlock, SEQ_TPB> : wide ? k_seq_T<kSeqSkew, SEQ_TPB_WIDE> : k_seq_T<kSeqSkew, SEQ_TPB>)<<<1, nt, 0, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
+    (!skewed ? k_seq_T<kSeqShared, SEQ_TPB> : wide ? k_seq_T<kSeqSkew, SEQ_TPB_WIDE> : k_seq_T<kSeqSkew, SEQ_TPB>)<<<1, nt, smc, s>>>(d, x->g, x->F, x->phys, x->ctl, S);
   if (skewed) k_seq_unskew<<<g1, BLK, 0, s>>>(d, S.skew, st, x->ctl);
   TRY(mark(x, "k_seq_T"));
   k_iter_end<<<1, 1, 0, s>>>(x->ctl, x->phys, 0);
@@ -450,18 +452,18 @@ int launch_iteration_seq(nim_ctx *x) {
 
 // a step's velocity constants in level order
 int seq_pack_velocity(nim_ctx *x) {
+  const int R = (x->phys.formulation == 1 ? kSeqV<1> : kSeqV<2>) + 12;
   const SeqTab &S = x->seqt;
   const int Nc = x->d.Nc;
   const bool one = x->phys.formulation == 1;
   const double *src[2] = {one ? x->F.AT : x->F.MF4, one ? x->F.AAv : x->F.MF};
   const int rows[2] = {one ? 9 : 8, one ? 45 : 15};
-  k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(src[0], S.vel, S.order, rows[0], Nc);
-  k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(src[1], S.vel + (size_t)rows[0] * Nc, S.order, rows[1], Nc);
-  double *quo = S.vel + (size_t)(one ? 54 : 23) * Nc;
+  k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(src[0], S.vel, S.order, rows[0], 0, R, Nc);
+  k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(src[1], S.vel, S.order, rows[1], rows[0], R, Nc);
   const double *A = x->F.AAv, *M = x->F.MF;
   const size_t n = Nc;
   k_seq_pack_quo<<<x->nblk_c, BLK, 0, x->stream>>>(one ? nullptr : x->F.MF4, one ? A + n : M, one ? A + 20 * n : M + 5 * n,
-                                                   one ? A + 39 * n : M + 10 * n, quo, x->phys, S.order, Nc);
+                                                   one ? A + 39 * n : M + 10 * n, S.vel, x->phys, S.order, R - 12, R, Nc);
   CK(cudaGetLastError());
   x->launches += 3;
   return NIM_OK;
@@ -470,7 +472,7 @@ int seq_pack_velocity(nim_ctx *x) {
 // constants and the wall faces' stencils
 int seq_pack_geometry(nim_ctx *x) {
   const SeqTab &S = x->seqt;
-  k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(x->g.dg, S.dg, S.order, 6, x->d.Nc);
+  k_seq_pack<<<x->nblk_c, BLK, 0, x->stream>>>(x->g.dg, S.dg, S.order, 6, 0, 6, x->d.Nc);
   k_seq_pack_p<<<x->nblk_c, BLK, 0, x->stream>>>(x->d, x->g, x->phys, S);
   k_seq_pack_wall<<<x->nblk_b, BLK, 0, x->stream>>>(x->d, S);
   CK(cudaGetLastError());
@@ -932,9 +934,10 @@ static int noalloc_setup(int device) {
 // numbers (the argument is in nim_kernels.cuh).  Wall faces, in BC-list
 // order bottom, top, inner, outer: level i + 2j on bottom and top, i + 2k on
 // inner and outer.  Also the sweep buffers and the cooperative grid sizes.
-// widest level swept by one block, and from where on it works on skewed copies
-// (measured beside the sweeps)
-constexpr int kSeqBlockMost = 1024, kSeqSkewFrom = 96;
+// widest level swept by one block, and the most its fields may take of its
+// shared memory (what 227 KB leave beside the block's reductions)
+constexpr int kSeqBlockMost = 1024;
+constexpr size_t kSeqSharedMost = 224 * 1024;
 static int setup_levels(nim_ctx *x) {
   const Dims &d = x->d;
   const size_t Nc = d.Nc;
@@ -980,12 +983,13 @@ static int setup_levels(nim_ctx *x) {
   TRY(dalloc(x, &S.border, (size_t)d.NBF));
   TRY(dalloc(x, &S.blev, blev.size()));
   TRY(dalloc(x, &S.wlev, wlev.size()));
-  TRY(dalloc(x, &S.dg, 6 * Nc));
-  TRY(dalloc(x, &S.vel, (x->phys.formulation == 1 ? 66 : 35) * Nc));
-  TRY(dalloc(x, &S.prs, 3 * kSeqP * Nc));
-  TRY(dalloc(x, &S.tmp, kSeqT * Nc));
-  TRY(dalloc(x, &S.wall, kSeqW * (size_t)d.NBF));
-  TRY(dalloc(x, &S.wface, kSeqI * (size_t)d.NBF));
+  auto table = [](int n, int rows) { return seq_at((n + 31) / 32 * 32, rows); };  // values of a table of n entries
+  TRY(dalloc(x, &S.dg, table(d.Nc, 6)));
+  TRY(dalloc(x, &S.vel, table(d.Nc, (x->phys.formulation == 1 ? kSeqV<1> : kSeqV<2>) + 12)));
+  TRY(dalloc(x, &S.prs, table(d.Nc, 3 * kSeqP)));
+  TRY(dalloc(x, &S.tmp, table(d.Nc, kSeqT)));
+  TRY(dalloc(x, &S.wall, table(d.NBF, kSeqW)));
+  TRY(dalloc(x, &S.wface, table(d.NBF, kSeqI)));
   CK(cudaMemcpy(S.order, order.data(), sizeof(int4) * Nc, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(S.lstart, lstart.data(), sizeof(int) * (nlev + 1), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(S.border, border.data(), sizeof(int) * d.NBF, cudaMemcpyHostToDevice));
@@ -998,8 +1002,19 @@ static int setup_levels(nim_ctx *x) {
   for (size_t L = 0; L + 1 < blev.size(); ++L) wmax = std::max(wmax, blev[L + 1] - blev[L]);
   x->seq_threads = warps(maxlev, SEQ_TPB_WIDE);
   x->wall_threads = warps(wmax, BLK);
-  x->seq_mode = maxlev > kSeqBlockMost ? kSeqGrid : maxlev > kSeqSkewFrom ? kSeqSkew : kSeqBlock;
-  if (x->seq_mode == kSeqBlock) return NIM_OK;
+  const size_t smc = sizeof(double) * ((size_t)d.NF + Nc);
+  x->seq_mode = maxlev > kSeqBlockMost ? kSeqGrid : smc <= kSeqSharedMost ? kSeqShared : kSeqSkew;
+  if (x->seq_mode == kSeqShared) {
+    x->seq_threads = std::min(x->seq_threads, SEQ_TPB);
+    auto room = [&](auto kern) {
+      return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSharedMost);
+    };
+    CK(room(x->phys.formulation == 1 ? k_seq_vel<1, kSeqShared, SEQ_TPB> : k_seq_vel<2, kSeqShared, SEQ_TPB>));
+    CK(room(k_seq_p<kSeqShared, SEQ_TPB>));
+    CK(room(k_seq_T<kSeqShared, SEQ_TPB>));
+    CK(room(k_seq_pbc<true>));
+    return NIM_OK;
+  }
   if (x->seq_mode == kSeqSkew) {
     S.skew.sk = d.NR + 1;
     S.skew.st = (d.NZ + 1) * S.skew.sk;

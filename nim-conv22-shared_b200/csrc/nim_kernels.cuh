@@ -4457,19 +4457,22 @@ __global__ void __launch_bounds__(BLK) k_convert(CvtList L) {
 // Levels that fit a block run in one block per swept field, whose barrier is
 // the SM's own and whose loads hit its L1; wider ones on a cooperative grid
 // (the three velocity components side by side), which reads through L2.
-// In one block a wide level is bound by L1 lines: its cells lie apart in the
-// fields, 32 lines a load.  From kSeqSkewFrom cells on the block therefore
-// works on skewed copies (below); a narrow level waits on latency instead,
-// neighbouring levels share the fields' lines, and the copies' six launches
-// do not come back (36x6x12, 66 wide: 443 us a pass without, 526 with;
-// 24x24x16 formulation 1, 168 wide: 896 without, 835 with).  The divisions by
+// Where a field's faces and averages fit the block's shared memory (up to
+// about 6800 cells), the block sweeps a copy there, whose loads take a tenth
+// of the first touch of an L2 line (36x6x12: 431 us a pass over the fields
+// themselves, 362 over the copy).  Else it works on skewed copies (below):
+// over the fields a wide level is bound by L1 lines, since its cells lie
+// apart, 32 lines a load (24x24x16 formulation 1, 168 wide: 896 us over the
+// fields, 835 over the copies; 48x48x32, 672 wide: 5.0 and 3.5 ms).
+// What is left is the issue of one or two warps: some 450 instructions a cell,
+// so the tables are laid out for constant offsets (seq_at), the divisions by
 // what a step or the run keeps are done once, with the packing, and nothing
 // is computed from a level's constants before the barrier, where it would
-// wait for their loads.
+// wait for their loads.  Fetching them two levels ahead gave nothing.
 // Time of a pass with dependent loads and a grid barrier a level, then loads
-// up front in one block, and now: 36x6x12 1891 -> 486 -> 431 us, 24x24x16
-// formulation 1 3882 -> 939 -> 824 us, 48x48x32 (672 wide) 10.3 -> 5.0 ->
-// 3.5 ms, 128x128x96 (grid) 35.2 -> 20.6 -> 19.8 ms.
+// up front in one block, and now: 36x6x12 1891 -> 486 -> 340 us, 24x24x16
+// formulation 1 3882 -> 939 -> 790 us, 48x48x32 (672 wide) 10.3 -> 5.0 ->
+// 3.4 ms, 128x128x96 (grid) 35.2 -> 20.6 -> 18.6 ms.
 
 // Skewed copies of the swept fields (one block over wide levels): cell (i, j, k) of
 // level t = i + 2j + 3k at t st + (k + 1) sk + j + 1, its +xi faces in three
@@ -4493,7 +4496,7 @@ struct SeqTab {
   int *lstart;          // level starts
   int nlev;
   int *border, *blev, *wlev;  // wall faces, levels, per-wall level ranges
-  // rows in level order, [row][Nc]: the face-metric differences dg (6); the
+  // tables in level order (seq_at): the face-metric differences dg (6); the
   // velocity constants of a step (formulation 2: M_F4 (8), M_F1..3 (15);
   // 1: a_t (9), AA_v (45)) and the relaxation factors of u, v, w over their
   // divisors (4 each); the pressure constants (kSeqP a direction); the
@@ -4501,41 +4504,51 @@ struct SeqTab {
   double *dg, *vel, *prs, *tmp;
   // in border order: the faces a wall face's update reads and the
   // constants of apply_pressure_bc in this pass
-  int *wface;    // [kSeqI][NBF]
-  double *wall;  // [kSeqW][NBF]
+  int *wface;    // kSeqI rows
+  double *wall;  // kSeqW rows
   // skewed copies of u, v, w, of p and of T (null where the sweeps work on
   // the fields themselves)
   Skew skew;
   double *skv, *skp, *skt;
 };
-// how a sweep runs: one block over the fields themselves, all blocks of a
-// cooperative launch, one block over skewed copies
-enum { kSeqBlock, kSeqGrid, kSeqSkew };
+// how a sweep runs: one block over a copy in its shared memory, all blocks of
+// a cooperative launch over the fields themselves, one block over skewed copies
+enum { kSeqShared, kSeqGrid, kSeqSkew };
 constexpr int kSeqI = 11;  // the face, its cell's other five, two stencils (a, b) along the wall, wall-end flags
+template <int FORM>
+constexpr int kSeqV = FORM == 1 ? 54 : 23;  // velocity rows before the 12 quotients
 constexpr int kSeqP = 9;   // m, a1, a2, mq, a1q, a2q, w/diag, b, bq of one direction
 constexpr int kSeqT = 24;  // w/MT_F4(0), MT_F4(1..7), (w/MT_F(0), MT_F(1..4)) x 3, R_D_T
 constexpr int kSeqW = 10;  // w/ap(pos), B1, body, the two bcg, the five ap of the other faces
 
-// dst[row][q] = src[row][order[q]]: rows of a per-cell array into level order
+// The level-order tables lie in groups of 32 entries with all their rows, 32
+// values a row: a warp's loads stay coalesced and a thread's rows are at
+// constant distances from the first, where [row][Nc] would cost the sweeps
+// an address a load (half of their instructions were integer; a pass at
+// 36x6x12 365 -> 340 us, at 128x128x96 19.4 -> 18.6 ms).  seq_at(q, R): where entry q of a table of R rows starts.
+__host__ __device__ __forceinline__ size_t seq_at(int q, int R) { return (size_t)(q >> 5) * (32 * R) + (q & 31); }
+// rows of a per-cell array into level order, to rows r0.. of a table of R rows
 __global__ void __launch_bounds__(BLK) k_seq_pack(const double *__restrict__ src, double *__restrict__ dst,
-                                                  const int4 *__restrict__ order, int rows, int Nc) {
+                                                  const int4 *__restrict__ order, int rows, int r0, int R, int Nc) {
   const int q = blockIdx.x * BLK + threadIdx.x;
   if (q >= Nc) return;
   const int c = order[q].x;
-  for (int r = 0; r < rows; ++r) dst[(size_t)r * Nc + q] = src[(size_t)r * Nc + c];
+  double *o = dst + seq_at(q, R) + 32 * r0;
+  for (int r = 0; r < rows; ++r) o[32 * r] = src[(size_t)r * Nc + c];
 }
-// w / div[order[q]] of the three components, for rows r of div: dst[4 v + r]
+// w / div[order[q]] of the three components, for rows r of div: row r0 + 4 v + r
 __global__ void __launch_bounds__(BLK) k_seq_pack_quo(const double *d0, const double *d1, const double *d2,
                                                       const double *d3, double *__restrict__ dst, Phys P,
-                                                      const int4 *__restrict__ order, int Nc) {
+                                                      const int4 *__restrict__ order, int r0, int R, int Nc) {
   const int q = blockIdx.x * BLK + threadIdx.x;
   if (q >= Nc) return;
   const int c = order[q].x;
+  double *o = dst + seq_at(q, R) + 32 * r0;
   const double *div[4] = {d0, d1, d2, d3};
   for (int r = 0; r < 4; ++r) {
     if (!div[r]) continue;
     const double v = div[r][c];
-    for (int n = 0; n < 3; ++n) dst[(size_t)(4 * n + r) * Nc + q] = P.w[n] / v;
+    for (int n = 0; n < 3; ++n) o[32 * (4 * n + r)] = P.w[n] / v;
   }
 }
 // the pressure sweep's constants in level order, once at init
@@ -4547,7 +4560,7 @@ __global__ void __launch_bounds__(BLK) k_seq_pack_p(Dims d, Geo g, Phys P, SeqTa
     if (!x.has_nb(d, 2 * dd)) continue;
     const PFaceCoef<double> K = p_face_coef(g, Nc, x.c, x.nb(d, 2 * dd).c, dd);
     const double v[kSeqP] = {K.m, K.a1, K.a2, K.mq, K.a1q, K.a2q, P.w_p / K.diag, K.b, K.bq};
-    for (int n = 0; n < kSeqP; ++n) S.prs[(size_t)(kSeqP * (dd - 1) + n) * Nc + q] = v[n];
+    for (int n = 0; n < kSeqP; ++n) S.prs[seq_at(q, 3 * kSeqP) + 32 * (kSeqP * (dd - 1) + n)] = v[n];
   }
 }
 // calculate_R_D_T (nse.f90:2000-2134) and the temperature sweep's constants
@@ -4568,19 +4581,19 @@ __global__ void __launch_bounds__(BLK) k_T_src(Dims d, Geo g, Fields F, Phys P, 
     p[n] = F.MT4[(3 * n + 2) * Nc + c];
   }
   T_form_F4(r, m, p, P.DT, F4);
-  double *o = S.tmp + q;
+  double *o = S.tmp + seq_at(q, kSeqT);
   o[0] = w / F4[0];
-  for (int k = 1; k < 8; ++k) o[k * Nc] = F4[k];
+  for (int k = 1; k < 8; ++k) o[32 * k] = F4[k];
   for (int dd = 1; dd <= 3; ++dd) {
     if (!x.has_nb(d, 2 * dd)) continue;
     double Fd[5];
     T_form_Fd(F, Nc, c, x.nb(d, 2 * dd).c, dd, Fd);
-    double *of = o + (8 + 5 * (dd - 1)) * Nc;
+    double *of = o + 32 * (8 + 5 * (dd - 1));
     of[0] = w / Fd[0];
-    for (int k = 1; k < 5; ++k) of[k * Nc] = Fd[k];
+    for (int k = 1; k < 5; ++k) of[32 * k] = Fd[k];
   }
   const double *T = F.f[4] + (size_t)parity(ctl) * d.NF;
-  o[23 * Nc] = P.alpha * diffusion_source(d, g, T, x, f);
+  o[32 * 23] = P.alpha * diffusion_source(d, g, T, x, f);
 }
 
 // a cell of a level: where its values are, and the index steps to those of
@@ -4758,18 +4771,13 @@ __device__ __forceinline__ void walk_levels(const Dims &d, const SeqTab &S, int 
     else
       return SeqCell(d, o);
   };
-  // the ends of this level, the next one and the one after, and the next
-  // level's cell: each looked up a level before it is needed
+  // the ends of this level and of the next ones, and the next levels' cells:
+  // each looked up a level before it is needed
   auto end = [&](int L) { return lstart[min(L + 1, S.nlev)]; };
-  int lo = 0, hi = end(0), hi1 = end(1), hi2 = end(2);
-  bool on = tid < hi, on1 = hi + tid < hi1;
-  SeqCell x = cell(order[on ? tid : 0]);
-  int4 o1 = order[on1 ? hi + tid : 0];
-  typename Sweep::Fixed st;
-  if (on) sw.fixed(tid, x, st);
-  for (int L = 0; L < S.nlev; ++L) {
-    if (on) {
-      sw.update(x, st);
+  auto entry = [&](int q, int hi) { return order[q < hi ? q : 0]; };
+  auto level = [&](int lo, int hi, const int4 o, const typename Sweep::Fixed &st) {
+    if (lo + tid < hi) {
+      sw.update(cell(o), st);
       for (int q = lo + tid + nth; q < hi; q += nth) {
         const SeqCell y = cell(order[q]);
         typename Sweep::Fixed s2;
@@ -4777,20 +4785,43 @@ __device__ __forceinline__ void walk_levels(const Dims &d, const SeqTab &S, int 
         sw.update(y, s2);
       }
     }
+  };
+  auto load = [&](int lo, int hi, const int4 o, typename Sweep::Fixed &st) {
+    if (lo + tid < hi) sw.fixed(lo + tid, cell(o), st);
+  };
+  int lo = 0, hi = end(0), hi1 = end(1), hi2 = end(2);
+  int4 o = entry(tid, hi), o1 = entry(hi + tid, hi1);
+  typename Sweep::Fixed st;
+  load(lo, hi, o, st);
+  for (int L = 0; L < S.nlev; ++L) {
+    level(lo, hi, o, st);
     lo = hi;
     hi = hi1;
     hi1 = hi2;
     hi2 = end(L + 3);
-    on = on1;
-    x = cell(o1);
-    if (on) sw.fixed(lo + tid, x, st);
-    on1 = hi + tid < hi1;
-    o1 = order[on1 ? hi + tid : 0];
+    o = o1;
+    load(lo, hi, o, st);
+    o1 = entry(hi + tid, hi1);
     if (MODE == kSeqGrid)
       cg::this_grid().sync();
     else
       __syncthreads();
   }
+}
+
+// n values into the block's shared memory and back, two a load where the
+// source allows it
+extern __shared__ double seq_sm[];
+__device__ __forceinline__ void seq_copy(double *__restrict__ dst, const double *__restrict__ src, int n) {
+  int a = 0;
+  if ((((size_t)src | (size_t)dst) & 15) == 0) {
+    a = n & ~1;
+    const double2 *v = (const double2 *)src;
+    double2 *o = (double2 *)dst;
+#pragma unroll 4
+    for (int q = threadIdx.x; q < a / 2; q += blockDim.x) o[q] = v[q];
+  }
+  for (int q = a + threadIdx.x; q < n; q += blockDim.x) dst[q] = src[q];
 }
 
 // velocity sweep of one component (integrate_velocity_field_formulation2_i,
@@ -4803,18 +4834,19 @@ struct SeqVel {
   const double *co, *Bq;
   double w, DT, ev;
   bool first;
-  const double *quo;  // [4][Nc] w over M_F4(1) and M_F(1) of the three faces (FORM 1: over AA_v's diagonals)
+  const double *quo;  // the component's rows of S.vel: w over M_F4(1) and M_F(1) of the three faces (FORM 1: over AA_v's diagonals)
   struct Fixed {
-    double a[FORM == 1 ? 54 : 23], wq[4], dg[6], B[4], oc[4];
+    double a[kSeqV<FORM>], wq[4], dg[6], B[4], oc[4];
   };
   __device__ __forceinline__ void fixed(int q, const SeqCell &x, Fixed &s) const {
-    const int Nc = d.Nc;
+    const size_t at = seq_at(q, kSeqV<FORM> + 12);
+    const double *A = S.vel + at, *W = quo + at, *G = S.dg + seq_at(q, 6);
 #pragma unroll
-    for (int n = 0; n < (FORM == 1 ? 54 : 23); ++n) s.a[n] = S.vel[n * Nc + q];
+    for (int n = 0; n < kSeqV<FORM>; ++n) s.a[n] = A[32 * n];
 #pragma unroll
-    for (int n = (FORM == 1 ? 1 : 0); n < 4; ++n) s.wq[n] = quo[n * Nc + q];
+    for (int n = (FORM == 1 ? 1 : 0); n < 4; ++n) s.wq[n] = W[32 * n];
 #pragma unroll
-    for (int n = 0; n < 6; ++n) s.dg[n] = S.dg[n * Nc + q];
+    for (int n = 0; n < 6; ++n) s.dg[n] = G[32 * n];
     s.B[0] = Bq[x.c];
     s.oc[0] = co[x.c];
 #pragma unroll
@@ -4894,11 +4926,22 @@ __global__ void __launch_bounds__(TPB, 1) k_seq_vel(Dims d, Geo g, Fields F, Phy
   const int par = parity(ctl), v = GRID ? threadIdx.y : blockIdx.x;
   double *b = SKEW ? S.skv + (size_t)(kSkewVel * v) * S.skew.L : nullptr;  // the component's skewed planes
   const size_t L = S.skew.L;
+  constexpr bool SH = MODE == kSeqShared;
+  double *const f = F.f[v] + (size_t)par * d.NF, *const c = F.c[v];
+  if (SH) {
+    seq_copy(seq_sm, f, d.NF);
+    seq_copy(seq_sm + d.NF, c, d.Nc);
+    __syncthreads();
+  }
   SeqVel<FORM, typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{
-      d, S, SKEW ? b : F.f[v] + (size_t)par * d.NF, SKEW ? b + 3 * L : F.c[v], SKEW ? b + 4 * L : F.co[v],
+      d, S, SH ? seq_sm : SKEW ? b : f, SH ? seq_sm + d.NF : SKEW ? b + 3 * L : c, SKEW ? b + 4 * L : F.co[v],
       SKEW ? b + 5 * L : F.Bv + (size_t)v * d.Nc, P.w[v], P.DT, 0., ctl->first != 0,
-      S.vel + (size_t)((FORM == 1 ? 54 : 23) + 4 * v) * d.Nc};
+      S.vel + 32 * (kSeqV<FORM> + 4 * v)};
   walk_levels<MODE>(d, S, GRID ? blockIdx.x * CB + threadIdx.x : threadIdx.x, GRID ? gridDim.x * CB : blockDim.x, sw);
+  if (SH) {
+    seq_copy(f, seq_sm, d.NF);
+    seq_copy(c, seq_sm + d.NF, d.Nc);
+  }
   double e[3] = {0., 0., 0.};
   e[v] = sw.ev;
   block_max<3, 0>(red, e, ctl->err[par]);
@@ -4917,17 +4960,17 @@ struct SeqP {
     double k[4][kSeqP], rp[4], dg[6];
   };
   __device__ __forceinline__ void fixed(int q, const SeqCell &x, Fixed &s) const {
-    const int Nc = d.Nc;
+    const double *G = S.dg + seq_at(q, 6);
     s.rp[0] = Rp[x.c];
 #pragma unroll
     for (int dd = 1; dd <= 3; ++dd) {
-      const double *A = S.prs + kSeqP * (dd - 1) * Nc + q;
+      const double *A = S.prs + seq_at(q, 3 * kSeqP) + 32 * (kSeqP * (dd - 1));
 #pragma unroll
-      for (int n = 0; n < kSeqP; ++n) s.k[dd][n] = A[n * Nc];
+      for (int n = 0; n < kSeqP; ++n) s.k[dd][n] = A[32 * n];
       s.rp[dd] = Rp[x.nb(dd)];
     }
 #pragma unroll
-    for (int n = 0; n < 6; ++n) s.dg[n] = S.dg[n * Nc + q];
+    for (int n = 0; n < 6; ++n) s.dg[n] = G[32 * n];
   }
   __device__ __forceinline__ void update(const SeqCell &x, const Fixed &s) {
     Hood h;
@@ -4965,13 +5008,19 @@ __global__ void __launch_bounds__(TPB, 1) k_seq_p(Dims d, Geo g, Fields F, Phys 
   __shared__ BlockRed red;
   red_init<1>(red);
   constexpr bool GRID = MODE == kSeqGrid, SKEW = MODE == kSeqSkew;
-  const int par = parity(ctl);
+  constexpr bool SH = MODE == kSeqShared;
+  double *const f = F.f[3] + (size_t)parity(ctl) * d.NF;
+  if (SH) {
+    seq_copy(seq_sm, f, d.NF);
+    __syncthreads();
+  }
   SeqP<typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{
-      d, S, SKEW ? S.skp : F.f[3] + (size_t)par * d.NF, SKEW ? S.skp + 3 * (size_t)S.skew.L : F.Rp, P.w_p, 0.,
+      d, S, SH ? seq_sm : SKEW ? S.skp : f, SKEW ? S.skp + 3 * (size_t)S.skew.L : F.Rp, P.w_p, 0.,
       ctl->first != 0};
   walk_levels<MODE>(d, S, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sw);
+  if (SH) seq_copy(f, seq_sm, d.NF);
   const double e[1] = {sw.ev};
-  block_max<1, 0>(red, e, ctl->err[par] + 3);
+  block_max<1, 0>(red, e, ctl->err[parity(ctl)] + 3);
 }
 
 // temperature sweep (integrate_temperature_field_formulation2_i, nse.f90:1009-1089)
@@ -4987,11 +5036,11 @@ struct SeqT {
     double a[kSeqT], dg[6], oc[4];
   };
   __device__ __forceinline__ void fixed(int q, const SeqCell &x, Fixed &s) const {
-    const int Nc = d.Nc;
+    const double *A = S.tmp + seq_at(q, kSeqT), *G = S.dg + seq_at(q, 6);
 #pragma unroll
-    for (int n = 0; n < kSeqT; ++n) s.a[n] = S.tmp[n * Nc + q];
+    for (int n = 0; n < kSeqT; ++n) s.a[n] = A[32 * n];
 #pragma unroll
-    for (int n = 0; n < 6; ++n) s.dg[n] = S.dg[n * Nc + q];
+    for (int n = 0; n < 6; ++n) s.dg[n] = G[32 * n];
     s.oc[0] = co[x.c];
 #pragma unroll
     for (int dd = 1; dd <= 3; ++dd) s.oc[dd] = co[x.nb(dd)];
@@ -5032,13 +5081,23 @@ __global__ void __launch_bounds__(TPB, 1) k_seq_T(Dims d, Geo g, Fields F, Phys 
   __shared__ BlockRed red;
   red_init<1>(red);
   constexpr bool GRID = MODE == kSeqGrid, SKEW = MODE == kSeqSkew;
-  const int par = parity(ctl);
+  constexpr bool SH = MODE == kSeqShared;
+  double *const f = F.f[4] + (size_t)parity(ctl) * d.NF, *const c = F.c[3];
+  if (SH) {
+    seq_copy(seq_sm, f, d.NF);
+    seq_copy(seq_sm + d.NF, c, d.Nc);
+    __syncthreads();
+  }
   SeqT<typename std::conditional<GRID, LdCoh, LdPlain>::type> sw{
-      d, S, SKEW ? S.skt : F.f[4] + (size_t)par * d.NF, SKEW ? S.skt + 3 * (size_t)S.skew.L : F.c[3],
+      d, S, SH ? seq_sm : SKEW ? S.skt : f, SH ? seq_sm + d.NF : SKEW ? S.skt + 3 * (size_t)S.skew.L : c,
       SKEW ? S.skt + 4 * (size_t)S.skew.L : F.co[3], P.w[3], 0., ctl->first != 0};
   walk_levels<MODE>(d, S, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sw);
+  if (SH) {
+    seq_copy(f, seq_sm, d.NF);
+    seq_copy(c, seq_sm + d.NF, d.Nc);
+  }
   const double e[1] = {sw.ev};
-  block_max<1, 0>(red, e, ctl->err[par] + 4);
+  block_max<1, 0>(red, e, ctl->err[parity(ctl)] + 4);
 }
 
 // apply_pressure_bc in the reference's BC-list order (bc.f90:148-340).  Within
@@ -5058,21 +5117,21 @@ __global__ void __launch_bounds__(BLK) k_seq_pack_wall(Dims d, SeqTab S) {
   const BFace B = bface(d, S.border[q]);
   const Cell &x = B.cell;
   const int pos = B.pos, dd = (pos + 1) / 2;
-  int *o = S.wface + q;
+  int *o = S.wface + seq_at(q, kSeqI);
   o[0] = x.face(d, pos);
   int n = 1, flags = 0;
   for (int k = 1; k <= 6; ++k)
-    if (k != pos) o[n++ * NB] = x.face(d, k);
+    if (k != pos) o[32 * n++] = x.face(d, k);
   for (int m = 0; m < 2; ++m) {
     const int e = m == 0 ? tr1(dd) : tr2(dd);
     const bool lo = !x.has_nb(d, 2 * e - 1), hi = !x.has_nb(d, 2 * e);
     const Cell p1 = x.nb(d, lo ? 2 * e : 2 * e - 1);
     const Cell p2 = lo ? p1.nb(d, 2 * e) : hi ? p1.nb(d, 2 * e - 1) : x.nb(d, 2 * e);
-    o[(6 + m) * NB] = p1.face(d, pos);
-    o[(8 + m) * NB] = p2.face(d, pos);
+    o[32 * (6 + m)] = p1.face(d, pos);
+    o[32 * (8 + m)] = p2.face(d, pos);
     flags |= (lo ? 1 : 0) << m | (hi ? 4 : 0) << m;
   }
-  o[10 * NB] = flags;
+  o[32 * 10] = flags;
 }
 __global__ void __launch_bounds__(BLK) k_p_bc_fixed(Dims d, Geo g, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
   if (ctl->done) return;
@@ -5084,24 +5143,29 @@ __global__ void __launch_bounds__(BLK) k_p_bc_fixed(Dims d, Geo g, Fields F, Phy
   const int par = parity(ctl), nh = newhalf(ctl);
   double B1, body;
   p_bc_fixed(d, g, F, P, F.f[0] + nh * NF, F.f[1] + nh * NF, F.f[2] + nh * NF, F.f[4] + par * NF, b, B, B1, body);
-  double *o = S.wall + q;
+  double *o = S.wall + seq_at(q, kSeqW);
   o[0] = P.w_p2 / (g.bcap[(B.pos - 1) * NB + b]);
-  o[NB] = B1;
-  o[2 * NB] = body;
-  o[3 * NB] = g.bcg[b];
-  o[4 * NB] = g.bcg[NB + b];
+  o[32] = B1;
+  o[32 * 2] = body;
+  o[32 * 3] = g.bcg[b];
+  o[32 * 4] = g.bcg[NB + b];
   int n = 5;
   for (int k = 1; k <= 6; ++k)
-    if (k != B.pos) o[n++ * NB] = g.bcap[(k - 1) * NB + b];
+    if (k != B.pos) o[32 * n++] = g.bcap[(k - 1) * NB + b];
 }
+template <bool SH>
 __global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl *ctl, SeqTab S, int wall0) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
-  const int par = parity(ctl), NB = d.NBF;
+  const int par = parity(ctl);
   const bool first = ctl->first;
   double e[1] = {0.};
-  double *pr = F.f[3] + (size_t)par * d.NF;
+  double *const pg = F.f[3] + (size_t)par * d.NF, *const pr = SH ? seq_sm : pg;
+  if (SH) {
+    seq_copy(seq_sm, pg, d.NF);
+    __syncthreads();
+  }
   const int *__restrict__ blev = S.blev;
   const double w = P.w_p2;
   const int wl = wall0 + blockIdx.x, L0 = S.wlev[wl], L1 = S.wlev[wl + 1], tid = threadIdx.x;
@@ -5110,10 +5174,12 @@ __global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl 
     double o[kSeqW];
   };
   auto look = [&](int q, Face &y) {
+    const int *I = S.wface + seq_at(q, kSeqI);
+    const double *O = S.wall + seq_at(q, kSeqW);
 #pragma unroll
-    for (int r = 0; r < kSeqI; ++r) y.i[r] = S.wface[r * NB + q];
+    for (int r = 0; r < kSeqI; ++r) y.i[r] = I[32 * r];
 #pragma unroll
-    for (int r = 0; r < kSeqW; ++r) y.o[r] = S.wall[r * NB + q];
+    for (int r = 0; r < kSeqW; ++r) y.o[r] = O[32 * r];
   };
   auto update = [&](const Face &y) {
     const double old = pr[y.i[0]];
@@ -5136,26 +5202,34 @@ __global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl 
     const double B2 = t[0] * y.o[3], B3 = t[1] * y.o[4];
     const double nw = (1 - w) * old + y.o[0] * (s + y.o[1] - B2 - B3 + y.o[2]);
     pr[y.i[0]] = nw;
+    if (SH) pg[y.i[0]] = nw;
     e[0] = nmax(e[0], errv(nw, old, first));
   };
-  int lo = blev[L0], hi = blev[L0 + 1];
-  Face y;
+  // two levels' faces in registers: one is updated, the other on its way
+  auto end = [&](int L) { return blev[min(L + 1, L1)]; };
+  int lo = blev[L0], hi = end(L0), hi1 = end(L0 + 1), hi2 = end(L0 + 2);
+  Face y, y1;
   if (lo + tid < hi) look(lo + tid, y);
-  for (int L = L0; L < L1; ++L) {
+  if (hi + tid < hi1) look(hi + tid, y1);
+  auto step = [&](int L, Face &cur) {
     if (lo + tid < hi) {
-      update(y);
+      update(cur);
       for (int q = lo + tid + blockDim.x; q < hi; q += blockDim.x) {
         Face z;
         look(q, z);
         update(z);
       }
     }
-    if (L + 1 < L1) {  // the next level's face, before the barrier
-      lo = hi;
-      hi = blev[L + 2];
-      if (lo + tid < hi) look(lo + tid, y);
-    }
+    if (hi1 + tid < hi2) look(hi1 + tid, cur);
+    lo = hi;
+    hi = hi1;
+    hi1 = hi2;
+    hi2 = end(L + 3);
     __syncthreads();
+  };
+  for (int L = L0; L < L1; L += 2) {
+    step(L, y);
+    if (L + 1 < L1) step(L + 1, y1);
   }
   block_max<1, 0>(red, e, ctl->err[par] + 3);
 }

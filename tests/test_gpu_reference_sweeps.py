@@ -1,6 +1,7 @@
 """The level-by-level sweeps of the reference-order schedule over every form
-they take: a level within a warp, within 256 threads, within 512, in several
-turns of a block, and on a cooperative grid; both formulations; theta counts
+they take: fields in a block's shared memory or in skewed copies, a level
+within a warp, within 256 threads, within 512, in several turns of a block,
+and on a cooperative grid; both formulations; theta counts
 even and odd, the smallest mesh.  Two passes of the loop body, bit for bit
 the oracle's sequential order (nse.f90:131-160)."""
 import numpy as np
@@ -26,6 +27,10 @@ def widest_level(nt, nr, nz):
 @pytest.mark.parametrize("dims,lo,hi,formulation", [
     ((6, 3, 4), 1, 32, 2), ((6, 3, 4), 1, 32, 1), ((7, 3, 5), 1, 32, 2),
     ((24, 24, 16), 33, 256, 1), ((41, 29, 24), 257, 512, 2), ((41, 29, 24), 257, 512, 1),
+    # the largest that fits a block's shared memory and the smallest that does
+    # not, an odd number of faces, narrow levels of a mesh that does not fit
+    ((36, 14, 13), 33, 256, 2), ((36, 14, 14), 33, 256, 2), ((21, 9, 7), 1, 64, 2), ((21, 9, 7), 1, 64, 1),
+    ((301, 5, 6), 1, 32, 2), ((301, 5, 6), 1, 32, 1),
     ((60, 40, 30), 513, 1024, 2), ((90, 70, 60), 1025, 4000, 2), ((90, 70, 60), 1025, 4000, 1),
 ])
 def test_two_passes_match_the_sequential_oracle(dims, lo, hi, formulation):
