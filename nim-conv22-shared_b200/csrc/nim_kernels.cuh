@@ -4470,9 +4470,11 @@ __global__ void __launch_bounds__(BLK) k_convert(CvtList L) {
 // is computed from a level's constants before the barrier, where it would
 // wait for their loads.  Fetching them two levels ahead gave nothing.
 // Time of a pass with dependent loads and a grid barrier a level, then loads
-// up front in one block, and now: 36x6x12 1891 -> 486 -> 340 us, 24x24x16
-// formulation 1 3882 -> 939 -> 790 us, 48x48x32 (672 wide) 10.3 -> 5.0 ->
-// 3.4 ms, 128x128x96 (grid) 35.2 -> 20.6 -> 18.6 ms.
+// up front in one block, then in these forms, and now, with the temperature
+// beside the pressure (launch_iteration_seq): 36x6x12 1891 -> 486 -> 340 ->
+// 253 us, 24x24x16 formulation 1 3882 -> 939 -> 790 -> 624 us, 48x48x32 (672
+// wide) 10.3 -> 5.0 -> 3.4 -> 2.5 ms, 128x128x96 (grid) 35.2 -> 20.6 -> 18.6
+// -> 13.9 ms.
 
 // Skewed copies of the swept fields (one block over wide levels): cell (i, j, k) of
 // level t = i + 2j + 3k at t st + (k + 1) sk + j + 1, its +xi faces in three

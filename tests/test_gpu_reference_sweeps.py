@@ -52,3 +52,30 @@ def test_two_passes_match_the_sequential_oracle(dims, lo, hi, formulation):
         a = gpu.download(f)
         assert np.array_equal(a, ref.get(f, a.size)), f
     gpu.close()
+
+
+def test_temperature_branches_of_several_contexts_at_once():
+    """Contexts of every form stepping together, each with its pressure and
+    temperature sweeps side by side, against the same contexts one at a time."""
+    dims = [(36, 14, 13), (41, 29, 24), (90, 70, 60), (21, 9, 7)]
+
+    def make():
+        out = []
+        for n, m in enumerate(dims):
+            case = config.small_case(*m)
+            s = nimgpu.NimSolver(nimgpu.Mesh(case.mesh_params()),
+                                 case.params(schedule=_abi.SCHEDULE_REFERENCE, formulation=1 + n % 2))
+            s.initialize_nse()
+            s.add_temperature_noise(case.noise, case.seed + n)
+            out.append(s)
+        return out
+
+    together, alone = make(), make()
+    rec = nimgpu.batch_step(together, 2)
+    for s, a, r in zip(together, alone, rec):
+        q = a.solve_nse(2)
+        assert [x.iters for x in r] == [x.iters for x in q]
+        for f in STATE:
+            assert np.array_equal(s.download(f), a.download(f)), f
+    for s in together + alone:
+        s.close()
