@@ -88,7 +88,7 @@ KERNEL_BYTES_PER_CELL = {
     "k_T_cell": 8 * 51,     # cells+old u,v,w (6) xi (9) g^ij (9) gfd (6) faces T (3) G (3) T,T_old (2); write T, MT_F terms (13)
     "k_T_face": 8 * 26,     # faces T (3) T,T_old (2) MT_F terms (12) dg (6); write faces T (3)
     # the reference-order sweeps (--schedule reference), in place
-    "k_seq_vel": 8 * 59,    # cells+old u,v,w (6) faces u,v,w (9) M_F4 (8) R sums (3) M_F1..3 (15) dg (6); write cells, faces (12)
+    "k_seq_vel": 8 * 67,    # cells+old u,v,w (6) faces u,v,w (9) R sums (3) M_F4, M_F1..3 (19) w over their divisors (12) dg (6); write cells, faces (12)
     "k_seq_p": 8 * 40,      # faces p (3) R_p (1) coefficients (27) dg (6); write faces p (3)
     "k_T_coef": 8 * 45,     # cells+old u,v,w (6) xi (9) g^ij diagonal (3) gfd (6); write MT_F, MT_F4 terms (21)
     "k_T_cell(src)": 8 * 57,  # MT_F, MT_F4 terms (21) faces T (3) G (3) g^ij (6); write the sweep's constants, R_D_T (24)

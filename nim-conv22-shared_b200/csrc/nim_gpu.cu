@@ -435,8 +435,7 @@ int launch_iteration_seq(nim_ctx *x) {
     CK(cudaEventRecord(x->fork, s));
     CK(cudaStreamWaitEvent(ts, x->fork, 0));
   }
-  (shared ? k_seq_pbc<true> : k_seq_pbc<false>)<<<2, x->wall_threads, smf, s>>>(d, x->F, x->phys, x->ctl, S, 0);
-  (shared ? k_seq_pbc<true> : k_seq_pbc<false>)<<<2, x->wall_threads, smf, s>>>(d, x->F, x->phys, x->ctl, S, 2);
+  (shared ? k_seq_pbc<true> : k_seq_pbc<false>)<<<1, x->wall_threads, smf, s>>>(d, x->F, x->phys, x->ctl, S);
   TRY(mark(x, "k_seq_pbc"));
   if (skewed) k_seq_skew<<<g1, BLK, 0, s>>>(d, S.skew, sp, x->ctl);
   if (grid_form)
@@ -469,7 +468,7 @@ int launch_iteration_seq(nim_ctx *x) {
   k_iter_end<<<1, 1, 0, s>>>(x->ctl, x->phys, 0);
   TRY(mark(x, "k_iter_end"));
   CK(cudaGetLastError());
-  x->kernels_per_iter = (x->phys.dpdx_tolerance ? 14 : 13) + (skewed ? 6 : 0);
+  x->kernels_per_iter = (x->phys.dpdx_tolerance ? 13 : 12) + (skewed ? 6 : 0);
   x->launches += x->kernels_per_iter;
   return NIM_OK;
 }
@@ -956,8 +955,8 @@ static int noalloc_setup(int device) {
 // Level orders of the reference-order sweeps.  Cells: level i + 2j + 3k,
 // which every dependence of a sweep crosses in the direction of the cell
 // numbers (the argument is in nim_kernels.cuh).  Wall faces, in BC-list
-// order bottom, top, inner, outer: level i + 2j on bottom and top, i + 2k on
-// inner and outer.  Also the sweep buffers and the cooperative grid sizes.
+// order bottom, top, inner, outer: level i + 2j on bottom and top, 1 + i + 2k
+// on inner, 2 (NR - 1) + 1 + i + 2k on outer.  Also the sweep buffers and the cooperative grid sizes.
 // widest level swept by one block, and the most its fields may take of its
 // shared memory (what 227 KB leave beside the block's reductions)
 constexpr int kSeqBlockMost = 1024;
@@ -984,29 +983,25 @@ static int setup_levels(nim_ctx *x) {
     const Cell q = Cell::of(d, c);
     order[fill[q.i + 2 * q.j + 3 * q.k]++] = make_int4(c, q.j, q.k, 0);
   }
-  // wall faces: per wall, counting sort by the in-wall level
-  const int nb1 = d.NT * d.NR, nb3 = d.NT * d.NZ;
-  const int w0[4] = {0, nb1, 2 * nb1, 2 * nb1 + nb3}, wn[4] = {nb1, nb1, nb3, nb3};
-  const int wl[4] = {d.NT + 2 * (d.NR - 1), d.NT + 2 * (d.NR - 1), d.NT + 2 * (d.NZ - 1), d.NT + 2 * (d.NZ - 1)};
-  std::vector<int> border(d.NBF), blev(1, 0), wlev(1, 0);
-  int q = 0;
-  for (int w = 0; w < 4; ++w) {
-    std::vector<int> cnt(wl[w] + 1, 0);
-    for (int r = 0; r < wn[w]; ++r) ++cnt[r % d.NT + 2 * (r / d.NT) + 1];
-    for (int L = 0; L < wl[w]; ++L) cnt[L + 1] += cnt[L];
-    std::vector<int> pos(cnt.begin(), cnt.end() - 1);
-    for (int r = 0; r < wn[w]; ++r) border[q + pos[r % d.NT + 2 * (r / d.NT)]++] = w0[w] + r;
-    for (int L = 1; L <= wl[w]; ++L) blev.push_back(q + cnt[L]);
-    q += wn[w];
-    wlev.push_back((int)blev.size() - 1);
-  }
+  // wall faces: counting sort by level
+  const int nb1 = d.NT * d.NR, nb3 = d.NT * d.NZ, nwall = d.NT + 2 * (d.NR - 1) + 2 * (d.NZ - 1) + 1;
+  auto wall_level = [&](int b) {
+    if (b < 2 * nb1) return b % nb1 % d.NT + 2 * (b % nb1 / d.NT);  // bottom, top
+    const int r = b - 2 * nb1, m = r % nb3;                         // inner, outer
+    return (r < nb3 ? 1 : 2 * (d.NR - 1) + 1) + m % d.NT + 2 * (m / d.NT);
+  };
+  std::vector<int> border(d.NBF), blev(nwall + 1, 0);
+  for (int b = 0; b < d.NBF; ++b) ++blev[wall_level(b) + 1];
+  for (int L = 0; L < nwall; ++L) blev[L + 1] += blev[L];
+  fill.assign(blev.begin(), blev.end() - 1);
+  for (int b = 0; b < d.NBF; ++b) border[fill[wall_level(b)]++] = b;
   SeqTab &S = x->seqt;
   S.nlev = nlev;
+  S.nwall = nwall;
   TRY(dalloc(x, &S.order, Nc));
   TRY(dalloc(x, &S.lstart, (size_t)nlev + 1));
   TRY(dalloc(x, &S.border, (size_t)d.NBF));
   TRY(dalloc(x, &S.blev, blev.size()));
-  TRY(dalloc(x, &S.wlev, wlev.size()));
   auto table = [](int n, int rows) { return seq_at((n + 31) / 32 * 32, rows); };  // values of a table of n entries
   TRY(dalloc(x, &S.dg, table(d.Nc, 6)));
   TRY(dalloc(x, &S.vel, table(d.Nc, (x->phys.formulation == 1 ? kSeqV<1> : kSeqV<2>) + 12)));
@@ -1018,14 +1013,13 @@ static int setup_levels(nim_ctx *x) {
   CK(cudaMemcpy(S.lstart, lstart.data(), sizeof(int) * (nlev + 1), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(S.border, border.data(), sizeof(int) * d.NBF, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(S.blev, blev.data(), sizeof(int) * blev.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(S.wlev, wlev.data(), sizeof(int) * wlev.size(), cudaMemcpyHostToDevice));
   // block sizes: whole warps for the widest level, at most SEQ_TPB_WIDE (a level
   // up to kSeqBlockMost wide then takes that many turns), or a cooperative grid
   auto warps = [](int n, int most) { return std::min(most, (n + 31) / 32 * 32); };
   int wmax = 1;
   for (size_t L = 0; L + 1 < blev.size(); ++L) wmax = std::max(wmax, blev[L + 1] - blev[L]);
   x->seq_threads = warps(maxlev, SEQ_TPB_WIDE);
-  x->wall_threads = warps(wmax, BLK);
+  x->wall_threads = warps(wmax, WALL_TPB);
   const size_t smc = sizeof(double) * ((size_t)d.NF + Nc);
   x->seq_mode = maxlev > kSeqBlockMost ? kSeqGrid : smc <= kSeqSharedMost ? kSeqShared : kSeqSkew;
   auto run_beside = [&]() -> int {

@@ -188,7 +188,7 @@ constexpr int BLK = 256;
 constexpr int LOOP_MINB = 2;  // resident blocks per SM of k_pass_loop at its widest (384 threads, 80 registers)
 // most threads of a reference-order sweep in one block: 256 keep a cell's
 // values in registers (255 a thread), 512 (128 a thread) serve wider levels
-constexpr int SEQ_TPB = 256, SEQ_TPB_WIDE = 512;
+constexpr int SEQ_TPB = 256, SEQ_TPB_WIDE = 512, WALL_TPB = 384;
 constexpr int VC2_MINB = 3;  // resident blocks per SM asked of k_vel_cell2 (56 registers)
 // resident blocks per SM the float instantiations of the pass kernels ask
 // for: computing in float they need about half the FP64 registers
@@ -4471,10 +4471,10 @@ __global__ void __launch_bounds__(BLK) k_convert(CvtList L) {
 // wait for their loads.  Fetching them two levels ahead gave nothing.
 // Time of a pass with dependent loads and a grid barrier a level, then loads
 // up front in one block, then in these forms, and now, with the temperature
-// beside the pressure (launch_iteration_seq): 36x6x12 1891 -> 486 -> 340 ->
-// 253 us, 24x24x16 formulation 1 3882 -> 939 -> 790 -> 624 us, 48x48x32 (672
-// wide) 10.3 -> 5.0 -> 3.4 -> 2.5 ms, 128x128x96 (grid) 35.2 -> 20.6 -> 18.6
-// -> 13.9 ms.
+// beside the pressure (launch_iteration_seq) and one walk over the walls:
+// 36x6x12 1891 -> 486 -> 340 -> 237 us, 24x24x16 formulation 1 3882 -> 939 ->
+// 790 -> 621 us, 48x48x32 (672 wide) 10.3 -> 5.0 -> 3.4 -> 2.5 ms, 128x128x96
+// (grid) 35.2 -> 20.6 -> 18.6 -> 13.6 ms.
 
 // Skewed copies of the swept fields (one block over wide levels): cell (i, j, k) of
 // level t = i + 2j + 3k at t st + (k + 1) sk + j + 1, its +xi faces in three
@@ -4497,7 +4497,8 @@ struct SeqTab {
   int4 *order;          // cells level by level: cell number, j, k
   int *lstart;          // level starts
   int nlev;
-  int *border, *blev, *wlev;  // wall faces, levels, per-wall level ranges
+  int *border, *blev;   // wall faces level by level, level starts
+  int nwall;
   // tables in level order (seq_at): the face-metric differences dg (6); the
   // velocity constants of a step (formulation 2: M_F4 (8), M_F1..3 (15);
   // 1: a_t (9), AA_v (45)) and the relaxation factors of u, v, w over their
@@ -5102,14 +5103,18 @@ __global__ void __launch_bounds__(TPB, 1) k_seq_T(Dims d, Geo g, Fields F, Phys 
   block_max<1, 0>(red, e, ctl->err[parity(ctl)] + 4);
 }
 
-// apply_pressure_bc in the reference's BC-list order (bc.f90:148-340).  Within
-// one wall a face reads its in-wall neighbours (+-1, +-2 along the wall), so
-// levels t = (in-wall theta index) + 2 (other in-wall index) reproduce the
-// order; bottom and top do not read each other, inner and outer read bottom
-// and top only, so one block per wall runs {bottom, top} and then
-// {inner, outer}.  border[] lists BC-list indices wall by wall and level by
-// level; wlev[w] .. wlev[w+1] are wall w's entries of blev[].  What no wall
-// pressure enters is formed for all faces at once by k_p_bc_fixed.
+// apply_pressure_bc in the reference's BC-list order (bc.f90:148-340): walls
+// bottom, top, inner, outer, each in face number order.  A face reads its
+// in-wall neighbours (+-1, +-2 along the wall) and, at a wall's edge, the face
+// of the other wall of its cell.  Levels i + 2j on bottom and top, 1 + i + 2k
+// on inner and 2 (NR - 1) + 1 + i + 2k on outer put each of them on a lower
+// level if its number is smaller and on a higher one if it is larger: inner
+// meets bottom and top at their i + 0, outer at their i + 2 (NR - 1).  One
+// block walks the levels of all four walls (36x6x12: 69 levels, where walls
+// in two launches of two blocks had 48 and 60: 75 -> 55 us; 128x128x96 898 -> 706).  border[] lists
+// BC-list indices level by level.  What no wall pressure enters is formed for
+// all faces at once by k_p_bc_fixed.
+//
 // the stencil of every wall face, once at init: flags bit m set where the
 // stencil along the m-th transverse direction starts at a low wall end, bit
 // 2 + m at a high one
@@ -5156,7 +5161,7 @@ __global__ void __launch_bounds__(BLK) k_p_bc_fixed(Dims d, Geo g, Fields F, Phy
     if (k != B.pos) o[32 * n++] = g.bcap[(k - 1) * NB + b];
 }
 template <bool SH>
-__global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl *ctl, SeqTab S, int wall0) {
+__global__ void __launch_bounds__(WALL_TPB) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl *ctl, SeqTab S) {
   if (ctl->done) return;
   __shared__ BlockRed red;
   red_init<1>(red);
@@ -5170,7 +5175,7 @@ __global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl 
   }
   const int *__restrict__ blev = S.blev;
   const double w = P.w_p2;
-  const int wl = wall0 + blockIdx.x, L0 = S.wlev[wl], L1 = S.wlev[wl + 1], tid = threadIdx.x;
+  const int nl = S.nwall, tid = threadIdx.x;
   struct Face {
     int i[kSeqI];
     double o[kSeqW];
@@ -5208,8 +5213,8 @@ __global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl 
     e[0] = nmax(e[0], errv(nw, old, first));
   };
   // two levels' faces in registers: one is updated, the other on its way
-  auto end = [&](int L) { return blev[min(L + 1, L1)]; };
-  int lo = blev[L0], hi = end(L0), hi1 = end(L0 + 1), hi2 = end(L0 + 2);
+  auto end = [&](int L) { return blev[min(L + 1, nl)]; };
+  int lo = 0, hi = end(0), hi1 = end(1), hi2 = end(2);
   Face y, y1;
   if (lo + tid < hi) look(lo + tid, y);
   if (hi + tid < hi1) look(hi + tid, y1);
@@ -5229,9 +5234,9 @@ __global__ void __launch_bounds__(BLK) k_seq_pbc(Dims d, Fields F, Phys P, Ctrl 
     hi2 = end(L + 3);
     __syncthreads();
   };
-  for (int L = L0; L < L1; L += 2) {
+  for (int L = 0; L < nl; L += 2) {
     step(L, y);
-    if (L + 1 < L1) step(L + 1, y1);
+    if (L + 1 < nl) step(L + 1, y1);
   }
   block_max<1, 0>(red, e, ctl->err[par] + 3);
 }
