@@ -213,6 +213,20 @@ void nim_params_reference(nim_params *p);
 int nim_gpu_create(const nim_mesh_desc *mesh, const nim_params *params,
                    nim_ctx **out);
 
+/* The form the ordered sweeps of NIM_SCHEDULE_REFERENCE take on a mesh (no
+   counterpart in the reference; a pure host function): NIM_REFERENCE_SHARED,
+   one block per swept field over a copy in its shared memory;
+   NIM_REFERENCE_GRID, a cooperative grid over the fields themselves;
+   NIM_REFERENCE_SKEWED, one block per swept field over skewed copies in
+   device memory.  The skewed form needs levels (cells of equal i + 2j + 3k)
+   of at most 1024 cells and copies of at most 8 values a cell and plane,
+   1.7 kB a cell: a tall or wide mesh with narrow levels takes the grid.  All
+   forms give the same bits.  copies, unless NULL: bytes of the skewed copies
+   (0 for the other forms).  NIM_ERR_BAD_ARG for counts nim_gpu_create
+   refuses. */
+enum { NIM_REFERENCE_SHARED = 0, NIM_REFERENCE_GRID = 1, NIM_REFERENCE_SKEWED = 2 };
+int nim_reference_form(int32_t n_theta, int32_t n_r, int32_t n_z, int64_t *copies);
+
 /* Init-time geometry and constants: evaluate_all_mesh_constants
    (geometry.f90:14-32), evaluate_pressure_bc_array (geometry.f90:879-975),
    calculate_pressure_nim_constants (nim.f90:556-743),

@@ -952,15 +952,67 @@ static int noalloc_setup(int device) {
   return NIM_OK;
 }
 
-// Level orders of the reference-order sweeps.  Cells: level i + 2j + 3k,
-// which every dependence of a sweep crosses in the direction of the cell
-// numbers (the argument is in nim_kernels.cuh).  Wall faces, in BC-list
-// order bottom, top, inner, outer: level i + 2j on bottom and top, 1 + i + 2k
-// on inner, 2 (NR - 1) + 1 + i + 2k on outer.  Also the sweep buffers and the cooperative grid sizes.
 // widest level swept by one block, and the most its fields may take of its
 // shared memory (what 227 KB leave beside the block's reductions)
 constexpr int kSeqBlockMost = 1024;
 constexpr size_t kSeqSharedMost = 224 * 1024;
+// Most values a plane of the skewed copies may have per cell.  A plane is the
+// box of the levels: (levels + 3)(NZ + 1)(NR + 1) values, and 27 planes are
+// kept, so the copies grow with the square of the longest direction while the
+// widest level does not.  48x48x32, 60x40x30 and 41x29x24, where the copies
+// pay (SeqTab), have 4 to 6 values a cell, 1.0 to 1.2 kB of copies a cell;
+// 36x80x400 has 38, 8 kB, and sweeps the fields themselves.
+constexpr int64_t kSkewMost = 8;
+// The form of the reference order's sweeps on a mesh: its widest level
+// (cells of equal i + 2j + 3k), the memory its fields take, and the values of
+// a plane of skewed copies.
+struct SeqForm {
+  int mode = kSeqGrid;
+  int64_t plane = 0;  // Skew::L (kSeqSkew)
+};
+static SeqForm seq_form(int64_t NT, int64_t NR, int64_t NZ) {
+  const int64_t nlev = (NT - 1) + 2 * (NR - 1) + 3 * (NZ - 1) + 1, Nc = NT * NR * NZ;
+  const int64_t NF = 3 * Nc + NT * NR + NT * NZ;
+  // a column (j, k) enters the level 2j + 3k and leaves after NT levels
+  std::vector<int32_t> step((size_t)nlev + 1, 0);
+  for (int64_t k = 0; k < NZ; ++k)
+    for (int64_t j = 0; j < NR; ++j) {
+      ++step[2 * j + 3 * k];
+      --step[2 * j + 3 * k + NT];
+    }
+  int64_t width = 0, most = 0;
+  for (int64_t L = 0; L < nlev; ++L) most = std::max(most, width += step[L]);
+  SeqForm f;
+  if (most > kSeqBlockMost) return f;
+  if (sizeof(double) * (uint64_t)(NF + Nc) <= kSeqSharedMost) {
+    f.mode = kSeqShared;
+    return f;
+  }
+  // the sweeps index three planes, and up to four levels beyond a cell, in
+  // 32 bits
+  const int64_t st = (NZ + 1) * (NR + 1), plane = (nlev + 3) * st;
+  if (plane <= kSkewMost * Nc && 3 * plane + 8 * st <= INT32_MAX) {
+    f.mode = kSeqSkew;
+    f.plane = plane;
+  }
+  return f;
+}
+extern "C" int nim_reference_form(int32_t n_theta, int32_t n_r, int32_t n_z, int64_t *copies) {
+  if (n_theta < 6 || n_r < 3 || n_z < 3 || (int64_t)n_theta * n_r * n_z > (int64_t)INT32_MAX / 4)
+    return NIM_ERR_BAD_ARG;
+  const SeqForm f = seq_form(n_theta, n_r, n_z);
+  if (copies) *copies = (int64_t)sizeof(double) * (3 * kSkewVel + kSkewP + kSkewTm) * f.plane;
+  return f.mode;
+}
+static_assert(kSeqShared == NIM_REFERENCE_SHARED && kSeqGrid == NIM_REFERENCE_GRID && kSeqSkew == NIM_REFERENCE_SKEWED,
+              "the header's forms");
+
+// Level orders of the reference-order sweeps.  Cells: level i + 2j + 3k,
+// which every dependence of a sweep crosses in the direction of the cell
+// numbers (the argument is in nim_kernels.cuh).  Wall faces, in BC-list
+// order bottom, top, inner, outer: level i + 2j on bottom and top, 1 + i + 2k
+// on inner, 2 (NR - 1) + 1 + i + 2k on outer.  Also the sweep buffers and the
+// cooperative grid sizes.
 static int setup_levels(nim_ctx *x) {
   const Dims &d = x->d;
   const size_t Nc = d.Nc;
@@ -1020,8 +1072,8 @@ static int setup_levels(nim_ctx *x) {
   for (size_t L = 0; L + 1 < blev.size(); ++L) wmax = std::max(wmax, blev[L + 1] - blev[L]);
   x->seq_threads = warps(maxlev, SEQ_TPB_WIDE);
   x->wall_threads = warps(wmax, WALL_TPB);
-  const size_t smc = sizeof(double) * ((size_t)d.NF + Nc);
-  x->seq_mode = maxlev > kSeqBlockMost ? kSeqGrid : smc <= kSeqSharedMost ? kSeqShared : kSeqSkew;
+  const SeqForm form = seq_form(d.NT, d.NR, d.NZ);
+  x->seq_mode = form.mode;
   auto run_beside = [&]() -> int {
     CK(cudaStreamCreateWithFlags(&x->side, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&x->fork, cudaEventDisableTiming));
@@ -1043,7 +1095,7 @@ static int setup_levels(nim_ctx *x) {
   if (x->seq_mode == kSeqSkew) {
     S.skew.sk = d.NR + 1;
     S.skew.st = (d.NZ + 1) * S.skew.sk;
-    S.skew.L = (nlev + 3) * S.skew.st;  // levels from -3 (the low z wall's layer)
+    S.skew.L = (int)form.plane;  // levels from -3 (the low z wall's layer)
     TRY(dalloc(x, &S.skv, 3 * kSkewVel * (size_t)S.skew.L));
     TRY(dalloc(x, &S.skp, kSkewP * (size_t)S.skew.L));
     TRY(dalloc(x, &S.skt, kSkewTm * (size_t)S.skew.L));
