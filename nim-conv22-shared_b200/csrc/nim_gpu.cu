@@ -149,8 +149,9 @@ struct nim_ctx {
   bool halo_ok[2] = {false, false};
   int64_t halo_recv[2][8] = {}, halo_send[2][8] = {};
   // a time step driven without blocking (the synchronous calls and
-  // nim_batch_step share it): graph launches so far, the cap, the event that
-  // marks the last control-block (or sums) copy
+  // nim_batch_step share it): the host's own cap on its passes, the event that
+  // marks the last control-block (or sums) copy; launched: passes the fused
+  // batch has queued
   struct Run {
     long long launched = 0, cap = 0;
     bool capped = false;
@@ -1636,7 +1637,6 @@ int iterations_launch(nim_ctx *x, int batches) {
   const int G = x->graph_G;
   if (x->loop && !x->in_batch) {
     TRY(x->phase == 1 ? launch_loop<float>(x, x->g32, x->F32, 1) : launch_loop<double>(x, x->g, x->F, 0));
-    x->run.launched += kLoopPasses;
     return ctrl_async(x);
   }
   if (x->seq) {
@@ -1646,7 +1646,6 @@ int iterations_launch(nim_ctx *x, int batches) {
     for (int k = 0; k < batches; ++k) CK(cudaGraphLaunch(graph, x->stream));
     x->launches += (long long)batches * G * x->kernels_per_iter;
   }
-  x->run.launched += (long long)batches * G;
   return ctrl_async(x);
 }
 
@@ -1668,9 +1667,9 @@ int integrate_start(nim_ctx *x) {
   const bool graphs = !x->seq && (!x->loop || x->in_batch);
   if (graphs && (!x->graph || x->graph_iters != G)) TRY(build_graph(x, G));
   if (graphs && x->mixed && (!x->graph32 || x->graph32_iters != G)) TRY(build_graph(x, G, true));
-  // with max_iters <= 0 the device never stops on its own; bound the host loop
-  x->run.cap = (x->params.max_iters > 0) ? (long long)x->params.max_iters + 2 * G : 100000000LL;
-  x->run.launched = 0;
+  // the device stops at max_iters on its own; with max_iters <= 0 it never
+  // does: bound the host loop
+  x->run.cap = (x->params.max_iters > 0) ? x->params.max_iters : 100000000LL;
   x->run.capped = false;
   if (x->mixed) {  // FP32 phase from the narrowed FP64 iterate
     TRY(mirror_state(x, 0));
@@ -1688,7 +1687,8 @@ int integrate_start(nim_ctx *x) {
 // the end-of-loop reductions are queued (wait for run.ev again)
 int integrate_advance(nim_ctx *x) {
   if (!x->ctl_host->done) {
-    if (x->run.launched < x->run.cap) {
+    // the cap counts passes that ran: those queued past a phase's end do nothing
+    if (x->ctl_host->step_iters < x->run.cap) {
       TRY(iterations_launch(x, 1));
       return 1;
     }
