@@ -3427,25 +3427,36 @@ __global__ void __launch_bounds__(BLK) k_p_dpdx(Dims d, GeoOf<R> g, FieldsT<R> F
 }
 
 // ---- K6: apply_zero_flux (bc.f90:345-390) on the z walls, into the next half
-// (the rest of the pass reads the z walls there; one half: in place)
+// (the rest of the pass reads the z walls there; one half: in place).  The
+// stencil of a wall reaches three faces in, which on three planes is the
+// other wall: one thread then forms both values of its column, the bottom's
+// from the old top and the top's from the new bottom, as the BC list runs.
 template <class R, class BI, class PS = LaunchPass>
 __device__ __forceinline__ void zero_flux_body(const Dims &d, const GeoOf<R> &g, const FieldsT<R> &F, Ctrl *ctl, const BI blockIdx, PS &&ps = PS{}) {
   if (!ps.template begin<1>(ctl)) return;
   const int par = ps.par, nh = ps.nh;
-  const bool first = ps.first;
+  const bool first = ps.first, both = d.NZ == 3;
   const int b = lin_index(blockIdx);
   double e[1] = {0.};
-  if (b < 2 * d.plane) {
+  if (b < (both ? 1 : 2) * d.plane) {
     const int NF = d.NF, NB = d.NBF;
     const BFace B = bface(d, b);
     const int in = (B.pos == 5) ? 6 : 5;
     const Cell c2 = B.cell.nb(d, in), c3 = c2.nb(d, in);
     const R *T = F.f[4] + par * NF;
-    const int f1 = B.cell.face(d, B.pos);
-    const Ar<R> nw = stored<R>((+g.zf[NB + b] * T[B.cell.face(d, in)] - g.zf[2 * NB + b] * T[c2.face(d, in)] +
-                                g.zf[3 * NB + b] * T[c3.face(d, in)]) / g.zf[b]);
+    R *Tn = F.f[4] + nh * NF;
+    auto value = [&](int w, const R &t2, const R &t3, const R &t4) {
+      return stored<R>((+g.zf[NB + w] * t2 - g.zf[2 * NB + w] * t3 + g.zf[3 * NB + w] * t4) / g.zf[w]);
+    };
+    const int f1 = B.cell.face(d, B.pos), f4 = c3.face(d, in);
+    const Ar<R> nw = value(b, T[B.cell.face(d, in)], T[c2.face(d, in)], T[f4]);
     e[0] = d.owns(B.cell.k) ? errv(nw, T[f1], first) : 0.;
-    F.f[4][nh * NF + f1] = nw;
+    if (both) {  // f4 is the top wall's face
+      const Ar<R> top = value(b + d.plane, T[c3.face(d, 5)], T[c2.face(d, 5)], (R)nw);
+      e[0] = nmax(e[0], errv(top, T[f4], first));
+      Tn[f4] = top;
+    }
+    Tn[f1] = nw;
   }
   ps.template end<BLK>(e, 4);
 }
