@@ -50,11 +50,12 @@ __device__ __forceinline__ bool div_ok(double b) {
   const uint32_t hi = (uint32_t)__double2hiint(b) & 0x7fffffffu;
   return (hi - ((1023u - E) << 20)) < ((2u * E) << 20) && (hi & 0xfffffu) != 0xfffffu;
 }
-// a's exponent within +-E, or a zero
+// a's exponent within +-E.  A zero is not: quot() adds a +0 remainder to the
+// quotient, so that -0 / b would come back as +0.
 template <int E>
 __device__ __forceinline__ bool num_ok(double a) {
   const uint32_t hi = (uint32_t)__double2hiint(a) & 0x7fffffffu;
-  return (hi - ((1023u - E) << 20)) < ((2u * E) << 20) || a == 0.0;
+  return (hi - ((1023u - E) << 20)) < ((2u * E) << 20);
 }
 
 }  // namespace nim
