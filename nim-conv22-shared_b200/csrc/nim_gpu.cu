@@ -469,7 +469,7 @@ int launch_iteration_seq(nim_ctx *x) {
   k_iter_end<<<1, 1, 0, s>>>(x->ctl, x->phys, 0);
   TRY(mark(x, "k_iter_end"));
   CK(cudaGetLastError());
-  x->kernels_per_iter = (x->phys.dpdx_tolerance ? 13 : 12) + (skewed ? 6 : 0);
+  x->kernels_per_iter = (x->phys.dpdx_tolerance ? 12 : 11) + (skewed ? 6 : 0);
   x->launches += x->kernels_per_iter;
   return NIM_OK;
 }
