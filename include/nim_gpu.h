@@ -492,6 +492,11 @@ int nim_gpu_tangent_get(nim_ctx *ctx, nim_field field, double *value, double *ta
    the context stays usable.  Between steps only. */
 int nim_gpu_selftest_wait_timeout(nim_ctx *ctx, int32_t tries);
 
+/* The same for the grid barrier of the inner loop's cooperative form: four
+   blocks wait for one arrival more than they make, at most `tries` (1..2^20)
+   polls each. */
+int nim_gpu_selftest_barrier_timeout(nim_ctx *ctx, int32_t tries);
+
 /* Self-test of the device exp (no counterpart in the reference): y[i] =
    the exp that the NIM coefficients use on the device, for n host values x
    (n <= 2^28; the call allocates and frees its device buffers and runs on

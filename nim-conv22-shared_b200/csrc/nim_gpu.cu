@@ -2977,6 +2977,21 @@ extern "C" int nim_gpu_selftest_wait_timeout(nim_ctx *x, int32_t tries) {
   return seen;
 }
 
+extern "C" int nim_gpu_selftest_barrier_timeout(nim_ctx *x, int32_t tries) {
+  if (!x || tries < 1 || tries > (1 << 20)) return NIM_ERR_BAD_ARG;
+  if (!x->initialized || x->in_step) return NIM_ERR_STATE;
+  CK(cudaSetDevice(x->device));
+  k_step_reset<<<1, 1, 0, x->stream>>>(x->ctl);
+  CK(cudaMemsetAsync(x->loop_bar, 0, sizeof(unsigned), x->stream));
+  k_barrier_selftest<<<4, dim3(32, 3), 0, x->stream>>>(x->ctl, x->loop_bar, tries);
+  CK(cudaGetLastError());
+  TRY(read_ctrl(x));
+  const int seen = x->ctl_host->status;
+  k_step_reset<<<1, 1, 0, x->stream>>>(x->ctl);  // the context stays usable
+  TRY(read_ctrl(x));
+  return seen;
+}
+
 extern "C" int nim_gpu_selftest_exp(const double *x, double *y, int64_t n) {
   if (n < 0 || (n > 0 && (!x || !y)) || n > (int64_t(1) << 28)) return NIM_ERR_BAD_ARG;
   if (n == 0) return NIM_OK;

@@ -4283,7 +4283,7 @@ struct LoopBarrier {
   unsigned target;   // arrivals that complete the next barrier
   __device__ __forceinline__ explicit LoopBarrier(unsigned *c) : count(c), target(gridDim.x) {}
   // false: the wait ran out (every block leaves, the step has timed out)
-  __device__ __forceinline__ bool sync(Ctrl *ctl) {
+  __device__ __forceinline__ bool sync(Ctrl *ctl, int tries = kBarTries) {
     __syncthreads();
     bool ok = true;
     if (threadIdx.x == 0 && threadIdx.y == 0) {
@@ -4292,9 +4292,9 @@ struct LoopBarrier {
       int n = 0;
       do {
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
-      } while ((int)(seen - target) < 0 && ++n < kBarTries);
+      } while ((int)(seen - target) < 0 && ++n < tries);
       asm volatile("fence.acq_rel.gpu;" ::: "memory");
-      if (n >= kBarTries) {
+      if (n >= tries) {
         ok = false;
         atomicCAS(&ctl->status, 0, -5);  // NIM_ERR_TIMEOUT
         *(volatile int *)&ctl->done = 1;
@@ -4304,6 +4304,16 @@ struct LoopBarrier {
     return __syncthreads_and(ok);
   }
 };
+// The give-up path of LoopBarrier::sync, without a fault: the blocks wait for
+// one arrival more than the grid makes, at most `tries` polls, and leave; the
+// step is then marked NIM_ERR_TIMEOUT and stopped.  No block waits for
+// another to be resident.
+__global__ void k_barrier_selftest(Ctrl *ctl, unsigned *arrivals, int tries) {
+  LoopBarrier bar(arrivals);
+  bar.target += 1;
+  bar.sync(ctl, tries);
+}
+
 // +xi_dd face updates of T, thread y = direction y+1 (T_face_body spread over
 // three threads a cell)
 template <class R, class PS>
@@ -4397,7 +4407,9 @@ __global__ void __launch_bounds__(CB3, LOOP_MINB) k_pass_loop(Dims d, GeoOf<R> g
     block_max<6, 0>(red, ps.m, ctl->err[ps.par]);
     if (!bar.sync(ctl)) return;
     if (tid == 0) {
-      // the other slot is accumulated into again only six barriers on
+      // clearing the other slot here is safe: every block read it before the
+      // first barrier of this pass, and adds to it again only after the fourth
+      // barrier of the next one
       for (int q = 0; q < 6; ++q) sc.err[ps.par][q] = __ldcg(&ctl->err[ps.par][q]);
       iter_end_body(&sc, P, lowp, LaunchBlock{});
       if (b0 == 0)

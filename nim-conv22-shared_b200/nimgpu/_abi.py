@@ -233,6 +233,8 @@ def gpu_lib() -> C.CDLL:
         lib.nim_gpu_selftest_nim_coef.restype = C.c_int
         lib.nim_gpu_selftest_wait_timeout.argtypes = [vp, C.c_int32]
         lib.nim_gpu_selftest_wait_timeout.restype = C.c_int
+        lib.nim_gpu_selftest_barrier_timeout.argtypes = [vp, C.c_int32]
+        lib.nim_gpu_selftest_barrier_timeout.restype = C.c_int
         lib.nim_gpu_nusselt_noalloc.argtypes = [vp, C.POINTER(C.c_double)]
         lib.nim_gpu_nusselt_noalloc.restype = C.c_int
         _gpu = lib
