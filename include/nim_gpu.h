@@ -207,9 +207,11 @@ void nim_params_reference(nim_params *p);
    TMA-staged form under the face sweep's n_theta conditions (not faster at
    the benchmark sizes, so off by default).  The inner loop of a small mesh
    (formulation 2, parallel schedule) runs as one cooperative launch instead
-   of a graph of launches; NIM_PASS_LOOP=on or =off overrides, and naming a
-   form of a sweep as above asks for launches.  All forms give identical
-   results. */
+   of a graph of launches, unless calls of other host threads are advancing
+   contexts on the device and the loops of all would not fit it side by side:
+   then as launches, which overlap; NIM_PASS_LOOP=on or =off overrides, and
+   naming a form of a sweep as above asks for launches.  All forms give
+   identical results. */
 int nim_gpu_create(const nim_mesh_desc *mesh, const nim_params *params,
                    nim_ctx **out);
 

@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstddef>
 #include <cstdio>
@@ -50,6 +51,18 @@ __device__ __align__(256) double g_noalloc_scratch[4 * kNoallocBlocks + 8];
 constexpr int kMaxDevices = 64;
 double *g_noalloc_ptr[kMaxDevices] = {nullptr};
 std::mutex g_noalloc_mutex;
+
+// Calls that are advancing contexts on a device at this moment, from all host
+// threads: k_pass_loop gives way to launches while its grid and theirs would
+// not be resident together (loop_now).
+std::atomic<int> g_advancing[kMaxDevices];
+struct Advancing {
+  const int device;
+  explicit Advancing(int d) : device(d) { ++g_advancing[device]; }
+  ~Advancing() { --g_advancing[device]; }
+  Advancing(const Advancing &) = delete;
+  Advancing &operator=(const Advancing &) = delete;
+};
 
 struct Buf {
   void *p = nullptr;
@@ -124,9 +137,10 @@ struct nim_ctx {
   VelCellMaps cmap64{}, cmap32{};
   // k_pass_loop: a small mesh's inner loop as one cooperative launch, block
   // (loop_bx, 3); off while the context advances in a batch (the enclosures
-  // share the GPU)
-  bool loop = false, in_batch = false, loop_pair = false;
-  int loop_bx = 0, loop_blocks = 0;
+  // share the GPU), and where other host threads need the room (loop_now):
+  // loop_room blocks are resident at once
+  bool loop = false, loop_forced = false, in_batch = false, loop_pair = false;
+  int loop_bx = 0, loop_blocks = 0, loop_room = 0;
   unsigned *loop_bar = nullptr;
   GeoT<float> g32{};
   FieldsT<float> F32{};
@@ -631,6 +645,7 @@ int choose_loop(nim_ctx *x) {
   const int most = !x->mixed && (x->flat1 || x->flat2) ? kLoopCellsFlat : kLoopCells;
   x->loop = !x->seq && x->phys.formulation == 2 && !x->slab_count && !x->cell_tile && force != "off" &&
             (force == "on" || (d.Nc <= most && env("NIM_CELL_SWEEP").empty() && env("NIM_FACE_SWEEP").empty()));
+  x->loop_forced = force == "on";
   if (!x->loop) return NIM_OK;
   int sms = 0, coop = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, x->device));
@@ -646,6 +661,7 @@ int choose_loop(nim_ctx *x) {
       per = std::min(per, nb);
     }
     x->loop_bx = bx;
+    x->loop_room = per * sms;
     x->loop_blocks = std::min(items(bx), per * sms);
     if (items(bx) <= per * sms) break;
   }
@@ -654,6 +670,21 @@ int choose_loop(nim_ctx *x) {
   x->loop_pair = x->cell_pair && items(x->loop_bx) > x->loop_blocks;
   if (!coop || x->loop_blocks < 1) x->loop = false;
   return NIM_OK;
+}
+
+// Whether this launch takes the loop form: cooperative launches that are not
+// resident together wait for one another, up to 256 passes each, where the
+// launches of several contexts overlap.  us a pass of all contexts together,
+// 1, 2, 4 and 8 host threads stepping FP64 contexts of one size: loops always,
+// launches always, this rule:
+//   36x6x12    34 17 9.4 6.4 | 44 25 13 7.3 | 34 17 9.5 5.9
+//   24x24x18   35 18  18  18 | 43 25 16  11 | 35 18  16  11
+//   45x37x29   49 50  51  50 | 57 46 38  37 | 50 46  38  37
+//   48x48x32   66 66  67  65 | 73 58 50  49 | 65 59  51  50
+//   64x48x32   91 91  91  91 | 87 68 62  62 | 90 68  61  62
+bool loop_now(const nim_ctx *x) {
+  if (!x->loop || x->in_batch) return false;
+  return x->loop_forced || (long long)g_advancing[x->device] * x->loop_blocks <= x->loop_room;
 }
 
 int build_graph(nim_ctx *x, int iters, bool lowp = false) {
@@ -1609,6 +1640,7 @@ static bool lone_slab(const nim_ctx *x) { return x->slab_count > 1; }
 extern "C" int nim_gpu_iterate(nim_ctx *x, int32_t n, nim_step_stats *s) {
   if (!x || n < 0 || lone_slab(x)) return NIM_ERR_BAD_ARG;
   if (!x->initialized) return NIM_ERR_STATE;
+  const Advancing here(x->device);
   // fixed number of passes: keep the stop flag clear and the cap out of reach
   const Phys keep = x->phys;
   x->phys.max_iters = 0;
@@ -1635,14 +1667,16 @@ int ctrl_async(nim_ctx *x) {
 
 int iterations_launch(nim_ctx *x, int batches) {
   const int G = x->graph_G;
-  if (x->loop && !x->in_batch) {
+  if (loop_now(x)) {
     TRY(x->phase == 1 ? launch_loop<float>(x, x->g32, x->F32, 1) : launch_loop<double>(x, x->g, x->F, 0));
     return ctrl_async(x);
   }
   if (x->seq) {
     for (int k = 0; k < batches * G; ++k) TRY(launch_iteration(x));
   } else {
-    cudaGraphExec_t graph = (x->phase == 1) ? x->graph32 : x->graph;
+    const bool lowp = x->phase == 1;
+    cudaGraphExec_t &graph = lowp ? x->graph32 : x->graph;
+    if (!graph || (lowp ? x->graph32_iters : x->graph_iters) != G) TRY(build_graph(x, G, lowp));
     for (int k = 0; k < batches; ++k) CK(cudaGraphLaunch(graph, x->stream));
     x->launches += (long long)batches * G * x->kernels_per_iter;
   }
@@ -1664,9 +1698,6 @@ int after_loop_start(nim_ctx *x) {
 // integrate_nse, first batch: launch ahead by the previous step's count
 int integrate_start(nim_ctx *x) {
   const int G = x->graph_G;
-  const bool graphs = !x->seq && (!x->loop || x->in_batch);
-  if (graphs && (!x->graph || x->graph_iters != G)) TRY(build_graph(x, G));
-  if (graphs && x->mixed && (!x->graph32 || x->graph32_iters != G)) TRY(build_graph(x, G, true));
   // the device stops at max_iters on its own; with max_iters <= 0 it never
   // does: bound the host loop
   x->run.cap = (x->params.max_iters > 0) ? x->params.max_iters : 100000000LL;
@@ -1768,9 +1799,8 @@ extern "C" int nim_gpu_set_graph_iters(nim_ctx *x, int32_t n) {
   return NIM_OK;
 }
 
-extern "C" int nim_gpu_integrate(nim_ctx *x, nim_step_stats *s) {
-  if (!x || lone_slab(x)) return NIM_ERR_BAD_ARG;
-  if (!x->initialized || !x->in_step) return NIM_ERR_STATE;
+// integrate_nse to its end, its caller counted as advancing (Advancing)
+static int integrate_wait(nim_ctx *x, nim_step_stats *s) {
   TRY(integrate_start(x));
   for (;;) {
     CK(cudaEventSynchronize(x->run.ev));
@@ -1780,6 +1810,13 @@ extern "C" int nim_gpu_integrate(nim_ctx *x, nim_step_stats *s) {
   }
   CK(cudaEventSynchronize(x->run.ev));
   return integrate_finish(x, s);
+}
+
+extern "C" int nim_gpu_integrate(nim_ctx *x, nim_step_stats *s) {
+  if (!x || lone_slab(x)) return NIM_ERR_BAD_ARG;
+  if (!x->initialized || !x->in_step) return NIM_ERR_STATE;
+  const Advancing here(x->device);
+  return integrate_wait(x, s);
 }
 
 extern "C" int nim_gpu_end_step(nim_ctx *x, nim_step_stats *s) {
@@ -1794,13 +1831,14 @@ extern "C" int nim_gpu_end_step(nim_ctx *x, nim_step_stats *s) {
 extern "C" int nim_gpu_step(nim_ctx *x, int32_t nsteps, nim_step_stats *per, int32_t *done) {
   if (!x || nsteps < 0 || lone_slab(x)) return NIM_ERR_BAD_ARG;
   if (!x->initialized) return NIM_ERR_STATE;
+  const Advancing here(x->device);
   int32_t k = 0;
   int st = NIM_OK;
   for (; k < nsteps; ++k) {
     nim_step_stats rec;
     std::memset(&rec, 0, sizeof(rec));
     TRY(nim_gpu_begin_step(x));
-    st = nim_gpu_integrate(x, &rec);
+    st = integrate_wait(x, &rec);
     rec.status = st;
     if (st != NIM_OK) {
       x->in_step = false;
@@ -1858,6 +1896,7 @@ extern "C" int nim_batch_step(int32_t n, nim_ctx *const *ctx, int32_t nsteps, ni
     for (int32_t i = 0; i < n; ++i) done[i] = 0;
   if (nsteps == 0) return NIM_OK;
   const InBatch share(n, ctx);
+  const Advancing here(ctx[0]->device);
   CK(cudaSetDevice(ctx[0]->device));
   enum { ITER, AFTER, END, FINISHED };
   std::vector<int> phase(n, ITER), k(n, 0);
@@ -2249,6 +2288,7 @@ extern "C" int nim_batch_step_fused(int32_t n, nim_ctx *const *ctx, int32_t nste
     for (int32_t i = 0; i < n; ++i) done[i] = 0;
   if (nsteps == 0) return NIM_OK;
   CK(cudaSetDevice(ctx[0]->device));
+  const Advancing here(ctx[0]->device);
   FusedBatch B;
   TRY(fused_setup(B, n, ctx));
   BatchState *state_dev = reinterpret_cast<BatchState *>(static_cast<char *>(B.dev) + B.state_dev_offset);
@@ -2646,6 +2686,7 @@ extern "C" int nim_slab_step(int32_t n, nim_ctx *const *X, int32_t nsteps, nim_s
     if (s > 0 && X[s]->slab_lo + X[s]->d.kown0 != X[s - 1]->slab_lo + X[s - 1]->d.kown1) return NIM_ERR_BAD_ARG;
   }
   CK(cudaSetDevice(X[0]->device));
+  const Advancing here(X[0]->device);
   for (int32_t s = 0; s < n; ++s) CK(cudaStreamSynchronize(X[s]->stream));
   // every halo from its owner: after nim_gpu_init, uploads or a previous call
   TRY(halo_exchange(X, n, X[0]->stream, kHaloAll));
@@ -3273,6 +3314,7 @@ extern "C" int nim_gpu_tangent_step(nim_ctx *x, int32_t nsteps, nim_step_stats *
   if (!x || nsteps < 0) return NIM_ERR_BAD_ARG;
   if (!x->dual_ready) return NIM_ERR_STATE;
   CK(cudaSetDevice(x->device));
+  const Advancing here(x->device);
   for (int32_t k = 0; k < nsteps; ++k) {
     nim_step_stats rec;
     std::memset(&rec, 0, sizeof(rec));
