@@ -1320,12 +1320,12 @@ void fill_integrate_stats(const nim_oracle &o, nim_step_stats *s, int iters) {
 
 // The visiting orders of the Gauss-Seidel sweeps.  SEQUENTIAL: cell number
 // and BC-list order, as the reference's loops run.  LEVELS: cells by the level
-// i + 2j + 3k (theta, r, z indices of the structured numbering) and wall faces
-// by i + 2j (bottom, top) or i + 2k (inner, outer), the order the CUDA
-// library's reference-order sweeps follow; inside a level the numbers run
-// downwards and the walls come as top, bottom, outer, inner, so that any
-// dependence between faces or cells the level order treats as independent
-// changes the result.
+// i + 2j + 3k (theta, r, z indices of the structured numbering) and the wall
+// faces of all four walls by one set of levels, i + 2j (bottom, top), 1 + i +
+// 2k (inner) and 2 (NR - 1) + 1 + i + 2k (outer): the order the CUDA library's
+// reference-order sweeps follow.  Inside a level the numbers run downwards,
+// outer wall first, so that any dependence between faces or cells the level
+// order treats as independent changes the result.
 void visiting_orders(nim_oracle &o, int NT, int NR, int NZ) {
   const int64_t N = o.NMESH, NB = o.NBF;
   o.cord.resize(N);
@@ -1346,15 +1346,14 @@ void visiting_orders(nim_oracle &o, int NT, int NR, int NZ) {
   by_level(v);
   for (int64_t q = 0; q < N; ++q) o.cord[q] = v[q].second;
   const int64_t nb1 = (int64_t)NT * NR, nb3 = (int64_t)NT * NZ;
-  const int64_t w0[4] = {nb1, 0, 2 * nb1 + nb3, 2 * nb1};  // top, bottom, outer, inner
-  const int64_t wn[4] = {nb1, nb1, nb3, nb3};
-  int64_t q = 0;
-  for (int w = 0; w < 4; ++w) {
-    v.clear();
-    for (int64_t r = 0; r < wn[w]; ++r) v.push_back({r % NT + 2 * (r / NT), w0[w] + r + 1});
-    by_level(v);
-    for (const auto &e : v) o.bord[q++] = e.second;
+  v.clear();
+  for (int64_t b = 0; b < NB; ++b) {
+    const int64_t r = b < 2 * nb1 ? b % nb1 : (b - 2 * nb1) % nb3;  // within its wall
+    const int64_t first = b < 2 * nb1 ? 0 : b < 2 * nb1 + nb3 ? 1 : 2 * (NR - 1) + 1;
+    v.push_back({first + r % NT + 2 * (r / NT), b + 1});
   }
+  by_level(v);
+  for (int64_t q = 0; q < NB; ++q) o.bord[q] = v[q].second;
 }
 
 }  // namespace

@@ -11,7 +11,7 @@
  * oracle is pinned only by its own invariants (tests/test_oracle.py) and by
  * the reference's structure it follows line by line.
  *
- * Two iteration schedules:
+ * Three iteration schedules:
  *   NIM_SCHED_SEQUENTIAL -- the reference's own order: one thread, cells in
  *     number order, Gauss-Seidel inside every sweep (run.sh:2 pins
  *     OMP_NUM_THREADS=1).  "faithful" mode.
@@ -20,8 +20,8 @@
  *     discrete fixed point, different path; used to check kernels step by
  *     step.
  *   NIM_SCHED_LEVELS     -- SEQUENTIAL's arithmetic with cells visited by
- *     the level i + 2j + 3k and wall faces by their in-wall level, the order
- *     of the library's reference-order sweeps.  Equal to SEQUENTIAL bit for
+ *     the level i + 2j + 3k and wall faces by the levels that merge the four
+ *     walls, the order of the library's reference-order sweeps.  Equal to SEQUENTIAL bit for
  *     bit when that order respects every dependence of the sweeps.
  */
 #ifndef NIM_ORACLE_H
