@@ -340,7 +340,7 @@ int launch_vel(nim_ctx *x, cudaStream_t s, const GeoOf<R> &g, const FieldsT<R> &
   } else if (std::is_same<R, float>::value && x->cell_quad) {
     if constexpr (std::is_same<R, float>::value) {
       if (x->flat4)
-        k_vel_cellN<R, 4, false, true><<<x->s4, t3, 0, s>>>(d, g, F, P, ctl);
+        k_vel_cellN<R, 4, true><<<x->s4, t3, 0, s>>>(d, g, F, P, ctl);
       else
         k_vel_cellN<R, 4><<<x->s4, t3, 0, s>>>(d, g, F, P, ctl);
       TRY(mark(x, "k_vel_cellN"));

@@ -1309,13 +1309,6 @@ __device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned coun
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-// dst and src 16-byte aligned, bytes a multiple of 16
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity) {
   unsigned ok;
   asm volatile(
@@ -1848,7 +1841,7 @@ __device__ __forceinline__ void stN(R *__restrict__ p, int i, const R (&v)[NP]) 
   *reinterpret_cast<typename VecN<R, NP>::T *>(p + i) = t;
 }
 
-template <class R, int NP, bool SLAB = false, bool FLAT = false>
+template <class R, int NP, bool FLAT = false>
 __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
   using V = Ar<R>;
   if (ctl->done) return;
@@ -2066,7 +2059,7 @@ __global__ void __launch_bounds__(CB3, VCN_MINB) k_vel_cellN(Dims d, GeoOf<R> g,
     }
     stN<R, NP>(F.c[q], c, out);
   }
-  if (!SLAB || d.owns(k)) block_max<3, CB3>(red, e, ctl->err[par]);
+  block_max<3, CB3>(red, e, ctl->err[par]);
 }
 
 // ---- K2: +xi face updates of u, v, w (nse.f90:878-1005).
@@ -2955,10 +2948,6 @@ __device__ __forceinline__ void p_bc_body(const Dims &d, const GeoOf<R> &g, cons
     e[0] = d.owns(B.cell.k) ? errv(nw, pr[fw0], first) : 0.;
   }
   ps.template end<BLK>(e, 3);
-}
-template <class R>
-__global__ void __launch_bounds__(BLK) k_p_bc(Dims d, GeoOf<R> g, FieldsT<R> F, Phys P, Ctrl *ctl) {
-  p_bc_body<R>(d, g, F, P, ctl, LaunchBlock{});
 }
 
 // (coefficient, face, cell) of the ten off-diagonal terms of the pressure
