@@ -1335,14 +1335,14 @@ extern "C" int nim_slab_halo(int32_t n_theta, int32_t n_r, int32_t n_z, int32_t 
   return NIM_OK;
 }
 
-// slab: null for the whole mesh, else {nslab, s}: the context holds z-slab s
-// of nslab (nim_slab_layout) with its halo planes
-// share of busy threads below which a sweep runs in cell order.  Both sides,
+// Share of busy threads below which a sweep runs in cell order.  Both sides,
 // us a pass of FP64: 131x97x83 (0.81 busy) 843 patches, 744 runs; 150x101x77
 // (pairs 0.77, one cell 0.91: runs for the pairs only) 820, 792; 72x72x54
 // (0.75) 261, 220; 128x128x96 (1.0) 890, 959: a patch keeps the r neighbours
 // of its cells in the block's cache lines.
 constexpr double kFlatBelow = 0.9;
+// slab: null for the whole mesh, else {nslab, s}: the context holds z-slab s
+// of nslab (nim_slab_layout) with its halo planes
 static int create_impl(const nim_mesh_desc *m, const nim_params *p, nim_ctx *x, const int32_t *slab = nullptr) {
   CK(cudaGetDevice(&x->device));
   TRY(noalloc_setup(x->device));

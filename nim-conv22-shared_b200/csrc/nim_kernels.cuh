@@ -757,9 +757,9 @@ __device__ __noinline__ void nim_direction_slow(double u, double k, double gminu
 // before; 150x101x77 237 -> 170 us.  And the series stops at the last term that can
 // change its sum: for |Re| <= 0.01, i.e. x = |u/k| <= 0.005, a term below a
 // quarter ulp of the partial sum it is added to leaves it as it is, which
-// holds from x^7/4725 (1.7e-20 of Kc<A>(1), Kc<A>(2)), x^6/945 (1.65e-17 against
-// sums of 0.5 whose half spacing is at least 2.7e-17, Kc<A>(3), Kc<A>(4)),
-// 3 x^6/4725 (1e-17 of Kc<A>(5)) and x^7/9450 (8.3e-21 against 0.5, Kc<A>(6)) on.
+// holds from x^7/4725 (1.7e-20 of A(1), A(2)), x^6/945 (1.65e-17 against
+// sums of 0.5 whose half spacing is at least 2.7e-17, A(3), A(4)),
+// 3 x^6/4725 (1e-17 of A(5)) and x^7/9450 (8.3e-21 against 0.5, A(6)) on.
 __device__ __forceinline__ void nim_direction_fast(double u, double k, double gminus, double gplus, double v_limit,
                                                    double A[6]) {
   const Recip rk = recip(k);
@@ -860,6 +860,7 @@ __device__ __forceinline__ void nim_direction_f32(float u, float k, float gminus
   }
 }
 
+// nim_exp over n arguments (self-test of the exp the NIM coefficients use)
 __global__ void k_exp_selftest(const double *x, double *y, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = nim_exp(x[i]);
@@ -1296,8 +1297,8 @@ __device__ __forceinline__ Ar<R> cell_update_f1(const R *__restrict__ fr, const 
                            (at[8]);
 }
 
-// ---- bulk copies into shared memory: cp.async.bulk rows whose completion
-// is counted in bytes on an mbarrier (phase 0, one arrival: the thread that
+// ---- bulk copies into shared memory: TMA boxes whose completion is counted
+// in bytes on an mbarrier (phase 0, one arrival: the thread that
 // posts the byte count).  Every wait is bounded; a wait that runs out marks
 // the step NIM_ERR_TIMEOUT and stopped, then waits (bounded) once more so
 // that no copy lands in shared memory after the block has left.
@@ -1340,8 +1341,6 @@ __global__ void k_wait_selftest(Ctrl *ctl, int tries) {
   mbar_expect_tx(&bar, 16);
   mbar_wait(&bar, 0, ctl, tries);
 }
-
-// nim_exp over n arguments (self-test of the exp the NIM coefficients use)
 
 // The block coordinates a pass kernel's body works on.  LaunchBlock reads
 // the launch's own blockIdx where the body uses a coordinate (the plain
@@ -4249,10 +4248,11 @@ __global__ void k_iter_end(Ctrl *ctl, Phys P, int lowp) {
 // ---- The inner loop of a small mesh as one cooperative launch: passes until
 // the stop test holds (at most `passes`), with a grid barrier between the
 // parts of a pass instead of a launch.  On small meshes a pass is a chain of
-// ten launches of a few microseconds each (launch, parity and stop flag,
+// eight launches of a few microseconds each (launch, parity and stop flag,
 // loads, a block's maxima); here it is five barriers: sweeps that read nothing
-// of each other's share a part, and the maxima are folded once a pass.  The parts run the plain kernels' bodies over runs of consecutive
-// cells (FlatBlock), so the results are theirs to the bit.
+// of each other's share a part, and the maxima are folded once a pass.  The
+// parts run the plain kernels' bodies over runs of consecutive cells
+// (FlatBlock), so the results are theirs to the bit.
 //
 // Block (BX, 3), BX = 32, 64 or 128 cells (host: choose_loop), all blocks
 // resident (a cooperative launch).  What one part writes, other SMs read in
@@ -4468,7 +4468,8 @@ __global__ void __launch_bounds__(BLK) k_convert(CvtList L) {
 // order (SeqTab), and look up the next level's cells before the barrier.
 // Levels that fit a block run in one block per swept field, whose barrier is
 // the SM's own and whose loads hit its L1; wider ones on a cooperative grid
-// (the three velocity components side by side), which reads through L2.
+// (the three velocity components side by side), which reads through L2, and so
+// do narrow levels of meshes too stretched for skewed copies (seq_form).
 // Where a field's faces and averages fit the block's shared memory (up to
 // about 6800 cells), the block sweeps a copy there, whose loads take a tenth
 // of the first touch of an L2 line (36x6x12: 431 us a pass over the fields
