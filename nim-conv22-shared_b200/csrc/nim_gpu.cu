@@ -503,7 +503,6 @@ int seq_pack_velocity(nim_ctx *x) {
   k_seq_pack_quo<<<x->nblk_c, BLK, 0, x->stream>>>(one ? nullptr : x->F.MF4, one ? A + n : M, one ? A + 20 * n : M + 5 * n,
                                                    one ? A + 39 * n : M + 10 * n, S.vel, x->phys, S.order, R - 12, R, Nc);
   CK(cudaGetLastError());
-  x->launches += 3;
   return NIM_OK;
 }
 // what stays as it is after init: the metric differences, the pressure
@@ -1587,7 +1586,12 @@ extern "C" int nim_gpu_init(nim_ctx *x) {
   k_wall_floor<<<x->nblk_b, BLK, 0, s>>>(d, x->g, x->ctl);
   CK(cudaGetLastError());
   if (x->mixed) TRY(mirror_geometry(x));
-  if (x->seq) TRY(seq_pack_geometry(x));
+  if (x->seq) {
+    TRY(seq_pack_geometry(x));
+    // passes before the first step find its constants zero, and their
+    // quotients not finite, as in the parallel schedule
+    TRY(seq_pack_velocity(x));
+  }
   CK(cudaStreamSynchronize(s));
   x->TI = x->params.DT;  // nse.f90:31
   x->STEP = 1;           // nse.f90:32
@@ -1613,7 +1617,10 @@ extern "C" int nim_gpu_begin_step(nim_ctx *x) {
   CK(cudaGetLastError());
   x->launches += 3;
   if (x->mixed) TRY(mirror_step_coefficients(x));
-  if (x->seq) TRY(seq_pack_velocity(x));
+  if (x->seq) {
+    TRY(seq_pack_velocity(x));
+    x->launches += 3;
+  }
   x->in_step = true;
   return NIM_OK;
 }
