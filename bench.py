@@ -94,14 +94,15 @@ KERNEL_BYTES_PER_CELL = {
     "k_T_cell(src)": 8 * 57,  # MT_F, MT_F4 terms (21) faces T (3) G (3) g^ij (6); write the sweep's constants, R_D_T (24)
     "k_seq_T": 8 * 39,      # T,T_old (2) faces T (3) constants, R_D_T (24) dg (6); write T, faces (4)
 }
-# DRAM bytes per cell and launch that ncu measured (dram__bytes_read.sum +
-# dram__bytes_write.sum, one --set full capture each); traffic grows with the
-# cells, so roofline.traffic scales these to the run's mesh
+# DRAM bytes per cell and launch that ncu measured (read and written, one
+# capture each); traffic grows with the cells, so roofline.traffic scales
+# these to the run's mesh
 NCU_DRAM_BYTES_PER_CELL = {
     "k_vel_cell": 425.2, "k_p_src": 324.4, "k_vel_face_tile": 361.4, "k_vel_face": 343.1, "k_vel_cell2": 441.0,
+    "k_p_faceN": 195.5, "k_T_cell": 379.1, "k_T_face": 195.2,
 }
 NCU_CAPTURE = {k: "128x128x96" for k in NCU_DRAM_BYTES_PER_CELL}
-for _k in ("k_vel_face", "k_vel_cell2"):
+for _k in ("k_vel_face", "k_vel_cell2", "k_p_faceN", "k_T_cell", "k_T_face"):
     NCU_CAPTURE[_k] = "96x96x64"
 # algorithmic bytes per cell-iteration and per cell-step of the whole pass
 # (FP64, every array read and written once, implicit connectivity)
