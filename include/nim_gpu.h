@@ -510,8 +510,9 @@ int nim_gpu_selftest_exp(const double *x, double *y, int64_t n);
 /* Self-test of the straight-line quotients the FP64 sweeps use in place of
    IEEE divisions (no counterpart in the reference): q[i] = a[i] / b[i], which
    must be the correctly rounded quotient, n <= 2^28.  Operands outside that
-   form's range (zero, subnormal, non-finite, exponents beyond +-480, divisors
-   with a significand above 2 - 2^-20) are divided.  Allocates and frees its
+   form's range (zero over a negative divisor, divisors zero, subnormal,
+   non-finite, exponents beyond +-480, divisors with a significand above
+   2 - 2^-20) are divided.  Allocates and frees its
    device buffers; default stream. */
 int nim_gpu_selftest_quot(const double *a, const double *b, double *q, int64_t n);
 

@@ -39,10 +39,13 @@ __device__ __forceinline__ Recip recip(double b) {
   y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
   return {b, y};
 }
+// (the remainder as b q - a: with b > 0 that is +0 where the quotient is exact
+// or a zero, and q - (+0) y leaves q as it is, -0 included; with b < 0 a +0
+// numerator's quotient loses its sign)
 __device__ __forceinline__ double quot(double a, const Recip &r) {
   double q = __dmul_rn(a, r.y);
-  q = __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
-  return __fma_rn(__fma_rn(-r.b, q, a), r.y, q);
+  q = __fma_rn(-__fma_rn(r.b, q, -a), r.y, q);
+  return __fma_rn(-__fma_rn(r.b, q, -a), r.y, q);
 }
 // b's exponent within +-E and its significand at most 2 - 2^-20
 template <int E>
@@ -50,12 +53,11 @@ __device__ __forceinline__ bool div_ok(double b) {
   const uint32_t hi = (uint32_t)__double2hiint(b) & 0x7fffffffu;
   return (hi - ((1023u - E) << 20)) < ((2u * E) << 20) && (hi & 0xfffffu) != 0xfffffu;
 }
-// a's exponent within +-E.  A zero is not: quot() adds a +0 remainder to the
-// quotient, so that -0 / b would come back as +0.
+// a's exponent within +-E, or a zero
 template <int E>
 __device__ __forceinline__ bool num_ok(double a) {
   const uint32_t hi = (uint32_t)__double2hiint(a) & 0x7fffffffu;
-  return (hi - ((1023u - E) << 20)) < ((2u * E) << 20);
+  return (hi - ((1023u - E) << 20)) < ((2u * E) << 20) || a == 0.0;
 }
 
 }  // namespace nim

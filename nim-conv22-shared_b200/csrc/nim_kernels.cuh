@@ -869,7 +869,7 @@ __global__ void k_exp_selftest(const double *x, double *y, int64_t n) {
 // quotients by nim_div.cuh where it accepts the operands, else a division
 __global__ void k_quot_selftest(const double *a, const double *b, double *q, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    q[i] = div_ok<480>(b[i]) && num_ok<480>(a[i]) ? quot(a[i], recip(b[i])) : a[i] / b[i];
+    q[i] = div_ok<480>(b[i]) && num_ok<480>(a[i]) && (b[i] > 0. || a[i] != 0.) ? quot(a[i], recip(b[i])) : a[i] / b[i];
 }
 
 // the six NIM coefficients of one direction (gminus = gplus = 1) for n
