@@ -221,9 +221,10 @@ int nim_gpu_create(const nim_mesh_desc *mesh, const nim_params *params,
    NIM_REFERENCE_GRID, a cooperative grid over the fields themselves;
    NIM_REFERENCE_SKEWED, one block per swept field over skewed copies in
    device memory.  The skewed form needs levels (cells of equal i + 2j + 3k)
-   of at most 1024 cells and copies of at most 8 values a cell and plane,
-   1.7 kB a cell: a tall or wide mesh with narrow levels takes the grid.  All
-   forms give the same bits.  copies, unless NULL: bytes of the skewed copies
+   of at most 1024 cells and copies of at most 8 values a cell and plane
+   (1.7 kB a cell) or 4 GiB in all; a stretched mesh beyond that takes the
+   grid, and so does nim_gpu_create when the device has no room left for the
+   copies.  All forms give the same bits.  copies, unless NULL: bytes of the skewed copies
    (0 for the other forms).  NIM_ERR_BAD_ARG for counts nim_gpu_create
    refuses. */
 enum { NIM_REFERENCE_SHARED = 0, NIM_REFERENCE_GRID = 1, NIM_REFERENCE_SKEWED = 2 };

@@ -987,13 +987,18 @@ static int noalloc_setup(int device) {
 // shared memory (what 227 KB leave beside the block's reductions)
 constexpr int kSeqBlockMost = 1024;
 constexpr size_t kSeqSharedMost = 224 * 1024;
-// Most values a plane of the skewed copies may have per cell.  A plane is the
-// box of the levels: (levels + 3)(NZ + 1)(NR + 1) values, and 27 planes are
-// kept, so the copies grow with the square of the longest direction while the
-// widest level does not.  48x48x32, 60x40x30 and 41x29x24, where the copies
-// pay (SeqTab), have 4 to 6 values a cell, 1.0 to 1.2 kB of copies a cell;
-// 36x80x400 has 38, 8 kB, and sweeps the fields themselves.
-constexpr int64_t kSkewMost = 8;
+// How far the skewed copies may outgrow the mesh: 8 values a cell and plane,
+// or kSkewBytes in all.  A plane is the box of the levels, (levels + 3)(NZ + 1)
+// (NR + 1) values, and 27 planes are kept, so the copies grow with the square
+// of the longest direction while the widest level does not: 48x48x32 has 5
+// values a cell (74 MB), 24x24x200 29 (0.7 GB), 36x80x400 39 (9.8 GB),
+// 36x80x2000 217 GB.  Where they fit they pay, on stretched meshes most; us a
+// pass of the copies and of the grid: 24x24x40 694, 2119; 24x24x200 3134,
+// 9255; 24x24x300 (1.5 GB) 4532, 13670; 16x60x300 (4.1 GB) 9390, 16620;
+// 36x80x100 (0.9 GB, 960 wide) 6988, 8881; 36x100x60 7255, 7257.  The limit
+// is a fiftieth of the device, for the context's neighbours.
+constexpr int64_t kSkewMost = 8, kSkewBytes = (int64_t)4 << 30;
+constexpr int kSkewPlanes = 3 * kSkewVel + kSkewP + kSkewTm;
 // The form of the reference order's sweeps on a mesh: its widest level
 // (cells of equal i + 2j + 3k), the memory its fields take, and the values of
 // a plane of skewed copies.
@@ -1022,7 +1027,8 @@ static SeqForm seq_form(int64_t NT, int64_t NR, int64_t NZ) {
   // the sweeps index three planes, and up to four levels beyond a cell, in
   // 32 bits
   const int64_t st = (NZ + 1) * (NR + 1), plane = (nlev + 3) * st;
-  if (plane <= kSkewMost * Nc && 3 * plane + 8 * st <= INT32_MAX) {
+  const bool small = plane <= kSkewMost * Nc || plane <= kSkewBytes / (int64_t)(kSkewPlanes * sizeof(double));
+  if (small && 3 * plane + 8 * st <= INT32_MAX) {
     f.mode = kSeqSkew;
     f.plane = plane;
   }
@@ -1032,7 +1038,7 @@ extern "C" int nim_reference_form(int32_t n_theta, int32_t n_r, int32_t n_z, int
   if (n_theta < 6 || n_r < 3 || n_z < 3 || (int64_t)n_theta * n_r * n_z > (int64_t)INT32_MAX / 4)
     return NIM_ERR_BAD_ARG;
   const SeqForm f = seq_form(n_theta, n_r, n_z);
-  if (copies) *copies = (int64_t)sizeof(double) * (3 * kSkewVel + kSkewP + kSkewTm) * f.plane;
+  if (copies) *copies = (int64_t)sizeof(double) * kSkewPlanes * f.plane;
   return f.mode;
 }
 static_assert(kSeqShared == NIM_REFERENCE_SHARED && kSeqGrid == NIM_REFERENCE_GRID && kSeqSkew == NIM_REFERENCE_SKEWED,
@@ -1105,6 +1111,24 @@ static int setup_levels(nim_ctx *x) {
   x->wall_threads = warps(wmax, WALL_TPB);
   const SeqForm form = seq_form(d.NT, d.NR, d.NZ);
   x->seq_mode = form.mode;
+  if (form.mode == kSeqSkew) {
+    // where the device has no room for the copies, the grid needs none
+    const size_t L = form.plane, bytes = sizeof(double) * kSkewPlanes * L;
+    void *q = nullptr;
+    if (cudaMalloc(&q, bytes) == cudaSuccess) {
+      x->allocs.push_back(q);
+      CK(cudaMemsetAsync(q, 0, bytes, x->stream));
+      S.skew.sk = d.NR + 1;
+      S.skew.st = (d.NZ + 1) * S.skew.sk;
+      S.skew.L = (int)L;  // levels from -3 (the low z wall's layer)
+      S.skv = static_cast<double *>(q);
+      S.skp = S.skv + 3 * kSkewVel * L;
+      S.skt = S.skp + kSkewP * L;
+    } else {
+      cudaGetLastError();
+      x->seq_mode = kSeqGrid;
+    }
+  }
   auto run_beside = [&]() -> int {
     CK(cudaStreamCreateWithFlags(&x->side, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&x->fork, cudaEventDisableTiming));
@@ -1123,15 +1147,7 @@ static int setup_levels(nim_ctx *x) {
     CK(room(k_seq_pbc<true>));
     return NIM_OK;
   }
-  if (x->seq_mode == kSeqSkew) {
-    S.skew.sk = d.NR + 1;
-    S.skew.st = (d.NZ + 1) * S.skew.sk;
-    S.skew.L = (int)form.plane;  // levels from -3 (the low z wall's layer)
-    TRY(dalloc(x, &S.skv, 3 * kSkewVel * (size_t)S.skew.L));
-    TRY(dalloc(x, &S.skp, kSkewP * (size_t)S.skew.L));
-    TRY(dalloc(x, &S.skt, kSkewTm * (size_t)S.skew.L));
-    return NIM_OK;
-  }
+  if (x->seq_mode == kSeqSkew) return NIM_OK;
   // cooperative grids: no more blocks than the widest level needs, and no
   // more than can be resident at once (cudaLaunchCooperativeKernel rejects
   // a larger grid rather than running it)

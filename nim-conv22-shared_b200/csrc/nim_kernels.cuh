@@ -4469,7 +4469,8 @@ __global__ void __launch_bounds__(BLK) k_convert(CvtList L) {
 // Levels that fit a block run in one block per swept field, whose barrier is
 // the SM's own and whose loads hit its L1; wider ones on a cooperative grid
 // (the three velocity components side by side), which reads through L2, and so
-// do narrow levels of meshes too stretched for skewed copies (seq_form).
+// do narrow levels of meshes too stretched for skewed copies (seq_form, with
+// both sides' times).
 // Where a field's faces and averages fit the block's shared memory (up to
 // about 6800 cells), the block sweeps a copy there, whose loads take a tenth
 // of the first touch of an L2 line (36x6x12: 431 us a pass over the fields

@@ -1,6 +1,6 @@
 """The reference order on meshes whose levels are narrow while the mesh is
-long in one direction (nim_reference_form: the cooperative grid, not the
-skewed copies): two passes of the loop body, bit for bit the oracle's
+long in one direction, on both sides of the limit of the skewed copies
+(nim_reference_form): two passes of the loop body, bit for bit the oracle's
 sequential order (nse.f90:131-160)."""
 import numpy as np
 import pytest
@@ -17,10 +17,11 @@ STATE = [
 ]
 
 
-@pytest.mark.parametrize("dims,formulation", [((24, 24, 200), 2), ((24, 24, 200), 1), ((6, 10, 150), 2), ((6, 90, 30), 2),
-                                              ((7, 8, 160), 1)])
-def test_two_passes_match_the_sequential_oracle(dims, formulation):
-    assert _abi.gpu_lib().nim_reference_form(*dims, None) == 1
+@pytest.mark.parametrize("dims,formulation,form", [
+    ((24, 24, 200), 2, 2), ((24, 24, 200), 1, 2), ((6, 10, 150), 2, 2), ((6, 90, 30), 2, 2), ((7, 8, 160), 1, 2),
+    ((6, 10, 900), 2, 1), ((7, 9, 850), 1, 1), ((24, 24, 600), 2, 1), ((24, 200, 110), 2, 1)])
+def test_two_passes_match_the_sequential_oracle(dims, formulation, form):
+    assert _abi.gpu_lib().nim_reference_form(*dims, None) == form
     case = config.small_case(*dims)
     params = case.params(schedule=_abi.SCHEDULE_REFERENCE, formulation=formulation)
     mesh = nimgpu.Mesh(case.mesh_params())

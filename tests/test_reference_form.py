@@ -1,6 +1,6 @@
 """The form the reference order's sweeps take on a mesh (nim_reference_form,
 include/nim_gpu.h): skewed copies only where they stay a small multiple of
-the fields and their planes can be indexed in 32 bits.  Pure host functions
+the fields or a few GB, and their planes can be indexed in 32 bits.  Pure host functions
 of libnimgpu.so: no GPU needed."""
 import ctypes as C
 import random
@@ -12,6 +12,7 @@ from nimgpu import _abi
 
 SHARED, GRID, SKEWED = 0, 1, 2
 PLANES = 27  # three components of 6 planes, the pressure's 4, the temperature's 5
+LIMIT = 4 << 30  # bytes of copies that outgrow 8 values a cell and plane
 
 
 @pytest.fixture(scope="module", autouse=True)
@@ -42,16 +43,17 @@ def widest_level(nt, nr, nz):
 # 32 bits, or both (36x80x4300 wraps to a small positive number, 24x120x2500
 # to a negative one, and 6x10x11410 to one smaller than the mesh)
 @pytest.mark.parametrize("dims", [(36, 80, 400), (36, 80, 2000), (36, 80, 4300), (24, 120, 2500), (6, 480, 2000),
-                                  (6, 10, 11410), (12, 60, 800), (12, 128, 2000), (24, 24, 200)])
+                                  (6, 10, 11410), (12, 60, 800), (12, 128, 2000), (24, 24, 600)])
 def test_narrow_levels_of_a_stretched_mesh_sweep_the_fields(dims):
     assert widest_level(*dims) <= 1024
-    assert plane(*dims) > 8 * np.prod(dims, dtype=np.int64)
+    assert plane(*dims) > 8 * np.prod(dims, dtype=np.int64) and 8 * PLANES * plane(*dims) > LIMIT
     assert form(*dims) == (GRID, 0)
 
 
 @pytest.mark.parametrize("dims,want", [
     ((36, 6, 12), SHARED), ((36, 14, 13), SHARED), ((36, 14, 14), SKEWED), ((24, 24, 16), SKEWED),
-    ((48, 48, 32), SKEWED), ((60, 40, 30), SKEWED), ((301, 5, 6), SKEWED), ((90, 70, 60), GRID), ((128, 128, 96), GRID)])
+    ((48, 48, 32), SKEWED), ((60, 40, 30), SKEWED), ((301, 5, 6), SKEWED), ((24, 24, 200), SKEWED), ((16, 60, 300), SKEWED),
+    ((6, 10, 600), SKEWED), ((90, 70, 60), GRID), ((128, 128, 96), GRID)])
 def test_the_measured_meshes_keep_their_form(dims, want):
     got, copies = form(*dims)
     assert got == want
@@ -73,7 +75,7 @@ def test_skewed_copies_stay_small_and_inside_32_bits():
             assert got == GRID
         if got == SKEWED:
             n = plane(nt, nr, nz)
-            assert copies == 8 * PLANES * n <= 8 * PLANES * 8 * nt * nr * nz
+            assert copies == 8 * PLANES * n <= max(8 * PLANES * 8 * nt * nr * nz, LIMIT)
             # the largest index of a sweep: three planes and the farthest neighbour
             assert 3 * n + 8 * (nz + 1) * (nr + 1) < 2 ** 31
         else:
